@@ -1,7 +1,7 @@
 // C ABI of the GB300 TRSK shallow-water step (include/imodel_swm.h).
 //
 // A handle owns the device copy of the mesh layout, the state buffers of
-// classic RK4 and one CUDA stream.  One RK4 step is 4 stages x 4 kernels;
+// classic RK4 and one CUDA stream.  One RK4 step is 4 stages x 3 or 4 kernels;
 // it is captured once into a CUDA graph per time step length and replayed.
 #include <cuda.h>  // pointer-attribute types only; the driver call is resolved at run time
 #include <cuda_runtime.h>
@@ -163,9 +163,12 @@ int alloc_work(Handle *H, Work<T> &W) {
   T **bufs_v[] = {&W.yn_h, &W.ya_h, &W.yb_h, &W.acc_h, &W.bern, &W.tend_h};
   for (T **b : bufs_v)
     if ((rc = dalloc(H, b, H->nv))) return rc;
-  T **bufs_e[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u, &W.h_ed, &W.uh, &W.q_ed, &W.tend_u};
+  T **bufs_e[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u, &W.uh, &W.q_ed, &W.tend_u};
   for (T **b : bufs_e)
     if ((rc = dalloc(H, b, H->ne))) return rc;
+  if (sizeof(T) == sizeof(double) ? (rc = dalloc(H, &W.fe, H->ne))
+                                  : (rc = dalloc(H, &W.h_ed, H->ne)))
+    return rc;
   if ((rc = dalloc(H, &W.q_tr, H->nt))) return rc;
   W.flags = H->d_flags;
   W.pv_on = H->testcase >= 2 ? 1 : 0;
@@ -797,6 +800,22 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
   if (H->precision == IMODEL_SWM_FP64 && !L.t_c.empty()) {
     if ((rc = upload(H, L.e_c, &M.e_c)) || (rc = upload(H, L.t_c, &M.t_c)) ||
         (rc = upload(H, L.c_p, &M.c_p)))
+      return rc;
+  }
+  if (H->precision == IMODEL_SWM_FP64) {
+    Layout64 D;
+    build_layout64(L, scheme, D);
+    M.rerad = D.rerad;
+    if ((rc = upload(H, D.c_rareag, &M.c_rareag)) ||
+        (rc = upload(H, D.c_rcellarea, &M.c_rcellarea)) || (rc = upload(H, D.c_eds, &M.c_eds)) ||
+        (rc = upload(H, D.e_rleng, &M.e_rleng)) || (rc = upload(H, D.e_rdleng, &M.e_rdleng)) ||
+        (rc = upload(H, D.e_d8, &M.e_d8)) || (rc = upload(H, D.e_dlerad, &M.e_dlerad)) ||
+        (rc = upload(H, D.e_rdlerad, &M.e_rdlerad)) || (rc = upload(H, D.t_rareag, &M.t_rareag)) ||
+        (rc = upload(H, D.c_nrm, &M.c_nrm)) || (rc = upload(H, D.c_rnrm, &M.c_rnrm)) ||
+        (rc = upload(H, D.t_nrm, &M.t_nrm)) || (rc = upload(H, D.t_rnrm, &M.t_rnrm)) ||
+        (rc = upload(H, D.e_nrm, &M.e_nrm)) || (rc = upload(H, D.e_rnrm, &M.e_rnrm)) ||
+        (rc = upload(H, D.e_dsum, &M.e_dsum)) || (rc = upload(H, D.e_rdsum, &M.e_rdsum)) ||
+        (rc = upload(H, D.c_off, &M.c_off)))
       return rc;
   }
   // the other method wrappers' geometry (empty vectors upload as NULL)
@@ -1535,7 +1554,7 @@ struct Moist {
   double q0 = 0.0;
   double *th = nullptr, *ex20 = nullptr, *qv = nullptr, *qc = nullptr, *qr = nullptr;
   double *q[5][4] = {};  // per tracer: y_n, two stage buffers, RK accumulator
-  double *uphi = nullptr;
+  double *uphi = nullptr, *gthb = nullptr;
   float *f_th = nullptr, *f_ex20 = nullptr, *f_qv = nullptr, *f_qc = nullptr, *f_qr = nullptr;
   float *f_q[5][4] = {};
   bool state_set = false;
@@ -1672,7 +1691,6 @@ void moist_step64(Moist *X, double dt) {
       A.u_in = u_in;
       A.tend_h = W.tend_h;
       A.tend_u = W.tend_u;
-      A.h_ed = W.h_ed;
       A.yn_h = W.yn_h;
       A.acc_h = W.acc_h;
       A.h_out = out(st, W.yn_h, W.ya_h, W.yb_h);
@@ -1688,12 +1706,12 @@ void moist_step64(Moist *X, double dt) {
         A.q_out[k] = out(st, q[0], q[1], q[2]);
       }
       A.uphi = X->uphi;
-      A.th = X->th;
-      A.ex20 = X->ex20;
+      A.rdt = dt >= 0x1p-500 && dt <= 0x1p500 ? 1.0 / dt : std::nan("");
+      A.gthb = X->gthb;
+      A.q0ex = X->ex20;
       A.qv = X->qv;
       A.qc = X->qc;
       A.qr = X->qr;
-      A.q0 = X->q0;
       A.flags = H->d_flags;
       imodel::launch_moist_stage(H->M, A, H->stream);
     }
@@ -1783,9 +1801,13 @@ int imodel_moist_create(const imodel_swm_mesh *m, const imodel_moist_opts *o, vo
     for (int k = 0; k < 5; ++k)
       for (int b = 0; b < 4; ++b)
         if ((rc = imodel::dalloc(H, &X->q[k][b], nv))) return rc;
-    if ((rc = imodel::dalloc(H, &X->uphi, 5 * ne))) return rc;
+    if ((rc = imodel::dalloc(H, &X->uphi, 5 * ne)) || (rc = imodel::dalloc(H, &X->gthb, ne)))
+      return rc;
     if ((rc = moist_in(H, o->theta, X->th, false)) || (rc = moist_in(H, ex.data(), X->ex20, false)))
       return rc;
+    imodel::launch_moist_consts(H->M, X->th, X->ex20, X->q0, X->gthb, H->stream);
+    if (cudaGetLastError() != cudaSuccess)
+      return imodel::set_error(H, IMODEL_SWM_ECUDA, "launch failed");
   }
   if (cudaStreamSynchronize(H->stream) != cudaSuccess)
     return imodel::set_error(H, IMODEL_SWM_ECUDA, "stream synchronize failed");

@@ -9,6 +9,15 @@ namespace imodel {
 struct DevMesh {
   int nv, ne, nt;
   double erad, grav;
+  double rerad;  // 1 / erad
+  // FP64 step: reciprocals of the divisors of its kernels (div_by), the
+  // slot's edge with its sign, d / 8, the norms of the projection points and
+  // pxt16's offsets (swm_layout.h)
+  const double *c_rareag, *c_rcellarea, *e_rleng, *e_rdleng, *t_rareag;
+  const double *e_dlerad, *e_rdlerad, *e_d8;
+  const double *c_nrm, *c_rnrm, *t_nrm, *t_rnrm, *e_nrm, *e_rnrm;
+  const double *e_dsum, *e_rdsum, *c_off;
+  const uint32_t *c_eds;
   // cells
   const int8_t *c_nnb;
   const int32_t *c_ed;
@@ -120,7 +129,8 @@ struct Work {
   T *yb_h, *yb_u;    // stage inputs (pong)
   T *acc_h, *acc_u;  // k0 + 2 k1 + 2 k2
   T *q_tr;           // [nt] potential vorticity at triangles
-  T *h_ed, *uh, *q_ed;  // [ne]
+  T *h_ed, *uh, *q_ed;  // [ne]; FP64: uh and q_ed hold 2 u h_e and 2 q_e, h_ed is not used
+  double2 *fe = nullptr;  // [ne] FP64: 2 u h_e d and the edge's kinetic-energy term
   T *bern;           // [nv] g (h + b) + K
   T *tend_h, *tend_u;   // tendency outputs (tendency-only evaluations)
   T *zflux;          // [6][nv] cell-centred PV flux of each cell edge (variants 1, 2)
@@ -174,7 +184,8 @@ void learned_launch(const DevMesh &M, const LearnedDev &L, const float *hd, cons
 // K div u and K_tr zeta (1 launch)
 inline int launches_per_stage(int precision_fp32, int variant, bool dif_on = false,
                               bool dif_k4 = false, bool apvm_on = false, int scheme = 0) {
-  int n = (precision_fp32 && variant >= 1) ? 3 : 4;
+  // FP64: triangles + edge fluxes, cells + edge PV, edges
+  int n = (precision_fp32 && variant == 0) ? 4 : 3;
   if (!precision_fp32 && scheme == 3) n += 1;  // dtred: the triangle reconstruction of uh q
   if (dif_on) n += (dif_k4 ? 3 : 1) + ((precision_fp32 && variant == 0) ? 1 : 0);
   // FP32 variants 1 and 2: the edge pre-pass for APVM's or gass18's edge PV
@@ -194,25 +205,29 @@ void launch_dif_coefs(const DevMesh &M, const double *kf, double k, bool take_sq
 // One RK stage of the moist shallow-water model (swm_moist.cu).  Tracer k of
 // {h theta, h qv, h qc, h qr, h tracer} is advanced when bit k of `active`
 // is set; swm != 0 adds the shallow-water terms (the caller has written
-// tend_h, tend_u and h_ed with a tendency evaluation of the stage input),
+// tend_h and tend_u with a tendency evaluation of the stage input),
 // the thermal momentum source and the water sources.
 struct MoistArgs {
   int stage = 0;
   double dt = 0.0;
   int swm = 0, active = 0;
   int upw1 = 0;  // tracer advection: 0 "trsk" (centred), 1 "upw1" (upwind)
-  const double *u_in = nullptr, *h_in = nullptr, *tend_u = nullptr, *tend_h = nullptr,
-               *h_ed = nullptr;
+  const double *u_in = nullptr, *h_in = nullptr, *tend_u = nullptr, *tend_h = nullptr;
   double *yn_u = nullptr, *acc_u = nullptr, *u_out = nullptr;
   double *yn_h = nullptr, *acc_h = nullptr, *h_out = nullptr;
   const double *q_in[5] = {};
   double *q_yn[5] = {}, *q_acc[5] = {}, *q_out[5] = {};
-  double *uphi = nullptr;  // [5][ne]
-  // theta (frozen), exp(20 theta), and qv, qc, qr of the last step [nv]
-  const double *th = nullptr, *ex20 = nullptr, *qv = nullptr, *qc = nullptr, *qr = nullptr;
-  double q0 = 0.0;
+  double *uphi = nullptr;  // [5][ne] "trsk": 2 u q_e d
+  // constants of the run (launch_moist_consts): g theta_e grad(b) [ne] and
+  // q0 exp(20 theta) [nv]; qv, qc, qr of the last step [nv]
+  const double *gthb = nullptr, *q0ex = nullptr, *qv = nullptr, *qc = nullptr, *qr = nullptr;
+  double rdt = 0.0;  // 1 / dt, for div_by
   int *flags = nullptr;
 };
+// gthb from theta and the topography (both frozen in a run); ex20 becomes
+// q0 ex20 in place
+void launch_moist_consts(const DevMesh &M, const double *th, double *ex20, double q0,
+                         double *gthb, cudaStream_t s);
 void launch_moist_stage(const DevMesh &M, const MoistArgs &A, cudaStream_t s);
 void launch_moist_q(int nv, const double *h, const double *hqv, const double *hqc,
                     const double *hqr, double *qv, double *qc, double *qr, int *flags,
@@ -265,6 +280,10 @@ void launch_store_host(int n, const int32_t *o2n, const T *src, double *dst, dou
 // Compensated FP64 integrals.  Scratch: partial sums, 2 doubles per block
 // and quantity; result[kDiagQ] on the device.
 constexpr int kDiagQ = 12;
+// threads per block of the FP64 kernels
+#ifndef BLOCK64
+#define BLOCK64 64
+#endif
 constexpr int kRedBlocks = 608;   // 4 blocks per SM on 152 SMs
 constexpr int kRedThreads = 256;
 // result indices

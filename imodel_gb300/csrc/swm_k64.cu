@@ -7,6 +7,7 @@
 // src/swm.f90:2416-2683 and src/swm_operators.f90 bit for bit.
 #include "imodel_swm.h"
 #include "swm_common.cuh"
+#include "swm_div.cuh"
 
 namespace imodel {
 namespace {
@@ -14,42 +15,77 @@ namespace {
 // constants.f90:45 -- eps = epsilon(1.) (float epsilon)
 constexpr double kEps = 1.1920928955078125e-07;
 
-template <class T>
-__device__ __forceinline__ T rk_stage(int stage, T k, T yn, T *acc, T dt) {
-  // ode_rk4, swm.f90:2647-2678
+// ode_rk4, swm.f90:2647-2678.  hdt = dt / 2: dt k / 2 and (dt / 2) k are the
+// same rounding (a power of two), and acc + 2 k is one fused operation with
+// an exact product.
+__device__ __forceinline__ double rk_stage(int stage, double k, double yn, double *acc,
+                                           double dt) {
   if (stage == 0) {
     *acc = k;
-    return yn + dt * k / T(2);
+    return yn + (dt * 0.5) * k;
   } else if (stage == 1) {
-    *acc = *acc + T(2) * k;
-    return yn + dt * k / T(2);
+    *acc = __fma_rn(2.0, k, *acc);
+    return yn + (dt * 0.5) * k;
   } else if (stage == 2) {
-    *acc = *acc + T(2) * k;
+    *acc = __fma_rn(2.0, k, *acc);
     return yn + dt * k;
   }
-  return yn + dt * (*acc + k) / T(6);
+  return yn + div_by(dt * (*acc + k), 6.0, kThird2);
 }
 
-// vort_tr (:551-611) + scalar_hx2tr (:229-284) + scalar_elem_divide (:1579);
-// the depth at the triangle by the scheme's interpolation (swm.f90:2459-2464):
-// kite areas (trsk), barycentric weights of the circumcentre (bary, pxt16) or
-// scalar_edtr2trcc of h_ed (:286-343, gass18, which also keeps eta and h_tr
-// for the rhombus PV)
+// What bounds the FP64 step: GB300's FP64 pipe (2 operations per cycle and
+// SM), not memory -- the kernels below are counted in FP64 operations.  Three
+// things keep the count low without changing a bit of the results:
+//  * divisions by what is known in advance (areas, lengths, the earth's
+//    radius, 6) are three operations instead of about ten (div_by);
+//  * factors of two are left out of the per-edge fields and put into
+//    constants: uh2 = 2 u h_e = u (h_1 + h_2), q2 = 2 q_e, and the stencil's
+//    d / 8 takes the product's 8 back (scaling by a power of two commutes
+//    with rounding);
+//  * products that both cells of an edge form alike are formed once per edge
+//    (2 u h_e d and the kinetic-energy term) and added with the cell's sign.
+
+// Edge e's fluxes: uh2 = 2 u h_e (scalar_hx2ed :89-97, scalar_elem_product
+// :1546), fe = {2 u h_e d, (l d / 4) u^2}
+__device__ __forceinline__ void edge_flux64(const DevMesh &M, int e, const double *__restrict__ h,
+                                            const double *__restrict__ u,
+                                            double *__restrict__ uh2,
+                                            double2 *__restrict__ fe) {
+  const int ne = M.ne;
+  const double ue = u[e];
+  const double f = ue * (h[M.e_v[e]] + h[M.e_v[ne + e]]);
+  uh2[e] = f;
+  fe[e] = make_double2(f * M.e_dleng[e], M.e_kew[e] * (ue * ue));
+}
+
+// Blocks [0, nbt): vort_tr (:551-611) + scalar_hx2tr (:229-284) +
+// scalar_elem_divide (:1579); the depth at the triangle by the scheme's
+// interpolation (swm.f90:2459-2464): kite areas (trsk), barycentric weights
+// of the circumcentre (bary, pxt16) or scalar_edtr2trcc of h_ed (:286-343,
+// gass18, which also keeps eta and h_tr for the rhombus PV).  The blocks
+// after: the edges' fluxes, which the next launch reads beside q.
 __global__ void __launch_bounds__(256) k_tri64(DevMesh M, const double *__restrict__ h,
                                                const double *__restrict__ u,
                                                double *__restrict__ q_tr, int pv_on,
                                                int *flags, const double *__restrict__ kt,
                                                double *__restrict__ coefvort, int scheme,
                                                double *__restrict__ eta_t,
-                                               double *__restrict__ h_trs) {
+                                               double *__restrict__ h_trs,
+                                               double *__restrict__ uh2,
+                                               double2 *__restrict__ fe, int nbt) {
+  if (static_cast<int>(blockIdx.x) >= nbt) {
+    const int e = (blockIdx.x - nbt) * blockDim.x + threadIdx.x;
+    if (e < M.ne) edge_flux64(M, e, h, u, uh2, fe);
+    return;
+  }
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = M.nt;
   if (t >= nt) return;
   double e = 0.0;
 #pragma unroll
   for (int s = 0; s < 3; ++s) e = e + u[M.t_ed[s * nt + t]] * M.t_lt[s * nt + t];
-  const double A = M.t_areag[t];
-  e = e / A / M.erad;
+  const double A = M.t_areag[t], rA = M.t_rareag[t];
+  e = div_by(div_by(e, A, rA), M.erad, M.rerad);
   // with diffusion on: rel_vort_tr(u) (:780-827) is this sum before f is
   // added; diffusion_ed's K_tr zeta
   if (coefvort) coefvort[t] = kt[t] * e;
@@ -66,13 +102,13 @@ __global__ void __launch_bounds__(256) k_tri64(DevMesh M, const double *__restri
       const double he = (h[M.e_v[ed]] + h[M.e_v[ne + ed]]) * 0.5;
       ht = ht + M.t_edarea[s * nt + t] * he;
     }
-    ht = ht / A;
+    ht = div_by(ht, A, rA);
     eta_t[t] = e;
     h_trs[t] = ht;
   } else {
 #pragma unroll
     for (int s = 0; s < 3; ++s) ht = ht + M.t_kite[s * nt + t] * h[M.t_v[s * nt + t]];
-    ht = ht / A;
+    ht = div_by(ht, A, rA);
   }
   double q = 0.0;
   if (pv_on) {
@@ -84,14 +120,21 @@ __global__ void __launch_bounds__(256) k_tri64(DevMesh M, const double *__restri
   q_tr[t] = q;
 }
 
-// proj_vec_sphere (smeshpack.f90:4419-4433): v - (v . p) p / |p|
+// proj_vec_sphere (smeshpack.f90:4419-4433): v - (v . p) p / |p|, with |p|
+// and its reciprocal from the layout
 __device__ __forceinline__ void proj_sphere(double &v0, double &v1, double &v2, double p0,
-                                            double p1, double p2) {
+                                            double p1, double p2, double np, double rnp) {
   const double vp = v0 * p0 + v1 * p1 + v2 * p2;
-  const double np = sqrt(p0 * p0 + p1 * p1 + p2 * p2);
-  v0 = v0 - vp * p0 / np;
-  v1 = v1 - vp * p1 / np;
-  v2 = v2 - vp * p2 / np;
+  v0 = v0 - div_by(vp * p0, np, rnp);
+  v1 = v1 - div_by(vp * p1, np, rnp);
+  v2 = v2 - div_by(vp * p2, np, rnp);
+}
+
+// +-x by the sign of s (a sign flip on the integer pipe instead of a
+// comparison and a product on the FP64 pipe)
+__device__ __forceinline__ double sign_of(double s, double x) {
+  return __hiloint2double(__double2hiint(x) ^ (__double2hiint(s) & 0x80000000),
+                          __double2loint(x));
 }
 
 // grad_tr2ed(q_tr) (:1427-1463), the PV gradient across each edge
@@ -100,8 +143,8 @@ __global__ void __launch_bounds__(256) k_qgrad64(DevMesh M, const double *__rest
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
-  double g = M.e_sgtg[e] * (q_tr[M.e_sh[ne + e]] - q_tr[M.e_sh[e]]);
-  qge[e] = g / M.e_dleng[e] / M.erad;
+  const double g = M.e_sgtg[e] * (q_tr[M.e_sh[ne + e]] - q_tr[M.e_sh[e]]);
+  qge[e] = div_by(div_by(g, M.e_dleng[e], M.e_rdleng[e]), M.erad, M.rerad);
 }
 
 // The two reconstructions apvm (:1465-1543) reads.  Blocks [0, nbt): the
@@ -123,17 +166,17 @@ __global__ void __launch_bounds__(256) k_apvm64(DevMesh M, const double *__restr
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
       const int ed = M.t_ed[s * nt + t];
-      const double sg = (M.t_lt[s * nt + t] < 0.0 ? 1.0 : -1.0) * qge[ed];
+      const double sg = sign_of(-M.t_lt[s * nt + t], qge[ed]);
       const double l = M.e_leng[ed];
       v0 = v0 + sg * (M.e_c[ed] - c0) * l;
       v1 = v1 + sg * (M.e_c[ne + ed] - c1) * l;
       v2 = v2 + sg * (M.e_c[2 * ne + ed] - c2) * l;
     }
-    const double A = M.t_areag[t];
-    v0 = v0 / A;
-    v1 = v1 / A;
-    v2 = v2 / A;
-    proj_sphere(v0, v1, v2, c0, c1, c2);
+    const double A = M.t_areag[t], rA = M.t_rareag[t];
+    v0 = div_by(v0, A, rA);
+    v1 = div_by(v1, A, rA);
+    v2 = div_by(v2, A, rA);
+    proj_sphere(v0, v1, v2, c0, c1, c2, M.t_nrm[t], M.t_rnrm[t]);
     qg[t] = v0;
     qg[nt + t] = v1;
     qg[2 * nt + t] = v2;
@@ -146,51 +189,40 @@ __global__ void __launch_bounds__(256) k_apvm64(DevMesh M, const double *__restr
     const int n = M.c_nnb[i];
     for (int j = 0; j < n; ++j) {
       const int ed = M.c_ed[j * nv + i];
-      const double su = (M.c_sd[j * nv + i] < 0.0 ? -1.0 : 1.0) * u[ed];
+      const double su = sign_of(M.c_sd[j * nv + i], u[ed]);
       const double d = M.e_dleng[ed];
       v0 = v0 + su * (M.e_c[ed] - p0) * d;
       v1 = v1 + su * (M.e_c[ne + ed] - p1) * d;
       v2 = v2 + su * (M.e_c[2 * ne + ed] - p2) * d;
     }
-    const double A = M.c_areag[i];
-    v0 = v0 / A;
-    v1 = v1 / A;
-    v2 = v2 / A;
-    proj_sphere(v0, v1, v2, p0, p1, p2);
+    const double A = M.c_areag[i], rA = M.c_rareag[i];
+    v0 = div_by(v0, A, rA);
+    v1 = div_by(v1, A, rA);
+    v2 = div_by(v2, A, rA);
+    proj_sphere(v0, v1, v2, p0, p1, p2, M.c_nrm[i], M.c_rnrm[i]);
     vhx[i] = v0;
     vhx[nv + i] = v1;
     vhx[2 * nv + i] = v2;
   }
 }
 
-// scalar_hx2ed (:89-97), scalar_elem_product (:1546), scalar_tr2ed (:124-176:
-// the plain average for trsk, circumcentre-distance weights for bary) or,
-// for gass18, scalar_elem_divide of the rhombus averages of eta and h_tr
-// (swm.f90:2475-2480); with qg != NULL the apvm correction of q_ed
-// (:1495-1502), coef = pvspar dt
-__global__ void __launch_bounds__(256) k_edge_pre64(DevMesh M, const double *__restrict__ h,
-                                                    const double *__restrict__ u,
-                                                    const double *__restrict__ q_tr,
-                                                    double *__restrict__ h_ed,
-                                                    double *__restrict__ uh,
-                                                    double *__restrict__ q_ed,
-                                                    const double *__restrict__ qg,
-                                                    const double *__restrict__ vhx,
-                                                    double coef, int scheme,
-                                                    const double *__restrict__ eta_t,
-                                                    const double *__restrict__ h_trs,
-                                                    int pv_on, int *flags) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+// Twice the PV of edge e: scalar_tr2ed (:124-176: the plain average for trsk,
+// circumcentre-distance weights for bary) or, for gass18, scalar_elem_divide
+// of the rhombus averages of eta and h_tr (swm.f90:2475-2480); with qg !=
+// NULL the apvm correction of q_ed (:1495-1502), coef = pvspar dt
+__device__ __forceinline__ double edge_pv2(const DevMesh &M, int e,
+                                           const double *__restrict__ q_tr,
+                                           const double *__restrict__ qg,
+                                           const double *__restrict__ vhx, double coef,
+                                           int scheme, const double *__restrict__ eta_t,
+                                           const double *__restrict__ h_trs, int pv_on,
+                                           int *flags) {
   const int ne = M.ne;
-  if (e >= ne) return;
-  const double he = (h[M.e_v[e]] + h[M.e_v[ne + e]]) * 0.5;
-  h_ed[e] = he;
-  uh[e] = u[e] * he;
   const int t1 = M.e_sh[e], t2 = M.e_sh[ne + e];
   double q;
   if (scheme == IMODEL_SWM_PXT16) {
     const double d1 = M.e_dist[e], d2 = M.e_dist[ne + e];
-    q = (d2 * q_tr[t1] + d1 * q_tr[t2]) / (d1 + d2);
+    q = div_by(d2 * q_tr[t1] + d1 * q_tr[t2], M.e_dsum[e], M.e_rdsum[e]);
   } else if (scheme == IMODEL_SWM_GASS18) {
     const double a1 = M.t_areag[t1], a2 = M.t_areag[t2];
     const double eta_ed = (a1 * eta_t[t1] + a2 * eta_t[t2]) / (a1 + a2);
@@ -203,7 +235,9 @@ __global__ void __launch_bounds__(256) k_edge_pre64(DevMesh M, const double *__r
         q = eta_ed / h_rhb;
     }
   } else {
-    q = 0.5 * (q_tr[t1] + q_tr[t2]);
+    const double q2 = q_tr[t1] + q_tr[t2];
+    if (!qg) return q2;
+    q = 0.5 * q2;
   }
   if (qg) {
     const int nt = M.nt, nv = M.nv;
@@ -214,59 +248,73 @@ __global__ void __launch_bounds__(256) k_edge_pre64(DevMesh M, const double *__r
                  b2 = vhx[2 * nv + c1] + vhx[2 * nv + c2];
     q = q - coef * (a0 * b0 + a1 * b1 + a2 * b2);
   }
-  q_ed[e] = q;
+  return q + q;
 }
 
-// div_hx(uh) (:613-661), kinetic_energy_hx trsk (:1162-1171), Bernoulli
-// potential (swm.f90:2533-2536) and the mass-equation RK stage
-__global__ void __launch_bounds__(256) k_cell64(DevMesh M, const double *__restrict__ h,
-                                                const double *__restrict__ u,
-                                                const double *__restrict__ uh,
-                                                double *__restrict__ bern,
-                                                const double *__restrict__ yn,
-                                                double *__restrict__ acc,
-                                                double *__restrict__ yout,
-                                                double *__restrict__ tend, int stage,
-                                                double dt, const double *__restrict__ kcv,
-                                                double *__restrict__ coefdiv, int perot_ke) {
+// Blocks [0, nbc): div_hx(uh) (:613-661), kinetic_energy_hx trsk
+// (:1162-1171), Bernoulli potential (swm.f90:2533-2536) and the
+// mass-equation RK stage.  The blocks after: q2, twice the edges' PV.  The
+// two do not read each other; sharing a launch fills the chip on small grids.
+__global__ void __launch_bounds__(256)
+    k_cell64(DevMesh M, const double *__restrict__ h, const double *__restrict__ u,
+             const double2 *__restrict__ fe, double *__restrict__ bern,
+             const double *__restrict__ yn, double *__restrict__ acc, double *__restrict__ yout,
+             double *__restrict__ tend, int stage, double dt, const double *__restrict__ kcv,
+             double *__restrict__ coefdiv, int nbc, double *__restrict__ q2,
+             const double *__restrict__ q_tr, const double *__restrict__ qg,
+             const double *__restrict__ vhx, double coef, int scheme,
+             const double *__restrict__ eta_t, const double *__restrict__ h_trs, int pv_on,
+             int *flags) {
+  if (static_cast<int>(blockIdx.x) >= nbc) {
+    const int e = (blockIdx.x - nbc) * blockDim.x + threadIdx.x;
+    if (e < M.ne) q2[e] = edge_pv2(M, e, q_tr, qg, vhx, coef, scheme, eta_t, h_trs, pv_on, flags);
+    return;
+  }
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nv = M.nv;
   if (i >= nv) return;
   const int n = M.c_nnb[i];
-  double d = 0.0, k = 0.0, du = 0.0;
-  for (int j = 0; j < n; ++j) {
-    const int e = M.c_ed[j * nv + i];
-    d = d + uh[e] * M.c_sd[j * nv + i];
-    const double ue = u[e];
-    k = k + M.e_kew[e] * (ue * ue);
-    if (coefdiv) du = du + ue * M.c_sd[j * nv + i];
+  const double A = M.c_areag[i], rA = M.c_rareag[i];
+  // c_eds: the slot's edge with ttgout < 0 in bit 31; d is twice the sum
+  double d = 0.0, k = 0.0;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    if (j >= n) break;
+    const uint32_t es = M.c_eds[j * nv + i];
+    const double2 f = fe[es & 0x7FFFFFFFu];
+    d = d + __hiloint2double(__double2hiint(f.x) ^ (es & 0x80000000u), __double2loint(f.x));
+    k = k + f.y;
   }
   // with diffusion on: div_hx(u) (:613-661), diffusion_ed's K div u
-  if (coefdiv) coefdiv[i] = kcv[i] * (du / M.c_areag[i] / M.erad);
-  const double divuh = d / M.c_areag[i] / M.erad;
+  if (coefdiv) {
+    double du = 0.0;
+    for (int j = 0; j < n; ++j) du = du + u[M.c_ed[j * nv + i]] * M.c_sd[j * nv + i];
+    coefdiv[i] = kcv[i] * div_by(div_by(du, A, rA), M.erad, M.rerad);
+  }
+  const double divuh = div_by(div_by(d * 0.5, A, rA), M.erad, M.rerad);
   double ke;
-  if (perot_ke) {
+  if (scheme == IMODEL_SWM_PXT16) {
     // kinetic_energy_hx, perhx branch (:1172-1173): half the squared
-    // vector_edhx2hx_perot (:454-509, HTC) of u
-    const int ne = M.ne;
-    const double p0 = M.c_p[i], p1 = M.c_p[nv + i], p2 = M.c_p[2 * nv + i];
+    // vector_edhx2hx_perot (:454-509, HTC) of u; c_off = ed%c%p - v%p
     double v0 = 0.0, v1 = 0.0, v2 = 0.0;
     for (int j = 0; j < n; ++j) {
-      const int ed = M.c_ed[j * nv + i];
-      const double su = (M.c_sd[j * nv + i] < 0.0 ? -1.0 : 1.0) * u[ed];
+      const uint32_t es = M.c_eds[j * nv + i];
+      const int ed = static_cast<int>(es & 0x7FFFFFFFu);
+      const double ue = u[ed];
+      const double su = __hiloint2double(__double2hiint(ue) ^ (es & 0x80000000u),
+                                         __double2loint(ue));
       const double dl = M.e_dleng[ed];
-      v0 = v0 + su * (M.e_c[ed] - p0) * dl;
-      v1 = v1 + su * (M.e_c[ne + ed] - p1) * dl;
-      v2 = v2 + su * (M.e_c[2 * ne + ed] - p2) * dl;
+      v0 = v0 + su * M.c_off[(3 * j) * nv + i] * dl;
+      v1 = v1 + su * M.c_off[(3 * j + 1) * nv + i] * dl;
+      v2 = v2 + su * M.c_off[(3 * j + 2) * nv + i] * dl;
     }
-    const double A = M.c_areag[i];
-    v0 = v0 / A;
-    v1 = v1 / A;
-    v2 = v2 / A;
-    proj_sphere(v0, v1, v2, p0, p1, p2);
-    ke = (v0 * v0 + v1 * v1 + v2 * v2) / 2.0;
+    v0 = div_by(v0, A, rA);
+    v1 = div_by(v1, A, rA);
+    v2 = div_by(v2, A, rA);
+    proj_sphere(v0, v1, v2, M.c_p[i], M.c_p[nv + i], M.c_p[2 * nv + i], M.c_nrm[i], M.c_rnrm[i]);
+    ke = (v0 * v0 + v1 * v1 + v2 * v2) * 0.5;
   } else {
-    ke = k / M.c_cellarea[i];
+    ke = div_by(k, M.c_cellarea[i], M.c_rcellarea[i]);
   }
   bern[i] = M.grav * (h[i] + M.c_bt[i]) + ke;
   const double masseq = -divuh;
@@ -276,36 +324,15 @@ __global__ void __launch_bounds__(256) k_cell64(DevMesh M, const double *__restr
     yout[i] = rk_stage(stage, masseq, yn[i], acc + i, dt);
 }
 
-// grad_ed (:511-548) + coriolis_ed TRSK (:1283-1308) and the momentum RK stage
-__global__ void __launch_bounds__(256) k_edge64(DevMesh M, const double *__restrict__ bern,
-                                                const double *__restrict__ uh,
-                                                const double *__restrict__ q_ed,
-                                                const double *__restrict__ yn,
-                                                double *__restrict__ acc,
-                                                double *__restrict__ yout,
-                                                double *__restrict__ tend, int stage,
-                                                double dt, int mom_on,
-                                                const double *__restrict__ dif1,
-                                                const double *__restrict__ dif2,
-                                                const int32_t *__restrict__ stq) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ne = M.ne;
-  if (e >= ne) return;
-  const double l = M.e_leng[e];
-  double g = bern[M.e_v[ne + e]] - bern[M.e_v[e]];
-  g = g / l / M.erad;
-  const double qe = q_ed[e];
-  const int ns = M.e_nst[e];
-  double q = 0.0;
-  for (int s = 0; s < ns; ++s) {
-    const int k = M.e_stk[s * ne + e];
-    // gass18 (:1378-1410): the PV of the edge connecting e and k when there
-    // is one (stq != NULL), else the TRSK average
-    const int c3 = stq ? stq[s * ne + e] : -1;
-    const double qtmp = c3 >= 0 ? q_ed[c3] : 0.5 * (qe + q_ed[k]);
-    q = q + uh[k] * qtmp * M.e_dleng[k] * M.e_stw[s * ne + e];
-  }
-  q = q / l;
+// the momentum tendency from its two terms (swm.f90:2578-2594) and the RK
+// stage
+__device__ __forceinline__ void edge_update64(int e, double g, double q,
+                                              const double *__restrict__ yn,
+                                              double *__restrict__ acc,
+                                              double *__restrict__ yout,
+                                              double *__restrict__ tend, int stage, double dt,
+                                              int mom_on, const double *__restrict__ dif1,
+                                              const double *__restrict__ dif2) {
   double momeq = -g - q;
   // diffusion, then hyperdiffusion (swm.f90:2578-2589)
   if (dif1) momeq = momeq + dif1[e];
@@ -317,10 +344,52 @@ __global__ void __launch_bounds__(256) k_edge64(DevMesh M, const double *__restr
     yout[e] = rk_stage(stage, momeq, yn[e], acc + e, dt);
 }
 
+// grad_ed (:511-548) + coriolis_ed TRSK (:1283-1308) and the momentum RK stage
+__global__ void __launch_bounds__(256) k_edge64(DevMesh M, const double *__restrict__ bern,
+                                                const double *__restrict__ uh2,
+                                                const double *__restrict__ q2,
+                                                const double *__restrict__ yn,
+                                                double *__restrict__ acc,
+                                                double *__restrict__ yout,
+                                                double *__restrict__ tend, int stage,
+                                                double dt, int mom_on,
+                                                const double *__restrict__ dif1,
+                                                const double *__restrict__ dif2,
+                                                const int32_t *__restrict__ stq) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int ne = M.ne;
+  if (e >= ne) return;
+  const double l = M.e_leng[e], rl = M.e_rleng[e];
+  double g = bern[M.e_v[ne + e]] - bern[M.e_v[e]];
+  g = div_by(div_by(g, l, rl), M.erad, M.rerad);
+  const double qe = q2[e];
+  const int ns = M.e_nst[e];
+  double q = 0.0;
+  // per slot: F_k (q_e + q_k) / 2 d_k w, in that order; 2 F, 2 q and d / 8
+  auto slot = [&](int s) {
+    const int k = M.e_stk[s * ne + e];
+    // gass18 (:1378-1410): the PV of the edge connecting e and k when there
+    // is one (stq != NULL), else the TRSK average
+    const int c3 = stq ? stq[s * ne + e] : -1;
+    const double qs = c3 >= 0 ? q2[c3] + q2[c3] : qe + q2[k];
+    q = q + uh2[k] * qs * M.e_d8[k] * M.e_stw[s * ne + e];
+  };
+  if (ns == 10) {
+    // hexagons on both sides (all but 60 edges): unrolled, so that the
+    // gathers of all slots are in flight together
+#pragma unroll
+    for (int s = 0; s < 10; ++s) slot(s);
+  } else {
+    for (int s = 0; s < ns; ++s) slot(s);
+  }
+  q = div_by(q, l, rl);
+  edge_update64(e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
+}
+
 // dtred: vector_edhx2tr_perot (:345-406, HTC) of uh at the triangle
 // circumcentres, cross(tr%c, v) / tr%areag, times q_tr (vector_elem_product,
 // :1617-1649); signcor = dsign(1, tr%tg) is the sign of t_lt
-__global__ void __launch_bounds__(256) k_vhq64(DevMesh M, const double *__restrict__ uh,
+__global__ void __launch_bounds__(256) k_vhq64(DevMesh M, const double *__restrict__ uh2,
                                                const double *__restrict__ q_tr,
                                                double *__restrict__ vhq) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -331,24 +400,24 @@ __global__ void __launch_bounds__(256) k_vhq64(DevMesh M, const double *__restri
 #pragma unroll
   for (int s = 0; s < 3; ++s) {
     const int ed = M.t_ed[s * nt + t];
-    const double su = (M.t_lt[s * nt + t] < 0.0 ? -1.0 : 1.0) * uh[ed];
+    const double su = sign_of(M.t_lt[s * nt + t], uh2[ed]) * 0.5;
     const double l = M.e_leng[ed];
     v0 = v0 + su * (M.e_c[ed] - c0) * l;
     v1 = v1 + su * (M.e_c[ne + ed] - c1) * l;
     v2 = v2 + su * (M.e_c[2 * ne + ed] - c2) * l;
   }
   const double w0 = c1 * v2 - c2 * v1, w1 = c2 * v0 - c0 * v2, w2 = c0 * v1 - c1 * v0;
-  const double A = M.t_areag[t], q = q_tr[t];
-  vhq[t] = w0 / A * q;
-  vhq[nt + t] = w1 / A * q;
-  vhq[2 * nt + t] = w2 / A * q;
+  const double A = M.t_areag[t], rA = M.t_rareag[t], q = q_tr[t];
+  vhq[t] = div_by(w0, A, rA) * q;
+  vhq[nt + t] = div_by(w1, A, rA) * q;
+  vhq[2 * nt + t] = div_by(w2, A, rA) * q;
 }
 
 // grad_ed (:511-548) + coriolis_ed's dtred (:1310-1329) or pered
 // (:1330-1377) branch, HTC, and the momentum RK stage
 __global__ void __launch_bounds__(256) k_edge64r(DevMesh M, const double *__restrict__ bern,
-                                                 const double *__restrict__ uh,
-                                                 const double *__restrict__ q_ed,
+                                                 const double *__restrict__ uh2,
+                                                 const double *__restrict__ q2,
                                                  const double *__restrict__ vhq,
                                                  const double *__restrict__ yn,
                                                  double *__restrict__ acc,
@@ -360,62 +429,60 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh M, const double *__rest
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne, nv = M.nv, nt = M.nt;
   if (e >= ne) return;
-  const double l = M.e_leng[e];
   double g = bern[M.e_v[ne + e]] - bern[M.e_v[e]];
-  g = g / l / M.erad;
+  g = div_by(div_by(g, M.e_leng[e], M.e_rleng[e]), M.erad, M.rerad);
   double v0, v1, v2;
   if (scheme == IMODEL_SWM_DTRED) {
     // the dual-triangle reconstructions of the edge's two triangles,
     // weighted by the other triangle's circumcentre distance
     const int k1 = M.e_sh[e], k2 = M.e_sh[ne + e];
     const double d1 = M.e_dist[e], d2 = M.e_dist[ne + e];
-    v0 = (d2 * vhq[k1] + d1 * vhq[k2]) / (d1 + d2);
-    v1 = (d2 * vhq[nt + k1] + d1 * vhq[nt + k2]) / (d1 + d2);
-    v2 = (d2 * vhq[2 * nt + k1] + d1 * vhq[2 * nt + k2]) / (d1 + d2);
+    const double ds = M.e_dsum[e], rds = M.e_rdsum[e];
+    v0 = div_by(d2 * vhq[k1] + d1 * vhq[k2], ds, rds);
+    v1 = div_by(d2 * vhq[nt + k1] + d1 * vhq[nt + k2], ds, rds);
+    v2 = div_by(d2 * vhq[2 * nt + k1] + d1 * vhq[2 * nt + k2], ds, rds);
   } else {
     // pered: at each of the edge's cells the Perot reconstruction of
     // uh (q_e + q_k) / 2 over the cell's edges, projected on the tangent
-    // plane; their average
-    const double qe = q_ed[e];
+    // plane; their average (halved together: 0.5 x + 0.5 y and 0.5 (x + y)
+    // are the same rounding)
+    const double qe = q2[e];
     double vc[2][3];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int c = M.e_v[i * ne + e];
-      const double p0 = M.c_p[c], p1 = M.c_p[nv + c], p2 = M.c_p[2 * nv + c];
       double a0 = 0.0, a1 = 0.0, a2 = 0.0;
       const int n = M.c_nnb[c];
-      for (int j = 0; j < n; ++j) {
-        const int l2 = M.c_ed[j * nv + c];
-        const double qtmp = 0.5 * (qe + q_ed[l2]);
-        const double f = (M.c_sd[j * nv + c] < 0.0 ? -1.0 : 1.0) * uh[l2] * qtmp;
-        const double d = M.e_dleng[l2];
-        a0 = a0 + f * (M.e_c[l2] - p0) * d;
-        a1 = a1 + f * (M.e_c[ne + l2] - p1) * d;
-        a2 = a2 + f * (M.e_c[2 * ne + l2] - p2) * d;
+#pragma unroll
+      for (int j = 0; j < 6; ++j) {
+        if (j >= n) break;
+        const uint32_t es = M.c_eds[j * nv + c];
+        const int l2 = static_cast<int>(es & 0x7FFFFFFFu);
+        const double x = uh2[l2];
+        const double f = __hiloint2double(__double2hiint(x) ^ (es & 0x80000000u),
+                                          __double2loint(x)) * (qe + q2[l2]);
+        const double d = M.e_d8[l2];
+        a0 = a0 + f * M.c_off[(3 * j) * nv + c] * d;
+        a1 = a1 + f * M.c_off[(3 * j + 1) * nv + c] * d;
+        a2 = a2 + f * M.c_off[(3 * j + 2) * nv + c] * d;
       }
-      const double A = M.c_areag[c];
-      a0 = a0 / A;
-      a1 = a1 / A;
-      a2 = a2 / A;
-      proj_sphere(a0, a1, a2, p0, p1, p2);
+      const double A = M.c_areag[c], rA = M.c_rareag[c];
+      a0 = div_by(a0, A, rA);
+      a1 = div_by(a1, A, rA);
+      a2 = div_by(a2, A, rA);
+      proj_sphere(a0, a1, a2, M.c_p[c], M.c_p[nv + c], M.c_p[2 * nv + c], M.c_nrm[c],
+                  M.c_rnrm[c]);
       vc[i][0] = a0;
       vc[i][1] = a1;
       vc[i][2] = a2;
     }
-    v0 = 0.5 * vc[0][0] + 0.5 * vc[1][0];
-    v1 = 0.5 * vc[0][1] + 0.5 * vc[1][1];
-    v2 = 0.5 * vc[0][2] + 0.5 * vc[1][2];
+    v0 = 0.5 * (vc[0][0] + vc[1][0]);
+    v1 = 0.5 * (vc[0][1] + vc[1][1]);
+    v2 = 0.5 * (vc[0][2] + vc[1][2]);
   }
-  proj_sphere(v0, v1, v2, M.e_c[e], M.e_c[ne + e], M.e_c[2 * ne + e]);
+  proj_sphere(v0, v1, v2, M.e_c[e], M.e_c[ne + e], M.e_c[2 * ne + e], M.e_nrm[e], M.e_rnrm[e]);
   const double q = -(v0 * M.e_nr[e] + v1 * M.e_nr[ne + e] + v2 * M.e_nr[2 * ne + e]);
-  double momeq = -g - q;
-  if (dif1) momeq = momeq + dif1[e];
-  if (dif2) momeq = momeq - dif2[e];
-  if (!mom_on) momeq = 0.0;
-  if (stage < 0)
-    tend[e] = momeq;
-  else
-    yout[e] = rk_stage(stage, momeq, yn[e], acc + e, dt);
+  edge_update64(e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
 }
 
 // diffusion_ed (swm_operators.f90:855-895), first half: coefdiv = K
@@ -434,7 +501,7 @@ __global__ void __launch_bounds__(256) k_difcv64(DevMesh M, const double *__rest
     const int n = M.c_nnb[i];
     double d = 0.0;
     for (int j = 0; j < n; ++j) d = d + x[M.c_ed[j * nv + i]] * M.c_sd[j * nv + i];
-    const double divx = d / M.c_areag[i] / M.erad;
+    const double divx = div_by(div_by(d, M.c_areag[i], M.c_rareag[i]), M.erad, M.rerad);
     coefdiv[i] = kcv[i] * divx;
   } else {
     const int t = (blockIdx.x - nbc) * blockDim.x + threadIdx.x;
@@ -443,7 +510,7 @@ __global__ void __launch_bounds__(256) k_difcv64(DevMesh M, const double *__rest
     double z = 0.0;
 #pragma unroll
     for (int s = 0; s < 3; ++s) z = z + x[M.t_ed[s * nt + t]] * M.t_lt[s * nt + t];
-    z = z / M.t_areag[t] / M.erad;
+    z = div_by(div_by(z, M.t_areag[t], M.t_rareag[t]), M.erad, M.rerad);
     coefvort[t] = kt[t] * z;
   }
 }
@@ -457,9 +524,9 @@ __global__ void __launch_bounds__(256) k_diflap64(DevMesh M, const double *__res
   const int ne = M.ne;
   if (e >= ne) return;
   double g = coefdiv[M.e_v[ne + e]] - coefdiv[M.e_v[e]];
-  g = g / M.e_leng[e] / M.erad;
+  g = div_by(div_by(g, M.e_leng[e], M.e_rleng[e]), M.erad, M.rerad);
   double gt = M.e_sgtg[e] * (coefvort[M.e_sh[ne + e]] - coefvort[M.e_sh[e]]);
-  gt = gt / (M.e_dleng[e] * M.erad);
+  gt = div_by(gt, M.e_dlerad[e], M.e_rdlerad[e]);
   lap[e] = g - gt;
 }
 
@@ -859,6 +926,7 @@ __global__ void __launch_bounds__(kRedThreads) k_errors(DevMesh M, const T *__re
 }
 
 inline int nblocks(int n, int t) { return (n + t - 1) / t; }
+inline int block64(int) { return BLOCK64; }
 
 }  // namespace
 
@@ -871,45 +939,44 @@ void launch_stage64(const DevMesh &M, const Work<double> &W, const double *h_in,
   // second application), before the edge kernel
   const Diffusion<double> &D = W.dif;
   const int sch = W.scheme;
-  k_tri64<<<nblocks(M.nt, 256), 256, 0, s>>>(M, h_in, u_in, W.q_tr, W.pv_on, W.flags, D.kt,
-                                              D.on ? D.coefvort : nullptr, sch, W.eta_t,
-                                              W.h_trs);
+  const int bt = block64(M.nt), bc = block64(M.nv), be = block64(M.ne);
+  const int nbt = nblocks(M.nt, bt);
+  k_tri64<<<nbt + nblocks(M.ne, bt), bt, 0, s>>>(M, h_in, u_in, W.q_tr, W.pv_on, W.flags, D.kt,
+                                                  D.on ? D.coefvort : nullptr, sch, W.eta_t,
+                                                  W.h_trs, W.uh, W.fe, nbt);
   if (ev) cudaEventRecord(ev[1], s);
   const Apvm<double> &A = W.apvm;
   if (A.on) {
-    const int nbt = nblocks(M.nt, 256);
-    k_qgrad64<<<nblocks(M.ne, 256), 256, 0, s>>>(M, W.q_tr, A.qge);
-    k_apvm64<<<nbt + nblocks(M.nv, 256), 256, 0, s>>>(M, A.qge, u_in, A.qg, A.vhx, nbt);
+    k_qgrad64<<<nblocks(M.ne, be), be, 0, s>>>(M, W.q_tr, A.qge);
+    k_apvm64<<<nbt + nblocks(M.nv, bt), bt, 0, s>>>(M, A.qge, u_in, A.qg, A.vhx, nbt);
   }
-  k_edge_pre64<<<nblocks(M.ne, 256), 256, 0, s>>>(M, h_in, u_in, W.q_tr, W.h_ed, W.uh, W.q_ed,
-                                                   A.on ? A.qg : nullptr, A.vhx, A.coef, sch,
-                                                   W.eta_t, W.h_trs, W.pv_on, W.flags);
   if (sch == IMODEL_SWM_DTRED)
-    k_vhq64<<<nblocks(M.nt, 256), 256, 0, s>>>(M, W.uh, W.q_tr, W.vhq);
+    k_vhq64<<<nblocks(M.nt, bt), bt, 0, s>>>(M, W.uh, W.q_tr, W.vhq);
   if (ev) cudaEventRecord(ev[2], s);
-  k_cell64<<<nblocks(M.nv, 256), 256, 0, s>>>(M, h_in, u_in, W.uh, W.bern, W.yn_h, W.acc_h,
-                                               h_out, W.tend_h, stage, dt, D.kcv,
-                                               D.on ? D.coefdiv : nullptr,
-                                               sch == IMODEL_SWM_PXT16 ? 1 : 0);
+  const int nbc = nblocks(M.nv, bc);
+  k_cell64<<<nbc + nblocks(M.ne, bc), bc, 0, s>>>(
+      M, h_in, u_in, W.fe, W.bern, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, D.kcv,
+      D.on ? D.coefdiv : nullptr, nbc, W.q_ed, W.q_tr, A.on ? A.qg : nullptr, A.vhx, A.coef, sch,
+      W.eta_t, W.h_trs, W.pv_on, W.flags);
   if (D.on) {
-    k_diflap64<<<nblocks(M.ne, 256), 256, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap);
+    k_diflap64<<<nblocks(M.ne, be), be, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap);
     if (D.k4) {
-      const int nbc = nblocks(M.nv, 256), nbt = nblocks(M.nt, 256);
-      k_difcv64<<<nbc + nbt, 256, 0, s>>>(M, D.lap, D.kcv, D.kt, D.coefdiv, D.coefvort, nbc);
-      k_diflap64<<<nblocks(M.ne, 256), 256, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap2);
+      k_difcv64<<<nbc + nblocks(M.nt, bc), bc, 0, s>>>(M, D.lap, D.kcv, D.kt, D.coefdiv,
+                                                        D.coefvort, nbc);
+      k_diflap64<<<nblocks(M.ne, be), be, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap2);
     }
   }
   if (ev) cudaEventRecord(ev[3], s);
   if (sch == IMODEL_SWM_PXT16 || sch == IMODEL_SWM_DTRED)
-    k_edge64r<<<nblocks(M.ne, 256), 256, 0, s>>>(M, W.bern, W.uh, W.q_ed, W.vhq, W.yn_u, W.acc_u,
-                                                  u_out, W.tend_u, stage, dt, W.mom_on,
-                                                  D.k2 ? D.lap : nullptr,
-                                                  D.k4 ? D.lap2 : nullptr, sch);
+    k_edge64r<<<nblocks(M.ne, be), be, 0, s>>>(M, W.bern, W.uh, W.q_ed, W.vhq, W.yn_u, W.acc_u,
+                                                u_out, W.tend_u, stage, dt, W.mom_on,
+                                                D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 : nullptr,
+                                                sch);
   else
-    k_edge64<<<nblocks(M.ne, 256), 256, 0, s>>>(M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u, u_out,
-                                                 W.tend_u, stage, dt, W.mom_on,
-                                                 D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 : nullptr,
-                                                 sch == IMODEL_SWM_GASS18 ? M.e_stq : nullptr);
+    k_edge64<<<nblocks(M.ne, be), be, 0, s>>>(M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u, u_out,
+                                               W.tend_u, stage, dt, W.mom_on,
+                                               D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 : nullptr,
+                                               sch == IMODEL_SWM_GASS18 ? M.e_stq : nullptr);
   if (ev) cudaEventRecord(ev[4], s);
 }
 

@@ -8,6 +8,7 @@
 // sources, exp(20 theta) in qsat, is formed once on the host (theta keeps its
 // initial value in the reference's RK4 path) and read here.
 #include "swm_common.cuh"
+#include "swm_div.cuh"
 
 namespace imodel {
 namespace {
@@ -17,29 +18,47 @@ constexpr double kEps = 1.1920928955078125e-07;
 // initialize_moist_swm_fields (moist_swm.f90:730-732)
 constexpr double kLscale = 10.0, kGammaR = 0.001, kQprecip = 0.0001;
 
+// dt k / 2 as (dt / 2) k and acc + 2 k as one fused operation with an exact
+// product: the same roundings (moist_swm.f90:1880-1960)
 __device__ __forceinline__ double rk_stage(int stage, double k, double yn, double *acc, double dt) {
-  // ode_rk4_moist_swm, moist_swm.f90:1880-1960
   if (stage == 0) {
     *acc = k;
-    return yn + dt * k / 2.0;
+    return yn + (dt * 0.5) * k;
   } else if (stage == 1) {
-    *acc = *acc + 2.0 * k;
-    return yn + dt * k / 2.0;
+    *acc = __fma_rn(2.0, k, *acc);
+    return yn + (dt * 0.5) * k;
   } else if (stage == 2) {
-    *acc = *acc + 2.0 * k;
+    *acc = __fma_rn(2.0, k, *acc);
     return yn + dt * k;
   }
-  return yn + dt * (*acc + k) / 6.0;
+  return yn + div_by(dt * (*acc + k), 6.0, kThird2);
 }
 // Fortran max(0, x) / min(a, b) as std::max / std::min evaluate them
 __device__ __forceinline__ double fmax0(double x) { return (0.0 < x) ? x : 0.0; }
 __device__ __forceinline__ double fminq(double a, double b) { return (b < a) ? b : a; }
 
-// Edges: u q_e for every advanced tracer with advmtd = "trsk" (scalar_hx2ed
-// + scalar_elem_product, divhx; "upw1" forms its fluxes in the cell
-// kernel); with the shallow-water terms on, the thermal momentum source
-// (source, moist_swm.f90:1299-1315) added to the momentum tendency and u's
-// RK stage.
+// what the sources read that stays fixed in a run: g theta_e grad(b) of
+// moist_swm.f90:1299-1315 at the edges, q0 exp(20 theta) of qsat at the cells
+__global__ void __launch_bounds__(256) k_moist_consts(DevMesh M, const double *__restrict__ th,
+                                                      double *__restrict__ ex20, double q0,
+                                                      double *__restrict__ gthb) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < M.nv) ex20[e] = q0 * ex20[e];
+  if (e >= M.ne) return;
+  const int v1 = M.e_v[e], v2 = M.e_v[M.ne + e];
+  double gb = M.c_bt[v2] - M.c_bt[v1];
+  gb = gb / M.e_leng[e] / M.erad;
+  const double th_ed = (th[v1] + th[v2]) * 0.5;
+  gthb[e] = M.grav * (th_ed * gb);
+}
+
+// Edges: twice u q_e times d for every advanced tracer with advmtd = "trsk"
+// (scalar_hx2ed + scalar_elem_product, divhx, and div_hx's product with the
+// edge length, which both cells form alike up to the sign; "upw1" forms its
+// fluxes in the cell kernel); with the shallow-water terms on, the thermal
+// momentum source (source, moist_swm.f90:1299-1315) added to the momentum
+// tendency and u's RK stage.  FP64-pipe bound like the FP64 step: divisions by
+// div_by, factors of two left out until the sums, run constants formed once.
 __global__ void __launch_bounds__(256) k_moist_edge(DevMesh M, MoistArgs A) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
@@ -47,27 +66,24 @@ __global__ void __launch_bounds__(256) k_moist_edge(DevMesh M, MoistArgs A) {
   const int v1 = M.e_v[e], v2 = M.e_v[ne + e];
   const double ue = A.u_in[e];
   if (!A.upw1) {
+    const double dl = M.e_dleng[e];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       if (!((A.active >> k) & 1)) continue;
-      const double qe = (A.q_in[k][v1] + A.q_in[k][v2]) * 0.5;
-      A.uphi[static_cast<size_t>(k) * ne + e] = ue * qe;
+      A.uphi[static_cast<size_t>(k) * ne + e] = ue * (A.q_in[k][v1] + A.q_in[k][v2]) * dl;
     }
   }
   if (!A.swm) return;
-  const double l = M.e_leng[e], erad = M.erad, grav = M.grav;
-  double g = A.h_in[v2] * A.q_in[0][v2] - A.h_in[v1] * A.q_in[0][v1];
-  g = g / l / erad;
-  const double hed = A.h_ed[e];
+  const double h1 = A.h_in[v1], h2 = A.h_in[v2];
+  double g = h2 * A.q_in[0][v2] - h1 * A.q_in[0][v1];
+  g = div_by(div_by(g, M.e_leng[e], M.e_rleng[e]), M.erad, M.rerad);
+  const double hed = (h1 + h2) * 0.5;
   double gpi_oh = 0.0;
   if (fabs(hed) < kEps / 100000.0)
     atomicOr(A.flags, 1);
   else
     gpi_oh = g / hed;
-  double gb = M.c_bt[v2] - M.c_bt[v1];
-  gb = gb / l / erad;
-  const double th_ed = (A.th[v1] + A.th[v2]) * 0.5;
-  const double su = (grav * 0.5) * gpi_oh + grav * (th_ed * gb);
+  const double su = (M.grav * 0.5) * gpi_oh + A.gthb[e];
   const double momeq = A.tend_u[e] + su;
   A.u_out[e] = rk_stage(A.stage, momeq, A.yn_u[e], A.acc_u + e, A.dt);
 }
@@ -84,22 +100,25 @@ __global__ void __launch_bounds__(256) k_moist_cell(DevMesh M, MoistArgs A) {
   if (A.swm) {
     A.h_out[i] = rk_stage(A.stage, A.tend_h[i], A.yn_h[i], A.acc_h + i, A.dt);
     const double hi = A.h_in[i];
-    const double qs = A.q0 * A.ex20[i] / ((hi + M.c_bt[i]) * M.grav);
+    const double qs = A.q0ex[i] / ((hi + M.c_bt[i]) * M.grav);
     double gamma_v = 1.0 + kLscale * (20.0 * qs);
     gamma_v = 1.0 / gamma_v;
     const double qv = A.qv[i], qc = A.qc[i];
-    double dqv = gamma_v * (qv - qs);
-    dqv = fmax0(dqv) / A.dt;
-    double dqc = fmax0(-gamma_v * (qv - qs));
-    dqc = fminq(qc, dqc) / A.dt;
-    const double dqr = fmax0(kGammaR * (qc - kQprecip)) / A.dt;
+    const double r = gamma_v * (qv - qs);
+    const double dqv = div_by(fmax0(r), A.dt, A.rdt);
+    const double dqc = div_by(fminq(qc, fmax0(-r)), A.dt, A.rdt);
+    const double dqr = div_by(fmax0(kGammaR * (qc - kQprecip)), A.dt, A.rdt);
     hs[1] = hi * (dqc - dqv);
     hs[2] = hi * (dqv - dqc - dqr);
     hs[3] = hi * dqr;
     hs[0] = hi * (kLscale * (dqv - dqc));
   }
   const int n = M.c_nnb[i];
-  const double A_i = M.c_areag[i], erad = M.erad;
+  const double A_i = M.c_areag[i], rA = M.c_rareag[i];
+  // the slots' edges with ttgout < 0 in bit 31
+  uint32_t es[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) es[j] = j < n ? M.c_eds[j * nv + i] : 0u;
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
     if (!((A.active >> k) & 1)) continue;
@@ -119,16 +138,23 @@ __global__ void __launch_bounds__(256) k_moist_cell(DevMesh M, MoistArgs A) {
       }
     } else {
       const double *uphi = A.uphi + static_cast<size_t>(k) * ne;
-      for (int j = 0; j < n; ++j) d = d + uphi[M.c_ed[j * nv + i]] * M.c_sd[j * nv + i];
+#pragma unroll
+      for (int j = 0; j < 6; ++j) {
+        if (j >= n) break;
+        const double f = uphi[es[j] & 0x7FFFFFFFu];
+        d = d + __hiloint2double(__double2hiint(f) ^ (es[j] & 0x80000000u), __double2loint(f));
+      }
+      d = d * 0.5;
     }
-    double t = -(d / A_i / erad);
+    double t = -div_by(div_by(d, A_i, rA), M.erad, M.rerad);
     if (A.swm && k < 4) t = t + hs[k];
     A.q_out[k][i] = rk_stage(A.stage, t, A.q_yn[k][i], A.q_acc[k] + i, A.dt);
   }
 }
 
 // after a step: qv, qc, qr = h qv / h etc. (scalar_elem_divide, with its
-// guard), the fields the next step's sources read
+// guard), the fields the next step's sources read; one reciprocal (rounded
+// to nearest) serves the three divisions where it is normal
 __global__ void k_moist_q(int nv, const double *__restrict__ h, const double *__restrict__ hqv,
                           const double *__restrict__ hqc, const double *__restrict__ hqr,
                           double *__restrict__ qv, double *__restrict__ qc,
@@ -140,9 +166,10 @@ __global__ void k_moist_q(int nv, const double *__restrict__ h, const double *__
     atomicOr(flags, 1);
     return;
   }
-  qv[i] = hqv[i] / hi;
-  qc[i] = hqc[i] / hi;
-  qr[i] = hqr[i] / hi;
+  const double r = fabs(hi) <= 0x1p500 ? 1.0 / hi : __longlong_as_double(0x7FF8000000000000LL);
+  qv[i] = div_by(hqv[i], hi, r);
+  qc[i] = div_by(hqc[i], hi, r);
+  qr[i] = div_by(hqr[i], hi, r);
 }
 
 // ---- FP32 --------------------------------------------------------------------
@@ -283,9 +310,18 @@ void launch_moist_q32(int nv, const float *hd, float h_ref, const float *hqv, co
   k_moist_q32<<<nblocks(nv, 256), 256, 0, s>>>(nv, hd, h_ref, hqv, hqc, hqr, qv, qc, qr, flags);
 }
 
+void launch_moist_consts(const DevMesh &M, const double *th, double *ex20, double q0,
+                         double *gthb, cudaStream_t s) {
+  // every cell has at least three edges on these grids, two cells an edge, so
+  // ne >= nv; the larger count covers both either way
+  const int n = M.ne > M.nv ? M.ne : M.nv;
+  k_moist_consts<<<nblocks(n, 256), 256, 0, s>>>(M, th, ex20, q0, gthb);
+}
+
 void launch_moist_stage(const DevMesh &M, const MoistArgs &A, cudaStream_t s) {
-  k_moist_edge<<<nblocks(M.ne, 256), 256, 0, s>>>(M, A);
-  k_moist_cell<<<nblocks(M.nv, 256), 256, 0, s>>>(M, A);
+  const int b = BLOCK64;
+  k_moist_edge<<<nblocks(M.ne, b), b, 0, s>>>(M, A);
+  k_moist_cell<<<nblocks(M.nv, b), b, 0, s>>>(M, A);
 }
 
 void launch_moist_q(int nv, const double *h, const double *hqv, const double *hqc,
