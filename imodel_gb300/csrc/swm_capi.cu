@@ -36,7 +36,7 @@ struct Handle {
   std::vector<double> h_areag;                 // reference order, for h_ref
   bool href_fixed = false;
   double h_ref = 0.0;
-  DevMesh M{};
+  DevMesh64 M{};
   std::vector<void *> allocs;
   int32_t *d_cell_n2o = nullptr, *d_edge_n2o = nullptr;
   int32_t *d_cell_o2n = nullptr, *d_edge_o2n = nullptr;
@@ -163,12 +163,11 @@ int alloc_work(Handle *H, Work<T> &W) {
   T **bufs_v[] = {&W.yn_h, &W.ya_h, &W.yb_h, &W.acc_h, &W.bern, &W.tend_h};
   for (T **b : bufs_v)
     if ((rc = dalloc(H, b, H->nv))) return rc;
-  T **bufs_e[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u, &W.uh, &W.q_ed, &W.tend_u};
+  T **bufs_e[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u, &W.h_ed, &W.uh, &W.q_ed, &W.tend_u};
+  constexpr bool fp64 = sizeof(T) == sizeof(double);
   for (T **b : bufs_e)
-    if ((rc = dalloc(H, b, H->ne))) return rc;
-  if (sizeof(T) == sizeof(double) ? (rc = dalloc(H, &W.fe, H->ne))
-                                  : (rc = dalloc(H, &W.h_ed, H->ne)))
-    return rc;
+    if (!(fp64 && b == &W.h_ed) && (rc = dalloc(H, b, H->ne))) return rc;
+  if (fp64 && (rc = dalloc(H, &W.fe, H->ne))) return rc;
   if ((rc = dalloc(H, &W.q_tr, H->nt))) return rc;
   W.flags = H->d_flags;
   W.pv_on = H->testcase >= 2 ? 1 : 0;
@@ -730,7 +729,7 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
     H->href_fixed = true;
   }
   CK(cudaStreamCreateWithFlags(&H->stream, cudaStreamNonBlocking));
-  DevMesh &M = H->M;
+  DevMesh64 &M = H->M;
   M.nv = L.nv;
   M.ne = L.ne;
   M.nt = L.nt;
@@ -802,22 +801,6 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
         (rc = upload(H, L.c_p, &M.c_p)))
       return rc;
   }
-  if (H->precision == IMODEL_SWM_FP64) {
-    Layout64 D;
-    build_layout64(L, scheme, D);
-    M.rerad = D.rerad;
-    if ((rc = upload(H, D.c_rareag, &M.c_rareag)) ||
-        (rc = upload(H, D.c_rcellarea, &M.c_rcellarea)) || (rc = upload(H, D.c_eds, &M.c_eds)) ||
-        (rc = upload(H, D.e_rleng, &M.e_rleng)) || (rc = upload(H, D.e_rdleng, &M.e_rdleng)) ||
-        (rc = upload(H, D.e_d8, &M.e_d8)) || (rc = upload(H, D.e_dlerad, &M.e_dlerad)) ||
-        (rc = upload(H, D.e_rdlerad, &M.e_rdlerad)) || (rc = upload(H, D.t_rareag, &M.t_rareag)) ||
-        (rc = upload(H, D.c_nrm, &M.c_nrm)) || (rc = upload(H, D.c_rnrm, &M.c_rnrm)) ||
-        (rc = upload(H, D.t_nrm, &M.t_nrm)) || (rc = upload(H, D.t_rnrm, &M.t_rnrm)) ||
-        (rc = upload(H, D.e_nrm, &M.e_nrm)) || (rc = upload(H, D.e_rnrm, &M.e_rnrm)) ||
-        (rc = upload(H, D.e_dsum, &M.e_dsum)) || (rc = upload(H, D.e_rdsum, &M.e_rdsum)) ||
-        (rc = upload(H, D.c_off, &M.c_off)))
-      return rc;
-  }
   // the other method wrappers' geometry (empty vectors upload as NULL)
   if (H->precision == IMODEL_SWM_FP32 &&
       ((rc = upload(H, L.c_C32, &M.c_C32)) || (rc = upload(H, L.c_gout, &M.c_gout)) ||
@@ -836,6 +819,13 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
     if ((rc = upload(H, L.t_apw32, &M.t_apw32)) || (rc = upload(H, L.t_cc32, &M.t_cc32)) ||
         (rc = upload(H, L.c_apw32, &M.c_apw32)) || (rc = upload(H, L.c_p32, &M.c_p32)))
       return rc;
+  }
+  if (H->precision == IMODEL_SWM_FP64) {
+    // the FP64 kernels' derived constants, formed on the GPU
+    double *p = nullptr;
+    if ((rc = dalloc(H, &p, consts64_size(M)))) return rc;
+    launch_consts64(M, p, nullptr);  // the stream of the uploads and the zero-fill
+    CK(cudaGetLastError());
   }
   H->d_cell_n2o = const_cast<int32_t *>(cn2o);
   H->d_edge_n2o = const_cast<int32_t *>(en2o);
@@ -1803,6 +1793,9 @@ int imodel_moist_create(const imodel_swm_mesh *m, const imodel_moist_opts *o, vo
         if ((rc = imodel::dalloc(H, &X->q[k][b], nv))) return rc;
     if ((rc = imodel::dalloc(H, &X->uphi, 5 * ne)) || (rc = imodel::dalloc(H, &X->gthb, ne)))
       return rc;
+    // the buffers' zero-fill (default stream) comes before what H->stream writes
+    if (cudaStreamSynchronize(nullptr) != cudaSuccess)
+      return imodel::set_error(H, IMODEL_SWM_ECUDA, "stream synchronize failed");
     if ((rc = moist_in(H, o->theta, X->th, false)) || (rc = moist_in(H, ex.data(), X->ex20, false)))
       return rc;
     imodel::launch_moist_consts(H->M, X->th, X->ex20, X->q0, X->gthb, H->stream);

@@ -9,15 +9,6 @@ namespace imodel {
 struct DevMesh {
   int nv, ne, nt;
   double erad, grav;
-  double rerad;  // 1 / erad
-  // FP64 step: reciprocals of the divisors of its kernels (div_by), the
-  // slot's edge with its sign, d / 8, the norms of the projection points and
-  // pxt16's offsets (swm_layout.h)
-  const double *c_rareag, *c_rcellarea, *e_rleng, *e_rdleng, *t_rareag;
-  const double *e_dlerad, *e_rdlerad, *e_d8;
-  const double *c_nrm, *c_rnrm, *t_nrm, *t_rnrm, *e_nrm, *e_rnrm;
-  const double *e_dsum, *e_rdsum, *c_off;
-  const uint32_t *c_eds;
   // cells
   const int8_t *c_nnb;
   const int32_t *c_ed;
@@ -80,6 +71,27 @@ struct DevMesh {
   const uint8_t *t_dopp;
 };
 
+// What the FP64 kernels read besides (a type of its own: the FP32 kernels'
+// parameters, and with them their code, stay as they are)
+struct DevMesh64 : DevMesh {
+  // FP64 step, formed on the GPU at create (launch_consts64): the
+  // reciprocals, rounded to nearest, of what its kernels divide by (div_by;
+  // NaN where the divisor is zero, not finite or outside 2^-500 .. 2^500: the
+  // kernel then divides) and factors they would otherwise form at every call
+  double rerad;                                // 1 / erad
+  const double *c_rareag, *c_rcellarea;        // [nv]
+  const uint32_t *c_eds;                       // [6][nv] slot's edge, bit 31: ttgout < 0; unused
+                                               // slots: edge 0
+  const double *e_rleng, *e_rdleng, *e_d8;     // [ne] 1 / l, 1 / d, d / 8
+  const double *e_dlerad, *e_rdlerad;          // [ne] d erad and its reciprocal
+  const double *t_rareag;                      // [nt]
+  // |p| of the points of the tangent-plane projections and its reciprocal
+  // (NULL without ed%nr)
+  const double *c_nrm, *c_rnrm, *t_nrm, *t_rnrm, *e_nrm, *e_rnrm;
+  const double *e_dsum, *e_rdsum;              // [ne] pxt16, dtred: d1 + d2
+  const double *c_off;                         // [18][nv] pxt16: (ed%c%p - v%p)_k of slot j at 3 j + k
+};
+
 // Launch configuration of the FP32 stage kernels, chosen by the autotuner.
 //   variant 0: triangle -> edge pre-pass -> cell -> edge (10-entry stencil)
 //   variant 1: triangle -> cell (cell-centred TRSK, writes the PV flux
@@ -93,6 +105,50 @@ struct Tune {
 };
 
 struct LearnedDev;
+
+// Programmatic dependent launch: a kernel of a step may start while its
+// predecessor still runs, load what is fixed (indices, geometry) and then
+// wait for it.  after_prior(x, ...) is that wait; every pointer to data that a
+// kernel of the step writes must be passed to it, so that no load through it
+// can be moved above the wait (a __restrict__ const pointer's loads count as
+// invariant otherwise).
+//
+// early (the FP32 kernels): on grids of fewer than kPdlGrid blocks let the
+// successor start at once rather than as this kernel's blocks end.  Per step:
+// FP32 level 5 27.0 us with plain launches, 24.1 with the wait alone, 20.9
+// with the early start; level 7 50.7, 49.3, 43.7; the moist FP32 step at level
+// 8 432, 422, 412.  At level 9 (10,000 blocks and more) nothing is gained and
+// the early start costs 3 % of the cell kernel.  The FP64 kernels keep the
+// wait alone (level 5 69.9 us plain, 57.7 with the wait, 63.6 early; pxt16 at
+// level 6 325, 323, 422): their blocks must spread evenly over the FP64 pipes,
+// and blocks that start early take the places first freed.
+constexpr unsigned kPdlGrid = 8192;
+template <class P>
+__device__ __forceinline__ void pin_ptr(P &p) {
+  asm volatile("" : "+l"(p));
+}
+template <bool early, class... P>
+__device__ __forceinline__ void after_prior(P &...p) {
+  if (early && gridDim.x < kPdlGrid) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (pin_ptr(p), ...);
+}
+inline bool pdl_grid(int grid) { return static_cast<unsigned>(grid) < kPdlGrid; }
+// launches k, which calls after_prior, so that it may start before the kernel
+// before it in the stream has finished (on grids below kPdlGrid)
+template <class... P, class... A>
+inline void launch_pdl(void (*k)(P...), int grid, int block, cudaStream_t s, A &&...a) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = pdl_grid(grid) ? 1 : 0;
+  cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
+}
 
 // Laplacian diffusion and hyperdiffusion of the momentum (diffusion_ed,
 // hyperdiffusion_ed, swm_operators.f90:855-975; coefficients swm.f90:169-205,
@@ -148,11 +204,15 @@ struct Work {
   int mom_on;        // testcase >= 2: momentum tendency kept, else zeroed
 };
 
+// M's derived FP64 constants, in consts64_size(M) doubles at p
+size_t consts64_size(const DevMesh64 &M);
+void launch_consts64(DevMesh64 &M, double *p, cudaStream_t s);
+
 // One tendency evaluation (stage < 0: write masseq/momeq to tend_*), or RK4
 // stage `stage` (0..3) of classic RK4 reading y_in and writing y_out.
 // ev (may be NULL): 5 events recorded before, between and after the four
 // kernels of the stage, for per-kernel timing outside graph capture.
-void launch_stage64(const DevMesh &M, const Work<double> &W, const double *h_in,
+void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_in,
                     const double *u_in, double *h_out, double *u_out, int stage,
                     double dt, cudaStream_t s, cudaEvent_t *ev = nullptr);
 // The learned corrections' error proxy: per block part[2 b] = sum w (a -
@@ -226,9 +286,9 @@ struct MoistArgs {
 };
 // gthb from theta and the topography (both frozen in a run); ex20 becomes
 // q0 ex20 in place
-void launch_moist_consts(const DevMesh &M, const double *th, double *ex20, double q0,
+void launch_moist_consts(const DevMesh64 &M, const double *th, double *ex20, double q0,
                          double *gthb, cudaStream_t s);
-void launch_moist_stage(const DevMesh &M, const MoistArgs &A, cudaStream_t s);
+void launch_moist_stage(const DevMesh64 &M, const MoistArgs &A, cudaStream_t s);
 void launch_moist_q(int nv, const double *h, const double *hqv, const double *hqc,
                     const double *hqr, double *qv, double *qc, double *qr, int *flags,
                     cudaStream_t s);
@@ -280,6 +340,7 @@ void launch_store_host(int n, const int32_t *o2n, const T *src, double *dst, dou
 // Compensated FP64 integrals.  Scratch: partial sums, 2 doubles per block
 // and quantity; result[kDiagQ] on the device.
 constexpr int kDiagQ = 12;
+constexpr int kMaxStencil = 10;  // slots of the TRSK stencil (swm_layout.h, kMaxSt)
 // threads per block of the FP64 kernels
 #ifndef BLOCK64
 #define BLOCK64 64

@@ -12,6 +12,7 @@ namespace imodel {
 namespace {
 
 // q_t = (curl u / A + f) / h_t  (vort_tr + scalar_hx2tr + scalar_elem_divide)
+template <class Wait>
 __global__ void __launch_bounds__(512) k_tri32(DevMesh M, const float *__restrict__ hd,
                                                const float *__restrict__ u,
                                                float *__restrict__ q_tr, float h_ref,
@@ -21,7 +22,7 @@ __global__ void __launch_bounds__(512) k_tri32(DevMesh M, const float *__restric
                                                float *__restrict__ ht_out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= M.nt) return;
-  tri_body(M, t, OneRun{}, hd, u, q_tr, h_ref, pv_on, flags, kt, coefvort, ht_out);
+  tri_body<OneRun, LdPlain, Wait>(M, t, OneRun{}, hd, u, q_tr, h_ref, pv_on, flags, kt, coefvort, ht_out);
 }
 
 // h_e (deviation), flux F_e = u_e (h_ref + h_e), q_e: the TRSK average
@@ -40,6 +41,7 @@ __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__re
                                                     const float *__restrict__ qw,
                                                     const float *__restrict__ ht, int pv_on,
                                                     int *flags) {
+  after_prior<true>(hd, u, q_tr, h_ed, uh, q_ed, qg, vhx, ht);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -86,6 +88,7 @@ __global__ void __launch_bounds__(256) k_apvm32(DevMesh M, const float *__restri
                                                 const float *__restrict__ u,
                                                 float *__restrict__ qg,
                                                 float *__restrict__ vhx, int nbt) {
+  after_prior<true>(q_tr, u, qg, vhx);
   const int ne = M.ne;
   float v[3] = {0.0f, 0.0f, 0.0f}, p[3];
   int n, i, stride;
@@ -139,6 +142,7 @@ __global__ void __launch_bounds__(512) k_cell32(DevMesh M, const float *__restri
                                                 float *__restrict__ yout,
                                                 float *__restrict__ tend, int stage, float dt,
                                                 float grav, int perot) {
+  after_prior<true>(hd, u, uh, bern, yn, acc, yout, tend);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nv = M.nv;
   if (i >= nv) return;
@@ -184,6 +188,7 @@ __global__ void __launch_bounds__(512) k_edge32(DevMesh M, const float *__restri
                                                 const float *__restrict__ dif2,
                                                 const int32_t *__restrict__ stq,
                                                 const float *__restrict__ q_tr, int dtred) {
+  after_prior<true>(bern, uh, q_ed, yn, acc, yout, tend, dif1, dif2, q_tr);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -233,6 +238,7 @@ __global__ void __launch_bounds__(256) k_difcv32(DevMesh M, const float *__restr
                                                  const float *__restrict__ kt,
                                                  float *__restrict__ coefdiv,
                                                  float *__restrict__ coefvort, int nbc) {
+  after_prior<true>(x, coefdiv, coefvort);
   if (static_cast<int>(blockIdx.x) < nbc) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int nv = M.nv;
@@ -257,6 +263,7 @@ __global__ void __launch_bounds__(256) k_difcv32(DevMesh M, const float *__restr
 __global__ void __launch_bounds__(256) k_diflap32(DevMesh M, const float *__restrict__ coefdiv,
                                                   const float *__restrict__ coefvort,
                                                   float *__restrict__ lap) {
+  after_prior<true>(coefdiv, coefvort, lap);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -270,7 +277,7 @@ __global__ void __launch_bounds__(256) k_diflap32(DevMesh M, const float *__rest
 // ---- cell-centred TRSK (variant 1), bodies in swm_k32_body.cuh ------------
 // kEdgePV: q_tr is the edges' PV from the edge pre-pass (APVM); kZ false:
 // no PV-flux terms (dtred forms its PV flux at the triangles)
-template <bool kEdgePV, bool kZ = true>
+template <class Wait, bool kEdgePV, bool kZ = true>
 __global__ void __launch_bounds__(512) k_cell32v2(DevMesh M, const float *__restrict__ hd,
                                                   const float *__restrict__ u,
                                                   const float *__restrict__ q_tr,
@@ -285,7 +292,7 @@ __global__ void __launch_bounds__(512) k_cell32v2(DevMesh M, const float *__rest
                                                   float *__restrict__ coefdiv) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M.nv) return;
-  cell_body<OneRun, LdPlain, kEdgePV, kZ>(M, i, OneRun{}, hd, u, q_tr, bern, zflux, yn, acc,
+  cell_body<OneRun, LdPlain, kEdgePV, kZ, Wait>(M, i, OneRun{}, hd, u, q_tr, bern, zflux, yn, acc,
                                           yout, tend, stage, dt, grav, h_ref, kcv, coefdiv);
 }
 
@@ -326,6 +333,7 @@ __global__ void __launch_bounds__(512) k_cell32p(DevMesh M, const float *__restr
     nb[j] = pk.y;
     tr[j] = pk.z;
   }
+  after_prior<true>(hd, u, q_ed, bern, zflux, yn, acc, yout, tend, coefdiv);
   const float hi = hd[i], bt = __ldg(&M.c_bt32[i]), inva = __ldg(&M.c_inva32[i]);
   const float ynv = stage >= 0 ? yn[i] : 0.0f, accv = stage >= 1 ? acc[i] : 0.0f;
   float ue[6], hn[6], qs[6];
@@ -451,6 +459,7 @@ __global__ void __launch_bounds__(512) k_cell32g(DevMesh M, const float *__restr
     R[j] = __int_as_float(pk.w);
     og[j] = __ldg(&M.c_gout[j * nv + i]);
   }
+  after_prior<true>(hd, u, q_ed, bern, zflux, yn, acc, yout, tend, coefdiv);
   const float hi = hd[i], bt = __ldg(&M.c_bt32[i]), inva = __ldg(&M.c_inva32[i]);
   const float ynv = stage >= 0 ? yn[i] : 0.0f, accv = stage >= 1 ? acc[i] : 0.0f;
   float ue[6], hn[6], qs[6], qo[6];
@@ -513,8 +522,9 @@ __global__ void __launch_bounds__(512) k_tri32d(DevMesh M, const float *__restri
   const int ed[3] = {a.x, a.y, a.z}, cv[3] = {a.w, b.x, b.y};
   const float circ[3] = {__int_as_float(b.z), __int_as_float(b.w), c.x};
   const float kite[3] = {c.y, c.z, c.w};
-  tri_core<OneRun, LdPlain>(t, OneRun{}, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u, q_tr,
-                            h_ref, pv_on, flags, kt, coefvort, nullptr);
+  after_prior<true>(hd, u, q_tr, coefvort, wq);
+  tri_core<OneRun, LdPlain, NoWait>(t, OneRun{}, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u,
+                                    q_tr, h_ref, pv_on, flags, kt, coefvort, nullptr);
   const float q = q_tr[t];
   const unsigned opp = __ldg(&M.t_dopp[t]);
   const float hc[3] = {hd[cv[0]], hd[cv[1]], hd[cv[2]]};
@@ -540,6 +550,7 @@ __global__ void __launch_bounds__(512) k_edge32d(DevMesh M, const float *__restr
                                                  float *__restrict__ tend, int stage, float dt,
                                                  int mom_on, const float *__restrict__ dif1,
                                                  const float *__restrict__ dif2) {
+  after_prior<true>(bern, wq, yn, acc, yout, tend, dif1, dif2);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne, nt = M.nt;
   if (e >= ne) return;
@@ -563,6 +574,7 @@ __global__ void __launch_bounds__(512) k_edge32d(DevMesh M, const float *__restr
 }
 
 // ---- variant 2: the triangle kernel on records with 16-bit indices -------
+template <class Wait>
 __global__ void __launch_bounds__(512) k_tri32c(DevMesh M, const float *__restrict__ hd,
                                                 const float *__restrict__ u,
                                                 float *__restrict__ q_tr, float h_ref,
@@ -571,7 +583,7 @@ __global__ void __launch_bounds__(512) k_tri32c(DevMesh M, const float *__restri
                                                 float *__restrict__ coefvort) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= M.nt) return;
-  tri_body16(M, t, hd, u, q_tr, h_ref, pv_on, flags, kt, coefvort);
+  tri_body16<Wait>(M, t, hd, u, q_tr, h_ref, pv_on, flags, kt, coefvort);
 }
 
 // the momentum tendency of edge e (edge_body's arithmetic): -grad B -
@@ -589,6 +601,7 @@ __device__ __forceinline__ float edge_momeq(uint32_t wa, uint32_t wb, float g,
 // two consecutive edges per thread: one 16-byte load of their cell words,
 // 8-byte loads and stores of their per-edge values, and twice the
 // independent gathers in flight
+template <class Wait>
 __global__ void __launch_bounds__(512) k_edge32v2(DevMesh M, const float *__restrict__ bern,
                                                   const float *__restrict__ zflux,
                                                   const float *__restrict__ yn,
@@ -605,6 +618,7 @@ __global__ void __launch_bounds__(512) k_edge32v2(DevMesh M, const float *__rest
   if (e0 + 1 < M.ne) {
     const uint4 w = __ldg(reinterpret_cast<const uint4 *>(M.e_vs2) + p);
     const float2 g = __ldg(reinterpret_cast<const float2 *>(M.e_grad32) + p);
+    IMODEL_WAIT(Wait, bern, zflux, yn, acc, yout, tend, corr, dif1, dif2);
     float m0 = edge_momeq(w.x, w.y, g.x, bern, zflux, erad);
     float m1 = edge_momeq(w.z, w.w, g.y, bern, zflux, erad);
     // learned correction of the PV flux (frozen over the RK step)
@@ -637,6 +651,7 @@ __global__ void __launch_bounds__(512) k_edge32v2(DevMesh M, const float *__rest
       reinterpret_cast<float2 *>(yout)[p] = make_float2(o0, o1);
     }
   } else {
+    IMODEL_WAIT(Wait, bern, zflux, yn, acc, yout, tend, corr, dif1, dif2);
     edge_body(M, e0, OneRun{}, __ldg(&M.e_vs2[e0]), bern, zflux, yn, acc, yout, tend, stage, dt,
               mom_on, erad, corr, dif1, dif2);
   }
@@ -679,6 +694,17 @@ __global__ void __launch_bounds__(256) k_departure(DevMesh M, const float *__res
 
 inline int nblocks(int n, int t) { return (n + t - 1) / t; }
 
+// kp, the instance that waits for its predecessor itself, on small grids; kn
+// without the wait on large ones
+template <class... P, class... A>
+void launch_wait(void (*kp)(P...), void (*kn)(P...), int grid, int block, cudaStream_t s,
+                 A &&...a) {
+  if (pdl_grid(grid))
+    launch_pdl(kp, grid, block, s, a...);
+  else
+    kn<<<grid, block, 0, s>>>(static_cast<P>(a)...);
+}
+
 }  // namespace
 
 void launch_departure(const DevMesh &M, const float *a, const float *b, const float *c,
@@ -699,28 +725,28 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
   // hyperdiffusion) once K div u and K_tr zeta are written
   auto diffusion_tail = [&]() {
     if (!D.on) return;
-    k_diflap32<<<nblocks(M.ne, 256), 256, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap);
+    launch_pdl(k_diflap32, nblocks(M.ne, 256), 256, s, M, D.coefdiv, D.coefvort, D.lap);
     if (D.k4) {
-      k_difcv32<<<nbc + nbt, 256, 0, s>>>(M, D.lap, D.kcv, D.kt, D.coefdiv, D.coefvort, nbc);
-      k_diflap32<<<nblocks(M.ne, 256), 256, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap2);
+      launch_pdl(k_difcv32, nbc + nbt, 256, s, M, D.lap, D.kcv, D.kt, D.coefdiv, D.coefvort, nbc);
+      launch_pdl(k_diflap32, nblocks(M.ne, 256), 256, s, M, D.coefdiv, D.coefvort, D.lap2);
     }
   };
   if (T.variant == 0 && D.on)  // variant 0: K div u and K_tr zeta in their own pass
-    k_difcv32<<<nbc + nbt, 256, 0, s>>>(M, u_in, D.kcv, D.kt, D.coefdiv, D.coefvort, nbc);
+    launch_pdl(k_difcv32, nbc + nbt, 256, s, M, u_in, D.kcv, D.kt, D.coefdiv, D.coefvort, nbc);
   float *cvort = (T.variant >= 1 && D.on) ? D.coefvort : nullptr;
   const bool dtred1 = T.variant >= 1 && W.scheme == IMODEL_SWM_DTRED;
   // gass18 needs the triangle depths of the 32-bit triangle kernel, dtred
   // the Perot vectors of its own
   if (dtred1)
-    k_tri32d<<<nblocks(M.nt, T.bs_tri), T.bs_tri, 0, s>>>(M, h_in, u_in, W.q_tr, W.h_ref,
-                                                           W.pv_on, W.flags, D.kt, cvort, W.vhq);
+    launch_pdl(k_tri32d, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M, h_in, u_in, W.q_tr, W.h_ref,
+               W.pv_on, W.flags, D.kt, cvort, W.vhq);
   else if (T.variant == 2 && W.scheme != IMODEL_SWM_GASS18)
-    k_tri32c<<<nblocks(M.nt, T.bs_tri), T.bs_tri, 0, s>>>(M, h_in, u_in, W.q_tr, W.h_ref,
-                                                           W.pv_on, W.flags, D.kt, cvort);
+    launch_wait(k_tri32c<PriorWait>, k_tri32c<NoWait>, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M,
+               h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort);
   else
-    k_tri32<<<nblocks(M.nt, T.bs_tri), T.bs_tri, 0, s>>>(
-        M, h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort,
-        W.scheme == IMODEL_SWM_GASS18 ? W.h_trs : nullptr);
+    launch_wait(k_tri32<PriorWait>, k_tri32<NoWait>, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M,
+               h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort, W.scheme ==
+               IMODEL_SWM_GASS18 ? W.h_trs : nullptr);
   if (T.variant >= 1) {
     if (ev) cudaEventRecord(ev[1], s);
     // learned correction: formed once per step from the first stage's state
@@ -732,45 +758,48 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
     // the PV of every edge from the edge pre-pass, read by the cells in
     // place of the triangle average
     if (A.on)
-      k_apvm32<<<nbt + nblocks(M.nv, 256), 256, 0, s>>>(M, W.q_tr, u_in, A.qg, A.vhx, nbt);
+      launch_pdl(k_apvm32, nbt + nblocks(M.nv, 256), 256, s, M, W.q_tr, u_in, A.qg, A.vhx, nbt);
     if (A.on || gass)
-      k_edge_pre32<<<nblocks(M.ne, T.bs_pre), T.bs_pre, 0, s>>>(
-          M, h_in, u_in, W.q_tr, W.h_ed, W.uh, W.q_ed, W.h_ref, A.on ? A.qg : nullptr, A.vhx,
-          A.coef, pxt || gass ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
+      launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr,
+                 W.h_ed, W.uh, W.q_ed, W.h_ref, A.on ? A.qg : nullptr, A.vhx, A.coef, pxt || gass
+                 ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
     if (ev) cudaEventRecord(ev[2], s);
     if (gass)
-      k_cell32g<<<nblocks(M.nv, T.bs_cell), T.bs_cell, 0, s>>>(
-          M, h_in, u_in, W.q_ed, W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt,
-          grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
+      launch_pdl(k_cell32g, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern,
+                 W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on
+                 ? D.coefdiv : nullptr);
     else if (pxt && A.on)
-      k_cell32p<true><<<nblocks(M.nv, T.bs_cell), T.bs_cell, 0, s>>>(
-          M, h_in, u_in, W.q_ed, W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt,
-          grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
+      launch_pdl(k_cell32p<true>, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed,
+                 W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref,
+                 D.kcv, D.on ? D.coefdiv : nullptr);
     else if (pxt)
-      k_cell32p<false><<<nblocks(M.nv, T.bs_cell), T.bs_cell, 0, s>>>(
-          M, h_in, u_in, W.q_tr, W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt,
-          grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
+      launch_pdl(k_cell32p<false>, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr,
+                 W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref,
+                 D.kcv, D.on ? D.coefdiv : nullptr);
     else if (dtred1)
-      k_cell32v2<false, false><<<nblocks(M.nv, T.bs_cell), T.bs_cell, 0, s>>>(
-          M, h_in, u_in, W.q_tr, W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt,
-          grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
+      launch_wait(k_cell32v2<PriorWait, false, false>, k_cell32v2<NoWait, false, false>,
+                 nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux,
+                 W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ?
+                 D.coefdiv : nullptr);
     else if (A.on)
-      k_cell32v2<true><<<nblocks(M.nv, T.bs_cell), T.bs_cell, 0, s>>>(
-          M, h_in, u_in, W.q_ed, W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt,
-          grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
+      launch_wait(k_cell32v2<PriorWait, true>, k_cell32v2<NoWait, true>, nblocks(M.nv, T.bs_cell),
+                 T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern, W.zflux, W.yn_h, W.acc_h, h_out,
+                 W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
     else
-      k_cell32v2<false><<<nblocks(M.nv, T.bs_cell), T.bs_cell, 0, s>>>(
-          M, h_in, u_in, W.q_tr, W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt,
-          grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
+      launch_wait(k_cell32v2<PriorWait, false>, k_cell32v2<NoWait, false>, nblocks(M.nv,
+                 T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux, W.yn_h,
+                 W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv :
+                 nullptr);
     diffusion_tail();
     if (ev) cudaEventRecord(ev[3], s);
     if (dtred1)
-      k_edge32d<<<nblocks(M.ne, T.bs_edge), T.bs_edge, 0, s>>>(
-          M, W.bern, W.vhq, W.yn_u, W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2);
+      launch_pdl(k_edge32d, nblocks(M.ne, T.bs_edge), T.bs_edge, s, M, W.bern, W.vhq, W.yn_u,
+                 W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2);
     else
-      k_edge32v2<<<nblocks((M.ne + 1) / 2, T.bs_edge), T.bs_edge, 0, s>>>(
-          M, W.bern, W.zflux, W.yn_u, W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on,
-          static_cast<float>(M.erad), W.learned ? W.learned->corr : nullptr, dif1, dif2);
+      launch_wait(k_edge32v2<PriorWait>, k_edge32v2<NoWait>, nblocks((M.ne + 1) / 2, T.bs_edge),
+                 T.bs_edge, s, M, W.bern, W.zflux, W.yn_u, W.acc_u, u_out, W.tend_u, stage, dt,
+                 W.mom_on, static_cast<float>(M.erad), W.learned ? W.learned->corr : nullptr,
+                 dif1, dif2);
     if (ev) cudaEventRecord(ev[4], s);
     return;
   }
@@ -778,24 +807,23 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
   const Apvm<float> &A = W.apvm;
   if (A.on) {
     const int nbt = nblocks(M.nt, 256);
-    k_apvm32<<<nbt + nblocks(M.nv, 256), 256, 0, s>>>(M, W.q_tr, u_in, A.qg, A.vhx, nbt);
+    launch_pdl(k_apvm32, nbt + nblocks(M.nv, 256), 256, s, M, W.q_tr, u_in, A.qg, A.vhx, nbt);
   }
   // the method wrappers (variant 0 only): pxt16 (distance-weighted q_e,
   // Perot KE, pered), gass18 (rhombus PV, connecting-edge PV), dtred
   const int sch = W.scheme;
   const bool pxt = sch == IMODEL_SWM_PXT16, gass = sch == IMODEL_SWM_GASS18;
-  k_edge_pre32<<<nblocks(M.ne, T.bs_pre), T.bs_pre, 0, s>>>(
-      M, h_in, u_in, W.q_tr, W.h_ed, W.uh, W.q_ed, W.h_ref, A.on ? A.qg : nullptr, A.vhx, A.coef,
-      pxt || gass ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
+  launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr, W.h_ed,
+             W.uh, W.q_ed, W.h_ref, A.on ? A.qg : nullptr, A.vhx, A.coef, pxt || gass ? M.e_qw32 :
+             nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
   if (ev) cudaEventRecord(ev[2], s);
-  k_cell32<<<nblocks(M.nv, T.bs_cell), T.bs_cell, 0, s>>>(M, h_in, u_in, W.uh, W.bern, W.yn_h,
-                                                           W.acc_h, h_out, W.tend_h, stage, dt,
-                                                           grav, pxt ? 1 : 0);
+  launch_pdl(k_cell32, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.uh, W.bern,
+             W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, pxt ? 1 : 0);
   diffusion_tail();
   if (ev) cudaEventRecord(ev[3], s);
-  k_edge32<<<nblocks(M.ne, T.bs_edge), T.bs_edge, 0, s>>>(
-      M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2,
-      gass ? M.e_stq : nullptr, W.q_tr, sch == IMODEL_SWM_DTRED ? 1 : 0);
+  launch_pdl(k_edge32, nblocks(M.ne, T.bs_edge), T.bs_edge, s, M, W.bern, W.uh, W.q_ed, W.yn_u,
+             W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2, gass ? M.e_stq : nullptr,
+             W.q_tr, sch == IMODEL_SWM_DTRED ? 1 : 0);
   if (ev) cudaEventRecord(ev[4], s);
 }
 

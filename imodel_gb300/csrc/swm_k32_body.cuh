@@ -30,6 +30,20 @@ struct LdL2 {
   static __device__ __forceinline__ float ld(const float *p) { return __ldcg(p); }
 };
 
+// Called between the loads of the fixed records and the first load of a
+// changing field: nothing in the persistent kernel, the wait for the kernel
+// before in the single-run kernels (after_prior).
+struct NoWait {
+  static constexpr bool kWaits = false;
+};
+struct PriorWait {
+  static constexpr bool kWaits = true;
+};
+// (discarded without a wait: taking the pointers by reference alone made the
+// cell kernel 2 % slower at level 9)
+#define IMODEL_WAIT(Wait, ...) \
+  if constexpr (Wait::kWaits) after_prior<true>(__VA_ARGS__)
+
 // ode_rk4 stage update (swm.f90:2647-2678) in FP32
 __device__ __forceinline__ float rk_stage32(int stage, float k, float yn, float *acc, float dt) {
   if (stage == 0) {
@@ -48,7 +62,7 @@ __device__ __forceinline__ float rk_stage32(int stage, float k, float yn, float 
 // q_t = (curl u / A + f) / h_t  (vort_tr + scalar_hx2tr + scalar_elem_divide)
 // from a triangle's decoded record: edges, cells, circulation and kite
 // coefficients, Coriolis parameter; the sums run in slot order 0, 1, 2
-template <class Ix, class Ld>
+template <class Ix, class Ld, class Wait>
 __device__ __forceinline__ void tri_core(int t, Ix ix, const int (&ed)[3], const int (&cv)[3],
                                          const float (&circ)[3], const float (&kite)[3],
                                          float f, const float *__restrict__ hd,
@@ -57,6 +71,7 @@ __device__ __forceinline__ void tri_core(int t, Ix ix, const int (&ed)[3], const
                                          const float *__restrict__ kt = nullptr,
                                          float *__restrict__ coefvort = nullptr,
                                          float *__restrict__ ht_out = nullptr) {
+  IMODEL_WAIT(Wait, hd, u, q_tr, coefvort, ht_out);
   float eta = f;
   float ht = 0.0f, z = 0.0f;
 #pragma unroll
@@ -82,7 +97,7 @@ __device__ __forceinline__ void tri_core(int t, Ix ix, const int (&ed)[3], const
   q_tr[ix(t)] = q;
 }
 
-template <class Ix, class Ld = LdPlain>
+template <class Ix, class Ld = LdPlain, class Wait = NoWait>
 __device__ __forceinline__ void tri_body(const DevMesh &M, int t, Ix ix,
                                          const float *__restrict__ hd,
                                          const float *__restrict__ u, float *__restrict__ q_tr,
@@ -97,7 +112,7 @@ __device__ __forceinline__ void tri_body(const DevMesh &M, int t, Ix ix,
   const int ed[3] = {a.x, a.y, a.z}, cv[3] = {a.w, b.x, b.y};
   const float circ[3] = {__int_as_float(b.z), __int_as_float(b.w), c.x};
   const float kite[3] = {c.y, c.z, c.w};
-  tri_core<Ix, Ld>(t, ix, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u, q_tr, h_ref, pv_on,
+  tri_core<Ix, Ld, Wait>(t, ix, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u, q_tr, h_ref, pv_on,
                    flags, kt, coefvort, ht_out);
 }
 
@@ -106,6 +121,7 @@ __device__ __forceinline__ void tri_body(const DevMesh &M, int t, Ix ix,
 // span more than 65,536 takes its indices from the 32-bit records instead
 // (warp-uniform branch).  The records and the bases are loaded together, so
 // that the gathers wait for one round trip, as with the 32-bit records.
+template <class Wait>
 __device__ __forceinline__ void tri_body16(const DevMesh &M, int t, const float *__restrict__ hd,
                                            const float *__restrict__ u,
                                            float *__restrict__ q_tr, float h_ref, int pv_on,
@@ -134,7 +150,7 @@ __device__ __forceinline__ void tri_body16(const DevMesh &M, int t, const float 
   }
   const float circ[3] = {__uint_as_float(a.w), b.x, b.y};
   const float kite[3] = {b.z, b.w, c.x};
-  tri_core<OneRun, LdPlain>(t, OneRun{}, ed, cv, circ, kite, c.y, hd, u, q_tr, h_ref, pv_on,
+  tri_core<OneRun, LdPlain, Wait>(t, OneRun{}, ed, cv, circ, kite, c.y, hd, u, q_tr, h_ref, pv_on,
                             flags, kt, coefvort);
 }
 
@@ -270,7 +286,8 @@ __device__ __forceinline__ void cell_own(const DevMesh &M, int i, Ix ix,
   accv = stage >= 1 ? Ld::ld(acc + ix(i)) : 0.0f;
 }
 
-template <class Ix, class Ld = LdPlain, bool kEdgePV = false, bool kZ = true>
+template <class Ix, class Ld = LdPlain, bool kEdgePV = false, bool kZ = true,
+          class Wait = NoWait>
 __device__ __forceinline__ void cell_body(const DevMesh &M, int i, Ix ix,
                                           const float *__restrict__ hd,
                                           const float *__restrict__ u,
@@ -297,6 +314,7 @@ __device__ __forceinline__ void cell_body(const DevMesh &M, int i, Ix ix,
     tr[j] = pk.z;
     R[j] = __int_as_float(pk.w);
   }
+  IMODEL_WAIT(Wait, hd, u, q_tr, bern, zflux, yn, acc, yout, tend, coefdiv);
   float hi, bt, inva, ynv, accv;
   cell_own<Ix, Ld>(M, i, ix, hd, yn, acc, stage, hi, bt, inva, ynv, accv);
   cell_core<Ix, Ld, kEdgePV, kZ>(i, ix, meta, ed, nb, tr, R, kd, hi, bt, inva, ynv, accv, hd, u,

@@ -5,6 +5,8 @@
 // below is rounded on its own, as in the Fortran built without contraction,
 // so that the FP64 step reproduces the reference arithmetic of
 // src/swm.f90:2416-2683 and src/swm_operators.f90 bit for bit.
+#include <cmath>
+
 #include "imodel_swm.h"
 #include "swm_common.cuh"
 #include "swm_div.cuh"
@@ -47,7 +49,7 @@ __device__ __forceinline__ double rk_stage(int stage, double k, double yn, doubl
 
 // Edge e's fluxes: uh2 = 2 u h_e (scalar_hx2ed :89-97, scalar_elem_product
 // :1546), fe = {2 u h_e d, (l d / 4) u^2}
-__device__ __forceinline__ void edge_flux64(const DevMesh &M, int e, const double *__restrict__ h,
+__device__ __forceinline__ void edge_flux64(const DevMesh64 &M, int e, const double *__restrict__ h,
                                             const double *__restrict__ u,
                                             double *__restrict__ uh2,
                                             double2 *__restrict__ fe) {
@@ -64,7 +66,7 @@ __device__ __forceinline__ void edge_flux64(const DevMesh &M, int e, const doubl
 // of the circumcentre (bary, pxt16) or scalar_edtr2trcc of h_ed (:286-343,
 // gass18, which also keeps eta and h_tr for the rhombus PV).  The blocks
 // after: the edges' fluxes, which the next launch reads beside q.
-__global__ void __launch_bounds__(256) k_tri64(DevMesh M, const double *__restrict__ h,
+__global__ void __launch_bounds__(256) k_tri64(DevMesh64 M, const double *__restrict__ h,
                                                const double *__restrict__ u,
                                                double *__restrict__ q_tr, int pv_on,
                                                int *flags, const double *__restrict__ kt,
@@ -73,6 +75,7 @@ __global__ void __launch_bounds__(256) k_tri64(DevMesh M, const double *__restri
                                                double *__restrict__ h_trs,
                                                double *__restrict__ uh2,
                                                double2 *__restrict__ fe, int nbt) {
+  after_prior<false>(h, u, q_tr, coefvort, eta_t, h_trs, uh2, fe);
   if (static_cast<int>(blockIdx.x) >= nbt) {
     const int e = (blockIdx.x - nbt) * blockDim.x + threadIdx.x;
     if (e < M.ne) edge_flux64(M, e, h, u, uh2, fe);
@@ -137,9 +140,15 @@ __device__ __forceinline__ double sign_of(double s, double x) {
                           __double2loint(x));
 }
 
+// x with its sign changed where bit 31 of es is set
+__device__ __forceinline__ double flip(uint32_t es, double x) {
+  return __hiloint2double(__double2hiint(x) ^ (es & 0x80000000u), __double2loint(x));
+}
+
 // grad_tr2ed(q_tr) (:1427-1463), the PV gradient across each edge
-__global__ void __launch_bounds__(256) k_qgrad64(DevMesh M, const double *__restrict__ q_tr,
+__global__ void __launch_bounds__(256) k_qgrad64(DevMesh64 M, const double *__restrict__ q_tr,
                                                  double *__restrict__ qge) {
+  after_prior<false>(q_tr, qge);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -152,10 +161,11 @@ __global__ void __launch_bounds__(256) k_qgrad64(DevMesh M, const double *__rest
 // dsign(1, tr%nr) = -tr%tg (smeshpack.f90:853-859), the sign of t_lt.
 // The blocks after: the velocity at the cells, vector_edhx2hx_perot
 // (:454-509, HTC, hx%areag); ttgout is the sign of c_sd.
-__global__ void __launch_bounds__(256) k_apvm64(DevMesh M, const double *__restrict__ qge,
+__global__ void __launch_bounds__(256) k_apvm64(DevMesh64 M, const double *__restrict__ qge,
                                                 const double *__restrict__ u,
                                                 double *__restrict__ qg,
                                                 double *__restrict__ vhx, int nbt) {
+  after_prior<false>(qge, u, qg, vhx);
   const int ne = M.ne;
   if (static_cast<int>(blockIdx.x) < nbt) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -210,7 +220,7 @@ __global__ void __launch_bounds__(256) k_apvm64(DevMesh M, const double *__restr
 // circumcentre-distance weights for bary) or, for gass18, scalar_elem_divide
 // of the rhombus averages of eta and h_tr (swm.f90:2475-2480); with qg !=
 // NULL the apvm correction of q_ed (:1495-1502), coef = pvspar dt
-__device__ __forceinline__ double edge_pv2(const DevMesh &M, int e,
+__device__ __forceinline__ double edge_pv2(const DevMesh64 &M, int e,
                                            const double *__restrict__ q_tr,
                                            const double *__restrict__ qg,
                                            const double *__restrict__ vhx, double coef,
@@ -256,7 +266,7 @@ __device__ __forceinline__ double edge_pv2(const DevMesh &M, int e,
 // mass-equation RK stage.  The blocks after: q2, twice the edges' PV.  The
 // two do not read each other; sharing a launch fills the chip on small grids.
 __global__ void __launch_bounds__(256)
-    k_cell64(DevMesh M, const double *__restrict__ h, const double *__restrict__ u,
+    k_cell64(DevMesh64 M, const double *__restrict__ h, const double *__restrict__ u,
              const double2 *__restrict__ fe, double *__restrict__ bern,
              const double *__restrict__ yn, double *__restrict__ acc, double *__restrict__ yout,
              double *__restrict__ tend, int stage, double dt, const double *__restrict__ kcv,
@@ -266,6 +276,7 @@ __global__ void __launch_bounds__(256)
              const double *__restrict__ eta_t, const double *__restrict__ h_trs, int pv_on,
              int *flags) {
   if (static_cast<int>(blockIdx.x) >= nbc) {
+    after_prior<false>(q2, q_tr, qg, vhx, eta_t, h_trs);
     const int e = (blockIdx.x - nbc) * blockDim.x + threadIdx.x;
     if (e < M.ne) q2[e] = edge_pv2(M, e, q_tr, qg, vhx, coef, scheme, eta_t, h_trs, pv_on, flags);
     return;
@@ -275,16 +286,23 @@ __global__ void __launch_bounds__(256)
   if (i >= nv) return;
   const int n = M.c_nnb[i];
   const double A = M.c_areag[i], rA = M.c_rareag[i];
-  // c_eds: the slot's edge with ttgout < 0 in bit 31; d is twice the sum
+  // c_eds: the slot's edge with ttgout < 0 in bit 31 (unused slots: edge 0);
+  // all slots are read before the sums, so that the loads wait once and not
+  // slot by slot (a guarded loop took 7.6 us at level 5).  d is twice the sum
+  uint32_t es[6];
+  double2 f[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) es[j] = M.c_eds[j * nv + i];
+  after_prior<false>(h, u, fe, bern, yn, acc, yout, tend, coefdiv);
+#pragma unroll
+  for (int j = 0; j < 6; ++j) f[j] = fe[es[j] & 0x7FFFFFFFu];
   double d = 0.0, k = 0.0;
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    if (j >= n) break;
-    const uint32_t es = M.c_eds[j * nv + i];
-    const double2 f = fe[es & 0x7FFFFFFFu];
-    d = d + __hiloint2double(__double2hiint(f.x) ^ (es & 0x80000000u), __double2loint(f.x));
-    k = k + f.y;
-  }
+  for (int j = 0; j < 6; ++j)
+    if (j < n) {
+      d = d + flip(es[j], f[j].x);
+      k = k + f[j].y;
+    }
   // with diffusion on: div_hx(u) (:613-661), diffusion_ed's K div u
   if (coefdiv) {
     double du = 0.0;
@@ -296,18 +314,20 @@ __global__ void __launch_bounds__(256)
   if (scheme == IMODEL_SWM_PXT16) {
     // kinetic_energy_hx, perhx branch (:1172-1173): half the squared
     // vector_edhx2hx_perot (:454-509, HTC) of u; c_off = ed%c%p - v%p
-    double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-    for (int j = 0; j < n; ++j) {
-      const uint32_t es = M.c_eds[j * nv + i];
-      const int ed = static_cast<int>(es & 0x7FFFFFFFu);
-      const double ue = u[ed];
-      const double su = __hiloint2double(__double2hiint(ue) ^ (es & 0x80000000u),
-                                         __double2loint(ue));
-      const double dl = M.e_dleng[ed];
-      v0 = v0 + su * M.c_off[(3 * j) * nv + i] * dl;
-      v1 = v1 + su * M.c_off[(3 * j + 1) * nv + i] * dl;
-      v2 = v2 + su * M.c_off[(3 * j + 2) * nv + i] * dl;
+    double v0 = 0.0, v1 = 0.0, v2 = 0.0, su[6], dl[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      const int ed = static_cast<int>(es[j] & 0x7FFFFFFFu);
+      su[j] = flip(es[j], u[ed]);
+      dl[j] = M.e_dleng[ed];
     }
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+      if (j < n) {
+        v0 = v0 + su[j] * M.c_off[(3 * j) * nv + i] * dl[j];
+        v1 = v1 + su[j] * M.c_off[(3 * j + 1) * nv + i] * dl[j];
+        v2 = v2 + su[j] * M.c_off[(3 * j + 2) * nv + i] * dl[j];
+      }
     v0 = div_by(v0, A, rA);
     v1 = div_by(v1, A, rA);
     v2 = div_by(v2, A, rA);
@@ -345,7 +365,7 @@ __device__ __forceinline__ void edge_update64(int e, double g, double q,
 }
 
 // grad_ed (:511-548) + coriolis_ed TRSK (:1283-1308) and the momentum RK stage
-__global__ void __launch_bounds__(256) k_edge64(DevMesh M, const double *__restrict__ bern,
+__global__ void __launch_bounds__(256) k_edge64(DevMesh64 M, const double *__restrict__ bern,
                                                 const double *__restrict__ uh2,
                                                 const double *__restrict__ q2,
                                                 const double *__restrict__ yn,
@@ -360,27 +380,32 @@ __global__ void __launch_bounds__(256) k_edge64(DevMesh M, const double *__restr
   const int ne = M.ne;
   if (e >= ne) return;
   const double l = M.e_leng[e], rl = M.e_rleng[e];
-  double g = bern[M.e_v[ne + e]] - bern[M.e_v[e]];
+  const int v1 = M.e_v[e], v2 = M.e_v[ne + e];
+  const int ns = M.e_nst[e];
+  // slots past ns hold edge 0 and weight 0 and are left out of the sum; all
+  // are read at once, the fixed ones before the wait for the cells' kernel
+  int k[kMaxStencil];
+  double w[kMaxStencil], d8[kMaxStencil];
+#pragma unroll
+  for (int s = 0; s < kMaxStencil; ++s) {
+    k[s] = M.e_stk[s * ne + e];
+    w[s] = M.e_stw[s * ne + e];
+  }
+#pragma unroll
+  for (int s = 0; s < kMaxStencil; ++s) d8[s] = M.e_d8[k[s]];
+  after_prior<false>(bern, uh2, q2, yn, acc, yout, tend, dif1, dif2);
+  double g = bern[v2] - bern[v1];
   g = div_by(div_by(g, l, rl), M.erad, M.rerad);
   const double qe = q2[e];
-  const int ns = M.e_nst[e];
   double q = 0.0;
   // per slot: F_k (q_e + q_k) / 2 d_k w, in that order; 2 F, 2 q and d / 8
-  auto slot = [&](int s) {
-    const int k = M.e_stk[s * ne + e];
+#pragma unroll
+  for (int s = 0; s < kMaxStencil; ++s) {
     // gass18 (:1378-1410): the PV of the edge connecting e and k when there
     // is one (stq != NULL), else the TRSK average
     const int c3 = stq ? stq[s * ne + e] : -1;
-    const double qs = c3 >= 0 ? q2[c3] + q2[c3] : qe + q2[k];
-    q = q + uh2[k] * qs * M.e_d8[k] * M.e_stw[s * ne + e];
-  };
-  if (ns == 10) {
-    // hexagons on both sides (all but 60 edges): unrolled, so that the
-    // gathers of all slots are in flight together
-#pragma unroll
-    for (int s = 0; s < 10; ++s) slot(s);
-  } else {
-    for (int s = 0; s < ns; ++s) slot(s);
+    const double qs = c3 >= 0 ? q2[c3] + q2[c3] : qe + q2[k[s]];
+    if (s < ns) q = q + uh2[k[s]] * qs * d8[s] * w[s];
   }
   q = div_by(q, l, rl);
   edge_update64(e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
@@ -389,9 +414,10 @@ __global__ void __launch_bounds__(256) k_edge64(DevMesh M, const double *__restr
 // dtred: vector_edhx2tr_perot (:345-406, HTC) of uh at the triangle
 // circumcentres, cross(tr%c, v) / tr%areag, times q_tr (vector_elem_product,
 // :1617-1649); signcor = dsign(1, tr%tg) is the sign of t_lt
-__global__ void __launch_bounds__(256) k_vhq64(DevMesh M, const double *__restrict__ uh2,
+__global__ void __launch_bounds__(256) k_vhq64(DevMesh64 M, const double *__restrict__ uh2,
                                                const double *__restrict__ q_tr,
                                                double *__restrict__ vhq) {
+  after_prior<false>(uh2, q_tr, vhq);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = M.nt, ne = M.ne;
   if (t >= nt) return;
@@ -415,7 +441,7 @@ __global__ void __launch_bounds__(256) k_vhq64(DevMesh M, const double *__restri
 
 // grad_ed (:511-548) + coriolis_ed's dtred (:1310-1329) or pered
 // (:1330-1377) branch, HTC, and the momentum RK stage
-__global__ void __launch_bounds__(256) k_edge64r(DevMesh M, const double *__restrict__ bern,
+__global__ void __launch_bounds__(256) k_edge64r(DevMesh64 M, const double *__restrict__ bern,
                                                  const double *__restrict__ uh2,
                                                  const double *__restrict__ q2,
                                                  const double *__restrict__ vhq,
@@ -429,6 +455,7 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh M, const double *__rest
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne, nv = M.nv, nt = M.nt;
   if (e >= ne) return;
+  after_prior<false>(bern, uh2, q2, vhq, yn, acc, yout, tend, dif1, dif2);
   double g = bern[M.e_v[ne + e]] - bern[M.e_v[e]];
   g = div_by(div_by(g, M.e_leng[e], M.e_rleng[e]), M.erad, M.rerad);
   double v0, v1, v2;
@@ -453,19 +480,21 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh M, const double *__rest
       const int c = M.e_v[i * ne + e];
       double a0 = 0.0, a1 = 0.0, a2 = 0.0;
       const int n = M.c_nnb[c];
+      double f[6], d[6];
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
-        if (j >= n) break;
         const uint32_t es = M.c_eds[j * nv + c];
         const int l2 = static_cast<int>(es & 0x7FFFFFFFu);
-        const double x = uh2[l2];
-        const double f = __hiloint2double(__double2hiint(x) ^ (es & 0x80000000u),
-                                          __double2loint(x)) * (qe + q2[l2]);
-        const double d = M.e_d8[l2];
-        a0 = a0 + f * M.c_off[(3 * j) * nv + c] * d;
-        a1 = a1 + f * M.c_off[(3 * j + 1) * nv + c] * d;
-        a2 = a2 + f * M.c_off[(3 * j + 2) * nv + c] * d;
+        f[j] = flip(es, uh2[l2]) * (qe + q2[l2]);
+        d[j] = M.e_d8[l2];
       }
+#pragma unroll
+      for (int j = 0; j < 6; ++j)
+        if (j < n) {
+          a0 = a0 + f[j] * M.c_off[(3 * j) * nv + c] * d[j];
+          a1 = a1 + f[j] * M.c_off[(3 * j + 1) * nv + c] * d[j];
+          a2 = a2 + f[j] * M.c_off[(3 * j + 2) * nv + c] * d[j];
+        }
       const double A = M.c_areag[c], rA = M.c_rareag[c];
       a0 = div_by(a0, A, rA);
       a1 = div_by(a1, A, rA);
@@ -489,11 +518,12 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh M, const double *__rest
 // div_hx(x) at the cells (blocks [0, nbc)), coefvort = K_tr rel_vort_tr(x)
 // at the triangles (the blocks after), HTC branches of div_hx (:613-661) and
 // rel_vort_tr (:780-827)
-__global__ void __launch_bounds__(256) k_difcv64(DevMesh M, const double *__restrict__ x,
+__global__ void __launch_bounds__(256) k_difcv64(DevMesh64 M, const double *__restrict__ x,
                                                  const double *__restrict__ kcv,
                                                  const double *__restrict__ kt,
                                                  double *__restrict__ coefdiv,
                                                  double *__restrict__ coefvort, int nbc) {
+  after_prior<false>(x, coefdiv, coefvort);
   if (static_cast<int>(blockIdx.x) < nbc) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int nv = M.nv;
@@ -517,9 +547,10 @@ __global__ void __launch_bounds__(256) k_difcv64(DevMesh M, const double *__rest
 
 // second half: lap = grad_ed(coefdiv) - grad_ed_tg(coefvort) (grad_ed
 // :511-548, grad_ed_tg :738-777, HTC)
-__global__ void __launch_bounds__(256) k_diflap64(DevMesh M, const double *__restrict__ coefdiv,
+__global__ void __launch_bounds__(256) k_diflap64(DevMesh64 M, const double *__restrict__ coefdiv,
                                                   const double *__restrict__ coefvort,
                                                   double *__restrict__ lap) {
+  after_prior<false>(coefdiv, coefvort, lap);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -554,6 +585,67 @@ __global__ void k_dif_coefs(DevMesh M, const double *__restrict__ kf, double k, 
     if (take_sqrt) f = sqrt(f);
     kt64[t] = f;
     if (kt32) kt32[t] = static_cast<float>(f);
+  }
+}
+
+// RN(1 / b) for div_by, NaN where its three operations could leave the
+// normal range
+__device__ __forceinline__ double recip(double b) {
+  const double a = fabs(b);
+  return a >= 0x1p-500 && a <= 0x1p500 ? 1.0 / b : __longlong_as_double(0x7FF8000000000000LL);
+}
+__device__ __forceinline__ double norm3(const double *p, int n, int i) {
+  const double p0 = p[i], p1 = p[n + i], p2 = p[2 * n + i];
+  return sqrt(p0 * p0 + p1 * p1 + p2 * p2);
+}
+
+// the derived constants of DevMesh (entity i of each kind)
+__global__ void __launch_bounds__(256) k_consts64(DevMesh64 M) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nv = M.nv, ne = M.ne, nt = M.nt;
+  auto w = [](const double *p, int k, double v) { const_cast<double *>(p)[k] = v; };
+  if (i < nv) {
+    w(M.c_rareag, i, recip(M.c_areag[i]));
+    w(M.c_rcellarea, i, recip(M.c_cellarea[i]));
+    for (int j = 0; j < 6; ++j) {
+      const int k = j * nv + i;
+      const bool live = j < M.c_nnb[i];
+      const int e = live ? M.c_ed[k] : 0;
+      // c_sd = ttgout d
+      const bool neg = live && (M.c_sd[k] < 0.0) != (M.e_dleng[e] < 0.0);
+      const_cast<uint32_t *>(M.c_eds)[k] = static_cast<uint32_t>(e) | (neg ? 0x80000000u : 0u);
+      if (M.c_off)
+        for (int c = 0; c < 3; ++c)
+          w(M.c_off, (3 * j + c) * nv + i, live ? M.e_c[c * ne + e] - M.c_p[c * nv + i] : 0.0);
+    }
+    if (M.c_nrm) {
+      w(M.c_nrm, i, norm3(M.c_p, nv, i));
+      w(M.c_rnrm, i, recip(M.c_nrm[i]));
+    }
+  }
+  if (i < nt) {
+    w(M.t_rareag, i, recip(M.t_areag[i]));
+    if (M.t_nrm) {
+      w(M.t_nrm, i, norm3(M.t_c, nt, i));
+      w(M.t_rnrm, i, recip(M.t_nrm[i]));
+    }
+  }
+  if (i < ne) {
+    const double d = M.e_dleng[i], dr = d * M.erad;
+    w(M.e_rleng, i, recip(M.e_leng[i]));
+    w(M.e_rdleng, i, recip(d));
+    w(M.e_d8, i, d * 0.125);
+    w(M.e_dlerad, i, dr);
+    w(M.e_rdlerad, i, recip(dr));
+    if (M.e_nrm) {
+      w(M.e_nrm, i, norm3(M.e_c, ne, i));
+      w(M.e_rnrm, i, recip(M.e_nrm[i]));
+    }
+    if (M.e_dsum) {
+      const double ds = M.e_dist[i] + M.e_dist[ne + i];
+      w(M.e_dsum, i, ds);
+      w(M.e_rdsum, i, recip(ds));
+    }
   }
 }
 
@@ -930,7 +1022,7 @@ inline int block64(int) { return BLOCK64; }
 
 }  // namespace
 
-void launch_stage64(const DevMesh &M, const Work<double> &W, const double *h_in,
+void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_in,
                     const double *u_in, double *h_out, double *u_out, int stage, double dt,
                     cudaStream_t s, cudaEvent_t *ev) {
   if (ev) cudaEventRecord(ev[0], s);
@@ -941,43 +1033,81 @@ void launch_stage64(const DevMesh &M, const Work<double> &W, const double *h_in,
   const int sch = W.scheme;
   const int bt = block64(M.nt), bc = block64(M.nv), be = block64(M.ne);
   const int nbt = nblocks(M.nt, bt);
-  k_tri64<<<nbt + nblocks(M.ne, bt), bt, 0, s>>>(M, h_in, u_in, W.q_tr, W.pv_on, W.flags, D.kt,
-                                                  D.on ? D.coefvort : nullptr, sch, W.eta_t,
-                                                  W.h_trs, W.uh, W.fe, nbt);
+  launch_pdl(k_tri64, nbt + nblocks(M.ne, bt), bt, s, M, h_in, u_in, W.q_tr, W.pv_on, W.flags,
+             D.kt, D.on ? D.coefvort : nullptr, sch, W.eta_t, W.h_trs, W.uh, W.fe, nbt);
   if (ev) cudaEventRecord(ev[1], s);
   const Apvm<double> &A = W.apvm;
   if (A.on) {
-    k_qgrad64<<<nblocks(M.ne, be), be, 0, s>>>(M, W.q_tr, A.qge);
-    k_apvm64<<<nbt + nblocks(M.nv, bt), bt, 0, s>>>(M, A.qge, u_in, A.qg, A.vhx, nbt);
+    launch_pdl(k_qgrad64, nblocks(M.ne, be), be, s, M, W.q_tr, A.qge);
+    launch_pdl(k_apvm64, nbt + nblocks(M.nv, bt), bt, s, M, A.qge, u_in, A.qg, A.vhx, nbt);
   }
   if (sch == IMODEL_SWM_DTRED)
-    k_vhq64<<<nblocks(M.nt, bt), bt, 0, s>>>(M, W.uh, W.q_tr, W.vhq);
+    launch_pdl(k_vhq64, nblocks(M.nt, bt), bt, s, M, W.uh, W.q_tr, W.vhq);
   if (ev) cudaEventRecord(ev[2], s);
   const int nbc = nblocks(M.nv, bc);
-  k_cell64<<<nbc + nblocks(M.ne, bc), bc, 0, s>>>(
-      M, h_in, u_in, W.fe, W.bern, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, D.kcv,
-      D.on ? D.coefdiv : nullptr, nbc, W.q_ed, W.q_tr, A.on ? A.qg : nullptr, A.vhx, A.coef, sch,
-      W.eta_t, W.h_trs, W.pv_on, W.flags);
+  launch_pdl(k_cell64, nbc + nblocks(M.ne, bc), bc, s, M, h_in, u_in, W.fe, W.bern, W.yn_h,
+             W.acc_h, h_out, W.tend_h, stage, dt, D.kcv, D.on ? D.coefdiv : nullptr, nbc, W.q_ed,
+             W.q_tr, A.on ? A.qg : nullptr, A.vhx, A.coef, sch, W.eta_t, W.h_trs, W.pv_on,
+             W.flags);
   if (D.on) {
-    k_diflap64<<<nblocks(M.ne, be), be, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap);
+    launch_pdl(k_diflap64, nblocks(M.ne, be), be, s, M, D.coefdiv, D.coefvort, D.lap);
     if (D.k4) {
-      k_difcv64<<<nbc + nblocks(M.nt, bc), bc, 0, s>>>(M, D.lap, D.kcv, D.kt, D.coefdiv,
-                                                        D.coefvort, nbc);
-      k_diflap64<<<nblocks(M.ne, be), be, 0, s>>>(M, D.coefdiv, D.coefvort, D.lap2);
+      launch_pdl(k_difcv64, nbc + nblocks(M.nt, bc), bc, s, M, D.lap, D.kcv, D.kt, D.coefdiv,
+                 D.coefvort, nbc);
+      launch_pdl(k_diflap64, nblocks(M.ne, be), be, s, M, D.coefdiv, D.coefvort, D.lap2);
     }
   }
   if (ev) cudaEventRecord(ev[3], s);
   if (sch == IMODEL_SWM_PXT16 || sch == IMODEL_SWM_DTRED)
-    k_edge64r<<<nblocks(M.ne, be), be, 0, s>>>(M, W.bern, W.uh, W.q_ed, W.vhq, W.yn_u, W.acc_u,
-                                                u_out, W.tend_u, stage, dt, W.mom_on,
-                                                D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 : nullptr,
-                                                sch);
+    launch_pdl(k_edge64r, nblocks(M.ne, be), be, s, M, W.bern, W.uh, W.q_ed, W.vhq, W.yn_u,
+               W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, D.k2 ? D.lap : nullptr, D.k4 ?
+               D.lap2 : nullptr, sch);
   else
-    k_edge64<<<nblocks(M.ne, be), be, 0, s>>>(M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u, u_out,
-                                               W.tend_u, stage, dt, W.mom_on,
-                                               D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 : nullptr,
-                                               sch == IMODEL_SWM_GASS18 ? M.e_stq : nullptr);
+    launch_pdl(k_edge64, nblocks(M.ne, be), be, s, M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u,
+               u_out, W.tend_u, stage, dt, W.mom_on, D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 :
+               nullptr, sch == IMODEL_SWM_GASS18 ? M.e_stq : nullptr);
   if (ev) cudaEventRecord(ev[4], s);
+}
+
+size_t consts64_size(const DevMesh64 &M) {
+  const size_t nv = M.nv, ne = M.ne, nt = M.nt;
+  return nv * 5 + ne * 5 + nt + (M.t_c ? 2 * (nv + ne + nt) : 0) + (M.e_dist ? 2 * ne : 0) +
+         (M.t_bary ? 18 * nv : 0);
+}
+
+void launch_consts64(DevMesh64 &M, double *p, cudaStream_t s) {
+  const size_t nv = M.nv, ne = M.ne, nt = M.nt;
+  auto take = [&p](size_t n) {
+    double *q = p;
+    p += n;
+    return q;
+  };
+  M.rerad = M.erad >= 0x1p-500 && M.erad <= 0x1p500 ? 1.0 / M.erad : std::nan("");
+  M.c_rareag = take(nv);
+  M.c_rcellarea = take(nv);
+  M.c_eds = reinterpret_cast<const uint32_t *>(take(3 * nv));
+  M.e_rleng = take(ne);
+  M.e_rdleng = take(ne);
+  M.e_d8 = take(ne);
+  M.e_dlerad = take(ne);
+  M.e_rdlerad = take(ne);
+  M.t_rareag = take(nt);
+  if (M.t_c) {
+    M.c_nrm = take(nv);
+    M.c_rnrm = take(nv);
+    M.e_nrm = take(ne);
+    M.e_rnrm = take(ne);
+    M.t_nrm = take(nt);
+    M.t_rnrm = take(nt);
+  }
+  if (M.e_dist) {
+    M.e_dsum = take(ne);
+    M.e_rdsum = take(ne);
+  }
+  if (M.t_bary) M.c_off = take(18 * nv);
+  int n = M.nv > M.ne ? M.nv : M.ne;
+  if (M.nt > n) n = M.nt;
+  k_consts64<<<nblocks(n, 256), 256, 0, s>>>(M);
 }
 
 void launch_dif_coefs(const DevMesh &M, const double *kf, double k, bool take_sqrt, double *kc64,

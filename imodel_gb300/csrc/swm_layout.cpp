@@ -5,7 +5,6 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
-#include <limits>
 #include <numeric>
 #ifdef _OPENMP
 #include <omp.h>
@@ -966,82 +965,6 @@ uint16_t bf16_bits(float v) {
   if ((b & 0x7F800000u) == 0x7F800000u && (b & 0x007FFFFFu)) return static_cast<uint16_t>(b >> 16);
   const uint64_t r = (static_cast<uint64_t>(b) + 0x7FFFu + ((b >> 16) & 1u)) >> 16;
   return static_cast<uint16_t>(r & 0xFFFFu);
-}
-
-namespace {
-// RN(1 / b) for div_by (swm_div.cuh), NaN where its three operations could
-// leave the normal range
-double recip(double b) {
-  const double a = std::fabs(b);
-  if (!(a >= 0x1p-500 && a <= 0x1p500)) return std::numeric_limits<double>::quiet_NaN();
-  return 1.0 / b;
-}
-// |p| of n points [3][n], summed as proj_vec_sphere does
-void norms(const HVec<double> &p, HVec<double> &nrm, HVec<double> &rnrm) {
-  const size_t n = p.size() / 3;
-  nrm.resize(n);
-  rnrm.resize(n);
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < static_cast<int64_t>(n); ++i) {
-    nrm[i] = std::sqrt(p[i] * p[i] + p[n + i] * p[n + i] + p[2 * n + i] * p[2 * n + i]);
-    rnrm[i] = recip(nrm[i]);
-  }
-}
-}  // namespace
-
-void build_layout64(const Layout &L, int scheme, Layout64 &D) {
-  const size_t NV = L.nv, NE = L.ne, NT = L.nt;
-  D.rerad = recip(L.erad);
-  D.c_rareag.resize(NV);
-  D.c_rcellarea.resize(NV);
-  D.c_eds.resize(kMaxNb * NV);
-  D.t_rareag.resize(NT);
-  for (HVec<double> *v : {&D.e_rleng, &D.e_rdleng, &D.e_d8, &D.e_dlerad, &D.e_rdlerad})
-    v->resize(NE);
-#pragma omp parallel for schedule(static)
-  for (int i = 0; i < L.nv; ++i) {
-    D.c_rareag[i] = recip(L.c_areag[i]);
-    D.c_rcellarea[i] = recip(L.c_cellarea[i]);
-    for (int j = 0; j < kMaxNb; ++j) {
-      const int e = L.c_ed[j * NV + i];
-      // c_sd = ttgout d
-      const bool neg = j < L.c_nnb[i] && (L.c_sd[j * NV + i] < 0.0) != (L.e_dleng[e] < 0.0);
-      D.c_eds[j * NV + i] =
-          j < L.c_nnb[i] ? static_cast<uint32_t>(e) | (neg ? 0x80000000u : 0u) : 0u;
-    }
-  }
-#pragma omp parallel for schedule(static)
-  for (int e = 0; e < L.ne; ++e) {
-    D.e_rleng[e] = recip(L.e_leng[e]);
-    D.e_rdleng[e] = recip(L.e_dleng[e]);
-    D.e_d8[e] = L.e_dleng[e] * 0.125;
-    D.e_dlerad[e] = L.e_dleng[e] * L.erad;
-    D.e_rdlerad[e] = recip(D.e_dlerad[e]);
-  }
-#pragma omp parallel for schedule(static)
-  for (int t = 0; t < L.nt; ++t) D.t_rareag[t] = recip(L.t_areag[t]);
-  if (!L.t_c.empty()) {
-    norms(L.c_p, D.c_nrm, D.c_rnrm);
-    norms(L.t_c, D.t_nrm, D.t_rnrm);
-    norms(L.e_c, D.e_nrm, D.e_rnrm);
-  }
-  if (!L.e_dist.empty()) {
-    D.e_dsum.resize(NE);
-    D.e_rdsum.resize(NE);
-#pragma omp parallel for schedule(static)
-    for (int e = 0; e < L.ne; ++e) {
-      D.e_dsum[e] = L.e_dist[e] + L.e_dist[NE + e];
-      D.e_rdsum[e] = recip(D.e_dsum[e]);
-    }
-  }
-  if (scheme == IMODEL_SWM_PXT16) {
-    fill(D.c_off, 3 * kMaxNb * NV, 0.0);
-#pragma omp parallel for schedule(static)
-    for (int i = 0; i < L.nv; ++i)
-      for (int j = 0; j < L.c_nnb[i]; ++j)
-        for (int k = 0; k < 3; ++k)
-          D.c_off[(3 * j + k) * NV + i] = L.e_c[k * NE + L.c_ed[j * NV + i]] - L.c_p[k * NV + i];
-  }
 }
 
 // Same inputs as imodel_gb300/learned.py (stencil, geometry_features): for

@@ -203,25 +203,6 @@ struct Layout {
 std::string build_layout(const imodel_swm_mesh &m, const double *bt, Layout &L,
                          int scheme = IMODEL_SWM_TRSK10, int fsphere = 0, double fcte = 0.0);
 
-// Constants of the FP64 kernels (device order) beside the layout's: the
-// reciprocals, rounded to nearest, of what those kernels divide by (NaN where
-// the divisor is zero, not finite or outside 2^-500 .. 2^500: the kernel then
-// divides), and factors that it would otherwise form at every call.
-struct Layout64 {
-  HVec<double> c_rareag, c_rcellarea;  // [nv]
-  HVec<uint32_t> c_eds;                // [6][nv] edge of slot j, bit 31: ttgout < 0
-  HVec<double> e_rleng, e_rdleng, e_d8;  // [ne] 1 / l, 1 / d, d / 8
-  HVec<double> e_dlerad, e_rdlerad;    // [ne] d erad and its reciprocal
-  HVec<double> t_rareag;               // [nt]
-  // |p| of the points of the tangent-plane projections and its reciprocal
-  // (empty without ed%nr)
-  HVec<double> c_nrm, c_rnrm, t_nrm, t_rnrm, e_nrm, e_rnrm;
-  HVec<double> e_dsum, e_rdsum;        // [ne] pxt16, dtred: d1 + d2
-  HVec<double> c_off;                  // [18][nv] pxt16: (ed%c%p - v%p)_k of slot j at 3 j + k
-  double rerad = 0;
-};
-void build_layout64(const Layout &L, int scheme, Layout64 &D);
-
 // Inputs of the learned TRSK correction (imodel_gb300/learned.py), device
 // order: per edge the 10 stencil edges as sign * (index + 1) (0 = padding),
 // slot-major [10][ne], and the 14 geometry inputs as BF16 bit patterns,

@@ -39,7 +39,7 @@ __device__ __forceinline__ double fminq(double a, double b) { return (b < a) ? b
 
 // what the sources read that stays fixed in a run: g theta_e grad(b) of
 // moist_swm.f90:1299-1315 at the edges, q0 exp(20 theta) of qsat at the cells
-__global__ void __launch_bounds__(256) k_moist_consts(DevMesh M, const double *__restrict__ th,
+__global__ void __launch_bounds__(256) k_moist_consts(DevMesh64 M, const double *__restrict__ th,
                                                       double *__restrict__ ex20, double q0,
                                                       double *__restrict__ gthb) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(256) k_moist_consts(DevMesh M, const double *_
 // momentum source (source, moist_swm.f90:1299-1315) added to the momentum
 // tendency and u's RK stage.  FP64-pipe bound like the FP64 step: divisions by
 // div_by, factors of two left out until the sums, run constants formed once.
-__global__ void __launch_bounds__(256) k_moist_edge(DevMesh M, MoistArgs A) {
+__global__ void __launch_bounds__(256) k_moist_edge(DevMesh64 M, MoistArgs A) {
+  after_prior<false>();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -92,7 +93,8 @@ __global__ void __launch_bounds__(256) k_moist_edge(DevMesh M, MoistArgs A) {
 // div_hx_upw1 with the upwind fluxes formed here), the
 // condensation, evaporation and precipitation sources (source, :1317-1351)
 // and the RK stages of h and the tracers.
-__global__ void __launch_bounds__(256) k_moist_cell(DevMesh M, MoistArgs A) {
+__global__ void __launch_bounds__(256) k_moist_cell(DevMesh64 M, MoistArgs A) {
+  after_prior<false>();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nv = M.nv, ne = M.ne;
   if (i >= nv) return;
@@ -115,10 +117,10 @@ __global__ void __launch_bounds__(256) k_moist_cell(DevMesh M, MoistArgs A) {
   }
   const int n = M.c_nnb[i];
   const double A_i = M.c_areag[i], rA = M.c_rareag[i];
-  // the slots' edges with ttgout < 0 in bit 31
+  // the slots' edges with ttgout < 0 in bit 31 (unused slots: edge 0)
   uint32_t es[6];
 #pragma unroll
-  for (int j = 0; j < 6; ++j) es[j] = j < n ? M.c_eds[j * nv + i] : 0u;
+  for (int j = 0; j < 6; ++j) es[j] = M.c_eds[j * nv + i];
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
     if (!((A.active >> k) & 1)) continue;
@@ -138,12 +140,14 @@ __global__ void __launch_bounds__(256) k_moist_cell(DevMesh M, MoistArgs A) {
       }
     } else {
       const double *uphi = A.uphi + static_cast<size_t>(k) * ne;
+      double f[6];
 #pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        if (j >= n) break;
-        const double f = uphi[es[j] & 0x7FFFFFFFu];
-        d = d + __hiloint2double(__double2hiint(f) ^ (es[j] & 0x80000000u), __double2loint(f));
-      }
+      for (int j = 0; j < 6; ++j) f[j] = uphi[es[j] & 0x7FFFFFFFu];
+#pragma unroll
+      for (int j = 0; j < 6; ++j)
+        if (j < n)
+          d = d + __hiloint2double(__double2hiint(f[j]) ^ (es[j] & 0x80000000u),
+                                   __double2loint(f[j]));
       d = d * 0.5;
     }
     double t = -div_by(div_by(d, A_i, rA), M.erad, M.rerad);
@@ -159,6 +163,7 @@ __global__ void k_moist_q(int nv, const double *__restrict__ h, const double *__
                           const double *__restrict__ hqc, const double *__restrict__ hqr,
                           double *__restrict__ qv, double *__restrict__ qc,
                           double *__restrict__ qr, int *flags) {
+  after_prior<false>(h, hqv, hqc, hqr, qv, qc, qr);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
   const double hi = h[i];
@@ -203,6 +208,7 @@ __device__ __forceinline__ float rk_stage32m(int stage, float k, float yn, float
 
 // the thermal momentum source and u's RK stage (shallow-water cases only)
 __global__ void __launch_bounds__(256) k_moist_edge32(DevMesh M, MoistArgs32 A) {
+  after_prior<true>();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -227,6 +233,7 @@ __global__ void __launch_bounds__(256) k_moist_edge32(DevMesh M, MoistArgs32 A) 
 }
 
 __global__ void __launch_bounds__(256) k_moist_cell32(DevMesh M, MoistArgs32 A) {
+  after_prior<true>();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nv = M.nv;
   if (i >= nv) return;
@@ -283,6 +290,7 @@ __global__ void k_moist_q32(int nv, const float *__restrict__ hd, float h_ref,
                             const float *__restrict__ hqv, const float *__restrict__ hqc,
                             const float *__restrict__ hqr, float *__restrict__ qv,
                             float *__restrict__ qc, float *__restrict__ qr, int *flags) {
+  after_prior<true>(hd, hqv, hqc, hqr, qv, qc, qr);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
   const float hi = h_ref + hd[i];
@@ -300,17 +308,18 @@ inline int nblocks(int n, int t) { return (n + t - 1) / t; }
 }  // namespace
 
 void launch_moist_stage32(const DevMesh &M, const MoistArgs32 &A, cudaStream_t s) {
-  if (A.swm) k_moist_edge32<<<nblocks(M.ne, 256), 256, 0, s>>>(M, A);
-  k_moist_cell32<<<nblocks(M.nv, 256), 256, 0, s>>>(M, A);
+  if (A.swm) launch_pdl(k_moist_edge32, nblocks(M.ne, 256), 256, s, M, A);
+  launch_pdl(k_moist_cell32, nblocks(M.nv, 256), 256, s, M, A);
 }
 
 void launch_moist_q32(int nv, const float *hd, float h_ref, const float *hqv, const float *hqc,
                       const float *hqr, float *qv, float *qc, float *qr, int *flags,
                       cudaStream_t s) {
-  k_moist_q32<<<nblocks(nv, 256), 256, 0, s>>>(nv, hd, h_ref, hqv, hqc, hqr, qv, qc, qr, flags);
+  launch_pdl(k_moist_q32, nblocks(nv, 256), 256, s, nv, hd, h_ref, hqv, hqc, hqr, qv, qc, qr,
+             flags);
 }
 
-void launch_moist_consts(const DevMesh &M, const double *th, double *ex20, double q0,
+void launch_moist_consts(const DevMesh64 &M, const double *th, double *ex20, double q0,
                          double *gthb, cudaStream_t s) {
   // every cell has at least three edges on these grids, two cells an edge, so
   // ne >= nv; the larger count covers both either way
@@ -318,16 +327,16 @@ void launch_moist_consts(const DevMesh &M, const double *th, double *ex20, doubl
   k_moist_consts<<<nblocks(n, 256), 256, 0, s>>>(M, th, ex20, q0, gthb);
 }
 
-void launch_moist_stage(const DevMesh &M, const MoistArgs &A, cudaStream_t s) {
+void launch_moist_stage(const DevMesh64 &M, const MoistArgs &A, cudaStream_t s) {
   const int b = BLOCK64;
-  k_moist_edge<<<nblocks(M.ne, b), b, 0, s>>>(M, A);
-  k_moist_cell<<<nblocks(M.nv, b), b, 0, s>>>(M, A);
+  launch_pdl(k_moist_edge, nblocks(M.ne, b), b, s, M, A);
+  launch_pdl(k_moist_cell, nblocks(M.nv, b), b, s, M, A);
 }
 
 void launch_moist_q(int nv, const double *h, const double *hqv, const double *hqc,
                     const double *hqr, double *qv, double *qc, double *qr, int *flags,
                     cudaStream_t s) {
-  k_moist_q<<<nblocks(nv, 256), 256, 0, s>>>(nv, h, hqv, hqc, hqr, qv, qc, qr, flags);
+  launch_pdl(k_moist_q, nblocks(nv, 256), 256, s, nv, h, hqv, hqc, hqr, qv, qc, qr, flags);
 }
 
 }  // namespace imodel
