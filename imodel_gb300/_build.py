@@ -99,6 +99,7 @@ def build_swm_lib(force: bool = False) -> str:
         # FP64 reference-order kernels: no multiply-add contraction
         "swm_k64.cu": ["--fmad=false"],
         "swm_k32.cu": [],
+        "swm_stage32.cu": [],
         "swm_capi.cu": [],
         "swm_ens.cu": [],
         "mlp.cu": [],
@@ -115,11 +116,12 @@ def build_swm_lib(force: bool = False) -> str:
         objs.append(obj)
         if force or _stale(obj, [src] + headers):
             jobs.append([nvcc] + NVCC_COMMON + extra + ["-c", src, "-o", obj])
-    src = os.path.join(CSRC, "swm_layout.cpp")
-    obj = os.path.join(OBJ_DIR, "swm_layout.o")
-    objs.append(obj)
-    if force or _stale(obj, [src] + headers):
-        jobs.append(["g++"] + CXX_COMMON + ["-fopenmp", "-I" + CSRC, "-c", src, "-o", obj])
+    for name in ("swm_layout", "swm_tiles"):
+        src = os.path.join(CSRC, name + ".cpp")
+        obj = os.path.join(OBJ_DIR, name + ".o")
+        objs.append(obj)
+        if force or _stale(obj, [src] + headers):
+            jobs.append(["g++"] + CXX_COMMON + ["-fopenmp", "-I" + CSRC, "-c", src, "-o", obj])
     if jobs:
         _run_parallel(jobs)
     if force or _stale(out, objs):

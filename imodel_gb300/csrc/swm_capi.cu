@@ -27,6 +27,7 @@ struct Handle {
   // gass18 on a grid whose connecting edges do not follow the cells'
   // structure (Layout::gass_cells false): the stencil variant only
   bool v0_only = false;
+  int ntiles = 0;  // tiles of the fused FP32 stage
   std::string err;
   int device = 0;
   int precision = IMODEL_SWM_FP64;
@@ -157,6 +158,29 @@ int dalloc(Handle *H, T **p, size_t n) {
   return IMODEL_SWM_OK;
 }
 
+// the tiles of the fused FP32 stage (none when the layout does not fit)
+int upload_tiles(Handle *H, const Layout &L) {
+  TileLayout T;
+  if (!build_tiles(L, tile_cap(L.nv), T)) return IMODEL_SWM_OK;
+  TileDev D;
+  D.cap = T.cap;
+  D.ntiles = T.ntiles;
+  D.max_h = T.max_h;
+  D.max_u = T.max_u;
+  D.max_t = T.max_t;
+  D.max_bytes = T.max_bytes;
+  if (!fused_prepare(D)) return IMODEL_SWM_OK;
+  const TileHead *head = nullptr;
+  const uint32_t *data = nullptr;
+  int rc;
+  if ((rc = upload(H, T.head, &head)) || (rc = upload(H, T.data, &data))) return rc;
+  D.head = reinterpret_cast<const int4 *>(head);
+  D.data = reinterpret_cast<const uint4 *>(data);
+  H->W32.tiles = D;
+  H->ntiles = D.ntiles;
+  return IMODEL_SWM_OK;
+}
+
 template <class T>
 int alloc_work(Handle *H, Work<T> &W) {
   int rc;
@@ -262,6 +286,9 @@ void learned_switch(Handle *H, bool on) {
     H->M.e_stc32 = w.e_stc32;
     H->M.c_R32 = w.c_R32;
     H->M.c_pk = w.c_pk;
+    // the tiles hold the learned fractions: the plain scheme takes variant
+    // 1's three kernels
+    H->W32.tiles.ntiles = on ? H->ntiles : 0;
   }
   if (H->graph) {
     cudaGraphExecDestroy(H->graph);
@@ -385,6 +412,9 @@ int flags_status(Handle *H, int f) {
   if (f & (8 | 16))
     return set_error(H, IMODEL_SWM_ECUDA,
                      "the learned-correction kernel's pipeline gave up on a bounded wait");
+  // bit 32: the same in the fused stage (swm_stage32.cu)
+  if (f & 32)
+    return set_error(H, IMODEL_SWM_ECUDA, "the fused stage gave up on a bounded wait");
   return IMODEL_SWM_OK;
 }
 
@@ -473,6 +503,7 @@ int error_proxy(Handle *H, int steps, bool *trip) {
     Mp.e_stc32 = H->w_plain.e_stc32;
     Mp.c_R32 = H->w_plain.c_R32;
     Mp.c_pk = H->w_plain.c_pk;
+    Wp.tiles.ntiles = 0;
   } else {
     Wp.learned = nullptr;
   }
@@ -827,6 +858,9 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
     launch_consts64(M, p, nullptr);  // the stream of the uploads and the zero-fill
     CK(cudaGetLastError());
   }
+  if (H->precision == IMODEL_SWM_FP32 && scheme == IMODEL_SWM_TRSK10 &&
+      (rc = upload_tiles(H, L)))
+    return rc;
   H->d_cell_n2o = const_cast<int32_t *>(cn2o);
   H->d_edge_n2o = const_cast<int32_t *>(en2o);
   const int32_t *co2n = nullptr, *eo2n = nullptr;
@@ -1495,9 +1529,9 @@ int imodel_swm_launch_count(void *handle, int32_t nsteps, int64_t *count) {
   const bool on = fp32 ? H->W32.dif.on : H->W64.dif.on;
   const bool k4 = fp32 ? H->W32.dif.k4 : H->W64.dif.k4;
   *count = static_cast<int64_t>(nsteps) * 4 *
-           imodel::launches_per_stage(fp32, fp32 ? H->W32.tune.variant : 0, on, k4,
+           (fp32 && imodel::fused_stage(H->W32) ? 1 : imodel::launches_per_stage(fp32, fp32 ? H->W32.tune.variant : 0, on, k4,
                                       fp32 ? H->W32.apvm.on : H->W64.apvm.on,
-                                      fp32 ? H->W32.scheme : H->W64.scheme);
+                                      fp32 ? H->W32.scheme : H->W64.scheme));
   // the learned correction adds one network launch per step while it is on
   if (fp32 && H->W32.learned) *count += nsteps;
   return IMODEL_SWM_OK;
@@ -1510,6 +1544,7 @@ const char *imodel_swm_main_kernel(void *handle) {
     return H->W64.scheme == IMODEL_SWM_PXT16 || H->W64.scheme == IMODEL_SWM_DTRED ? "k_edge64r"
                                                                                   : "k_edge64";
   const int v = H->W32.tune.variant;
+  if (imodel::fused_stage(H->W32)) return "k_stage32";
   if (v >= 1 && H->W32.scheme == IMODEL_SWM_PXT16) return "k_cell32p";
   if (v >= 1 && H->W32.scheme == IMODEL_SWM_GASS18) return "k_cell32g";
   if (v >= 1 && H->W32.scheme == IMODEL_SWM_DTRED) return "k_cell32v2";

@@ -95,7 +95,8 @@ struct DevMesh64 : DevMesh {
 // Launch configuration of the FP32 stage kernels, chosen by the autotuner.
 //   variant 0: triangle -> edge pre-pass -> cell -> edge (10-entry stencil)
 //   variant 1: triangle -> cell (cell-centred TRSK, writes the PV flux
-//              contribution of each cell edge) -> edge (sums two cells)
+//              contribution of each cell edge) -> edge (sums two cells); one
+//              kernel over tiles where fused_stage() holds (the same bits)
 //   variant 2: variant 1 reading the triangle records with 16-bit indices
 //              (40 instead of 52 bytes per triangle)
 struct Tune {
@@ -105,6 +106,14 @@ struct Tune {
 };
 
 struct LearnedDev;
+
+// Device copy of a handle's tiles (swm_layout.h); ntiles 0: none
+struct TileDev {
+  int ntiles = 0, cap = 0;
+  int max_h = 0, max_u = 0, max_t = 0, max_bytes = 0;
+  const int4 *head = nullptr;  // [ntiles][5]
+  const uint4 *data = nullptr;
+};
 
 // Programmatic dependent launch: a kernel of a step may start while its
 // predecessor still runs, load what is fixed (indices, geometry) and then
@@ -137,10 +146,12 @@ inline bool pdl_grid(int grid) { return static_cast<unsigned>(grid) < kPdlGrid; 
 // launches k, which calls after_prior, so that it may start before the kernel
 // before it in the stream has finished (on grids below kPdlGrid)
 template <class... P, class... A>
-inline void launch_pdl(void (*k)(P...), int grid, int block, cudaStream_t s, A &&...a) {
+inline void launch_pdl_smem(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                            A &&...a) {
   cudaLaunchConfig_t c{};
   c.gridDim = dim3(grid);
   c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
   c.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -148,6 +159,10 @@ inline void launch_pdl(void (*k)(P...), int grid, int block, cudaStream_t s, A &
   c.attrs = &at;
   c.numAttrs = pdl_grid(grid) ? 1 : 0;
   cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
+}
+template <class... P, class... A>
+inline void launch_pdl(void (*k)(P...), int grid, int block, cudaStream_t s, A &&...a) {
+  launch_pdl_smem(k, grid, block, 0, s, a...);
 }
 
 // Laplacian diffusion and hyperdiffusion of the momentum (diffusion_ed,
@@ -193,6 +208,7 @@ struct Work {
   Diffusion<T> dif;
   Apvm<T> apvm;
   Tune tune;
+  TileDev tiles;     // FP32 trsk10: the fused stage's tiles
   int *flags;        // bit 0: PV division by ~0
   // method wrapper (IMODEL_SWM_TRSK10 ... IMODEL_SWM_DTRED; FP64 handles)
   int scheme = 0;
@@ -223,6 +239,19 @@ void launch_departure(const DevMesh &M, const float *a, const float *b, const fl
 void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
                     const float *u_in, float *h_out, float *u_out, int stage, float dt,
                     cudaStream_t s, cudaEvent_t *ev = nullptr);
+// The fused stage (swm_stage32.cu) runs in place of variant 1's three kernels
+// where nothing needs their intermediate fields
+inline bool fused_stage(const Work<float> &W) {
+  return W.tiles.ntiles > 0 && W.tune.variant == 1 && W.scheme == 0 && !W.apvm.on && !W.dif.on &&
+         !W.learned;
+}
+int tile_cap(int nv);  // cells with flux terms per tile (threads per block) on a grid of nv cells
+// whether the fused stage's block fits an SM with these tiles; prepares the
+// kernel for its shared memory
+bool fused_prepare(const TileDev &T);
+void launch_stage32_fused(const DevMesh &M, const Work<float> &W, const float *h_in,
+                          const float *u_in, float *h_out, float *u_out, int stage, float dt,
+                          cudaStream_t s);
 // The learned TRSK correction inside the FP32 step (mlp.cu): once per step,
 // after the first stage's PV, corr[e] = q_e h_e sigma_e y_e is formed from the
 // network output; the edge kernel adds it to the momentum tendency of every

@@ -593,9 +593,7 @@ __device__ __forceinline__ float edge_momeq(uint32_t wa, uint32_t wb, float g,
                                            const float *__restrict__ zflux, float erad) {
   const int c1 = static_cast<int>(wa & 0x0FFFFFFFu), c2 = static_cast<int>(wb & 0x0FFFFFFFu);
   const int s1 = static_cast<int>(wa >> 28), s2 = static_cast<int>(wb >> 28);
-  const float grad = (bern[c2] - bern[c1]) * g;
-  const float q = (zflux[6 * c1 + s1] + zflux[6 * c2 + s2]) * (g * erad);
-  return -grad - q;
+  return edge_terms(bern[c1], bern[c2], zflux[6 * c1 + s1], zflux[6 * c2 + s2], g, erad);
 }
 
 // two consecutive edges per thread: one 16-byte load of their cell words,
@@ -718,6 +716,14 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
   const Tune &T = W.tune;
   const float grav = static_cast<float>(M.grav);
   if (ev) cudaEventRecord(ev[0], s);
+  if (fused_stage(W)) {
+    if (ev) cudaEventRecord(ev[1], s);
+    if (ev) cudaEventRecord(ev[2], s);
+    launch_stage32_fused(M, W, h_in, u_in, h_out, u_out, stage, dt, s);
+    if (ev) cudaEventRecord(ev[3], s);
+    if (ev) cudaEventRecord(ev[4], s);
+    return;
+  }
   const Diffusion<float> &D = W.dif;
   const float *dif1 = D.k2 ? D.lap : nullptr, *dif2 = D.k4 ? D.lap2 : nullptr;
   const int nbc = nblocks(M.nv, 256), nbt = nblocks(M.nt, 256);

@@ -44,19 +44,23 @@ struct PriorWait {
 #define IMODEL_WAIT(Wait, ...) \
   if constexpr (Wait::kWaits) after_prior<true>(__VA_ARGS__)
 
+// Which products are fused into a sum is written out in the functions below,
+// not left to the compiler: the separate kernels, the fused stage and the
+// ensemble kernel give the same bits.
+
 // ode_rk4 stage update (swm.f90:2647-2678) in FP32
 __device__ __forceinline__ float rk_stage32(int stage, float k, float yn, float *acc, float dt) {
   if (stage == 0) {
     *acc = k;
-    return yn + 0.5f * dt * k;
+    return fmaf(0.5f * dt, k, yn);
   } else if (stage == 1) {
-    *acc = *acc + 2.0f * k;
-    return yn + 0.5f * dt * k;
+    *acc = fmaf(2.0f, k, *acc);
+    return fmaf(0.5f * dt, k, yn);
   } else if (stage == 2) {
-    *acc = *acc + 2.0f * k;
-    return yn + dt * k;
+    *acc = fmaf(2.0f, k, *acc);
+    return fmaf(dt, k, yn);
   }
-  return yn + dt * (*acc + k) * (1.0f / 6.0f);
+  return fmaf(__fmul_rn(dt, __fadd_rn(*acc, k)), 1.0f / 6.0f, yn);
 }
 
 // q_t = (curl u / A + f) / h_t  (vort_tr + scalar_hx2tr + scalar_elem_divide)
@@ -77,9 +81,9 @@ __device__ __forceinline__ void tri_core(int t, Ix ix, const int (&ed)[3], const
 #pragma unroll
   for (int s = 0; s < 3; ++s) {
     const float us = Ld::ld(u + ix(ed[s]));
-    eta += circ[s] * us;
-    z += circ[s] * us;
-    ht += kite[s] * Ld::ld(hd + ix(cv[s]));
+    eta = fmaf(circ[s], us, eta);
+    z = fmaf(circ[s], us, z);
+    ht = fmaf(kite[s], Ld::ld(hd + ix(cv[s])), ht);
   }
   // with diffusion on: K_tr times the relative vorticity
   if (coefvort) coefvort[ix(t)] = kt[t] * z;
@@ -163,39 +167,50 @@ __device__ __forceinline__ void tri_body16(const DevMesh &M, int t, const float 
 // kite fractions R_c; the edge kernel adds the two cells' Z and divides by
 // l_e.  The 10-entry stencil (40 B of indices and 40 B of weights per edge)
 // becomes n fractions per cell.
+//
+// The fractions sum to one, so w_c(j, i) = -w_c(i, j): a pair of edges
+// shares its weight and q_i + q_j between both its terms (five operations a
+// pair, where summing each edge's row took ten), and the pair's work cancels
+// exactly in the weight.  S(j) = R(0) + ... + R(j - 1), w = (S(j) - 1/2) - S(i).
 template <int N>
 __device__ __forceinline__ void trsk_cell(const float (&G)[6], const float (&qs)[6],
                                           const float (&R)[6], unsigned tneg, float (&Z)[6]) {
+  float S[N], a[N];
+  S[0] = 0.0f;
+#pragma unroll
+  for (int j = 1; j < N; ++j) S[j] = S[j - 1] + R[j - 1];
+#pragma unroll
+  for (int i = 0; i < N; ++i) a[i] = 0.0f;
+#pragma unroll
+  for (int j = 1; j < N; ++j) {
+    const float Sh = S[j] - 0.5f;
+#pragma unroll
+    for (int i = 0; i < j; ++i) {
+      const float t = __fmul_rn(Sh - S[i], __fadd_rn(qs[i], qs[j]));
+      a[i] = fmaf(t, G[j], a[i]);
+      a[j] = fmaf(-t, G[i], a[j]);
+    }
+  }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    float c = 0.0f, acc = 0.0f;
-#pragma unroll
-    for (int s = 1; s < N; ++s) {
-      const int j = (i + s) % N;
-      c += R[(i + s - 1) % N];
-      acc += (c - 0.5f) * G[j] * (qs[i] + qs[j]);
-    }
-    const float z = 0.5f * acc;
+    const float z = 0.5f * a[i];
     Z[i] = ((tneg >> i) & 1u) ? -z : z;
   }
 }
 
 // the arithmetic of one cell from its gathered values: div F, K, the
-// Bernoulli potential, the PV-flux contributions Z (cell-major zflux) and
-// the mass RK stage.  kEdgePV: qt holds the PV of the cell's edges (formed
-// by the edge pre-pass, APVM's upwinding included) instead of the PV of its
-// triangles.
+// Bernoulli potential, the PV-flux contributions Z (cell-major zflux);
+// returns the sum of the fluxes out of the cell.  kEdgePV: qt holds the PV of
+// the cell's edges (formed by the edge pre-pass, APVM's upwinding included)
+// instead of the PV of its triangles.
 template <class Ix = OneRun, bool kEdgePV = false, bool kZ = true>
-__device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)[6],
-                                          const float2 (&kd)[6], const float (&ue)[6],
-                                          const float (&hn)[6], const float (&qt)[6], float hi,
-                                          float bt, float inva, float ynv, float accv,
-                                          float *__restrict__ bern, float *__restrict__ zflux,
-                                          float *__restrict__ acc, float *__restrict__ yout,
-                                          float *__restrict__ tend, int stage, float dt,
-                                          float grav, float h_ref, Ix ix = Ix{},
-                                          const float *__restrict__ kcv = nullptr,
-                                          float *__restrict__ coefdiv = nullptr) {
+__device__ __forceinline__ float cell_terms(int i, uint32_t meta, const float (&R)[6],
+                                            const float2 (&kd)[6], const float (&ue)[6],
+                                            const float (&hn)[6], const float (&qt)[6], float hi,
+                                            float bt, float inva, float *__restrict__ bern,
+                                            float *__restrict__ zflux, float grav, float h_ref,
+                                            Ix ix = Ix{}, const float *__restrict__ kcv = nullptr,
+                                            float *__restrict__ coefdiv = nullptr) {
   const int n = static_cast<int>(meta & 7u);
   const unsigned tneg = meta >> 8;
   float G[6], qs[6];
@@ -204,17 +219,17 @@ __device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
     // F_e = u_e h_e, h_e the two-cell average (scalar_hx2ed)
-    const float F = ue[j] * (h_ref + 0.5f * (hi + hn[j]));
-    G[j] = F * kd[j].y;
+    const float F = __fmul_rn(ue[j], fmaf(0.5f, hi + hn[j], h_ref));
+    G[j] = __fmul_rn(F, kd[j].y);
     // q_e: edge j lies between triangles j-1 and j (scalar_tr2ed)
     qs[j] = kEdgePV ? qt[j] : 0.5f * ((j == 0 ? qlast : qt[j - 1]) + qt[j]);
-    div += G[j];
-    ke += kd[j].x * (ue[j] * ue[j]);
-    du += ue[j] * kd[j].y;
+    div = __fadd_rn(div, G[j]);
+    ke = fmaf(kd[j].x, __fmul_rn(ue[j], ue[j]), ke);
+    du = fmaf(ue[j], kd[j].y, du);
   }
   // with diffusion on: K times the divergence of u
   if (coefdiv) coefdiv[ix(i)] = kcv[ix(i)] * (du * inva);
-  bern[ix(i)] = grav * (hi + bt) + ke;
+  bern[ix(i)] = fmaf(grav, hi + bt, ke);
   // kZ false (dtred): the edges form their PV flux from the triangles
   if (kZ) {
     float Z[6];
@@ -230,7 +245,24 @@ __device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)
     for (int j = 0; j < 6; ++j)
       if (j < n) zflux[ix(6 * i + j)] = Z[j];
   }
-  const float masseq = -div * inva;
+  return div;
+}
+
+// cell_terms and the mass RK stage
+template <class Ix = OneRun, bool kEdgePV = false, bool kZ = true>
+__device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)[6],
+                                          const float2 (&kd)[6], const float (&ue)[6],
+                                          const float (&hn)[6], const float (&qt)[6], float hi,
+                                          float bt, float inva, float ynv, float accv,
+                                          float *__restrict__ bern, float *__restrict__ zflux,
+                                          float *__restrict__ acc, float *__restrict__ yout,
+                                          float *__restrict__ tend, int stage, float dt,
+                                          float grav, float h_ref, Ix ix = Ix{},
+                                          const float *__restrict__ kcv = nullptr,
+                                          float *__restrict__ coefdiv = nullptr) {
+  const float div = cell_terms<Ix, kEdgePV, kZ>(i, meta, R, kd, ue, hn, qt, hi, bt, inva, bern,
+                                                zflux, grav, h_ref, ix, kcv, coefdiv);
+  const float masseq = __fmul_rn(-div, inva);
   if (stage < 0) {
     tend[ix(i)] = masseq;
   } else {
@@ -322,6 +354,13 @@ __device__ __forceinline__ void cell_body(const DevMesh &M, int i, Ix ix,
                                  coefdiv);
 }
 
+// -grad B - (Z_c1 + Z_c2) / l_e of an edge
+__device__ __forceinline__ float edge_terms(float b1, float b2, float z1, float z2, float g,
+                                            float erad) {
+  const float grad = __fmul_rn(b2 - b1, g);
+  return -fmaf(z1 + z2, __fmul_rn(g, erad), grad);
+}
+
 // -grad B - (Z_c1 + Z_c2) / l_e and the momentum RK stage of edge e
 template <class Ix, class Ld = LdPlain>
 __device__ __forceinline__ void edge_body(const DevMesh &M, int e, Ix ix, uint2 w,
@@ -336,9 +375,9 @@ __device__ __forceinline__ void edge_body(const DevMesh &M, int e, Ix ix, uint2 
   const int c1 = static_cast<int>(w.x & 0x0FFFFFFFu), c2 = static_cast<int>(w.y & 0x0FFFFFFFu);
   const int s1 = static_cast<int>(w.x >> 28), s2 = static_cast<int>(w.y >> 28);
   const float g = __ldg(&M.e_grad32[e]);  // 1 / (l_e a)
-  const float grad = (Ld::ld(bern + ix(c2)) - Ld::ld(bern + ix(c1))) * g;
-  const float q = (Ld::ld(zflux + ix(6 * c1 + s1)) + Ld::ld(zflux + ix(6 * c2 + s2))) * (g * erad);
-  float momeq = -grad - q;
+  float momeq = edge_terms(Ld::ld(bern + ix(c1)), Ld::ld(bern + ix(c2)),
+                           Ld::ld(zflux + ix(6 * c1 + s1)), Ld::ld(zflux + ix(6 * c2 + s2)), g,
+                           erad);
   // learned correction of the PV flux (frozen over the RK step)
   if (corr) momeq += corr[ix(e)];
   // diffusion, then hyperdiffusion

