@@ -1,15 +1,22 @@
 // Batched ensembles: several grids, each with several members, advanced by
 // one persistent cooperative launch (FP32, cell-centred TRSK).
 //
-// Members of a grid share its geometry; their state is interleaved with the
-// member index fastest (entity i, member m at i*M + m), so the threads of a
-// warp that share an entity read its geometry once and the members' values
-// from contiguous memory.  The kernel loops over "macro steps": the grid with
-// the most steps steps every time, the others are spread evenly over the same
-// macro steps.  Each RK stage is three phases (triangles, cells, edges) over
-// the work of every grid that steps, separated by grid-wide barriers; each
-// barrier's wait is bounded and reports a timeout through the error flag
-// instead of waiting forever.
+// The kernel loops over "macro steps": the grid with the most steps steps
+// every time, the others are spread evenly over the same macro steps.  An RK
+// stage is one pass over work items, a tile of a grid (swm_layout.h) for a
+// group of its members: the block fetches the tile's records into shared
+// memory once and steps each member's tile there, as the fused stage of a
+// single run does (swm_tile.cuh, with the same bits).  No intermediate field
+// goes through memory and one grid-wide barrier ends the stage; the barrier's
+// wait is bounded and reports a timeout through the error flag instead of
+// waiting forever.  Each member's state is stored like a single run's.
+//
+// Before, a stage was three phases (triangles, cells, edges) over members
+// interleaved in memory with a barrier after each, bound by the latency of
+// two dependent loads per entity at 32 warps per SM.  32 members on level 6
+// for 32 steps with 8 on level 7 for 64 took 54 ms (36 ms tuned) that way and
+// take 23.5 ms now, 5.4e9 member-cell-steps a second; what bounds them is the
+// issue of a tile's instructions, and a stage of few items the barrier.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -20,42 +27,25 @@
 
 #include "imodel_swm.h"
 #include "swm_common.cuh"
-#include "swm_k32_body.cuh"
 #include "swm_layout.h"
+#include "swm_tile.cuh"
 
 namespace imodel {
 namespace {
 
 constexpr int kMaxGrids = 8;
 
-// Division of 0 <= n < 2^31 by an invariant d >= 1 with one multiply-high
-// (Granlund and Montgomery, "Division by invariant integers using
-// multiplication", PLDI 1994, fig. 4.1): l = ceil(log2 d),
-// m = floor(2^32 (2^l - d) / d) + 1, n / d = (umulhi(m, n) + n) >> l; the sum
-// cannot overflow 32 bits for n < 2^31.
-struct FastDiv {
-  uint32_t m = 1, l = 0;
-  __device__ __forceinline__ int operator()(int n) const {
-    const uint32_t u = static_cast<uint32_t>(n);
-    return static_cast<int>((__umulhi(m, u) + u) >> l);
-  }
-};
-inline FastDiv make_fastdiv(uint32_t d) {
-  FastDiv f;
-  while ((1ull << f.l) < d) ++f.l;
-  f.m = static_cast<uint32_t>(((1ull << 32) * ((1ull << f.l) - d)) / d + 1);
-  return f;
-}
+constexpr int kEnsThreads = 256;
 
 struct GridDev {
-  DevMesh M;
-  int members;
-  FastDiv per_member;  // entity index = item / members
-  float h_ref;
+  TileDev tiles;
+  int nv, ne;
+  int members, group, ngroups;  // members per work item, items per tile
+  float h_ref, grav, erad;
   int nsteps;  // steps this launch
   float dt;
+  // [members][nv] and [members][ne]
   float *yn_h, *yn_u, *ya_h, *ya_u, *yb_h, *yb_u, *acc_h, *acc_u;
-  float *q_tr, *bern, *zflux;
 };
 
 struct EnsArgs {
@@ -63,40 +53,39 @@ struct EnsArgs {
   int macro_steps;
   int pv_on, mom_on;
   GridDev g[kMaxGrids];
+  int smem_block, smem_h, smem_u, smem_t;  // shared memory: the largest tile's sizes
   unsigned *bar_count;
-  unsigned *bar_gen;
-  int *flags;  // bit 0: PV division by ~0, bit 2: barrier timed out
+  int *flags;  // bit 0: PV division by ~0, bit 2: barrier timed out, bit 32: copy timed out
   // test hook: block stall_block (-1: none) leaves before its first
   // barrier; spin_limit bounds every barrier wait (polls of ~64 ns)
   int stall_block;
   unsigned long long spin_limit;
 };
 
-// grid-wide barrier with a bounded wait (cooperative launch: all blocks are
-// resident).  Returns false, with bit 2 of *flags set, if it gave up.
-__device__ bool grid_barrier(const EnsArgs &A) {
+// grid-wide barrier number `epoch` (0, 1, ...) with a bounded wait
+// (cooperative launch: all blocks are resident).  The counter only grows, so
+// the arrival that completes the barrier is also what the others poll.  The
+// fences order the block's writes before its arrival and, behind the wait,
+// drop the SM's L1 lines, so plain loads after the barrier see every block's
+// writes.  Returns false, with bit 2 of *flags set, if it gave up.
+__device__ bool grid_barrier(const EnsArgs &A, unsigned epoch) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
-    volatile unsigned *gen = A.bar_gen;
-    const unsigned g0 = *gen;
     __threadfence();
-    const unsigned arrived = atomicAdd(A.bar_count, 1u);
-    if (arrived == gridDim.x - 1) {
-      atomicExch(A.bar_count, 0u);
-      __threadfence();
-      atomicAdd(A.bar_gen, 1u);
-    } else {
-      unsigned long long spins = 0;
-      while (*gen == g0) {
-        if (++spins > A.spin_limit) {  // 2^26: several seconds; a phase takes < 10 ms
-          atomicOr(A.flags, 4);
-          ok = 0;
-          break;
-        }
-        __nanosleep(64);
+    const unsigned target = (epoch + 1) * gridDim.x;
+    atomicAdd(A.bar_count, 1u);
+    const volatile unsigned *count = A.bar_count;
+    unsigned long long spins = 0;
+    // wraps with the counter: fewer than 2^31 arrivals apart
+    while (static_cast<int>(*count - target) < 0) {
+      if (++spins > A.spin_limit) {  // 2^26: several seconds; a phase takes < 10 ms
+        atomicOr(A.flags, 4);
+        ok = 0;
+        break;
       }
+      __nanosleep(64);
     }
     __threadfence();
     s_ok = ok;
@@ -110,79 +99,96 @@ __device__ __forceinline__ bool steps_now(int s, int n, int S) {
   return (static_cast<long long>(s + 1) * n) / S > (static_cast<long long>(s) * n) / S;
 }
 
-// MINB = 1: registers as the compiler likes them; MINB = 2: capped at 64 per
-// thread for twice the resident warps (the tuner times both)
-template <int MINB>
-__global__ void __launch_bounds__(512, MINB) k_ensemble(EnsArgs A) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nthr = gridDim.x * blockDim.x;
+__global__ void __launch_bounds__(kEnsThreads, 3) k_ensemble(EnsArgs A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint64_t mbar;
   if (static_cast<int>(blockIdx.x) == A.stall_block) return;  // test hook
+  if (threadIdx.x == 0) tc05::mbar_init(&mbar, 1);
+  TileShared S;
+  S.block = smem;
+  S.sh = reinterpret_cast<float *>(smem + A.smem_block);
+  S.su = S.sh + A.smem_h;
+  S.sq = S.su + A.smem_u;
+  S.sb = S.sq + A.smem_t;
+  S.sz = S.sb + kEnsThreads;
+  __syncthreads();
+  uint32_t parity = 0;
+  unsigned epoch = 0;
   for (int s = 0; s < A.macro_steps; ++s) {
-    bool on[kMaxGrids];
-    for (int k = 0; k < A.ngrids; ++k) on[k] = steps_now(s, A.g[k].nsteps, A.macro_steps);
+    unsigned on = 0;
+    int total = 0;
+    for (int k = 0; k < A.ngrids; ++k)
+      if (steps_now(s, A.g[k].nsteps, A.macro_steps)) {
+        on |= 1u << k;
+        total += A.g[k].tiles.ntiles * A.g[k].ngroups;
+      }
     for (int st = 0; st < 4; ++st) {
-      // Each phase walks the grids that step now; item r of a grid is
-      // entity r / members, member r % members (all counts < 2^31).
-      // phase 1: potential vorticity at triangles
-      for (int k = 0; k < A.ngrids; ++k) {
-        if (!on[k]) continue;
+      for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        int k = 0, r = item;
+        for (;; ++k) {
+          if (!(on >> k & 1u)) continue;
+          const int n = A.g[k].tiles.ntiles * A.g[k].ngroups;
+          if (r < n) break;
+          r -= n;
+        }
         const GridDev &G = A.g[k];
-        const float *hin = st == 0 ? G.yn_h : (st == 2 ? G.yb_h : G.ya_h);
-        const float *uin = st == 0 ? G.yn_u : (st == 2 ? G.yb_u : G.ya_u);
-        const int n = G.M.nt * G.members;
-        for (int r = tid; r < n; r += nthr) {
-          const int t = G.per_member(r), m = r - t * G.members;
-          tri_body<Member, LdL2>(G.M, t, Member{G.members, m}, hin, uin, G.q_tr, G.h_ref,
-                                 A.pv_on, A.flags);
+        const int grp = r / G.tiles.ntiles, tile = r - grp * G.tiles.ntiles;
+        const Tile T(G.tiles.head + 5 * tile);
+        if (threadIdx.x == 0) {
+          // the last item's records have been read (barrier below); order
+          // those reads before the copy's writes
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          bulk_load(smem, G.tiles.data + T.block, T.bytes, &mbar);
+        }
+        const int m0 = grp * G.group, m1 = min(G.members, m0 + G.group);
+        for (int m = m0; m < m1; ++m) {
+          const size_t oh = static_cast<size_t>(m) * G.nv, ou = static_cast<size_t>(m) * G.ne;
+          TileFields F;
+          F.hd = (st == 0 ? G.yn_h : (st == 2 ? G.yb_h : G.ya_h)) + oh;
+          F.u = (st == 0 ? G.yn_u : (st == 2 ? G.yb_u : G.ya_u)) + ou;
+          F.h_out = (st == 0 ? G.ya_h : (st == 1 ? G.yb_h : (st == 2 ? G.ya_h : G.yn_h))) + oh;
+          F.u_out = (st == 0 ? G.ya_u : (st == 1 ? G.yb_u : (st == 2 ? G.ya_u : G.yn_u))) + ou;
+          F.yn_h = G.yn_h + oh;
+          F.yn_u = G.yn_u + ou;
+          F.acc_h = G.acc_h + oh;
+          F.acc_u = G.acc_u + ou;
+          F.tend_h = F.tend_u = nullptr;
+          TileOwn<kEnsThreads> own;
+          own.load(T, F, st);
+          if (m == m0) {
+            if (!tc05::mbar_wait(&mbar, parity, A.flags, 32)) return;
+            parity ^= 1u;
+          }
+          own.rim(T, F, S);
+          own.store(T, F, S);
+          __syncthreads();
+          tile_triangles<kEnsThreads>(T, S, G.h_ref, A.pv_on, A.flags);
+          __syncthreads();
+          tile_cells(T, S, F, own, st, G.dt, G.grav, G.h_ref);
+          __syncthreads();
+          tile_edges(T, S, F, own, st, G.dt, G.erad, A.mom_on);
+          // the next member (or tile) overwrites depths, velocities, records;
+          // the edges read neither depths nor velocities
+          if (m + 1 == m1) __syncthreads();
         }
       }
-      if (!grid_barrier(A)) return;
-      // phase 2: cells
-      for (int k = 0; k < A.ngrids; ++k) {
-        if (!on[k]) continue;
-        const GridDev &G = A.g[k];
-        const float *hin = st == 0 ? G.yn_h : (st == 2 ? G.yb_h : G.ya_h);
-        const float *uin = st == 0 ? G.yn_u : (st == 2 ? G.yb_u : G.ya_u);
-        float *hout = st == 0 ? G.ya_h : (st == 1 ? G.yb_h : (st == 2 ? G.ya_h : G.yn_h));
-        const int n = G.M.nv * G.members;
-        for (int r = tid; r < n; r += nthr) {
-          const int i = G.per_member(r), m = r - i * G.members;
-          cell_body<Member, LdL2>(G.M, i, Member{G.members, m}, hin, uin, G.q_tr, G.bern,
-                                  G.zflux, G.yn_h, G.acc_h, hout, nullptr, st, G.dt,
-                                  static_cast<float>(G.M.grav), G.h_ref);
-        }
-      }
-      if (!grid_barrier(A)) return;
-      // phase 3: edges
-      for (int k = 0; k < A.ngrids; ++k) {
-        if (!on[k]) continue;
-        const GridDev &G = A.g[k];
-        float *uout = st == 0 ? G.ya_u : (st == 1 ? G.yb_u : (st == 2 ? G.ya_u : G.yn_u));
-        const int n = G.M.ne * G.members;
-        for (int r = tid; r < n; r += nthr) {
-          const int e = G.per_member(r), m = r - e * G.members;
-          edge_body<Member, LdL2>(G.M, e, Member{G.members, m}, __ldg(&G.M.e_vs2[e]), G.bern,
-                                  G.zflux, G.yn_u, G.acc_u, uout, nullptr, st, G.dt, A.mom_on,
-                                  static_cast<float>(G.M.erad));
-        }
-      }
-      if (!grid_barrier(A)) return;
+      if (!grid_barrier(A, epoch++)) return;
     }
   }
 }
 
-// member m of a grid <-> reference-ordered FP64 arrays
-__global__ void k_ens_gather(int n, int M, int m, const int32_t *__restrict__ n2o,
+// a member's fields <-> reference-ordered FP64 arrays
+__global__ void k_ens_gather(int n, const int32_t *__restrict__ n2o,
                              const double *__restrict__ src, float *__restrict__ dst, double shift) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i * M + m] = static_cast<float>(src[n2o[i]] - shift);
+  if (i < n) dst[i] = static_cast<float>(src[n2o[i]] - shift);
 }
-__global__ void k_ens_scatter(int n, int M, int m, const int32_t *__restrict__ n2o,
+__global__ void k_ens_scatter(int n, const int32_t *__restrict__ n2o,
                               const float *__restrict__ src, double *__restrict__ dst,
                               double shift, int *flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    const double v = static_cast<double>(src[i * M + m]) + shift;
+    const double v = static_cast<double>(src[i]) + shift;
     dst[n2o[i]] = v;
     if (!isfinite(v)) atomicOr(flags, 2);
   }
@@ -205,11 +211,13 @@ struct Ens {
   GridHost g[kMaxGrids];
   std::vector<void *> allocs;
   double *stage_h = nullptr, *stage_u = nullptr;
-  unsigned *bar = nullptr;  // [0] count, [1] generation
+  unsigned *bar = nullptr;  // arrivals at the grid-wide barriers
   int *flags = nullptr;
   int *h_flags = nullptr;
   cudaStream_t stream = nullptr;
-  int block = 256, blocks_per_sm = 0, variant = 0;
+  int blocks_per_sm = 0;  // 0: as many as fit
+  size_t smem = 0;
+  EnsArgs args{};         // the parts that stay: sizes, members
   bool any_state = false;
   // test hook for the next launch only (imodel_swm_ensemble_test_stall)
   int test_stall_block = -1;
@@ -259,6 +267,11 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
   E->ngrids = ngrids;
   size_t maxn = 0;
   int rc;
+  int64_t cells = 0;
+  for (int k = 0; k < ngrids; ++k)
+    cells += static_cast<int64_t>(std::max(0, meshes[k].nv)) * std::max(0, members[k]);
+  const int cap = std::min(tile_cap(static_cast<int>(std::min<int64_t>(cells, INT32_MAX))),
+                           kEnsThreads);
   for (int k = 0; k < ngrids; ++k) {
     if (members[k] < 1) return fail(E, IMODEL_SWM_EINVAL, "every grid needs at least one member");
     Layout L;
@@ -275,52 +288,68 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
     G.members = members[k];
     G.areag.assign(meshes[k].hx_areag, meshes[k].hx_areag + L.nv);
     maxn = std::max(maxn, static_cast<size_t>(std::max(L.nv, L.ne)));
-    DevMesh &D = G.dev.M;
-    std::memset(&D, 0, sizeof(D));
-    D.nv = L.nv;
-    D.ne = L.ne;
-    D.nt = L.nt;
-    D.erad = L.erad;
-    D.grav = L.grav;
-    std::vector<float> bt32(L.nv, 0.0f);
-    const int32_t *ra = nullptr, *rb = nullptr, *rcc = nullptr;
-    if ((rc = up(E, L.t_recA, &ra)) || (rc = up(E, L.t_recB, &rb)) ||
-        (rc = up(E, L.t_recC, &rcc)))
-      return rc;
-    D.t_recA = reinterpret_cast<const int4 *>(ra);
-    D.t_recB = reinterpret_cast<const int4 *>(rb);
-    D.t_recC = reinterpret_cast<const float4 *>(rcc);
-    const int32_t *pk = nullptr;
-    const float *kd = nullptr;
-    const uint32_t *vs2 = nullptr;
+    GridDev &W = G.dev;
+    W.nv = L.nv;
+    W.ne = L.ne;
+    W.members = G.members;
+    W.grav = static_cast<float>(L.grav);
+    W.erad = static_cast<float>(L.erad);
+    // a tile's limits shrink with its size: one of these always fits
+    TileLayout T;
+    bool fits = false;
+    for (int c : {cap, 128, 64})
+      if (!fits && c <= cap) fits = build_tiles(L, c, T);
+    if (!fits) return fail(E, IMODEL_SWM_EINVAL, "grid " + std::to_string(k) + ": no tiling");
+    TileDev &D = W.tiles;
+    D.cap = T.cap;
+    D.ntiles = T.ntiles;
+    const TileHead *head = nullptr;
+    const uint32_t *data = nullptr;
     const int32_t *cn2o = nullptr, *en2o = nullptr;
-    if ((rc = up(E, L.t_ed, &D.t_ed)) || (rc = up(E, L.t_v, &D.t_v)) ||
-        (rc = up(E, L.t_f32, &D.t_f32)) || (rc = up(E, L.c_meta, &D.c_meta)) ||
-        (rc = up(E, L.c_inva32, &D.c_inva32)) || (rc = up(E, bt32, &D.c_bt32)) ||
-        (rc = up(E, L.e_grad32, &D.e_grad32)) || (rc = up(E, L.c_pk, &pk)) ||
-        (rc = up(E, L.c_kd, &kd)) || (rc = up(E, L.e_vs2, &vs2)) ||
+    if ((rc = up(E, T.head, &head)) || (rc = up(E, T.data, &data)) ||
         (rc = up(E, L.cell_n2o, &cn2o)) || (rc = up(E, L.edge_n2o, &en2o)))
       return rc;
-    D.c_pk = reinterpret_cast<const int4 *>(pk);
-    D.c_kd = reinterpret_cast<const float2 *>(kd);
-    D.e_vs2 = reinterpret_cast<const uint2 *>(vs2);
+    D.head = reinterpret_cast<const int4 *>(head);
+    D.data = reinterpret_cast<const uint4 *>(data);
     G.cell_n2o = const_cast<int32_t *>(cn2o);
     G.edge_n2o = const_cast<int32_t *>(en2o);
-    GridDev &W = G.dev;
-    W.members = G.members;
-    W.per_member = make_fastdiv(static_cast<uint32_t>(G.members));
-    float **bv[] = {&W.yn_h, &W.ya_h, &W.yb_h, &W.acc_h, &W.bern};
+    EnsArgs &A = E->args;
+    A.smem_block = std::max(A.smem_block, T.max_bytes);
+    A.smem_h = std::max(A.smem_h, T.max_h);
+    A.smem_u = std::max(A.smem_u, T.max_u);
+    A.smem_t = std::max(A.smem_t, T.max_t);
+    float **bv[] = {&W.yn_h, &W.ya_h, &W.yb_h, &W.acc_h};
     for (float **b : bv)
       if ((rc = zalloc(E, b, static_cast<size_t>(L.nv) * M))) return rc;
     float **be[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u};
     for (float **b : be)
       if ((rc = zalloc(E, b, static_cast<size_t>(L.ne) * M))) return rc;
-    if ((rc = zalloc(E, &W.q_tr, static_cast<size_t>(L.nt) * M)) ||
-        (rc = zalloc(E, &W.zflux, static_cast<size_t>(L.nv) * 6 * M)))
-      return rc;
+  }
+  EnsArgs &A = E->args;
+  E->smem = A.smem_block + sizeof(float) * (static_cast<size_t>(A.smem_h) + A.smem_u + A.smem_t +
+                                            kEnsThreads + 6 * kEnsThreads);
+  constexpr int kMost = 227 * 1024 - 1024;
+  if (E->smem > kMost) return fail(E, IMODEL_SWM_EINVAL, "a tile does not fit an SM");
+  EK(cudaFuncSetAttribute(k_ensemble, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  // Members per work item: a tile's records come in once for all of them,
+  // but every block should have several items for the blocks to end a stage
+  // together.  One eighth of a block's tile-members is the step of the
+  // longest share over the mean.
+  int sms = 0, occ = 0;
+  EK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
+  EK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, kEnsThreads, E->smem));
+  int64_t visits = 0;
+  for (int k = 0; k < ngrids; ++k)
+    visits += static_cast<int64_t>(E->g[k].dev.tiles.ntiles) * members[k];
+  const int64_t want = std::max<int64_t>(1, visits / (8 * static_cast<int64_t>(sms) *
+                                                      std::max(1, occ)));
+  for (int k = 0; k < ngrids; ++k) {
+    GridDev &W = E->g[k].dev;
+    W.group = static_cast<int>(std::min<int64_t>(want, W.members));
+    W.ngroups = (W.members + W.group - 1) / W.group;
   }
   if ((rc = zalloc(E, &E->stage_h, maxn)) || (rc = zalloc(E, &E->stage_u, maxn)) ||
-      (rc = zalloc(E, &E->bar, 2)) || (rc = zalloc(E, &E->flags, 1)))
+      (rc = zalloc(E, &E->bar, 1)) || (rc = zalloc(E, &E->flags, 1)))
     return rc;
   EK(cudaMallocHost(&E->h_flags, sizeof(int)));
   return IMODEL_SWM_OK;
@@ -332,20 +361,14 @@ int ens_flags(Ens *E) {
   EK(cudaStreamSynchronize(E->stream));
   const int f = *E->h_flags;
   if (f & 4) return fail(E, IMODEL_SWM_ECUDA, "grid barrier timed out");
+  if (f & 32) return fail(E, IMODEL_SWM_ECUDA, "the ensemble kernel gave up on a bounded wait");
   if (f & 1) return fail(E, IMODEL_SWM_EDIVZERO, "division by zero in PV (|h_tr| < eps/1e5)");
   if (f & 2) return fail(E, IMODEL_SWM_EBLOWUP, "state holds NaN or Inf");
   return IMODEL_SWM_OK;
 }
 
-inline const void *ens_kernel(int variant) {
-  return variant == 1 ? reinterpret_cast<const void *>(k_ensemble<2>)
-                      : reinterpret_cast<const void *>(k_ensemble<1>);
-}
-
-int ens_launch(Ens *E, const double *dt, const int32_t *nsteps, int block, int bps,
-               int variant) {
-  EnsArgs A;
-  std::memset(&A, 0, sizeof(A));
+int ens_launch(Ens *E, const double *dt, const int32_t *nsteps, int bps) {
+  EnsArgs A = E->args;
   A.ngrids = E->ngrids;
   A.pv_on = E->testcase >= 2 ? 1 : 0;
   A.mom_on = E->testcase > 1 ? 1 : 0;
@@ -361,7 +384,6 @@ int ens_launch(Ens *E, const double *dt, const int32_t *nsteps, int block, int b
   if (S == 0) return IMODEL_SWM_OK;
   A.macro_steps = S;
   A.bar_count = E->bar;
-  A.bar_gen = E->bar + 1;
   A.flags = E->flags;
   A.stall_block = E->test_stall_block;
   A.spin_limit = E->test_spin_limit ? E->test_spin_limit : (1ull << 26);
@@ -371,13 +393,13 @@ int ens_launch(Ens *E, const double *dt, const int32_t *nsteps, int block, int b
   EK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   EK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   if (!coop) return fail(E, IMODEL_SWM_ECUDA, "device does not support cooperative launch");
-  EK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_kernel(variant), block, 0));
+  EK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, kEnsThreads, E->smem));
   if (occ < 1) return fail(E, IMODEL_SWM_ECUDA, "ensemble kernel does not fit an SM");
   const int per_sm = (bps > 0 && bps <= occ) ? bps : occ;
-  EK(cudaMemsetAsync(E->bar, 0, 2 * sizeof(unsigned), E->stream));
+  EK(cudaMemsetAsync(E->bar, 0, sizeof(unsigned), E->stream));
   void *args[] = {&A};
-  EK(cudaLaunchCooperativeKernel(ens_kernel(variant), dim3(sms * per_sm),
-                                 dim3(block), args, 0, E->stream));
+  EK(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_ensemble), dim3(sms * per_sm),
+                                 dim3(kEnsThreads), args, E->smem, E->stream));
   return IMODEL_SWM_OK;
 }
 
@@ -425,12 +447,10 @@ int imodel_swm_ensemble_set_state(void *ens, int32_t grid, int32_t member, const
   }
   EK(cudaMemcpyAsync(E->stage_h, h, sizeof(double) * G.nv, cudaMemcpyHostToDevice, E->stream));
   EK(cudaMemcpyAsync(E->stage_u, u, sizeof(double) * G.ne, cudaMemcpyHostToDevice, E->stream));
-  imodel::k_ens_gather<<<(G.nv + 255) / 256, 256, 0, E->stream>>>(G.nv, G.members, member,
-                                                                  G.cell_n2o, E->stage_h,
-                                                                  G.dev.yn_h, G.h_ref);
-  imodel::k_ens_gather<<<(G.ne + 255) / 256, 256, 0, E->stream>>>(G.ne, G.members, member,
-                                                                  G.edge_n2o, E->stage_u,
-                                                                  G.dev.yn_u, 0.0);
+  imodel::k_ens_gather<<<(G.nv + 255) / 256, 256, 0, E->stream>>>(
+      G.nv, G.cell_n2o, E->stage_h, G.dev.yn_h + static_cast<size_t>(member) * G.nv, G.h_ref);
+  imodel::k_ens_gather<<<(G.ne + 255) / 256, 256, 0, E->stream>>>(
+      G.ne, G.edge_n2o, E->stage_u, G.dev.yn_u + static_cast<size_t>(member) * G.ne, 0.0);
   EK(cudaGetLastError());
   EK(cudaStreamSynchronize(E->stream));
   E->any_state = true;
@@ -445,9 +465,11 @@ int imodel_swm_ensemble_get_state(void *ens, int32_t grid, int32_t member, doubl
   if (member < 0 || member >= G.members) return imodel::fail(E, IMODEL_SWM_EINVAL, "bad member");
   if (cudaSetDevice(E->device) != cudaSuccess) return IMODEL_SWM_ECUDA;
   imodel::k_ens_scatter<<<(G.nv + 255) / 256, 256, 0, E->stream>>>(
-      G.nv, G.members, member, G.cell_n2o, G.dev.yn_h, E->stage_h, G.h_ref, E->flags);
+      G.nv, G.cell_n2o, G.dev.yn_h + static_cast<size_t>(member) * G.nv, E->stage_h, G.h_ref,
+      E->flags);
   imodel::k_ens_scatter<<<(G.ne + 255) / 256, 256, 0, E->stream>>>(
-      G.ne, G.members, member, G.edge_n2o, G.dev.yn_u, E->stage_u, 0.0, E->flags);
+      G.ne, G.edge_n2o, G.dev.yn_u + static_cast<size_t>(member) * G.ne, E->stage_u, 0.0,
+      E->flags);
   EK(cudaGetLastError());
   EK(cudaMemcpyAsync(h, E->stage_h, sizeof(double) * G.nv, cudaMemcpyDeviceToHost, E->stream));
   EK(cudaMemcpyAsync(u, E->stage_u, sizeof(double) * G.ne, cudaMemcpyDeviceToHost, E->stream));
@@ -459,7 +481,7 @@ int imodel_swm_ensemble_advance(void *ens, const double *dt, const int32_t *nste
   if (!E || !dt || !nsteps) return IMODEL_SWM_EINVAL;
   if (!E->any_state) return imodel::fail(E, IMODEL_SWM_ESTATE, "no state set");
   if (cudaSetDevice(E->device) != cudaSuccess) return IMODEL_SWM_ECUDA;
-  int rc = imodel::ens_launch(E, dt, nsteps, E->block, E->blocks_per_sm, E->variant);
+  int rc = imodel::ens_launch(E, dt, nsteps, E->blocks_per_sm);
   if (rc) return rc;
   return imodel::ens_flags(E);
 }
@@ -502,30 +524,23 @@ int imodel_swm_ensemble_tune(void *ens, const double *dt, int32_t nsteps, int32_
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   float best = 1e30f;
-  int bb = E->block, bbps = E->blocks_per_sm, bv = E->variant;
+  int bbps = E->blocks_per_sm, occ = 0;
   int rc = IMODEL_SWM_OK;
-  const int blocks[3] = {128, 256, 512};
-  for (int v = 0; v < 2 && rc == IMODEL_SWM_OK; ++v)
-    for (int b : blocks) {
-      int occ = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, imodel::ens_kernel(v), b, 0);
-      for (int bps = occ; bps >= 1 && rc == IMODEL_SWM_OK; bps = bps > 1 ? bps / 2 : 0) {
-        cudaEventRecord(e0, E->stream);
-        rc = imodel::ens_launch(E, dt, ns.data(), b, bps, v);
-        cudaEventRecord(e1, E->stream);
-        if (rc) break;
-        rc = imodel::ens_flags(E);
-        float ms = 1e30f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (rc == IMODEL_SWM_OK && ms < best) {
-          best = ms;
-          bb = b;
-          bbps = bps;
-          bv = v;
-        }
-        if (bps == 1) break;
-      }
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, imodel::k_ensemble, imodel::kEnsThreads,
+                                                E->smem);
+  for (int bps = occ; bps >= 1 && rc == IMODEL_SWM_OK; --bps) {
+    cudaEventRecord(e0, E->stream);
+    rc = imodel::ens_launch(E, dt, ns.data(), bps);
+    cudaEventRecord(e1, E->stream);
+    if (rc) break;
+    rc = imodel::ens_flags(E);
+    float ms = 1e30f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    if (rc == IMODEL_SWM_OK && ms < best) {
+      best = ms;
+      bbps = bps;
     }
+  }
   for (size_t q = 0; q < bufs.size(); ++q)
     cudaMemcpyAsync(bufs[q], saved[q], sizes[q], cudaMemcpyDeviceToDevice, E->stream);
   cudaStreamSynchronize(E->stream);
@@ -533,12 +548,10 @@ int imodel_swm_ensemble_tune(void *ens, const double *dt, int32_t nsteps, int32_
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
-  E->block = bb;
   E->blocks_per_sm = bbps;
-  E->variant = bv;
-  choice[0] = bb;
+  choice[0] = imodel::kEnsThreads;
   choice[1] = bbps;
-  choice[2] = bv;
+  choice[2] = 0;
   return IMODEL_SWM_OK;
 }
 

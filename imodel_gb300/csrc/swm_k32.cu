@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(512) k_tri32(DevMesh M, const float *__restric
                                                float *__restrict__ ht_out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= M.nt) return;
-  tri_body<OneRun, LdPlain, Wait>(M, t, OneRun{}, hd, u, q_tr, h_ref, pv_on, flags, kt, coefvort, ht_out);
+  tri_body<Wait>(M, t, hd, u, q_tr, h_ref, pv_on, flags, kt, coefvort, ht_out);
 }
 
 // h_e (deviation), flux F_e = u_e (h_ref + h_e), q_e: the TRSK average
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(512) k_cell32v2(DevMesh M, const float *__rest
                                                   float *__restrict__ coefdiv) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M.nv) return;
-  cell_body<OneRun, LdPlain, kEdgePV, kZ, Wait>(M, i, OneRun{}, hd, u, q_tr, bern, zflux, yn, acc,
+  cell_body<kEdgePV, kZ, Wait>(M, i, hd, u, q_tr, bern, zflux, yn, acc,
                                           yout, tend, stage, dt, grav, h_ref, kcv, coefdiv);
 }
 
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(512) k_tri32d(DevMesh M, const float *__restri
   const float circ[3] = {__int_as_float(b.z), __int_as_float(b.w), c.x};
   const float kite[3] = {c.y, c.z, c.w};
   after_prior<true>(hd, u, q_tr, coefvort, wq);
-  tri_core<OneRun, LdPlain, NoWait>(t, OneRun{}, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u,
+  tri_core<NoWait>(t, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u,
                                     q_tr, h_ref, pv_on, flags, kt, coefvort, nullptr);
   const float q = q_tr[t];
   const unsigned opp = __ldg(&M.t_dopp[t]);
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(512) k_edge32v2(DevMesh M, const float *__rest
     }
   } else {
     IMODEL_WAIT(Wait, bern, zflux, yn, acc, yout, tend, corr, dif1, dif2);
-    edge_body(M, e0, OneRun{}, __ldg(&M.e_vs2[e0]), bern, zflux, yn, acc, yout, tend, stage, dt,
+    edge_body(M, e0, __ldg(&M.e_vs2[e0]), bern, zflux, yn, acc, yout, tend, stage, dt,
               mom_on, erad, corr, dif1, dif2);
   }
 }

@@ -1,38 +1,14 @@
 // Per-entity bodies of the FP32 cell-centred TRSK stage (internal header).
 //
-// Shared by the single-run kernels (swm_k32.cu) and the ensemble kernel
-// (swm_ens.cu).  The index policy maps an entity to its slot in a state
-// array: one run stores entity i at i, an ensemble stores member m of entity
-// i at i*M + m (members fastest), so that the threads of a warp that share
-// an entity read its geometry once and the members' values contiguously.
+// Shared by the single-run kernels (swm_k32.cu) and the tiles of the fused
+// stage and the ensemble kernel (swm_tile.cuh).
 #pragma once
 #include "swm_common.cuh"
 
 namespace imodel {
 
-struct OneRun {
-  __device__ __forceinline__ int operator()(int i) const { return i; }
-};
-struct Member {
-  int M, m;
-  __device__ __forceinline__ int operator()(int i) const { return i * M + m; }
-};
-
-// Loads of fields that change during a run.  Separate launches see each
-// other's writes, so plain loads are fine there; inside the persistent
-// ensemble kernel another block may have rewritten the value since this SM
-// cached it, so those loads go through L2 (ld.global.cg), never through the
-// incoherent L1 / read-only path.
-struct LdPlain {
-  static __device__ __forceinline__ float ld(const float *p) { return *p; }
-};
-struct LdL2 {
-  static __device__ __forceinline__ float ld(const float *p) { return __ldcg(p); }
-};
-
-// Called between the loads of the fixed records and the first load of a
-// changing field: nothing in the persistent kernel, the wait for the kernel
-// before in the single-run kernels (after_prior).
+// Between the loads of the fixed records and the first load of a changing
+// field: the wait for the kernel before (after_prior), or nothing.
 struct NoWait {
   static constexpr bool kWaits = false;
 };
@@ -66,8 +42,8 @@ __device__ __forceinline__ float rk_stage32(int stage, float k, float yn, float 
 // q_t = (curl u / A + f) / h_t  (vort_tr + scalar_hx2tr + scalar_elem_divide)
 // from a triangle's decoded record: edges, cells, circulation and kite
 // coefficients, Coriolis parameter; the sums run in slot order 0, 1, 2
-template <class Ix, class Ld, class Wait>
-__device__ __forceinline__ void tri_core(int t, Ix ix, const int (&ed)[3], const int (&cv)[3],
+template <class Wait>
+__device__ __forceinline__ void tri_core(int t, const int (&ed)[3], const int (&cv)[3],
                                          const float (&circ)[3], const float (&kite)[3],
                                          float f, const float *__restrict__ hd,
                                          const float *__restrict__ u, float *__restrict__ q_tr,
@@ -80,16 +56,16 @@ __device__ __forceinline__ void tri_core(int t, Ix ix, const int (&ed)[3], const
   float ht = 0.0f, z = 0.0f;
 #pragma unroll
   for (int s = 0; s < 3; ++s) {
-    const float us = Ld::ld(u + ix(ed[s]));
+    const float us = u[ed[s]];
     eta = fmaf(circ[s], us, eta);
     z = fmaf(circ[s], us, z);
-    ht = fmaf(kite[s], Ld::ld(hd + ix(cv[s])), ht);
+    ht = fmaf(kite[s], hd[cv[s]], ht);
   }
   // with diffusion on: K_tr times the relative vorticity
-  if (coefvort) coefvort[ix(t)] = kt[t] * z;
+  if (coefvort) coefvort[t] = kt[t] * z;
   ht += h_ref;
   // gass18: the depth at the triangle for the rhombus PV of the edges
-  if (ht_out) ht_out[ix(t)] = ht;
+  if (ht_out) ht_out[t] = ht;
   float q = 0.0f;
   if (pv_on) {
     // scalar_elem_divide guard, swm_operators.f90:1604-1606
@@ -98,11 +74,11 @@ __device__ __forceinline__ void tri_core(int t, Ix ix, const int (&ed)[3], const
     else
       q = eta / ht;
   }
-  q_tr[ix(t)] = q;
+  q_tr[t] = q;
 }
 
-template <class Ix, class Ld = LdPlain, class Wait = NoWait>
-__device__ __forceinline__ void tri_body(const DevMesh &M, int t, Ix ix,
+template <class Wait>
+__device__ __forceinline__ void tri_body(const DevMesh &M, int t,
                                          const float *__restrict__ hd,
                                          const float *__restrict__ u, float *__restrict__ q_tr,
                                          float h_ref, int pv_on, int *flags,
@@ -116,7 +92,7 @@ __device__ __forceinline__ void tri_body(const DevMesh &M, int t, Ix ix,
   const int ed[3] = {a.x, a.y, a.z}, cv[3] = {a.w, b.x, b.y};
   const float circ[3] = {__int_as_float(b.z), __int_as_float(b.w), c.x};
   const float kite[3] = {c.y, c.z, c.w};
-  tri_core<Ix, Ld, Wait>(t, ix, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u, q_tr, h_ref, pv_on,
+  tri_core<Wait>(t, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u, q_tr, h_ref, pv_on,
                    flags, kt, coefvort, ht_out);
 }
 
@@ -154,7 +130,7 @@ __device__ __forceinline__ void tri_body16(const DevMesh &M, int t, const float 
   }
   const float circ[3] = {__uint_as_float(a.w), b.x, b.y};
   const float kite[3] = {b.z, b.w, c.x};
-  tri_core<OneRun, LdPlain, Wait>(t, OneRun{}, ed, cv, circ, kite, c.y, hd, u, q_tr, h_ref, pv_on,
+  tri_core<Wait>(t, ed, cv, circ, kite, c.y, hd, u, q_tr, h_ref, pv_on,
                             flags, kt, coefvort);
 }
 
@@ -203,13 +179,13 @@ __device__ __forceinline__ void trsk_cell(const float (&G)[6], const float (&qs)
 // returns the sum of the fluxes out of the cell.  kEdgePV: qt holds the PV of
 // the cell's edges (formed by the edge pre-pass, APVM's upwinding included)
 // instead of the PV of its triangles.
-template <class Ix = OneRun, bool kEdgePV = false, bool kZ = true>
+template <bool kEdgePV = false, bool kZ = true>
 __device__ __forceinline__ float cell_terms(int i, uint32_t meta, const float (&R)[6],
                                             const float2 (&kd)[6], const float (&ue)[6],
                                             const float (&hn)[6], const float (&qt)[6], float hi,
                                             float bt, float inva, float *__restrict__ bern,
                                             float *__restrict__ zflux, float grav, float h_ref,
-                                            Ix ix = Ix{}, const float *__restrict__ kcv = nullptr,
+                                            const float *__restrict__ kcv = nullptr,
                                             float *__restrict__ coefdiv = nullptr) {
   const int n = static_cast<int>(meta & 7u);
   const unsigned tneg = meta >> 8;
@@ -228,8 +204,8 @@ __device__ __forceinline__ float cell_terms(int i, uint32_t meta, const float (&
     du = fmaf(ue[j], kd[j].y, du);
   }
   // with diffusion on: K times the divergence of u
-  if (coefdiv) coefdiv[ix(i)] = kcv[ix(i)] * (du * inva);
-  bern[ix(i)] = fmaf(grav, hi + bt, ke);
+  if (coefdiv) coefdiv[i] = kcv[i] * (du * inva);
+  bern[i] = fmaf(grav, hi + bt, ke);
   // kZ false (dtred): the edges form their PV flux from the triangles
   if (kZ) {
     float Z[6];
@@ -243,13 +219,13 @@ __device__ __forceinline__ float cell_terms(int i, uint32_t meta, const float (&
       trsk_cell<3>(G, qs, R, tneg, Z);
 #pragma unroll
     for (int j = 0; j < 6; ++j)
-      if (j < n) zflux[ix(6 * i + j)] = Z[j];
+      if (j < n) zflux[6 * i + j] = Z[j];
   }
   return div;
 }
 
 // cell_terms and the mass RK stage
-template <class Ix = OneRun, bool kEdgePV = false, bool kZ = true>
+template <bool kEdgePV = false, bool kZ = true>
 __device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)[6],
                                           const float2 (&kd)[6], const float (&ue)[6],
                                           const float (&hn)[6], const float (&qt)[6], float hi,
@@ -257,18 +233,18 @@ __device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)
                                           float *__restrict__ bern, float *__restrict__ zflux,
                                           float *__restrict__ acc, float *__restrict__ yout,
                                           float *__restrict__ tend, int stage, float dt,
-                                          float grav, float h_ref, Ix ix = Ix{},
+                                          float grav, float h_ref,
                                           const float *__restrict__ kcv = nullptr,
                                           float *__restrict__ coefdiv = nullptr) {
-  const float div = cell_terms<Ix, kEdgePV, kZ>(i, meta, R, kd, ue, hn, qt, hi, bt, inva, bern,
-                                                zflux, grav, h_ref, ix, kcv, coefdiv);
+  const float div = cell_terms<kEdgePV, kZ>(i, meta, R, kd, ue, hn, qt, hi, bt, inva, bern,
+                                                zflux, grav, h_ref, kcv, coefdiv);
   const float masseq = __fmul_rn(-div, inva);
   if (stage < 0) {
-    tend[ix(i)] = masseq;
+    tend[i] = masseq;
   } else {
     float a = accv;
-    yout[ix(i)] = rk_stage32(stage, masseq, ynv, &a, dt);
-    if (stage < 3) acc[ix(i)] = a;
+    yout[i] = rk_stage32(stage, masseq, ynv, &a, dt);
+    if (stage < 3) acc[i] = a;
   }
 }
 
@@ -279,8 +255,8 @@ __device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)
 // weights), gathering its neighbours' values.  The cell's own values come in
 // as arguments: h (deviation) hi, b bt, 1/(A a) inva, y_n ynv and the RK
 // accumulator accv (read for stages 1-3).
-template <class Ix, class Ld, bool kEdgePV = false, bool kZ = true>
-__device__ __forceinline__ void cell_core(int i, Ix ix, uint32_t meta,
+template <bool kEdgePV, bool kZ>
+__device__ __forceinline__ void cell_core(int i, uint32_t meta,
                                           const int (&ed)[6], const int (&nb)[6],
                                           const int (&tr)[6], const float (&R)[6],
                                           const float2 (&kd)[6], float hi, float bt, float inva,
@@ -295,32 +271,30 @@ __device__ __forceinline__ void cell_core(int i, Ix ix, uint32_t meta,
   float ue[6], hn[6], qt[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    ue[j] = Ld::ld(u + ix(ed[j]));
-    hn[j] = Ld::ld(hd + ix(nb[j]));
+    ue[j] = u[ed[j]];
+    hn[j] = hd[nb[j]];
     // kEdgePV: q_tr is the edges' PV, indexed by the slot's edge
-    qt[j] = Ld::ld(q_tr + ix(kEdgePV ? ed[j] : tr[j]));
+    qt[j] = q_tr[kEdgePV ? ed[j] : tr[j]];
   }
-  cell_math<Ix, kEdgePV, kZ>(i, meta, R, kd, ue, hn, qt, hi, bt, inva, ynv, accv, bern, zflux,
-                             acc, yout, tend, stage, dt, grav, h_ref, ix, kcv, coefdiv);
+  cell_math<kEdgePV, kZ>(i, meta, R, kd, ue, hn, qt, hi, bt, inva, ynv, accv, bern, zflux,
+                             acc, yout, tend, stage, dt, grav, h_ref, kcv, coefdiv);
 }
 
 // the cell's own values from global memory
-template <class Ix, class Ld>
-__device__ __forceinline__ void cell_own(const DevMesh &M, int i, Ix ix,
+__device__ __forceinline__ void cell_own(const DevMesh &M, int i,
                                          const float *__restrict__ hd,
                                          const float *__restrict__ yn,
                                          const float *__restrict__ acc, int stage, float &hi,
                                          float &bt, float &inva, float &ynv, float &accv) {
-  hi = Ld::ld(hd + ix(i));
+  hi = hd[i];
   bt = __ldg(&M.c_bt32[i]);
   inva = __ldg(&M.c_inva32[i]);
-  ynv = stage >= 0 ? Ld::ld(yn + ix(i)) : 0.0f;
-  accv = stage >= 1 ? Ld::ld(acc + ix(i)) : 0.0f;
+  ynv = stage >= 0 ? yn[i] : 0.0f;
+  accv = stage >= 1 ? acc[i] : 0.0f;
 }
 
-template <class Ix, class Ld = LdPlain, bool kEdgePV = false, bool kZ = true,
-          class Wait = NoWait>
-__device__ __forceinline__ void cell_body(const DevMesh &M, int i, Ix ix,
+template <bool kEdgePV, bool kZ, class Wait>
+__device__ __forceinline__ void cell_body(const DevMesh &M, int i,
                                           const float *__restrict__ hd,
                                           const float *__restrict__ u,
                                           const float *__restrict__ q_tr,
@@ -348,8 +322,8 @@ __device__ __forceinline__ void cell_body(const DevMesh &M, int i, Ix ix,
   }
   IMODEL_WAIT(Wait, hd, u, q_tr, bern, zflux, yn, acc, yout, tend, coefdiv);
   float hi, bt, inva, ynv, accv;
-  cell_own<Ix, Ld>(M, i, ix, hd, yn, acc, stage, hi, bt, inva, ynv, accv);
-  cell_core<Ix, Ld, kEdgePV, kZ>(i, ix, meta, ed, nb, tr, R, kd, hi, bt, inva, ynv, accv, hd, u,
+  cell_own(M, i, hd, yn, acc, stage, hi, bt, inva, ynv, accv);
+  cell_core<kEdgePV, kZ>(i, meta, ed, nb, tr, R, kd, hi, bt, inva, ynv, accv, hd, u,
                                  q_tr, bern, zflux, acc, yout, tend, stage, dt, grav, h_ref, kcv,
                                  coefdiv);
 }
@@ -362,8 +336,7 @@ __device__ __forceinline__ float edge_terms(float b1, float b2, float z1, float 
 }
 
 // -grad B - (Z_c1 + Z_c2) / l_e and the momentum RK stage of edge e
-template <class Ix, class Ld = LdPlain>
-__device__ __forceinline__ void edge_body(const DevMesh &M, int e, Ix ix, uint2 w,
+__device__ __forceinline__ void edge_body(const DevMesh &M, int e, uint2 w,
                                           const float *__restrict__ bern,
                                           const float *__restrict__ zflux,
                                           const float *__restrict__ yn, float *__restrict__ acc,
@@ -375,19 +348,19 @@ __device__ __forceinline__ void edge_body(const DevMesh &M, int e, Ix ix, uint2 
   const int c1 = static_cast<int>(w.x & 0x0FFFFFFFu), c2 = static_cast<int>(w.y & 0x0FFFFFFFu);
   const int s1 = static_cast<int>(w.x >> 28), s2 = static_cast<int>(w.y >> 28);
   const float g = __ldg(&M.e_grad32[e]);  // 1 / (l_e a)
-  float momeq = edge_terms(Ld::ld(bern + ix(c1)), Ld::ld(bern + ix(c2)),
-                           Ld::ld(zflux + ix(6 * c1 + s1)), Ld::ld(zflux + ix(6 * c2 + s2)), g,
+  float momeq = edge_terms(bern[c1], bern[c2],
+                           zflux[6 * c1 + s1], zflux[6 * c2 + s2], g,
                            erad);
   // learned correction of the PV flux (frozen over the RK step)
-  if (corr) momeq += corr[ix(e)];
+  if (corr) momeq += corr[e];
   // diffusion, then hyperdiffusion
-  if (dif1) momeq += dif1[ix(e)];
-  if (dif2) momeq -= dif2[ix(e)];
+  if (dif1) momeq += dif1[e];
+  if (dif2) momeq -= dif2[e];
   if (!mom_on) momeq = 0.0f;
   if (stage < 0)
-    tend[ix(e)] = momeq;
+    tend[e] = momeq;
   else
-    yout[ix(e)] = rk_stage32(stage, momeq, Ld::ld(yn + ix(e)), acc + ix(e), dt);
+    yout[e] = rk_stage32(stage, momeq, yn[e], acc + e, dt);
 }
 
 }  // namespace imodel

@@ -120,7 +120,7 @@ __device__ __forceinline__ void tile_triangles(const Tile &T, const TileShared &
                        static_cast<int>(iv >> 20)};
     const float circ[3] = {a.x, a.y, a.z};
     const float kite[3] = {__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z)};
-    tri_core<OneRun, LdPlain, NoWait>(k, OneRun{}, ed, cv, circ, kite, a.w, S.sh, S.su, S.sq,
+    tri_core<NoWait>(k, ed, cv, circ, kite, a.w, S.sh, S.su, S.sq,
                                       h_ref, pv_on, flags);
   }
 }
@@ -149,7 +149,7 @@ __device__ __forceinline__ void tile_cells(const Tile &T, const TileShared &S,
   const float bt = reinterpret_cast<const float *>(S.block + T.bt)[tid];
   const bool mine = tid < T.nc;
   const float inva = mine ? reinterpret_cast<const float *>(S.block + T.inva)[tid] : 0.0f;
-  const float div = cell_terms<OneRun>(tid, meta, R, kd, ue, hn, qt, S.sh[tid], bt, inva, S.sb,
+  const float div = cell_terms(tid, meta, R, kd, ue, hn, qt, S.sh[tid], bt, inva, S.sb,
                                        S.sz, grav, h_ref);
   if (!mine) return;
   const float masseq = __fmul_rn(-div, inva);

@@ -304,9 +304,9 @@ void *imodel_swm_stream(void *handle);
 /* ---- ensembles ----------------------------------------------------------- *
  * Many instances of the FP32 step on up to 8 grids (e.g. 64 members on one
  * level and 16 on another) advanced together by ONE persistent cooperative
- * launch.  Members of a grid share its geometry; their states are
- * interleaved member-fastest.  Each grid keeps its own dt and step count; the
- * grids' steps are spread evenly over the launch.  Member results equal the
+ * launch.  Members of a grid share its geometry, which a block reads once
+ * for several of them.  Each grid keeps its own dt and step count; the grids'
+ * steps are spread evenly over the launch.  Member results equal the
  * single-run FP32 path (variant 1) bit for bit when both store h against the
  * same reference depth (a grid's reference is the area mean of the first
  * state set on it; other members differ from their own single runs at the
@@ -322,10 +322,9 @@ int imodel_swm_ensemble_get_state(void *ens, int32_t grid, int32_t member, doubl
 /* dt[ngrids] seconds and nsteps[ngrids] RK4 steps per grid, one launch. */
 int imodel_swm_ensemble_advance(void *ens, const double *dt, const int32_t *nsteps);
 /* Autotuner of the persistent launch: times nsteps steps per grid for each
- * kernel variant (0: registers unconstrained, 1: at most 64 registers per
- * thread for more resident warps), block size and blocks-per-SM count, keeps
- * the fastest, restores the state.
- * choice = {block size, blocks per SM, variant}. */
+ * blocks-per-SM count, keeps the fastest, restores the state.
+ * choice = {block size, blocks per SM, variant}; there is one block size and
+ * one variant (0). */
 int imodel_swm_ensemble_tune(void *ens, const double *dt, int32_t nsteps, int32_t choice[3]);
 /* Test hook with no counterpart in the reference: in the next
  * imodel_swm_ensemble_advance launch only, block `block` of the persistent
