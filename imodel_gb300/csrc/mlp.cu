@@ -190,18 +190,23 @@ namespace imodel {
 namespace {
 
 // ---- fused forward + backward over a batch ---------------------------------
-// dynamic shared memory: A1 8K | B1 4K | A2 16K | B2 8K | B2T 8K | A3 16K |
-// AW 32K | BW 32K
-constexpr int TRN_SMEM = 8192 + 4096 + 16384 + 8192 + 8192 + 16384 + 32768 + 32768;
+// dynamic shared memory: B1 4K | B2 8K | B2T 8K | A2 16K | AW 32K | BW 32K.
+// A3 (dZ2) takes A2's place, whose product has been waited for, and A1 the
+// last rows of BW, which are written after it: 100 KB, so that two CTAs share
+// an SM (and its 512 TMEM columns) and hide each other's waits for products
+// and rows.  A batch of 65,536 rows is 512 tiles: one CTA an SM took four
+// rounds of them.
+constexpr int TRN_SMEM = 4096 + 8192 + 8192 + 16384 + 32768 + 32768;
+constexpr int TRN_CTAS = 2;  // per SM
 
-__global__ void __launch_bounds__(TM, 1)
+__global__ void __launch_bounds__(TM, TRN_CTAS)
     k_mlp_train(Weights W, const uint16_t *__restrict__ x, const float *__restrict__ t,
                 const float *__restrict__ wts,
                 int64_t n, int64_t batch, uint64_t seed, float inv_batch,
                 float *__restrict__ partials, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t *A1 = smem, *B1 = A1 + 8192, *A2 = B1 + 4096, *B2 = A2 + 16384, *B2T = B2 + 8192,
-          *A3 = B2T + 8192, *AW = A3 + 16384, *BW = AW + 32768;
+  uint8_t *B1 = smem, *B2 = B1 + 4096, *B2T = B2 + 8192, *A2 = B2T + 8192, *AW = A2 + 16384,
+          *BW = AW + 32768, *A3 = A2, *A1 = BW + 24576;
   __shared__ uint64_t mbar;
   __shared__ uint32_t tslot;
   __shared__ float sb1[NH], sb2[NH], sw3[NH];
@@ -406,26 +411,52 @@ __global__ void __launch_bounds__(TM, 1)
   if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
-// sum of the CTAs' partial gradients in a fixed order
-__global__ void k_reduce(const float *__restrict__ partials, int nblk, float *__restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= NPART) return;
+// Sum of the CTAs' partial gradients in a fixed order, in FP64: a block takes
+// 32 parameters, its warp w every kRed-th partial from w on, and the warps'
+// sums are added in order.  (One thread a parameter added 152 values in a row,
+// 27 us a step: FP64 additions are slow here and 5826 threads are few.)  With
+// ADAM the parameter's update follows at once, and its BF16 images with it.
+constexpr int kRed = 16;
+struct AdamArgs {
+  float *p, *m, *v, *loss;
+  uint16_t *w1img, *w2img, *w2timg;
+  float lr, b1, b2, eps, c1, c2;
+};
+template <bool ADAM>
+__global__ void __launch_bounds__(32 * kRed) k_reduce(const float *__restrict__ partials, int nblk,
+                                                      float *__restrict__ grad, AdamArgs A) {
+  __shared__ double part[kRed][32];
+  const int lane = threadIdx.x & 31, w0 = threadIdx.x >> 5, q = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += partials[static_cast<int64_t>(b) * NPART + p];
-  grad[p] = static_cast<float>(s);
-}
-
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                       float *__restrict__ v, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NPARAM) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  if (q < NPART)
+    for (int b = w0; b < nblk; b += kRed) s += partials[static_cast<int64_t>(b) * NPART + q];
+  part[w0][lane] = s;
+  __syncthreads();
+  if (w0 != 0 || q >= NPART) return;
+#pragma unroll
+  for (int k = 1; k < kRed; ++k) s += part[k][lane];
+  const float gi = static_cast<float>(s);
+  if (!ADAM) {
+    grad[q] = gi;
+    return;
+  }
+  if (q == NPARAM) {
+    *A.loss = gi;
+    return;
+  }
+  const float mi = A.b1 * A.m[q] + (1.0f - A.b1) * gi;
+  const float vi = A.b2 * A.v[q] + (1.0f - A.b2) * gi * gi;
+  A.m[q] = mi;
+  A.v[q] = vi;
+  const float w = A.p[q] - A.lr * (mi / A.c1) / (sqrtf(vi / A.c2) + A.eps);
+  A.p[q] = w;
+  if (q < OFF_B1) {
+    A.w1img[kmaj_off(q / NIN, q % NIN, K1) / 2] = bf16bits(w);
+  } else if (q >= OFF_W2 && q < OFF_B2) {
+    const int o = (q - OFF_W2) / NH, i = (q - OFF_W2) % NH;
+    A.w2img[kmaj_off(o, i, NH) / 2] = bf16bits(w);
+    A.w2timg[kmaj_off(i, o, NH) / 2] = bf16bits(w);
+  }
 }
 
 struct Mlp {
@@ -485,18 +516,22 @@ int check_err(Mlp *P) {
   return IMODEL_SWM_OK;
 }
 
+// one batch's gradient and loss sum into P->g or, with A, straight into an Adam
+// step and A->loss
 int run_grad(Mlp *P, const uint16_t *x, const float *t, const float *w, int64_t n, int64_t batch,
-             uint64_t seed,
-             int *nblk_out) {
+             uint64_t seed, const AdamArgs *A) {
   const int64_t ntiles = (batch + TM - 1) / TM;
-  const int nblk = static_cast<int>(std::min<int64_t>(ntiles, P->sms));
+  const int nblk = static_cast<int>(std::min<int64_t>(ntiles, TRN_CTAS * P->sms));
   k_mlp_train<<<nblk, TM, TRN_SMEM, P->stream>>>(weights(P), x, t, w, n, batch, seed,
                                                  1.0f / static_cast<float>(batch), P->partials,
                                                  P->d_err);
   MK(cudaGetLastError());
-  k_reduce<<<(NPART + 255) / 256, 256, 0, P->stream>>>(P->partials, nblk, P->g);
+  constexpr int blocks = (NPART + 31) / 32;
+  if (A)
+    k_reduce<true><<<blocks, 32 * kRed, 0, P->stream>>>(P->partials, nblk, nullptr, *A);
+  else
+    k_reduce<false><<<blocks, 32 * kRed, 0, P->stream>>>(P->partials, nblk, P->g, AdamArgs{});
   MK(cudaGetLastError());
-  *nblk_out = nblk;
   return IMODEL_SWM_OK;
 }
 
@@ -570,7 +605,8 @@ int imodel_mlp_create(int32_t device, void **mlp) {
   MK(cudaMalloc(&P->m, imodel::NPART * sizeof(float)));
   MK(cudaMalloc(&P->v, imodel::NPART * sizeof(float)));
   MK(cudaMalloc(&P->g, imodel::NPART * sizeof(float)));
-  MK(cudaMalloc(&P->partials, static_cast<size_t>(P->sms) * imodel::NPART * sizeof(float)));
+  MK(cudaMalloc(&P->partials, static_cast<size_t>(imodel::TRN_CTAS * P->sms) * imodel::NPART *
+                                  sizeof(float)));
   MK(cudaMalloc(&P->img, (imodel::NH * imodel::K1 + 2 * imodel::NH * imodel::NH) * 2));
   MK(cudaMalloc(&P->d_err, sizeof(int)));
   MK(cudaMemset(P->p, 0, imodel::NPART * sizeof(float)));
@@ -653,8 +689,7 @@ int imodel_mlp_grad(void *mlp, const uint16_t *x, const float *t, const float *w
                      P->stream));
   MK(cudaMemcpyAsync(dt, t, static_cast<size_t>(n) * sizeof(float), cudaMemcpyHostToDevice,
                      P->stream));
-  int nblk = 0;
-  int rc = imodel::run_grad(P, dx, dt, dwt, n, batch, seed, &nblk);
+  int rc = imodel::run_grad(P, dx, dt, dwt, n, batch, seed, nullptr);
   std::vector<float> g(imodel::NPART);
   if (!rc) {
     cudaError_t e = cudaMemcpyAsync(g.data(), P->g, imodel::NPART * sizeof(float),
@@ -713,18 +748,25 @@ int imodel_mlp_train(void *mlp, int64_t steps, int64_t batch, float lr, uint64_t
   MK(cudaMalloc(&dloss, static_cast<size_t>(steps) * sizeof(float)));
   int rc = IMODEL_SWM_OK;
   for (int64_t s = 0; s < steps && !rc; ++s) {
-    int nblk = 0;
-    rc = imodel::run_grad(P, P->dx, P->dt, P->dw, P->dn, batch,
-                          imodel::splitmix(seed + static_cast<uint64_t>(P->step)), &nblk);
-    if (rc) break;
+    const uint64_t draw = imodel::splitmix(seed + static_cast<uint64_t>(P->step));
     P->step += 1;
-    const float c1 = 1.0f - std::pow(b1, static_cast<float>(P->step));
-    const float c2 = 1.0f - std::pow(b2, static_cast<float>(P->step));
-    imodel::k_adam<<<(imodel::NPARAM + 255) / 256, 256, 0, P->stream>>>(P->p, P->g, P->m, P->v,
-                                                                        lr, b1, b2, eps, c1, c2);
-    cudaMemcpyAsync(dloss + s, P->g + imodel::NPARAM, sizeof(float), cudaMemcpyDeviceToDevice,
-                    P->stream);
-    rc = imodel::images(P);
+    const imodel::Weights W = imodel::weights(P);
+    imodel::AdamArgs A;
+    A.p = P->p;
+    A.m = P->m;
+    A.v = P->v;
+    A.loss = dloss + s;
+    A.w1img = const_cast<uint16_t *>(W.w1img);
+    A.w2img = const_cast<uint16_t *>(W.w2img);
+    A.w2timg = const_cast<uint16_t *>(W.w2timg);
+    A.lr = lr;
+    A.b1 = b1;
+    A.b2 = b2;
+    A.eps = eps;
+    A.c1 = 1.0f - std::pow(b1, static_cast<float>(P->step));
+    A.c2 = 1.0f - std::pow(b2, static_cast<float>(P->step));
+    rc = imodel::run_grad(P, P->dx, P->dt, P->dw, P->dn, batch, draw, &A);
+    if (rc) P->step -= 1;
   }
   if (!rc) {
     cudaError_t e = cudaMemcpyAsync(lossbuf.data(), dloss, static_cast<size_t>(steps) * sizeof(float),
