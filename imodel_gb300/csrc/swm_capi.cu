@@ -171,11 +171,24 @@ int upload_tiles(Handle *H, const Layout &L) {
   D.max_bytes = T.max_bytes;
   if (!fused_prepare(D)) return IMODEL_SWM_OK;
   const TileHead *head = nullptr;
-  const uint32_t *data = nullptr;
+  double *data = nullptr;
   int rc;
-  if ((rc = upload(H, T.head, &head)) || (rc = upload(H, T.data, &data))) return rc;
+  if ((rc = upload(H, T.head, &head)) || (rc = dalloc(H, &data, T.data_bytes / sizeof(double))))
+    return rc;
   D.head = reinterpret_cast<const int4 *>(head);
   D.data = reinterpret_cast<const uint4 *>(data);
+  // the lists are not kept (default stream, like the uploads before)
+  int32_t *lists = nullptr;
+  const size_t bytes = T.lists.size() * sizeof(int32_t);
+  CK(cudaMalloc(&lists, bytes));
+  cudaError_t e = cudaMemcpy(lists, T.lists.data(), bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    launch_fill_tiles(H->M, T.ntiles, D.head, lists, reinterpret_cast<uint4 *>(data), nullptr);
+    e = cudaGetLastError();
+  }
+  const cudaError_t f = cudaFree(lists);
+  CK(e);
+  CK(f);
   H->W32.tiles = D;
   H->ntiles = D.ntiles;
   return IMODEL_SWM_OK;

@@ -246,6 +246,9 @@ inline bool fused_stage(const Work<float> &W) {
          !W.learned;
 }
 int tile_cap(int nv);  // cells with flux terms per tile (threads per block) on a grid of nv cells
+// writes the tiles' blocks from their lists (swm_layout.h) and M's FP32 arrays
+void launch_fill_tiles(const DevMesh &M, int ntiles, const int4 *head, const int32_t *lists,
+                       uint4 *data, cudaStream_t s);
 // whether the fused stage's block fits an SM with these tiles; prepares the
 // kernel for its shared memory
 bool fused_prepare(const TileDev &T);

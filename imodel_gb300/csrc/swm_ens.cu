@@ -257,6 +257,41 @@ int zalloc(Ens *E, T **p, size_t n) {
   return IMODEL_SWM_OK;
 }
 
+// the tiles' blocks, from a copy of the layout's arrays that is not kept
+int fill_tiles(Ens *E, const Layout &L, const TileLayout &T, const int4 *head, uint4 *data) {
+  const size_t kept = E->allocs.size();
+  DevMesh M;
+  std::memset(&M, 0, sizeof(M));
+  M.nv = L.nv;
+  M.ne = L.ne;
+  M.nt = L.nt;
+  const std::vector<float> bt32(L.nv, 0.0f);
+  const int32_t *ra = nullptr, *rb = nullptr, *rc3 = nullptr, *pk = nullptr, *lists = nullptr;
+  const float *kd = nullptr;
+  const uint32_t *vs2 = nullptr;
+  int rc;
+  if ((rc = up(E, L.t_recA, &ra)) || (rc = up(E, L.t_recB, &rb)) || (rc = up(E, L.t_recC, &rc3)) ||
+      (rc = up(E, L.t_f32, &M.t_f32)) || (rc = up(E, L.c_meta, &M.c_meta)) ||
+      (rc = up(E, L.c_inva32, &M.c_inva32)) || (rc = up(E, bt32, &M.c_bt32)) ||
+      (rc = up(E, L.e_grad32, &M.e_grad32)) || (rc = up(E, L.c_pk, &pk)) ||
+      (rc = up(E, L.c_kd, &kd)) || (rc = up(E, L.e_vs2, &vs2)) || (rc = up(E, T.lists, &lists)))
+    return rc;
+  M.t_recA = reinterpret_cast<const int4 *>(ra);
+  M.t_recB = reinterpret_cast<const int4 *>(rb);
+  M.t_recC = reinterpret_cast<const float4 *>(rc3);
+  M.c_pk = reinterpret_cast<const int4 *>(pk);
+  M.c_kd = reinterpret_cast<const float2 *>(kd);
+  M.e_vs2 = reinterpret_cast<const uint2 *>(vs2);
+  launch_fill_tiles(M, T.ntiles, head, lists, data, nullptr);
+  EK(cudaGetLastError());
+  EK(cudaStreamSynchronize(nullptr));
+  while (E->allocs.size() > kept) {
+    EK(cudaFree(E->allocs.back()));
+    E->allocs.pop_back();
+  }
+  return IMODEL_SWM_OK;
+}
+
 int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t *members) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
@@ -304,13 +339,14 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
     D.cap = T.cap;
     D.ntiles = T.ntiles;
     const TileHead *head = nullptr;
-    const uint32_t *data = nullptr;
+    uint4 *data = nullptr;
     const int32_t *cn2o = nullptr, *en2o = nullptr;
-    if ((rc = up(E, T.head, &head)) || (rc = up(E, T.data, &data)) ||
+    if ((rc = up(E, T.head, &head)) || (rc = zalloc(E, &data, T.data_bytes / sizeof(uint4))) ||
         (rc = up(E, L.cell_n2o, &cn2o)) || (rc = up(E, L.edge_n2o, &en2o)))
       return rc;
     D.head = reinterpret_cast<const int4 *>(head);
-    D.data = reinterpret_cast<const uint4 *>(data);
+    D.data = data;
+    if ((rc = fill_tiles(E, L, T, D.head, data))) return rc;
     G.cell_n2o = const_cast<int32_t *>(cn2o);
     G.edge_n2o = const_cast<int32_t *>(en2o);
     EnsArgs &A = E->args;

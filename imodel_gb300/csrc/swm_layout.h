@@ -262,13 +262,17 @@ struct TileHead {
   int32_t bt;      // [nz] topography
   int32_t inva;    // [nc] 1 / (A erad)
   int32_t bytes;
-  int32_t pad;
+  int32_t lists;   // where the tile's lists begin in TileLayout::lists
 };
 struct TileLayout {
   int cap = 0, ntiles = 0;
   int max_h = 0, max_u = 0, max_t = 0, max_bytes = 0;  // over the tiles
-  HVec<TileHead> head;  // [ntiles]
-  HVec<uint32_t> data;  // the blocks
+  size_t data_bytes = 0;  // of all blocks
+  HVec<TileHead> head;    // [ntiles]
+  // per tile the device indices of its other depths (the ring cells, then the
+  // rest), other edges and triangles, each ascending; from them
+  // launch_fill_tiles writes the blocks on the GPU
+  HVec<int32_t> lists;
 };
 // Cuts a trsk10 layout into tiles of at most cap cells with flux terms; false
 // when a tile has 1024 or more of something (the caller then does without).

@@ -73,6 +73,84 @@ __global__ void __launch_bounds__(kThr, kThr == 256 ? 3 : 4)
   tile_edges(T, S, F, own, kStage, dt, erad, mom_on);
 }
 
+// ---- the tiles' blocks -------------------------------------------------------
+// position of k in the ascending list v[n], which holds it
+__device__ __forceinline__ int place(const int32_t *v, int n, int k) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (v[mid] < k)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(256) k_fill_tiles(DevMesh M, const int4 *head,
+                                                    const int32_t *lists, unsigned char *data) {
+  // the lists (below 1024 entries each): ring cells and other depths, other
+  // edges, triangles
+  __shared__ int32_t lh[1024], lu[1024], lt[1024];
+  const Tile T(head + 5 * blockIdx.x);
+  const int nhx = T.nh - T.nc, nux = T.nu - T.ne, nring = T.nz - T.nc;
+  const int32_t *src = lists + __ldg(&head[5 * blockIdx.x + 4].w);
+  unsigned char *block = data + 16 * static_cast<size_t>(T.block);
+  int32_t *hx = reinterpret_cast<int32_t *>(block);
+  int32_t *ux = reinterpret_cast<int32_t *>(block + T.ux);
+  for (int k = threadIdx.x; k < nhx; k += blockDim.x) hx[k] = lh[k] = src[k];
+  for (int k = threadIdx.x; k < nux; k += blockDim.x) ux[k] = lu[k] = src[nhx + k];
+  for (int k = threadIdx.x; k < T.nt; k += blockDim.x) lt[k] = src[nhx + nux + k];
+  __syncthreads();
+  // local numbers: depths own, ring, others; edges own, others
+  auto cell = [&](int c) -> uint32_t {
+    if (c >= T.c0 && c < T.c0 + T.nc) return c - T.c0;
+    const int r = place(lh, nring, c);
+    if (r < nring && lh[r] == c) return T.nc + r;
+    return T.nz + place(lh + nring, nhx - nring, c);
+  };
+  auto edge = [&](int e) -> uint32_t {
+    return e >= T.e0 && e < T.e0 + T.ne ? e - T.e0 : T.ne + place(lu, nux, e);
+  };
+  uint4 *ta = reinterpret_cast<uint4 *>(block + T.triA);
+  uint4 *tb = reinterpret_cast<uint4 *>(block + T.triB);
+  uint32_t *tc = reinterpret_cast<uint32_t *>(block + T.triC);
+  for (int k = threadIdx.x; k < T.nt; k += blockDim.x) {
+    const int t = lt[k];
+    const int4 a = M.t_recA[t], b = M.t_recB[t];
+    const float4 c = M.t_recC[t];
+    ta[k] = make_uint4(b.z, b.w, __float_as_uint(c.x), __float_as_uint(M.t_f32[t]));
+    tb[k] = make_uint4(__float_as_uint(c.y), __float_as_uint(c.z), __float_as_uint(c.w),
+                       edge(a.x) | edge(a.y) << 10 | edge(a.z) << 20);
+    tc[k] = cell(a.w) | cell(b.x) << 10 | cell(b.y) << 20;
+  }
+  uint4 *slot = reinterpret_cast<uint4 *>(block + T.slot);
+  uint32_t *meta = reinterpret_cast<uint32_t *>(block + T.meta);
+  float *bt = reinterpret_cast<float *>(block + T.bt);
+  float *inva = reinterpret_cast<float *>(block + T.inva);
+  for (int z = threadIdx.x; z < T.nz; z += blockDim.x) {
+    const int c = z < T.nc ? T.c0 + z : lh[z - T.nc];
+    meta[z] = M.c_meta[c];
+    bt[z] = M.c_bt32[c];
+    if (z < T.nc) inva[z] = M.c_inva32[c];
+    for (int j = 0; j < 6; ++j) {
+      // {edge, neighbour, triangle, kite fraction}, {KE weight, ttgout d};
+      // unused slots repeat slot 0 with zero weights
+      const int4 pk = M.c_pk[j * M.nv + c];
+      const float2 kd = M.c_kd[j * M.nv + c];
+      slot[j * T.nz + z] = make_uint4(edge(pk.x) | cell(pk.y) << 10 | place(lt, T.nt, pk.z) << 20,
+                                      pk.w, __float_as_uint(kd.x), __float_as_uint(kd.y));
+    }
+  }
+  uint2 *ed = reinterpret_cast<uint2 *>(block + T.edge);
+  for (int k = threadIdx.x; k < T.ne; k += blockDim.x) {
+    const uint2 w = M.e_vs2[T.e0 + k];  // cell | slot << 28 of both cells
+    ed[k] = make_uint2(cell(w.x & 0x0FFFFFFF) | (w.x >> 28) << 10 | cell(w.y & 0x0FFFFFFF) << 13 |
+                           (w.y >> 28) << 23,
+                       __float_as_uint(M.e_grad32[T.e0 + k]));
+  }
+}
+
 size_t fused_smem(const TileDev &T) {
   return static_cast<size_t>(T.max_bytes) +
          sizeof(float) * (static_cast<size_t>(T.max_h) + T.max_u + T.max_t + T.cap);
@@ -105,6 +183,12 @@ inline Stage32 stage_kernel(const TileDev &T, int stage) {
   return threads(T) == 192 ? stage_kernel<192>(stage) : stage_kernel<256>(stage);
 }
 }  // namespace
+
+void launch_fill_tiles(const DevMesh &M, int ntiles, const int4 *head, const int32_t *lists,
+                       uint4 *data, cudaStream_t s) {
+  if (ntiles > 0)
+    k_fill_tiles<<<ntiles, 256, 0, s>>>(M, head, lists, reinterpret_cast<unsigned char *>(data));
+}
 
 bool fused_prepare(const TileDev &T) {
   constexpr int kMost = 227 * 1024 - 1024;

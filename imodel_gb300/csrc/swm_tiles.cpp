@@ -12,35 +12,32 @@
 namespace imodel {
 namespace {
 
-// Local numbers of one tile's entities, by device index: a value per index,
-// forgotten when the tile changes.  The memory is mapped zeroed and touched
-// only around the tiles that a thread works on.
-class LocalNumbers {
+// A set of entities by device index, emptied by a new tag.  The memory is
+// mapped zeroed and touched only around the tiles that a thread works on.
+class Marks {
  public:
-  explicit LocalNumbers(size_t n)
-      : v_(static_cast<uint64_t *>(std::calloc(n ? n : 1, sizeof(uint64_t)))) {}
-  ~LocalNumbers() { std::free(v_); }
-  LocalNumbers(const LocalNumbers &) = delete;
+  explicit Marks(size_t n)
+      : v_(static_cast<int32_t *>(std::calloc(n ? n : 1, sizeof(int32_t)))) {}
+  ~Marks() { std::free(v_); }
+  Marks(const Marks &) = delete;
   bool valid() const { return v_ != nullptr; }
-  void start(int tile) { tag_ = static_cast<uint64_t>(tile) + 1; }
-  bool has(int32_t k) const { return v_[k] >> 32 == tag_; }
-  void set(int32_t k, uint32_t local) { v_[k] = tag_ << 32 | local; }
+  void start(int tag) { tag_ = tag + 1; }
+  bool has(int32_t k) const { return v_[k] == tag_; }
   // true when k was not there
   bool add(int32_t k) {
     if (has(k)) return false;
-    set(k, 0);
+    v_[k] = tag_;
     return true;
   }
-  uint32_t operator[](int32_t k) const { return static_cast<uint32_t>(v_[k]); }
 
  private:
-  uint64_t *v_;
-  uint64_t tag_ = 0;
+  int32_t *v_;
+  int32_t tag_ = 0;
 };
 
 // cells whose flux terms a tile of the cells [c0, c1) needs: its own and the
 // higher-numbered neighbours; the last c1 <= end with at most cap of them
-int tile_end(const Layout &L, int c0, int end, int cap, LocalNumbers &ring) {
+int tile_end(const Layout &L, int c0, int end, int cap, Marks &ring) {
   const size_t NV = L.nv;
   ring.start(c0);
   int above = 0;  // ring cells >= c1
@@ -90,7 +87,7 @@ bool build_tiles(const Layout &L, int cap, TileLayout &T) {
   bool ok = true;
 #pragma omp parallel reduction(&& : ok) reduction(|| : oom)
   {
-    LocalNumbers ring(NV);
+    Marks ring(NV);
     oom = !ring.valid();
 #pragma omp for schedule(static)
     for (int s = 0; s < nseg; ++s) {
@@ -119,11 +116,11 @@ bool build_tiles(const Layout &L, int cap, TileLayout &T) {
   start.push_back(L.nv);
   T.ntiles = nt;
   T.head.resize(static_cast<size_t>(nt));
-  // pass 1: the lists of every tile; pass 2: their places; pass 3: the records
+  // the lists of every tile, then their places
   std::vector<TileLists> lists(nt);
 #pragma omp parallel reduction(&& : ok) reduction(|| : oom)
   {
-    LocalNumbers cells(NV), edges(NE), tris(NT);
+    Marks cells(NV), edges(NE), tris(NT);
     oom = !cells.valid() || !edges.valid() || !tris.valid();
 #pragma omp for schedule(static)
     for (int b = 0; b < nt; ++b) {
@@ -195,96 +192,28 @@ bool build_tiles(const Layout &L, int cap, TileLayout &T) {
   }
   if (oom) throw std::bad_alloc();
   if (!ok) return false;
-  size_t bytes = 0;
+  size_t bytes = 0, nlists = 0;
   for (TileHead &H : T.head) {
-    if (bytes / 16 > INT32_MAX) return false;
+    if (bytes / 16 > INT32_MAX || nlists > INT32_MAX) return false;
     H.block = static_cast<int32_t>(bytes / 16);
+    H.lists = static_cast<int32_t>(nlists);
     bytes += H.bytes;
+    nlists += (H.nh - H.nc) + (H.nu - H.ne) + H.nt;
     T.max_h = std::max(T.max_h, H.nh);
     T.max_u = std::max(T.max_u, H.nu);
     T.max_t = std::max(T.max_t, H.nt);
     T.max_bytes = std::max(T.max_bytes, H.bytes);
   }
-  T.data.resize(bytes / 4);
-  auto bits = [](float f) {
-    uint32_t v;
-    std::memcpy(&v, &f, sizeof(v));
-    return v;
-  };
-#pragma omp parallel reduction(|| : oom)
-  {
-    LocalNumbers cells(NV), edges(NE), tris(NT);
-    oom = !cells.valid() || !edges.valid() || !tris.valid();
-#pragma omp for schedule(static)
-    for (int b = 0; b < nt; ++b) {
-      if (oom) continue;
-      const TileHead &H = T.head[b];
-      const TileLists &Q = lists[b];
-      cells.start(b);
-      edges.start(b);
-      tris.start(b);
-      uint32_t *base = T.data.data() + 4 * static_cast<size_t>(H.block);
-      std::memset(base, 0, H.bytes);
-      auto part = [&](int off) { return base + off / 4; };
-      // local numbers: depths own, ring, others; edges own, others
-      for (int k = 0; k < H.nc; ++k) cells.set(H.c0 + k, k);
-      int n = H.nc;
-      for (const std::vector<int32_t> *list : {&Q.z, &Q.hx})
-        for (int c : *list) {
-          part(0)[n - H.nc] = static_cast<uint32_t>(c);
-          cells.set(c, n++);
-        }
-      for (int k = 0; k < H.ne; ++k) edges.set(H.e0 + k, k);
-      n = H.ne;
-      for (int e : Q.ux) {
-        part(H.ux)[n - H.ne] = static_cast<uint32_t>(e);
-        edges.set(e, n++);
-      }
-      n = 0;
-      for (int t : Q.tri) tris.set(t, n++);
-      for (int k = 0; k < H.nt; ++k) {
-        const int t = Q.tri[k];
-        uint32_t *A = part(H.triA) + 4 * k, *B = part(H.triB) + 4 * k;
-        uint32_t ie = 0, iv = 0;
-        for (int s = 0; s < 3; ++s) {
-          ie |= edges[L.t_ed[s * NT + t]] << (10 * s);
-          iv |= cells[L.t_v[s * NT + t]] << (10 * s);
-          A[s] = bits(L.t_circ32[s * NT + t]);
-          B[s] = bits(L.t_kite32[s * NT + t]);
-        }
-        A[3] = bits(L.t_f32[t]);
-        B[3] = ie;
-        part(H.triC)[k] = iv;
-      }
-      for (int z = 0; z < H.nz; ++z) {
-        const int c = z < H.nc ? H.c0 + z : Q.z[z - H.nc];
-        part(H.meta)[z] = L.c_meta[c];
-        part(H.bt)[z] = bits(static_cast<float>(L.c_bt[c]));
-        if (z < H.nc) part(H.inva)[z] = bits(L.c_inva32[c]);
-        for (int j = 0; j < kMaxNb; ++j) {
-          // c_pk: {edge, neighbour, triangle, kite fraction}; c_kd: {KE
-          // weight, ttgout d}; unused slots repeat slot 0 with zero weights
-          const size_t src = j * NV + c;
-          uint32_t *q = part(H.slot) + 4 * (j * H.nz + z);
-          q[0] = edges[L.c_pk[4 * src]] | cells[L.c_pk[4 * src + 1]] << 10 |
-                 tris[L.c_pk[4 * src + 2]] << 20;
-          q[1] = static_cast<uint32_t>(L.c_pk[4 * src + 3]);
-          q[2] = bits(L.c_kd[2 * src]);
-          q[3] = bits(L.c_kd[2 * src + 1]);
-        }
-      }
-      for (int k = 0; k < H.ne; ++k) {
-        const size_t e = H.e0 + k;
-        const uint32_t w1 = L.e_vs[e], w2 = L.e_vs[NE + e];
-        const uint32_t z1 = cells[static_cast<int32_t>(w1 & 0x0FFFFFFFu)];
-        const uint32_t z2 = cells[static_cast<int32_t>(w2 & 0x0FFFFFFFu)];
-        uint32_t *q = part(H.edge) + 2 * k;
-        q[0] = z1 | (w1 >> 28) << 10 | z2 << 13 | (w2 >> 28) << 23;
-        q[1] = bits(L.e_grad32[e]);
-      }
+  T.data_bytes = bytes;
+  T.lists.resize(nlists);
+#pragma omp parallel for schedule(static)
+  for (int b = 0; b < nt; ++b) {
+    int32_t *p = T.lists.data() + T.head[b].lists;
+    for (const std::vector<int32_t> *v : {&lists[b].z, &lists[b].hx, &lists[b].ux, &lists[b].tri}) {
+      std::copy(v->begin(), v->end(), p);
+      p += v->size();
     }
   }
-  if (oom) throw std::bad_alloc();
   return true;
 }
 
