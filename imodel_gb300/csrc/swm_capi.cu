@@ -67,7 +67,7 @@ struct Handle {
   // kite fractions and weights (reference layout) for export
   struct WeightSet {
     const double *e_stw = nullptr;
-    const float *e_stc32 = nullptr, *c_R32 = nullptr;
+    const float *e_stc32 = nullptr;
     const int4 *c_pk = nullptr;
   } w_learned, w_plain;
   imodel::HVec<double> kite_hxtr, kite_trskw;
@@ -200,11 +200,10 @@ int alloc_work(Handle *H, Work<T> &W) {
   T **bufs_v[] = {&W.yn_h, &W.ya_h, &W.yb_h, &W.acc_h, &W.bern, &W.tend_h};
   for (T **b : bufs_v)
     if ((rc = dalloc(H, b, H->nv))) return rc;
-  T **bufs_e[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u, &W.h_ed, &W.uh, &W.q_ed, &W.tend_u};
-  constexpr bool fp64 = sizeof(T) == sizeof(double);
+  T **bufs_e[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u, &W.uh, &W.q_ed, &W.tend_u};
   for (T **b : bufs_e)
-    if (!(fp64 && b == &W.h_ed) && (rc = dalloc(H, b, H->ne))) return rc;
-  if (fp64 && (rc = dalloc(H, &W.fe, H->ne))) return rc;
+    if ((rc = dalloc(H, b, H->ne))) return rc;
+  if (sizeof(T) == sizeof(double) && (rc = dalloc(H, &W.fe, H->ne))) return rc;
   if ((rc = dalloc(H, &W.q_tr, H->nt))) return rc;
   W.flags = H->d_flags;
   W.pv_on = H->testcase >= 2 ? 1 : 0;
@@ -281,7 +280,7 @@ void *host_view(Handle *H, const void *p, size_t bytes) {
   return static_cast<char *>(a.devicePointer);
 }
 
-// host FP64 arrays (reference order) -> device state yn, plus h_ed and the
+// host FP64 arrays (reference order) -> device state yn and the
 // "last stage input" ya, as after the reference's initial tendency call
 // (swm.f90:214)
 int learned_guard(Handle *H, bool *tripped = nullptr, int steps = 0);
@@ -297,7 +296,6 @@ void learned_switch(Handle *H, bool on) {
     const Handle::WeightSet &w = on ? H->w_learned : H->w_plain;
     H->M.e_stw = w.e_stw;
     H->M.e_stc32 = w.e_stc32;
-    H->M.c_R32 = w.c_R32;
     H->M.c_pk = w.c_pk;
     // the tiles hold the learned fractions: the plain scheme takes variant
     // 1's three kernels
@@ -514,7 +512,6 @@ int error_proxy(Handle *H, int steps, bool *trip) {
   if (H->learned_mode == 2) {
     Mp.e_stw = H->w_plain.e_stw;
     Mp.e_stc32 = H->w_plain.e_stc32;
-    Mp.c_R32 = H->w_plain.c_R32;
     Mp.c_pk = H->w_plain.c_pk;
     Wp.tiles.ntiles = 0;
   } else {
@@ -799,10 +796,8 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
     if ((rc = upload(H, L.c_div32, &M.c_div32)) || (rc = upload(H, L.c_kew32, &M.c_kew32)) ||
         (rc = upload(H, bt32, &M.c_bt32)) || (rc = upload(H, L.e_grad32, &M.e_grad32)) ||
         (rc = upload(H, L.e_stc32, &M.e_stc32)) || (rc = upload(H, L.t_f32, &M.t_f32)) ||
-        (rc = upload(H, L.c_nb, &M.c_nb)) || (rc = upload(H, L.c_tr, &M.c_tr)) ||
-        (rc = upload(H, L.c_R32, &M.c_R32)) || (rc = upload(H, L.c_dg32, &M.c_dg32)) ||
-        (rc = upload(H, L.c_inva32, &M.c_inva32)) || (rc = upload(H, L.c_meta, &M.c_meta)) ||
-        (rc = upload(H, L.e_vs, &M.e_vs)))
+        (rc = upload(H, L.c_nb, &M.c_nb)) || (rc = upload(H, L.c_inva32, &M.c_inva32)) ||
+        (rc = upload(H, L.c_meta, &M.c_meta)))
       return rc;
     const int32_t *ra = nullptr, *rb = nullptr, *rc32 = nullptr;
     if ((rc = upload(H, L.t_recA, &ra)) || (rc = upload(H, L.t_recB, &rb)) ||
@@ -859,10 +854,14 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
   if (H->precision == IMODEL_SWM_FP32 &&
       ((rc = upload(H, L.e_qw32, &M.e_qw32)) || (rc = upload(H, L.e_dtc32, &M.e_dtc32))))
     return rc;
-  if (H->precision == IMODEL_SWM_FP32 && !L.t_apw32.empty()) {
-    if ((rc = upload(H, L.t_apw32, &M.t_apw32)) || (rc = upload(H, L.t_cc32, &M.t_cc32)) ||
+  if (H->precision == IMODEL_SWM_FP32 && !L.t_ap32.empty()) {
+    const float *ap = nullptr;
+    const int32_t *across = nullptr;
+    if ((rc = upload(H, L.t_ap32, &ap)) || (rc = upload(H, L.t_across, &across)) ||
         (rc = upload(H, L.c_apw32, &M.c_apw32)) || (rc = upload(H, L.c_p32, &M.c_p32)))
       return rc;
+    M.t_ap32 = reinterpret_cast<const float4 *>(ap);
+    M.t_across = reinterpret_cast<const int4 *>(across);
   }
   if (H->precision == IMODEL_SWM_FP64) {
     // the FP64 kernels' derived constants, formed on the GPU
@@ -922,7 +921,7 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
     if (o && o->learned == 1 && (rc = setup_learned(H, m, L, o))) return rc;
   }
   if (H->learned_mode == 2) {
-    H->w_learned = {M.e_stw, M.e_stc32, M.c_R32, M.c_pk};
+    H->w_learned = {M.e_stw, M.e_stc32, M.c_pk};
     if (H->precision == IMODEL_SWM_FP32) {
       // the guard's fallback: the plain scheme's weight-dependent arrays
       WeightArrays Lp;
@@ -931,7 +930,7 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
       const int32_t *pk = nullptr;
       if ((rc = upload(H, Lp.e_stw, &H->w_plain.e_stw)) ||
           (rc = upload(H, Lp.e_stc32, &H->w_plain.e_stc32)) ||
-          (rc = upload(H, Lp.c_R32, &H->w_plain.c_R32)) || (rc = upload(H, Lp.c_pk, &pk)))
+          (rc = upload(H, Lp.c_pk, &pk)))
         return rc;
       H->w_plain.c_pk = reinterpret_cast<const int4 *>(pk);
       if ((rc = dalloc(H, &H->ck_h, static_cast<size_t>(L.nv))) ||
@@ -1030,8 +1029,9 @@ int setup_apvm(Handle *H, Work<T> &W, double pvspar, double dt) {
   A.on = false;
   if (!(pvspar > 0)) return IMODEL_SWM_OK;
   int rc;
-  if ((!A.qg && (rc = dalloc(H, &A.qg, 3 * static_cast<size_t>(H->nt)))) ||
-      (!A.vhx && (rc = dalloc(H, &A.vhx, 3 * static_cast<size_t>(H->nv)))) ||
+  const size_t k = sizeof(T) == sizeof(float) ? 4 : 3;
+  if ((!A.qg && (rc = dalloc(H, &A.qg, k * static_cast<size_t>(H->nt)))) ||
+      (!A.vhx && (rc = dalloc(H, &A.vhx, k * static_cast<size_t>(H->nv)))) ||
       (!A.qge && (rc = dalloc(H, &A.qge, static_cast<size_t>(H->ne)))))
     return rc;
   A.coef = static_cast<T>(pvspar * dt);
@@ -1521,7 +1521,7 @@ int imodel_swm_set_apvm(void *handle, double pvspar, double dt) {
   if (pvspar > 0 && (!(dt > 0) || !std::isfinite(dt)))
     return imodel::set_error(H, IMODEL_SWM_EINVAL, "apvm needs a finite dt > 0");
   const bool fp32 = H->precision == IMODEL_SWM_FP32;
-  if (pvspar > 0 && !(fp32 ? H->M.t_apw32 != nullptr : H->M.t_c != nullptr))
+  if (pvspar > 0 && !(fp32 ? H->M.t_ap32 != nullptr : H->M.t_c != nullptr))
     return imodel::set_error(H, IMODEL_SWM_EINVAL, "apvm needs the mesh's ed_nr and ed_c");
   if (cudaSetDevice(H->device) != cudaSuccess) return IMODEL_SWM_ECUDA;
   // FP32: the correction is applied in the edge pre-pass, which variants 1

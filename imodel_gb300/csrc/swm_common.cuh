@@ -31,10 +31,10 @@ struct DevMesh {
   const int4 *t_recA, *t_recB;  // [nt] packed triangle records (swm_layout.h)
   const float4 *t_recC;
   // cell-centred TRSK variant (FP32)
-  const int32_t *c_nb, *c_tr;
-  const float *c_R32, *c_dg32, *c_inva32;
+  const int32_t *c_nb;
+  const float *c_inva32;
   const float *c_area32, *e_area32;  // A_i and l_e d_e / 2 in FP32 (drift check)
-  const uint32_t *c_meta, *e_vs;
+  const uint32_t *c_meta;
   const int4 *c_pk;     // [6][nv] {edge, neighbour, triangle, kite fraction bits}
   const float2 *c_kd;   // [6][nv] {KE weight, ttgout*d}
   const uint2 *e_vs2;   // [ne] both cell words of an edge
@@ -50,7 +50,9 @@ struct DevMesh {
   // ed%nr): ed%c%p, tr%c%p (circumcentre), v%p
   const double *e_c, *t_c, *c_p;
   // the FP32 step's APVM weights and projection vectors (swm_layout.h)
-  const float *t_apw32, *t_cc32, *c_apw32, *c_p32;
+  const float4 *t_ap32;   // [3][nt]
+  const int4 *t_across;   // [nt]
+  const float *c_apw32, *c_p32;
   // geometry of the pxt16, gass18 and dtred method wrappers (FP64, NULL
   // for trsk10; swm_layout.h): barycentric weights [3][nt], circumcentre
   // distances [2][ne], edge areas [3][nt], connecting edges [10][ne], ed%nr
@@ -186,8 +188,10 @@ template <class T>
 struct Apvm {
   bool on = false;
   T coef = T(0);          // pvspar * dt
-  T *qg = nullptr;        // [3][nt] Perot reconstruction of grad_tr2ed(q_tr)
-  T *vhx = nullptr;       // [3][nv] Perot reconstruction of u at the cells
+  // Perot reconstructions of grad_tr2ed(q_tr) at the triangles and of u at
+  // the cells: [3][n] in FP64, [n][4] in FP32
+  T *qg = nullptr;
+  T *vhx = nullptr;
   T *qge = nullptr;       // [ne] grad_tr2ed(q_tr) (FP64 step)
 };
 
@@ -200,7 +204,7 @@ struct Work {
   T *yb_h, *yb_u;    // stage inputs (pong)
   T *acc_h, *acc_u;  // k0 + 2 k1 + 2 k2
   T *q_tr;           // [nt] potential vorticity at triangles
-  T *h_ed, *uh, *q_ed;  // [ne]; FP64: uh and q_ed hold 2 u h_e and 2 q_e, h_ed is not used
+  T *uh, *q_ed;      // [ne]; FP64: 2 u h_e and 2 q_e
   double2 *fe = nullptr;  // [ne] FP64: 2 u h_e d and the edge's kinetic-energy term
   T *bern;           // [nv] g (h + b) + K
   T *tend_h, *tend_u;   // tendency outputs (tendency-only evaluations)
@@ -279,7 +283,10 @@ inline int launches_per_stage(int precision_fp32, int variant, bool dif_on = fal
   // FP64: triangles + edge fluxes, cells + edge PV, edges
   int n = (precision_fp32 && variant == 0) ? 4 : 3;
   if (!precision_fp32 && scheme == 3) n += 1;  // dtred: the triangle reconstruction of uh q
-  if (dif_on) n += (dif_k4 ? 3 : 1) + ((precision_fp32 && variant == 0) ? 1 : 0);
+  // (the last gradients are formed in k_edge32v2)
+  const bool in_edge = precision_fp32 && variant >= 1 && scheme != 3;
+  if (dif_on)
+    n += (dif_k4 ? 3 : 1) - (in_edge ? 1 : 0) + ((precision_fp32 && variant == 0) ? 1 : 0);
   // FP32 variants 1 and 2: the edge pre-pass for APVM's or gass18's edge PV
   if (precision_fp32 && variant >= 1 && (apvm_on || scheme == 2)) n += 1;
   // the reconstructions

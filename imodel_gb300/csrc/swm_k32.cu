@@ -25,30 +25,31 @@ __global__ void __launch_bounds__(512) k_tri32(DevMesh M, const float *__restric
   tri_body<Wait>(M, t, hd, u, q_tr, h_ref, pv_on, flags, kt, coefvort, ht_out);
 }
 
-// h_e (deviation), flux F_e = u_e (h_ref + h_e), q_e: the TRSK average
+// flux F_e = u_e (h_ref + h_e), q_e: the TRSK average
 // (scalar_tr2ed), the circumcentre-distance weights of pxt16 (qw) or
 // gass18's rhombus PV (qw and the triangle depths ht: (w1 eta1 + w2 eta2) /
 // (w1 h1 + w2 h2), eta = q h, with scalar_elem_divide's guard)
 __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__restrict__ hd,
                                                     const float *__restrict__ u,
                                                     const float *__restrict__ q_tr,
-                                                    float *__restrict__ h_ed,
                                                     float *__restrict__ uh,
                                                     float *__restrict__ q_ed, float h_ref,
-                                                    const float *__restrict__ qg,
-                                                    const float *__restrict__ vhx,
+                                                    const float4 *__restrict__ qg,
+                                                    const float4 *__restrict__ vhx,
                                                     float coef,
                                                     const float *__restrict__ qw,
                                                     const float *__restrict__ ht, int pv_on,
                                                     int *flags) {
-  after_prior<true>(hd, u, q_tr, h_ed, uh, q_ed, qg, vhx, ht);
+  after_prior<true>(hd, u, q_tr, uh, q_ed, qg, vhx, ht);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
   const int c1 = __ldg(&M.e_v[e]), c2 = __ldg(&M.e_v[ne + e]);
-  const float he = 0.5f * (hd[c1] + hd[c2]);
-  h_ed[e] = he;
-  uh[e] = u[e] * (h_ref + he);
+  // the cell-centred variants form the flux in their cell kernel (uh NULL)
+  if (uh) {
+    const float he = 0.5f * (hd[c1] + hd[c2]);
+    uh[e] = u[e] * (h_ref + he);
+  }
   const int t1 = __ldg(&M.e_sh[e]), t2 = __ldg(&M.e_sh[ne + e]);
   float q;
   if (!qw) {
@@ -69,12 +70,9 @@ __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__re
   }
   if (qg) {
     // apvm (swm_operators.f90:1495-1502), coef = pvspar dt
-    const int nt = M.nt, nv = M.nv;
-    float d = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      d += (qg[k * nt + t1] + qg[k * nt + t2]) * (vhx[k * nv + c1] + vhx[k * nv + c2]);
-    q -= coef * d;
+    const float4 a1 = qg[t1], a2 = qg[t2], b1 = vhx[c1], b2 = vhx[c2];
+    q -= coef * ((a1.x + a2.x) * (b1.x + b2.x) + (a1.y + a2.y) * (b1.y + b2.y) +
+                 (a1.z + a2.z) * (b1.z + b2.z));
   }
   q_ed[e] = q;
 }
@@ -83,53 +81,61 @@ __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__re
 // (swm_layout.h): blocks [0, nbt) the PV gradient at the triangles,
 // vector_edtr2tr_perot (:408-452) of grad_tr2ed(q_tr) (:1427-1463); the
 // blocks after the velocity at the cells, vector_edhx2hx_perot (:454-509);
-// each then projected on the tangent plane of its unit point.
+// each then projected on the tangent plane of its unit point.  Bound by HBM
+// and the gathers: a triangle reads 64 B of records in four wide loads and the
+// PV across its three edges (it went through the edges' records for them, two
+// more dependent loads), and the vectors are written as 16-byte records, one
+// gather each for the edges.
 __global__ void __launch_bounds__(256) k_apvm32(DevMesh M, const float *__restrict__ q_tr,
                                                 const float *__restrict__ u,
-                                                float *__restrict__ qg,
-                                                float *__restrict__ vhx, int nbt) {
-  after_prior<true>(q_tr, u, qg, vhx);
-  const int ne = M.ne;
+                                                float4 *__restrict__ qg,
+                                                float4 *__restrict__ vhx, int nbt) {
   float v[3] = {0.0f, 0.0f, 0.0f}, p[3];
-  int n, i, stride;
-  float *out;
+  int i;
+  float4 *out;
   if (static_cast<int>(blockIdx.x) < nbt) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int nt = M.nt;
     if (t >= nt) return;
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-      const int ed = __ldg(&M.t_ed[s * nt + t]);
-      const float g = __ldg(&M.e_gtg32[ed]) *
-                      (q_tr[__ldg(&M.e_sh[ne + ed])] - q_tr[__ldg(&M.e_sh[ed])]);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) v[k] = fmaf(g, __ldg(&M.t_apw32[(3 * s + k) * nt + t]), v[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) p[k] = __ldg(&M.t_cc32[k * nt + t]);
+    const int4 nb = __ldg(&M.t_across[t]);
+    const float4 a = __ldg(&M.t_ap32[t]), b = __ldg(&M.t_ap32[nt + t]),
+                 c = __ldg(&M.t_ap32[2 * nt + t]);
+    after_prior<true>(q_tr, u, qg, vhx);
+    const float q = q_tr[t], g0 = q_tr[nb.x] - q, g1 = q_tr[nb.y] - q, g2 = q_tr[nb.z] - q;
+    v[0] = fmaf(g2, b.z, fmaf(g1, a.w, __fmul_rn(g0, a.x)));
+    v[1] = fmaf(g2, b.w, fmaf(g1, b.x, __fmul_rn(g0, a.y)));
+    v[2] = fmaf(g2, c.x, fmaf(g1, b.y, __fmul_rn(g0, a.z)));
+    p[0] = c.y;
+    p[1] = c.z;
+    p[2] = c.w;
     i = t;
-    stride = nt;
     out = qg;
   } else {
     const int c = (blockIdx.x - nbt) * blockDim.x + threadIdx.x;
     const int nv = M.nv;
     if (c >= nv) return;
-    n = M.c_nnb[c];
-    for (int j = 0; j < n; ++j) {
-      const float ue = u[__ldg(&M.c_ed[j * nv + c])];
+    const int n = M.c_nnb[c];
+    int ed[6];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) v[k] = fmaf(ue, __ldg(&M.c_apw32[(3 * j + k) * nv + c]), v[k]);
-    }
+    for (int j = 0; j < 6; ++j) ed[j] = j < n ? __ldg(&M.c_ed[j * nv + c]) : 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) p[k] = __ldg(&M.c_p32[k * nv + c]);
+    after_prior<true>(q_tr, u, qg, vhx);
+    float ue[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) ue[j] = j < n ? u[ed[j]] : 0.0f;
+    // a pentagon's sixth slot has zero weights
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        v[k] = fmaf(ue[j], __ldg(&M.c_apw32[(3 * j + k) * nv + c]), v[k]);
     i = c;
-    stride = nv;
     out = vhx;
   }
   // proj_vec_sphere (smeshpack.f90:4419-4433) with |p| = 1
   const float vp = v[0] * p[0] + v[1] * p[1] + v[2] * p[2];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) out[k * stride + i] = v[k] - vp * p[k];
+  out[i] = make_float4(v[0] - vp * p[0], v[1] - vp * p[1], v[2] - vp * p[2], 0.0f);
 }
 
 // -div F, K, Bernoulli potential g (h - h_ref + b) + K, mass RK stage
@@ -267,11 +273,8 @@ __global__ void __launch_bounds__(256) k_diflap32(DevMesh M, const float *__rest
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
-  const float g = (coefdiv[__ldg(&M.e_v[ne + e])] - coefdiv[__ldg(&M.e_v[e])]) *
-                  __ldg(&M.e_grad32[e]);
-  const float gt = (coefvort[__ldg(&M.e_sh[ne + e])] - coefvort[__ldg(&M.e_sh[e])]) *
-                   __ldg(&M.e_gtg32[e]);
-  lap[e] = g - gt;
+  lap[e] = edge_lap(M, e, __ldg(&M.e_v[e]), __ldg(&M.e_v[ne + e]), __ldg(&M.e_grad32[e]), coefdiv,
+                    coefvort);
 }
 
 // ---- cell-centred TRSK (variant 1), bodies in swm_k32_body.cuh ------------
@@ -607,16 +610,14 @@ __global__ void __launch_bounds__(512) k_edge32v2(DevMesh M, const float *__rest
                                                   float *__restrict__ yout,
                                                   float *__restrict__ tend, int stage, float dt,
                                                   int mom_on, float erad,
-                                                  const float *__restrict__ corr,
-                                                  const float *__restrict__ dif1,
-                                                  const float *__restrict__ dif2) {
+                                                  const float *__restrict__ corr, EdgeDif D) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   const int e0 = 2 * p;
   if (e0 >= M.ne) return;
   if (e0 + 1 < M.ne) {
     const uint4 w = __ldg(reinterpret_cast<const uint4 *>(M.e_vs2) + p);
     const float2 g = __ldg(reinterpret_cast<const float2 *>(M.e_grad32) + p);
-    IMODEL_WAIT(Wait, bern, zflux, yn, acc, yout, tend, corr, dif1, dif2);
+    IMODEL_WAIT(Wait, bern, zflux, yn, acc, yout, tend, corr);
     float m0 = edge_momeq(w.x, w.y, g.x, bern, zflux, erad);
     float m1 = edge_momeq(w.z, w.w, g.y, bern, zflux, erad);
     // learned correction of the PV flux (frozen over the RK step)
@@ -626,15 +627,15 @@ __global__ void __launch_bounds__(512) k_edge32v2(DevMesh M, const float *__rest
       m1 += c.y;
     }
     // diffusion, then hyperdiffusion
-    if (dif1) {
-      const float2 d = reinterpret_cast<const float2 *>(dif1)[p];
+    if (D.lap) {
+      const float2 d = reinterpret_cast<const float2 *>(D.lap)[p];
       m0 += d.x;
       m1 += d.y;
     }
-    if (dif2) {
-      const float2 d = reinterpret_cast<const float2 *>(dif2)[p];
-      m0 -= d.x;
-      m1 -= d.y;
+    if (D.coefdiv) {
+      constexpr uint32_t mask = 0x0FFFFFFFu;
+      m0 = fmaf(D.sgn, edge_lap(M, e0, w.x & mask, w.y & mask, g.x, D.coefdiv, D.coefvort), m0);
+      m1 = fmaf(D.sgn, edge_lap(M, e0 + 1, w.z & mask, w.w & mask, g.y, D.coefdiv, D.coefvort), m1);
     }
     if (!mom_on) m0 = m1 = 0.0f;
     if (stage < 0) {
@@ -649,9 +650,9 @@ __global__ void __launch_bounds__(512) k_edge32v2(DevMesh M, const float *__rest
       reinterpret_cast<float2 *>(yout)[p] = make_float2(o0, o1);
     }
   } else {
-    IMODEL_WAIT(Wait, bern, zflux, yn, acc, yout, tend, corr, dif1, dif2);
+    IMODEL_WAIT(Wait, bern, zflux, yn, acc, yout, tend, corr);
     edge_body(M, e0, __ldg(&M.e_vs2[e0]), bern, zflux, yn, acc, yout, tend, stage, dt,
-              mom_on, erad, corr, dif1, dif2);
+              mom_on, erad, corr, D);
   }
 }
 
@@ -727,14 +728,19 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
   const Diffusion<float> &D = W.dif;
   const float *dif1 = D.k2 ? D.lap : nullptr, *dif2 = D.k4 ? D.lap2 : nullptr;
   const int nbc = nblocks(M.nv, 256), nbt = nblocks(M.nt, 256);
+  const Apvm<float> &A = W.apvm;
+  float4 *qg4 = reinterpret_cast<float4 *>(A.qg), *vhx4 = reinterpret_cast<float4 *>(A.vhx);
   // the edge gradients of the diffusion (and the second application of
-  // hyperdiffusion) once K div u and K_tr zeta are written
-  auto diffusion_tail = [&]() {
+  // hyperdiffusion) once K div u and K_tr zeta are written; in_edge: the
+  // edge kernel forms the last of them itself
+  auto diffusion_tail = [&](bool in_edge) {
     if (!D.on) return;
-    launch_pdl(k_diflap32, nblocks(M.ne, 256), 256, s, M, D.coefdiv, D.coefvort, D.lap);
+    if (D.k4 || !in_edge)
+      launch_pdl(k_diflap32, nblocks(M.ne, 256), 256, s, M, D.coefdiv, D.coefvort, D.lap);
     if (D.k4) {
       launch_pdl(k_difcv32, nbc + nbt, 256, s, M, D.lap, D.kcv, D.kt, D.coefdiv, D.coefvort, nbc);
-      launch_pdl(k_diflap32, nblocks(M.ne, 256), 256, s, M, D.coefdiv, D.coefvort, D.lap2);
+      if (!in_edge)
+        launch_pdl(k_diflap32, nblocks(M.ne, 256), 256, s, M, D.coefdiv, D.coefvort, D.lap2);
     }
   };
   if (T.variant == 0 && D.on)  // variant 0: K div u and K_tr zeta in their own pass
@@ -758,17 +764,16 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
     // learned correction: formed once per step from the first stage's state
     if (W.learned && stage <= 0)
       learned_launch(M, *W.learned, h_in, u_in, W.q_tr, W.h_ref, T.mlp_gather, W.flags, s);
-    const Apvm<float> &A = W.apvm;
     const bool pxt = W.scheme == IMODEL_SWM_PXT16, gass = W.scheme == IMODEL_SWM_GASS18;
     // APVM (swm_operators.f90:1495-1502) and pxt16's distance-weighted q_e:
     // the PV of every edge from the edge pre-pass, read by the cells in
     // place of the triangle average
     if (A.on)
-      launch_pdl(k_apvm32, nbt + nblocks(M.nv, 256), 256, s, M, W.q_tr, u_in, A.qg, A.vhx, nbt);
+      launch_pdl(k_apvm32, nbt + nbc, 256, s, M, W.q_tr, u_in, qg4, vhx4, nbt);
     if (A.on || gass)
       launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr,
-                 W.h_ed, W.uh, W.q_ed, W.h_ref, A.on ? A.qg : nullptr, A.vhx, A.coef, pxt || gass
-                 ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
+                 nullptr, W.q_ed, W.h_ref, A.on ? qg4 : nullptr, vhx4, A.coef,
+                 pxt || gass ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
     if (ev) cudaEventRecord(ev[2], s);
     if (gass)
       launch_pdl(k_cell32g, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern,
@@ -796,7 +801,14 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
                  T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux, W.yn_h,
                  W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv :
                  nullptr);
-    diffusion_tail();
+    diffusion_tail(!dtred1);
+    EdgeDif E;
+    if (D.on) {
+      if (D.k2 && D.k4) E.lap = D.lap;
+      E.coefdiv = D.coefdiv;
+      E.coefvort = D.coefvort;
+      E.sgn = D.k4 ? -1.0f : 1.0f;
+    }
     if (ev) cudaEventRecord(ev[3], s);
     if (dtred1)
       launch_pdl(k_edge32d, nblocks(M.ne, T.bs_edge), T.bs_edge, s, M, W.bern, W.vhq, W.yn_u,
@@ -804,28 +816,23 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
     else
       launch_wait(k_edge32v2<PriorWait>, k_edge32v2<NoWait>, nblocks((M.ne + 1) / 2, T.bs_edge),
                  T.bs_edge, s, M, W.bern, W.zflux, W.yn_u, W.acc_u, u_out, W.tend_u, stage, dt,
-                 W.mom_on, static_cast<float>(M.erad), W.learned ? W.learned->corr : nullptr,
-                 dif1, dif2);
+                 W.mom_on, static_cast<float>(M.erad), W.learned ? W.learned->corr : nullptr, E);
     if (ev) cudaEventRecord(ev[4], s);
     return;
   }
   if (ev) cudaEventRecord(ev[1], s);
-  const Apvm<float> &A = W.apvm;
-  if (A.on) {
-    const int nbt = nblocks(M.nt, 256);
-    launch_pdl(k_apvm32, nbt + nblocks(M.nv, 256), 256, s, M, W.q_tr, u_in, A.qg, A.vhx, nbt);
-  }
+  if (A.on) launch_pdl(k_apvm32, nbt + nbc, 256, s, M, W.q_tr, u_in, qg4, vhx4, nbt);
   // the method wrappers (variant 0 only): pxt16 (distance-weighted q_e,
   // Perot KE, pered), gass18 (rhombus PV, connecting-edge PV), dtred
   const int sch = W.scheme;
   const bool pxt = sch == IMODEL_SWM_PXT16, gass = sch == IMODEL_SWM_GASS18;
-  launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr, W.h_ed,
-             W.uh, W.q_ed, W.h_ref, A.on ? A.qg : nullptr, A.vhx, A.coef, pxt || gass ? M.e_qw32 :
-             nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
+  launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr, W.uh,
+             W.q_ed, W.h_ref, A.on ? qg4 : nullptr, vhx4, A.coef, pxt || gass ? M.e_qw32 : nullptr,
+             gass ? W.h_trs : nullptr, W.pv_on, W.flags);
   if (ev) cudaEventRecord(ev[2], s);
   launch_pdl(k_cell32, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.uh, W.bern,
              W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, pxt ? 1 : 0);
-  diffusion_tail();
+  diffusion_tail(false);
   if (ev) cudaEventRecord(ev[3], s);
   launch_pdl(k_edge32, nblocks(M.ne, T.bs_edge), T.bs_edge, s, M, W.bern, W.uh, W.q_ed, W.yn_u,
              W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2, gass ? M.e_stq : nullptr,

@@ -335,6 +335,23 @@ __device__ __forceinline__ float edge_terms(float b1, float b2, float z1, float 
   return -fmaf(z1 + z2, __fmul_rn(g, erad), grad);
 }
 
+// grad_ed(K div x) - grad_ed_tg(K_tr zeta(x)) of an edge between the cells
+// c1, c2
+__device__ __forceinline__ float edge_lap(const DevMesh &M, int e, int c1, int c2, float g,
+                                          const float *__restrict__ coefdiv,
+                                          const float *__restrict__ coefvort) {
+  const int t1 = __ldg(&M.e_sh[e]), t2 = __ldg(&M.e_sh[M.ne + e]);
+  const float gt = __fmul_rn(coefvort[t2] - coefvort[t1], __ldg(&M.e_gtg32[e]));
+  return fmaf(coefdiv[c2] - coefdiv[c1], g, -gt);
+}
+
+// the diffusion terms that the edge kernel adds: + lap when given, then sgn
+// (1 or -1) times edge_lap of coefdiv and coefvort when given
+struct EdgeDif {
+  const float *lap = nullptr, *coefdiv = nullptr, *coefvort = nullptr;
+  float sgn = 0.0f;
+};
+
 // -grad B - (Z_c1 + Z_c2) / l_e and the momentum RK stage of edge e
 __device__ __forceinline__ void edge_body(const DevMesh &M, int e, uint2 w,
                                           const float *__restrict__ bern,
@@ -342,20 +359,16 @@ __device__ __forceinline__ void edge_body(const DevMesh &M, int e, uint2 w,
                                           const float *__restrict__ yn, float *__restrict__ acc,
                                           float *__restrict__ yout, float *__restrict__ tend,
                                           int stage, float dt, int mom_on, float erad,
-                                          const float *__restrict__ corr = nullptr,
-                                          const float *__restrict__ dif1 = nullptr,
-                                          const float *__restrict__ dif2 = nullptr) {
+                                          const float *__restrict__ corr, const EdgeDif &D) {
   const int c1 = static_cast<int>(w.x & 0x0FFFFFFFu), c2 = static_cast<int>(w.y & 0x0FFFFFFFu);
   const int s1 = static_cast<int>(w.x >> 28), s2 = static_cast<int>(w.y >> 28);
   const float g = __ldg(&M.e_grad32[e]);  // 1 / (l_e a)
-  float momeq = edge_terms(bern[c1], bern[c2],
-                           zflux[6 * c1 + s1], zflux[6 * c2 + s2], g,
-                           erad);
+  float momeq = edge_terms(bern[c1], bern[c2], zflux[6 * c1 + s1], zflux[6 * c2 + s2], g, erad);
   // learned correction of the PV flux (frozen over the RK step)
   if (corr) momeq += corr[e];
   // diffusion, then hyperdiffusion
-  if (dif1) momeq += dif1[e];
-  if (dif2) momeq -= dif2[e];
+  if (D.lap) momeq += D.lap[e];
+  if (D.coefdiv) momeq = fmaf(D.sgn, edge_lap(M, e, c1, c2, g, D.coefdiv, D.coefvort), momeq);
   if (!mom_on) momeq = 0.0f;
   if (stage < 0)
     tend[e] = momeq;

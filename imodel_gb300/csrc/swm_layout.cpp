@@ -797,20 +797,28 @@ std::string build_layout(const imodel_swm_mesh &m, const double *bt, Layout &L, 
 #pragma omp parallel for schedule(static)
     for (int i = 0; i < nv; ++i)
       for (int k = 0; k < 3; ++k) L.c_p[k * NV + i] = m.v_p[3 * static_cast<size_t>(L.cell_n2o[i]) + k];
-    fill(L.t_apw32, 9 * NT, 0.0f);
-    fill(L.t_cc32, 3 * NT, 0.0f);
+    L.t_ap32.resize(12 * NT);
+    fill(L.t_across, 4 * NT, 0);
 #pragma omp parallel for schedule(static)
     for (int i = 0; i < nt; ++i) {
       const int t = L.tri_n2o[i];
       for (int s = 0; s < 3; ++s) {
         const int e = m.tr_ed[3 * static_cast<size_t>(t) + s] - 1;
         const double sg = -static_cast<double>(m.tr_tg[3 * static_cast<size_t>(t) + s]);
+        // grad_tr2ed: sign (q(sh(2)) - q(sh(1))) / (edhx%leng erad)
+        const int ei = L.edge_o2n[e];
+        const bool is1 = L.e_sh[ei] == i;
+        L.t_across[4 * static_cast<size_t>(i) + s] = is1 ? L.e_sh[NE + ei] : L.e_sh[ei];
+        const double gr = (is1 ? L.e_sgtg[ei] : -L.e_sgtg[ei]) / (m.edhx_leng[e] * m.erad);
         for (int k = 0; k < 3; ++k) {
           const double d = m.ed_c[3 * static_cast<size_t>(e) + k] - L.t_c[k * NT + i];
-          L.t_apw32[(3 * s + k) * NT + i] = static_cast<float>(sg * d * m.ed_leng[e] / m.tr_areag[t]);
+          const int q = 3 * s + k;
+          L.t_ap32[4 * ((q / 4) * NT + i) + q % 4] =
+              static_cast<float>(sg * d * m.ed_leng[e] / m.tr_areag[t] * gr);
         }
       }
-      for (int k = 0; k < 3; ++k) L.t_cc32[k * NT + i] = static_cast<float>(L.t_c[k * NT + i]);
+      for (int k = 0; k < 3; ++k)
+        L.t_ap32[4 * (2 * NT + i) + 1 + k] = static_cast<float>(L.t_c[k * NT + i]);
     }
     fill(L.c_apw32, 18 * NV, 0.0f);
     fill(L.c_p32, 3 * NV, 0.0f);
@@ -1264,7 +1272,7 @@ extern "C" int imodel_swm_test_layout_digest(const imodel_swm_mesh *m, int32_t s
   IMODEL_DIGEST(e_nst) IMODEL_DIGEST(e_stk) IMODEL_DIGEST(e_stw) IMODEL_DIGEST(e_stc32)
   IMODEL_DIGEST(t_ed) IMODEL_DIGEST(t_v) IMODEL_DIGEST(t_lt) IMODEL_DIGEST(t_kite)
   IMODEL_DIGEST(t_areag) IMODEL_DIGEST(t_f) IMODEL_DIGEST(e_c) IMODEL_DIGEST(t_c)
-  IMODEL_DIGEST(c_p) IMODEL_DIGEST(t_apw32) IMODEL_DIGEST(t_cc32) IMODEL_DIGEST(c_apw32)
+  IMODEL_DIGEST(c_p) IMODEL_DIGEST(t_ap32) IMODEL_DIGEST(t_across) IMODEL_DIGEST(c_apw32)
   IMODEL_DIGEST(c_p32) IMODEL_DIGEST(t_recA) IMODEL_DIGEST(t_recB) IMODEL_DIGEST(t_recC)
   IMODEL_DIGEST(t_c16A) IMODEL_DIGEST(t_c16B) IMODEL_DIGEST(t_c16C) IMODEL_DIGEST(t_wb)
   IMODEL_DIGEST(t_circ32) IMODEL_DIGEST(t_kite32) IMODEL_DIGEST(t_f32) IMODEL_DIGEST(e_area)

@@ -169,13 +169,16 @@ __device__ __forceinline__ void tile_edges(const Tile &T, const TileShared &S,
                                            int stage, float dt, float erad, int mom_on) {
   const int tid = threadIdx.x;
   const uint2 *edge = reinterpret_cast<const uint2 *>(S.block + T.edge);
-  auto update = [&](int k, float yn, float ac) {
-    const int e = T.e0 + k;
+  auto tendency = [&](int k) {
     const uint2 w = edge[k];
-    float m = edge_terms(S.sb[w.x & 1023u], S.sb[w.x >> 13 & 1023u],
-                         S.sz[6 * (w.x & 1023u) + (w.x >> 10 & 7u)],
-                         S.sz[6 * (w.x >> 13 & 1023u) + (w.x >> 23)], __uint_as_float(w.y), erad);
-    if (!mom_on) m = 0.0f;
+    const float m = edge_terms(S.sb[w.x & 1023u], S.sb[w.x >> 13 & 1023u],
+                               S.sz[6 * (w.x & 1023u) + (w.x >> 10 & 7u)],
+                               S.sz[6 * (w.x >> 13 & 1023u) + (w.x >> 23)], __uint_as_float(w.y),
+                               erad);
+    return mom_on ? m : 0.0f;
+  };
+  auto update = [&](int k, float m, float yn, float ac) {
+    const int e = T.e0 + k;
     if (stage < 0) {
       F.tend_u[e] = m;
     } else {
@@ -183,12 +186,18 @@ __device__ __forceinline__ void tile_edges(const Tile &T, const TileShared &S,
       if (stage < 3) F.acc_u[e] = ac;
     }
   };
+  // all reads of the rounds before their writes, which could alias them for
+  // all the compiler knows
   constexpr int kE = TileOwn<nthr>::kE;
+  float m[kE];
+#pragma unroll
+  for (int r = 0; r < kE; ++r) m[r] = tid + r * nthr < T.ne ? tendency(tid + r * nthr) : 0.0f;
 #pragma unroll
   for (int r = 0; r < kE; ++r)
-    if (tid + r * nthr < T.ne) update(tid + r * nthr, own.ynu[r], own.acu[r]);
+    if (tid + r * nthr < T.ne) update(tid + r * nthr, m[r], own.ynu[r], own.acu[r]);
   for (int k = tid + kE * nthr; k < T.ne; k += nthr)
-    update(k, stage >= 0 ? F.yn_u[T.e0 + k] : 0.0f, stage >= 1 ? F.acc_u[T.e0 + k] : 0.0f);
+    update(k, tendency(k), stage >= 0 ? F.yn_u[T.e0 + k] : 0.0f,
+           stage >= 1 ? F.acc_u[T.e0 + k] : 0.0f);
 }
 
 }  // namespace imodel
