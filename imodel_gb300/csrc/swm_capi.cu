@@ -1593,7 +1593,8 @@ struct Moist {
   double *th = nullptr, *ex20 = nullptr, *qv = nullptr, *qc = nullptr, *qr = nullptr;
   double *q[5][4] = {};  // per tracer: y_n, two stage buffers, RK accumulator
   double *uphi = nullptr, *gthb = nullptr;
-  float *f_th = nullptr, *f_ex20 = nullptr, *f_qv = nullptr, *f_qc = nullptr, *f_qr = nullptr;
+  float *f_gthb = nullptr, *f_ex20 = nullptr, *f_qv = nullptr, *f_qc = nullptr, *f_qr = nullptr;
+  bool fused = false;  // FP32: the stage is one kernel over tiles
   float *f_q[5][4] = {};
   bool state_set = false;
   // one step's launches, captured once per dt and replayed
@@ -1657,6 +1658,7 @@ void moist_step32(Moist *X, double dt) {
   const float fdt = static_cast<float>(dt);
   const bool swm = X->testcase > 1;
   const int active = swm ? (0xF | (X->testcase == 2 ? 0x10 : 0)) : 0x10;
+  const bool fused = swm && X->fused && imodel::fused_stage(W);
   {
     for (int st = 0; st < 4; ++st) {
       imodel::MoistArgs32 A;
@@ -1668,7 +1670,8 @@ void moist_step32(Moist *X, double dt) {
       A.h_ref = W.h_ref;
       const float *h_in = swm ? stage_in(st, W.yn_h, W.ya_h, W.yb_h) : W.yn_h;
       const float *u_in = swm ? stage_in(st, W.yn_u, W.ya_u, W.yb_u) : W.yn_u;
-      if (swm) imodel::launch_stage32(H->M, W, h_in, u_in, nullptr, nullptr, -1, fdt, H->stream);
+      if (swm && !fused)
+        imodel::launch_stage32(H->M, W, h_in, u_in, nullptr, nullptr, -1, fdt, H->stream);
       A.h_in = h_in;
       A.u_in = u_in;
       A.tend_h = W.tend_h;
@@ -1687,15 +1690,18 @@ void moist_step32(Moist *X, double dt) {
         A.q_acc[k] = q[3];
         A.q_out[k] = stage_out(st, q[0], q[1], q[2]);
       }
-      A.th = X->f_th;
-      A.ex20 = X->f_ex20;
+      A.gthb = X->f_gthb;
+      A.q0ex = X->f_ex20;
       A.qv = X->f_qv;
       A.qc = X->f_qc;
       A.qr = X->f_qr;
-      A.q0 = static_cast<float>(X->q0);
       A.flags = H->d_flags;
-      imodel::launch_moist_stage32(H->M, A, H->stream);
+      if (fused)
+        imodel::launch_moist_stage32_fused(H->M, W, A, H->stream);
+      else
+        imodel::launch_moist_stage32(H->M, A, H->stream);
     }
+    if (fused) return;
     imodel::launch_moist_q32(H->nv, W.yn_h, W.h_ref, X->f_q[1][0], X->f_q[2][0], X->f_q[3][0],
                              X->f_qv, X->f_qc, X->f_qr, H->d_flags, H->stream);
   }
@@ -1825,14 +1831,24 @@ int imodel_moist_create(const imodel_swm_mesh *m, const imodel_moist_opts *o, vo
   std::vector<double> ex(nv);
   for (size_t i = 0; i < nv; ++i) ex[i] = std::exp(20.0 * o->theta[i]);
   if (X->fp32) {
-    for (float **p : {&X->f_th, &X->f_ex20, &X->f_qv, &X->f_qc, &X->f_qr})
+    float *th = nullptr;
+    for (float **p : {&th, &X->f_ex20, &X->f_qv, &X->f_qc, &X->f_qr})
       if ((rc = imodel::dalloc(H, p, nv))) return rc;
+    if ((rc = imodel::dalloc(H, &X->f_gthb, ne))) return rc;
     for (int k = 0; k < 5; ++k)
       for (int b = 0; b < 4; ++b)
         if ((rc = imodel::dalloc(H, &X->f_q[k][b], nv))) return rc;
-    if ((rc = moist_in32(H, o->theta, X->f_th, false, 0.0)) ||
+    // the buffers' zero-fill (default stream) comes before what H->stream writes
+    if (cudaStreamSynchronize(nullptr) != cudaSuccess)
+      return imodel::set_error(H, IMODEL_SWM_ECUDA, "stream synchronize failed");
+    if ((rc = moist_in32(H, o->theta, th, false, 0.0)) ||
         (rc = moist_in32(H, ex.data(), X->f_ex20, false, 0.0)))
       return rc;
+    imodel::launch_moist_consts32(H->M, th, X->f_ex20, static_cast<float>(X->q0), X->f_gthb,
+                                  H->stream);
+    if (cudaGetLastError() != cudaSuccess)
+      return imodel::set_error(H, IMODEL_SWM_ECUDA, "launch failed");
+    X->fused = imodel::fused_moist_ok(H->W32.tiles);
   } else {
     for (double **p : {&X->th, &X->ex20, &X->qv, &X->qc, &X->qr})
       if ((rc = imodel::dalloc(H, p, nv))) return rc;

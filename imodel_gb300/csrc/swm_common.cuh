@@ -345,11 +345,23 @@ struct MoistArgs32 {
   float *yn_h = nullptr, *acc_h = nullptr, *h_out = nullptr;
   const float *q_in[5] = {};
   float *q_yn[5] = {}, *q_acc[5] = {}, *q_out[5] = {};
-  const float *th = nullptr, *ex20 = nullptr, *qv = nullptr, *qc = nullptr, *qr = nullptr;
-  float q0 = 0.0f;
+  // constants of the run: g theta_e grad(b) [ne] and q0 exp(20 theta) [nv];
+  // qv, qc, qr of the last step [nv]
+  const float *gthb = nullptr, *q0ex = nullptr;
+  float *qv = nullptr, *qc = nullptr, *qr = nullptr;
   int *flags = nullptr;
 };
 void launch_moist_stage32(const DevMesh &M, const MoistArgs32 &A, cudaStream_t s);
+// gthb from theta and the topography (both frozen in a run); ex20 becomes
+// q0 ex20 in place
+void launch_moist_consts32(const DevMesh &M, const float *th, float *ex20, float q0, float *gthb,
+                           cudaStream_t s);
+// the shallow-water stage and the moist one in one kernel over tiles, where
+// fused_stage(W) holds and its shared memory fits (fused_moist_ok); after the
+// last stage qv, qc, qr are those of the new state
+bool fused_moist_ok(const TileDev &T);
+void launch_moist_stage32_fused(const DevMesh &M, const Work<float> &W, const MoistArgs32 &A,
+                                cudaStream_t s);
 void launch_moist_q32(int nv, const float *hd, float h_ref, const float *hqv, const float *hqc,
                       const float *hqr, float *qv, float *qc, float *qr, int *flags,
                       cudaStream_t s);

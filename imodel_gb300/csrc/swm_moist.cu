@@ -9,14 +9,13 @@
 // initial value in the reference's RK4 path) and read here.
 #include "swm_common.cuh"
 #include "swm_div.cuh"
+#include "swm_moist32.cuh"
 
 namespace imodel {
 namespace {
 
 // constants.f90:45 -- eps = epsilon(1.) (float epsilon)
 constexpr double kEps = 1.1920928955078125e-07;
-// initialize_moist_swm_fields (moist_swm.f90:730-732)
-constexpr double kLscale = 10.0, kGammaR = 0.001, kQprecip = 0.0001;
 
 // dt k / 2 as (dt / 2) k and acc + 2 k as one fused operation with an exact
 // product: the same roundings (moist_swm.f90:1880-1960)
@@ -192,18 +191,18 @@ __global__ void k_moist_q(int nv, const double *__restrict__ h, const double *__
 // q_i + q_nb and q_nb + q_i round alike, so no flux array goes through
 // memory.
 
-__device__ __forceinline__ float rk_stage32m(int stage, float k, float yn, float *acc, float dt) {
-  if (stage == 0) {
-    *acc = k;
-    return yn + dt * k * 0.5f;
-  } else if (stage == 1) {
-    *acc = *acc + 2.0f * k;
-    return yn + dt * k * 0.5f;
-  } else if (stage == 2) {
-    *acc = *acc + 2.0f * k;
-    return yn + dt * k;
-  }
-  return yn + dt * (*acc + k) * (1.0f / 6.0f);
+// what the sources read that stays fixed in a run: g theta_e grad(b) at the
+// edges, q0 exp(20 theta) at the cells
+__global__ void __launch_bounds__(256) k_moist_consts32(DevMesh M, const float *__restrict__ th,
+                                                        float *__restrict__ ex20, float q0,
+                                                        float *__restrict__ gthb) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < M.nv) ex20[e] = q0 * ex20[e];
+  if (e >= M.ne) return;
+  const int v1 = M.e_v[e], v2 = M.e_v[M.ne + e];
+  const float gb = (M.c_bt32[v2] - M.c_bt32[v1]) * M.e_grad32[e];
+  const float th_ed = (th[v1] + th[v2]) * 0.5f;
+  gthb[e] = static_cast<float>(M.grav) * (th_ed * gb);
 }
 
 // the thermal momentum source and u's RK stage (shallow-water cases only)
@@ -214,22 +213,10 @@ __global__ void __launch_bounds__(256) k_moist_edge32(DevMesh M, MoistArgs32 A) 
   if (e >= ne) return;
   const int v1 = __ldg(&M.e_v[e]), v2 = __ldg(&M.e_v[ne + e]);
   const float gr = __ldg(&M.e_grad32[e]), grav = static_cast<float>(M.grav);
-  const float hd1 = A.h_in[v1], hd2 = A.h_in[v2];
-  const float Q1 = A.q_in[0][v1], Q2 = A.q_in[0][v2];
-  const float h1 = A.h_ref + hd1, h2 = A.h_ref + hd2;
-  const float g = ((hd2 - hd1) * (Q1 + Q2) * 0.5f + (Q2 - Q1) * (h1 + h2) * 0.5f) * gr;
-  // scalar_hx2ed of h
-  const float hed = A.h_ref + 0.5f * (hd1 + hd2);
-  float gpi_oh = 0.0f;
-  if (fabsf(hed) < 1.1920928955078125e-12f)
-    atomicOr(A.flags, 1);
-  else
-    gpi_oh = g / hed;
-  const float gb = (__ldg(&M.c_bt32[v2]) - __ldg(&M.c_bt32[v1])) * gr;
-  const float th_ed = (A.th[v1] + A.th[v2]) * 0.5f;
-  const float su = (grav * 0.5f) * gpi_oh + grav * (th_ed * gb);
+  const float su = thermal32(A.h_in[v1], A.h_in[v2], A.q_in[0][v1], A.q_in[0][v2], A.h_ref, gr,
+                             grav, A.gthb[e], A.flags);
   const float momeq = A.tend_u[e] + su;
-  A.u_out[e] = rk_stage32m(A.stage, momeq, A.yn_u[e], A.acc_u + e, A.dt);
+  A.u_out[e] = rk_stage32(A.stage, momeq, A.yn_u[e], A.acc_u + e, A.dt);
 }
 
 __global__ void __launch_bounds__(256) k_moist_cell32(DevMesh M, MoistArgs32 A) {
@@ -239,19 +226,9 @@ __global__ void __launch_bounds__(256) k_moist_cell32(DevMesh M, MoistArgs32 A) 
   if (i >= nv) return;
   float hs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   if (A.swm) {
-    A.h_out[i] = rk_stage32m(A.stage, A.tend_h[i], A.yn_h[i], A.acc_h + i, A.dt);
-    const float hi = A.h_ref + A.h_in[i];
-    const float qs = A.q0 * A.ex20[i] / ((hi + __ldg(&M.c_bt32[i])) * static_cast<float>(M.grav));
-    const float gamma_v = 1.0f / (1.0f + kLscale * (20.0f * qs));
-    const float qv = A.qv[i], qc = A.qc[i];
-    const float r = gamma_v * (qv - qs);
-    const float dqv = fmaxf(r, 0.0f) / A.dt;
-    const float dqc = fminf(qc, fmaxf(-r, 0.0f)) / A.dt;
-    const float dqr = fmaxf(static_cast<float>(kGammaR) * (qc - static_cast<float>(kQprecip)), 0.0f) / A.dt;
-    hs[1] = hi * (dqc - dqv);
-    hs[2] = hi * (dqv - dqc - dqr);
-    hs[3] = hi * dqr;
-    hs[0] = hi * (static_cast<float>(kLscale) * (dqv - dqc));
+    A.h_out[i] = rk_stage32(A.stage, A.tend_h[i], A.yn_h[i], A.acc_h + i, A.dt);
+    sources32(A.h_ref + A.h_in[i], __ldg(&M.c_bt32[i]), A.q0ex[i], A.qv[i], A.qc[i], A.dt,
+              static_cast<float>(M.grav), hs);
   }
   // the cell's edges: the normal velocity times c_div32, and the neighbour
   const int n = M.c_nnb[i];
@@ -282,7 +259,7 @@ __global__ void __launch_bounds__(256) k_moist_cell32(DevMesh M, MoistArgs32 A) 
     }
     float t = -d;
     if (A.swm && k < 4) t = t + hs[k];
-    A.q_out[k][i] = rk_stage32m(A.stage, t, A.q_yn[k][i], A.q_acc[k] + i, A.dt);
+    A.q_out[k][i] = rk_stage32(A.stage, t, A.q_yn[k][i], A.q_acc[k] + i, A.dt);
   }
 }
 
@@ -325,6 +302,12 @@ void launch_moist_consts(const DevMesh64 &M, const double *th, double *ex20, dou
   // ne >= nv; the larger count covers both either way
   const int n = M.ne > M.nv ? M.ne : M.nv;
   k_moist_consts<<<nblocks(n, 256), 256, 0, s>>>(M, th, ex20, q0, gthb);
+}
+
+void launch_moist_consts32(const DevMesh &M, const float *th, float *ex20, float q0, float *gthb,
+                           cudaStream_t s) {
+  const int n = M.ne > M.nv ? M.ne : M.nv;
+  k_moist_consts32<<<nblocks(n, 256), 256, 0, s>>>(M, th, ex20, q0, gthb);
 }
 
 void launch_moist_stage(const DevMesh64 &M, const MoistArgs &A, cudaStream_t s) {

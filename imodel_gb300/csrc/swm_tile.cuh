@@ -3,6 +3,8 @@
 // (swm_ens.cu).  Tiles and their blocks: swm_layout.h; the arithmetic:
 // swm_k32_body.cuh, as in the separate kernels and with the same bits.
 #pragma once
+#include <type_traits>
+
 #include "swm_k32_body.cuh"
 #include "tc05.cuh"
 
@@ -126,19 +128,27 @@ __device__ __forceinline__ void tile_triangles(const Tile &T, const TileShared &
 }
 
 // Bernoulli potential and PV-flux terms of the tile's cells; the own cells'
-// depth
-template <int nthr>
+// depth.  For an own cell, cell(slot words, ue, kd, meta, bt, inva, new depth)
+// may do more with what was gathered.
+struct NoCell {
+  template <class... P>
+  __device__ __forceinline__ void operator()(const P &...) const {}
+};
+template <int nthr, class Cell = NoCell>
 __device__ __forceinline__ void tile_cells(const Tile &T, const TileShared &S,
                                            const TileFields &F, const TileOwn<nthr> &own,
-                                           int stage, float dt, float grav, float h_ref) {
+                                           int stage, float dt, float grav, float h_ref,
+                                           Cell cell = Cell{}) {
   const int tid = threadIdx.x;
   if (tid >= T.nz) return;
   const uint4 *slot = reinterpret_cast<const uint4 *>(S.block + T.slot) + tid;
   float R[6], ue[6], hn[6], qt[6];
   float2 kd[6];
+  uint32_t word[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
     const uint4 s = slot[j * T.nz];
+    word[j] = s.x;
     ue[j] = S.su[s.x & 1023u];
     hn[j] = S.sh[s.x >> 10 & 1023u];
     qt[j] = S.sq[s.x >> 20];
@@ -155,26 +165,35 @@ __device__ __forceinline__ void tile_cells(const Tile &T, const TileShared &S,
   const float masseq = __fmul_rn(-div, inva);
   if (stage < 0) {
     F.tend_h[T.c0 + tid] = masseq;
+    cell(word, ue, kd, meta, bt, inva, 0.0f);
   } else {
     float a = own.ach;
-    F.h_out[T.c0 + tid] = rk_stage32(stage, masseq, own.ynh, &a, dt);
+    const float hnew = rk_stage32(stage, masseq, own.ynh, &a, dt);
+    F.h_out[T.c0 + tid] = hnew;
     if (stage < 3) F.acc_h[T.c0 + tid] = a;
+    cell(word, ue, kd, meta, bt, inva, hnew);
   }
 }
 
-// the own edges' velocity
-template <int nthr>
+// the own edges' velocity; force(k, cell 1, cell 2, 1 / (l erad)) is added to
+// the momentum tendency of own edge k (cells by local number)
+struct NoForce {
+  __device__ __forceinline__ float operator()(int, int, int, float) const { return 0.0f; }
+};
+template <int nthr, class Force = NoForce>
 __device__ __forceinline__ void tile_edges(const Tile &T, const TileShared &S,
                                            const TileFields &F, const TileOwn<nthr> &own,
-                                           int stage, float dt, float erad, int mom_on) {
+                                           int stage, float dt, float erad, int mom_on,
+                                           Force force = Force{}) {
   const int tid = threadIdx.x;
   const uint2 *edge = reinterpret_cast<const uint2 *>(S.block + T.edge);
   auto tendency = [&](int k) {
     const uint2 w = edge[k];
-    const float m = edge_terms(S.sb[w.x & 1023u], S.sb[w.x >> 13 & 1023u],
-                               S.sz[6 * (w.x & 1023u) + (w.x >> 10 & 7u)],
-                               S.sz[6 * (w.x >> 13 & 1023u) + (w.x >> 23)], __uint_as_float(w.y),
-                               erad);
+    const int c1 = w.x & 1023u, c2 = w.x >> 13 & 1023u;
+    const float g = __uint_as_float(w.y);
+    float m = edge_terms(S.sb[c1], S.sb[c2], S.sz[6 * c1 + (w.x >> 10 & 7u)],
+                         S.sz[6 * c2 + (w.x >> 23)], g, erad);
+    if constexpr (!std::is_same<Force, NoForce>::value) m += force(k, c1, c2, g);
     return mom_on ? m : 0.0f;
   };
   auto update = [&](int k, float m, float yn, float ac) {

@@ -50,3 +50,27 @@ def test_fused_stage_reports_a_vanishing_depth(grid_at):
         m.ode_rk4(h, u, 600.0, 1)
     assert ei.value.code == 3
     m.close()
+
+
+@pytest.mark.parametrize("advection", ["trsk", "upw1"])
+@pytest.mark.parametrize("level,case", [(2, 2), (4, 3), (6, 2), (7, 3)])
+def test_fused_moist_stage_close_to_fp64(grid_at, level, case, advection):
+    """The fused FP32 moist stage at each tile size against the FP64 handle.
+    Four steps are sixteen evaluations of a few hundred FP32 roundings (6e-8
+    each), so 1e-5 of each field's norm bounds them; the cloud and rain water
+    begin at zero and are measured against the vapour they come from."""
+    from imodel_gb300.moist import FIELDS, Moist, moist_fields
+    g = grid_at(level)
+    f = moist_fields(g, case)
+    dt = min(900.0, 110.0 * 2.0 ** (8 - level))
+    out = []
+    for prec in ("fp64", "fp32"):
+        m = Moist(g, case, f, advection=advection, precision=prec)
+        m.set_state(f)
+        m.advance(dt, 4)
+        out.append(m.get_state())
+        m.close()
+    norm = {k: np.linalg.norm(out[0][k]) for k in FIELDS}
+    norm["hqc"] = norm["hqr"] = norm["hqv"]
+    for k in FIELDS:
+        assert np.linalg.norm(out[1][k] - out[0][k]) <= 1e-5 * norm[k], k
