@@ -82,9 +82,10 @@ __global__ void __launch_bounds__(kThr, kThr == 256 ? 3 : 4)
 // source.  After the last stage the own cells also form qv, qc, qr, which no
 // other cell reads.  In place of the tendency written and read back, two more
 // kernels that fetch indices, depths and velocities again and a third at the
-// end of the step: level 8 376 -> 280 us a step.
+// end of the step: level 8 376 -> 280 us a step, and 253 with the registers
+// held to three blocks on an SM (a few bytes spilled).
 template <int kStage, int kThr>
-__global__ void __launch_bounds__(kThr, 2)
+__global__ void __launch_bounds__(kThr, 3)
     k_moist_stage32(TileDev D, MoistArgs32 A, float grav, float erad, int pv_on, int mom_on) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t mbar[2];
