@@ -1750,6 +1750,8 @@ void moist_step64(Moist *X, double dt) {
         A.q_out[k] = out(st, q[0], q[1], q[2]);
       }
       A.uphi = X->uphi;
+      A.dts = st < 2 ? dt * 0.5 : dt;
+      A.hgrav = H->M.grav * 0.5;
       A.rdt = dt >= 0x1p-500 && dt <= 0x1p500 ? 1.0 / dt : std::nan("");
       A.gthb = X->gthb;
       A.q0ex = X->ex20;

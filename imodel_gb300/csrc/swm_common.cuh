@@ -321,6 +321,8 @@ struct MoistArgs {
   // q0 exp(20 theta) [nv]; qv, qc, qr of the last step [nv]
   const double *gthb = nullptr, *q0ex = nullptr, *qv = nullptr, *qc = nullptr, *qr = nullptr;
   double rdt = 0.0;  // 1 / dt, for div_by
+  double dts = 0.0;  // dt / 2 in stages 0 and 1, dt in the others
+  double hgrav = 0.0;  // grav / 2
   int *flags = nullptr;
 };
 // gthb from theta and the topography (both frozen in a run); ex20 becomes
@@ -392,10 +394,13 @@ void launch_store_host(int n, const int32_t *o2n, const T *src, double *dst, dou
 // and quantity; result[kDiagQ] on the device.
 constexpr int kDiagQ = 12;
 constexpr int kMaxStencil = 10;  // slots of the TRSK stencil (swm_layout.h, kMaxSt)
-// threads per block of the FP64 kernels
-#ifndef BLOCK64
-#define BLOCK64 64
-#endif
+// Threads per block of the FP64 kernels over n items.  A small grid's blocks
+// are dealt out unevenly over the SMs' FP64 pipes, so below 100,000 items they
+// are single warps (level 5: 53.6 us a step against 57.7 with two; level 6 in the
+// pxt16 scheme, with counts on both sides of the line, 320 either way).  Large
+// grids of single warps reach the limit of 32 blocks on an SM (level 8: 1764
+// against 1648; four warps 1648, eight 1653).
+inline int block64(int n) { return n < 100000 ? 32 : 64; }
 constexpr int kRedBlocks = 608;   // 4 blocks per SM on 152 SMs
 constexpr int kRedThreads = 256;
 // result indices

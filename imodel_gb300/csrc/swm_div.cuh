@@ -6,7 +6,7 @@
 namespace imodel {
 
 // RN(1 / 6), rounded on the host
-constexpr double kThird2 = 1.0 / 6.0;
+constexpr double kSixth = 1.0 / 6.0;
 
 static __device__ __noinline__ double div_full(double a, double b) { return a / b; }
 

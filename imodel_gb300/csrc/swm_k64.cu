@@ -17,22 +17,22 @@ namespace {
 // constants.f90:45 -- eps = epsilon(1.) (float epsilon)
 constexpr double kEps = 1.1920928955078125e-07;
 
-// ode_rk4, swm.f90:2647-2678.  hdt = dt / 2: dt k / 2 and (dt / 2) k are the
-// same rounding (a power of two), and acc + 2 k is one fused operation with
-// an exact product.
+// ode_rk4, swm.f90:2647-2678.  dt is half the time step in stages 0 and 1: dt
+// k / 2 and (dt / 2) k are the same rounding (a power of two), and acc + 2 k
+// is one fused operation with an exact product.
 __device__ __forceinline__ double rk_stage(int stage, double k, double yn, double *acc,
                                            double dt) {
   if (stage == 0) {
     *acc = k;
-    return yn + (dt * 0.5) * k;
+    return yn + dt * k;
   } else if (stage == 1) {
     *acc = __fma_rn(2.0, k, *acc);
-    return yn + (dt * 0.5) * k;
+    return yn + dt * k;
   } else if (stage == 2) {
     *acc = __fma_rn(2.0, k, *acc);
     return yn + dt * k;
   }
-  return yn + div_by(dt * (*acc + k), 6.0, kThird2);
+  return yn + div_by(dt * (*acc + k), 6.0, kSixth);
 }
 
 // What bounds the FP64 step: GB300's FP64 pipe (2 operations per cycle and
@@ -45,7 +45,8 @@ __device__ __forceinline__ double rk_stage(int stage, double k, double yn, doubl
 //    d / 8 takes the product's 8 back (scaling by a power of two commutes
 //    with rounding);
 //  * products that both cells of an edge form alike are formed once per edge
-//    (2 u h_e d and the kinetic-energy term) and added with the cell's sign.
+//    (2 u h_e d and the kinetic-energy term) and added with the cell's sign;
+//  * sums begin with their first term (0 + x is x but for the sign of a zero).
 
 // Edge e's fluxes: uh2 = 2 u h_e (scalar_hx2ed :89-97, scalar_elem_product
 // :1546), fe = {2 u h_e d, (l d / 4) u^2}
@@ -84,9 +85,9 @@ __global__ void __launch_bounds__(256) k_tri64(DevMesh64 M, const double *__rest
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = M.nt;
   if (t >= nt) return;
-  double e = 0.0;
+  double e = u[M.t_ed[t]] * M.t_lt[t];
 #pragma unroll
-  for (int s = 0; s < 3; ++s) e = e + u[M.t_ed[s * nt + t]] * M.t_lt[s * nt + t];
+  for (int s = 1; s < 3; ++s) e = e + u[M.t_ed[s * nt + t]] * M.t_lt[s * nt + t];
   const double A = M.t_areag[t], rA = M.t_rareag[t];
   e = div_by(div_by(e, A, rA), M.erad, M.rerad);
   // with diffusion on: rel_vort_tr(u) (:780-827) is this sum before f is
@@ -109,8 +110,9 @@ __global__ void __launch_bounds__(256) k_tri64(DevMesh64 M, const double *__rest
     eta_t[t] = e;
     h_trs[t] = ht;
   } else {
+    ht = M.t_kite[t] * h[M.t_v[t]];
 #pragma unroll
-    for (int s = 0; s < 3; ++s) ht = ht + M.t_kite[s * nt + t] * h[M.t_v[s * nt + t]];
+    for (int s = 1; s < 3; ++s) ht = ht + M.t_kite[s * nt + t] * h[M.t_v[s * nt + t]];
     ht = div_by(ht, A, rA);
   }
   double q = 0.0;
@@ -296,9 +298,9 @@ __global__ void __launch_bounds__(256)
   after_prior<false>(h, u, fe, bern, yn, acc, yout, tend, coefdiv);
 #pragma unroll
   for (int j = 0; j < 6; ++j) f[j] = fe[es[j] & 0x7FFFFFFFu];
-  double d = 0.0, k = 0.0;
+  double d = flip(es[0], f[0].x), k = f[0].y;
 #pragma unroll
-  for (int j = 0; j < 6; ++j)
+  for (int j = 1; j < 6; ++j)
     if (j < n) {
       d = d + flip(es[j], f[j].x);
       k = k + f[j].y;
@@ -405,7 +407,8 @@ __global__ void __launch_bounds__(256) k_edge64(DevMesh64 M, const double *__res
     // is one (stq != NULL), else the TRSK average
     const int c3 = stq ? stq[s * ne + e] : -1;
     const double qs = c3 >= 0 ? q2[c3] + q2[c3] : qe + q2[k[s]];
-    if (s < ns) q = q + uh2[k[s]] * qs * d8[s] * w[s];
+    const double t = uh2[k[s]] * qs * d8[s] * w[s];
+    if (s < ns) q = s == 0 ? t : q + t;
   }
   q = div_by(q, l, rl);
   edge_update64(e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
@@ -1018,7 +1021,6 @@ __global__ void __launch_bounds__(kRedThreads) k_errors(DevMesh M, const T *__re
 }
 
 inline int nblocks(int n, int t) { return (n + t - 1) / t; }
-inline int block64(int) { return BLOCK64; }
 
 }  // namespace
 
@@ -1031,6 +1033,7 @@ void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_i
   // second application), before the edge kernel
   const Diffusion<double> &D = W.dif;
   const int sch = W.scheme;
+  if (stage == 0 || stage == 1) dt = dt * 0.5;  // rk_stage
   const int bt = block64(M.nt), bc = block64(M.nv), be = block64(M.ne);
   const int nbt = nblocks(M.nt, bt);
   launch_pdl(k_tri64, nbt + nblocks(M.ne, bt), bt, s, M, h_in, u_in, W.q_tr, W.pv_on, W.flags,

@@ -17,20 +17,21 @@ namespace {
 // constants.f90:45 -- eps = epsilon(1.) (float epsilon)
 constexpr double kEps = 1.1920928955078125e-07;
 
-// dt k / 2 as (dt / 2) k and acc + 2 k as one fused operation with an exact
-// product: the same roundings (moist_swm.f90:1880-1960)
+// dt (half the time step in stages 0 and 1) times k for dt k / 2, and acc + 2 k
+// as one fused operation with an exact product: the same roundings
+// (moist_swm.f90:1880-1960)
 __device__ __forceinline__ double rk_stage(int stage, double k, double yn, double *acc, double dt) {
   if (stage == 0) {
     *acc = k;
-    return yn + (dt * 0.5) * k;
+    return yn + dt * k;
   } else if (stage == 1) {
     *acc = __fma_rn(2.0, k, *acc);
-    return yn + (dt * 0.5) * k;
+    return yn + dt * k;
   } else if (stage == 2) {
     *acc = __fma_rn(2.0, k, *acc);
     return yn + dt * k;
   }
-  return yn + div_by(dt * (*acc + k), 6.0, kThird2);
+  return yn + div_by(dt * (*acc + k), 6.0, kSixth);
 }
 // Fortran max(0, x) / min(a, b) as std::max / std::min evaluate them
 __device__ __forceinline__ double fmax0(double x) { return (0.0 < x) ? x : 0.0; }
@@ -83,9 +84,9 @@ __global__ void __launch_bounds__(256) k_moist_edge(DevMesh64 M, MoistArgs A) {
     atomicOr(A.flags, 1);
   else
     gpi_oh = g / hed;
-  const double su = (M.grav * 0.5) * gpi_oh + A.gthb[e];
+  const double su = A.hgrav * gpi_oh + A.gthb[e];
   const double momeq = A.tend_u[e] + su;
-  A.u_out[e] = rk_stage(A.stage, momeq, A.yn_u[e], A.acc_u + e, A.dt);
+  A.u_out[e] = rk_stage(A.stage, momeq, A.yn_u[e], A.acc_u + e, A.dts);
 }
 
 // Cells: the divergence of each advected tracer's flux (div_hx, or
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(256) k_moist_cell(DevMesh64 M, MoistArgs A) {
   if (i >= nv) return;
   double hs[4] = {0.0, 0.0, 0.0, 0.0};
   if (A.swm) {
-    A.h_out[i] = rk_stage(A.stage, A.tend_h[i], A.yn_h[i], A.acc_h + i, A.dt);
+    A.h_out[i] = rk_stage(A.stage, A.tend_h[i], A.yn_h[i], A.acc_h + i, A.dts);
     const double hi = A.h_in[i];
     const double qs = A.q0ex[i] / ((hi + M.c_bt[i]) * M.grav);
     double gamma_v = 1.0 + kLscale * (20.0 * qs);
@@ -141,17 +142,19 @@ __global__ void __launch_bounds__(256) k_moist_cell(DevMesh64 M, MoistArgs A) {
       const double *uphi = A.uphi + static_cast<size_t>(k) * ne;
       double f[6];
 #pragma unroll
-      for (int j = 0; j < 6; ++j) f[j] = uphi[es[j] & 0x7FFFFFFFu];
+      for (int j = 0; j < 6; ++j) {
+        const double x = uphi[es[j] & 0x7FFFFFFFu];
+        f[j] = __hiloint2double(__double2hiint(x) ^ (es[j] & 0x80000000u), __double2loint(x));
+      }
+      d = f[0];
 #pragma unroll
-      for (int j = 0; j < 6; ++j)
-        if (j < n)
-          d = d + __hiloint2double(__double2hiint(f[j]) ^ (es[j] & 0x80000000u),
-                                   __double2loint(f[j]));
+      for (int j = 1; j < 6; ++j)
+        if (j < n) d = d + f[j];
       d = d * 0.5;
     }
     double t = -div_by(div_by(d, A_i, rA), M.erad, M.rerad);
     if (A.swm && k < 4) t = t + hs[k];
-    A.q_out[k][i] = rk_stage(A.stage, t, A.q_yn[k][i], A.q_acc[k] + i, A.dt);
+    A.q_out[k][i] = rk_stage(A.stage, t, A.q_yn[k][i], A.q_acc[k] + i, A.dts);
   }
 }
 
@@ -311,9 +314,9 @@ void launch_moist_consts32(const DevMesh &M, const float *th, float *ex20, float
 }
 
 void launch_moist_stage(const DevMesh64 &M, const MoistArgs &A, cudaStream_t s) {
-  const int b = BLOCK64;
-  launch_pdl(k_moist_edge, nblocks(M.ne, b), b, s, M, A);
-  launch_pdl(k_moist_cell, nblocks(M.nv, b), b, s, M, A);
+  const int be = block64(M.ne), bc = block64(M.nv);
+  launch_pdl(k_moist_edge, nblocks(M.ne, be), be, s, M, A);
+  launch_pdl(k_moist_cell, nblocks(M.nv, bc), bc, s, M, A);
 }
 
 void launch_moist_q(int nv, const double *h, const double *hqv, const double *hqc,
