@@ -3,20 +3,21 @@
 //
 // The kernel loops over "macro steps": the grid with the most steps steps
 // every time, the others are spread evenly over the same macro steps.  An RK
-// stage is one pass over work items, a tile of a grid (swm_layout.h) for a
-// group of its members: the block fetches the tile's records into shared
-// memory once and steps each member's tile there, as the fused stage of a
-// single run does (swm_tile.cuh, with the same bits).  No intermediate field
-// goes through memory and one grid-wide barrier ends the stage; the barrier's
-// wait is bounded and reports a timeout through the error flag instead of
-// waiting forever.  Each member's state is stored like a single run's.
+// stage is one pass over work items, a tile of a grid (swm_layout.h) for one
+// member or two: the block fetches the tile's records into shared memory and
+// steps the members' tile there, as the fused stage of a single run does
+// (swm_tile.cuh, with the same bits).  No intermediate field goes through
+// memory and one grid-wide barrier ends the stage; the barrier's wait is
+// bounded and reports a timeout through the error flag instead of waiting
+// forever.  Each member's state is stored like a single run's.
 //
-// Before, a stage was three phases (triangles, cells, edges) over members
-// interleaved in memory with a barrier after each, bound by the latency of
-// two dependent loads per entity at 32 warps per SM.  32 members on level 6
-// for 32 steps with 8 on level 7 for 64 took 54 ms (36 ms tuned) that way and
-// take 23.5 ms now, 5.4e9 member-cell-steps a second; what bounds them is the
-// issue of a tile's instructions, and a stage of few items the barrier.
+// What bounds a stage is the issue of a tile's instructions and the latency
+// of its phases (a stage of few items: the barrier), so two members are
+// stepped together in packed arithmetic (swm_pair.cuh), which takes 0.7 of the
+// instructions.  32 members on level 6 for 32 steps with 8 on level 7 for 64:
+// 54 ms with a stage in three phases (triangles, cells, edges) over members
+// interleaved in memory, 24.0 by tiles a member at a time, 19.2 by pairs,
+// 6.6e9 member-cell-steps a second.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -35,12 +36,19 @@ namespace {
 
 constexpr int kMaxGrids = 8;
 
+// Threads of a block, and the most cells of its tiles.  By pairs the smaller
+// blocks keep more of them at different phases: 32 members on level 6 with 8 on
+// level 7, 32 and 64 steps, 21.3 ms with 256 threads (two blocks an SM), 20.7
+// with 192 (three), 19.4 with 128 (five).
+template <class V>
 constexpr int kEnsThreads = 256;
+template <>
+constexpr int kEnsThreads<Pair> = 128;
 
 struct GridDev {
   TileDev tiles;
   int nv, ne;
-  int members, group, ngroups;  // members per work item, items per tile
+  int members, group, ngroups;  // members per work item (1 or 2), items per tile
   float h_ref, grav, erad;
   int nsteps;  // steps this launch
   float dt;
@@ -52,6 +60,7 @@ struct EnsArgs {
   int ngrids;
   int macro_steps;
   int pv_on, mom_on;
+  int single;  // no grid has more than one member
   GridDev g[kMaxGrids];
   int smem_block, smem_h, smem_u, smem_t;  // shared memory: the largest tile's sizes
   unsigned *bar_count;
@@ -99,21 +108,62 @@ __device__ __forceinline__ bool steps_now(int s, int n, int S) {
   return (static_cast<long long>(s + 1) * n) / S > (static_cast<long long>(s) * n) / S;
 }
 
-__global__ void __launch_bounds__(kEnsThreads, 3) k_ensemble(EnsArgs A) {
+// item number r of a stage (grids in `on`, tile by tile, members innermost)
+struct Item {
+  int k, tile, m;
+  __device__ __forceinline__ Item(const EnsArgs &A, unsigned on, int r) {
+    for (k = 0;; ++k) {
+      if (!(on >> k & 1u)) continue;
+      const int n = A.g[k].tiles.ntiles * A.g[k].ngroups;
+      if (r < n) break;
+      r -= n;
+    }
+    tile = r / A.g[k].ngroups;
+    m = (r - tile * A.g[k].ngroups) * A.g[k].group;
+  }
+};
+
+__device__ __forceinline__ TileFields member_fields(const GridDev &G, int st, int m) {
+  const size_t oh = static_cast<size_t>(m) * G.nv, ou = static_cast<size_t>(m) * G.ne;
+  TileFields F;
+  F.hd = (st == 0 ? G.yn_h : (st == 2 ? G.yb_h : G.ya_h)) + oh;
+  F.u = (st == 0 ? G.yn_u : (st == 2 ? G.yb_u : G.ya_u)) + ou;
+  F.h_out = (st == 0 ? G.ya_h : (st == 1 ? G.yb_h : (st == 2 ? G.ya_h : G.yn_h))) + oh;
+  F.u_out = (st == 0 ? G.ya_u : (st == 1 ? G.yb_u : (st == 2 ? G.ya_u : G.yn_u))) + ou;
+  F.yn_h = G.yn_h + oh;
+  F.yn_u = G.yn_u + ou;
+  F.acc_h = G.acc_h + oh;
+  F.acc_u = G.acc_u + ou;
+  F.tend_h = F.tend_u = nullptr;
+  // a member alone is stepped as both of a pair
+  const bool two = G.group == 2 && m + 1 < G.members;
+  F.mh = two ? G.nv : 0;
+  F.mu = two ? G.ne : 0;
+  return F;
+}
+
+// V: float, a member at a time, or Pair, two
+template <class V>
+__global__ void __launch_bounds__(kEnsThreads<V>, std::is_same<V, Pair>::value ? 5 : 3)
+    k_ensemble(EnsArgs A) {
+  constexpr int kThr = kEnsThreads<V>;
+  constexpr bool kPair = std::is_same<V, Pair>::value;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t mbar;
   if (static_cast<int>(blockIdx.x) == A.stall_block) return;  // test hook
   if (threadIdx.x == 0) tc05::mbar_init(&mbar, 1);
-  TileShared S;
+  TileSharedOf<V> S;
   S.block = smem;
-  S.sh = reinterpret_cast<float *>(smem + A.smem_block);
+  S.sh = reinterpret_cast<V *>(smem + A.smem_block);
   S.su = S.sh + A.smem_h;
   S.sq = S.su + A.smem_u;
   S.sb = S.sq + A.smem_t;
-  S.sz = S.sb + kEnsThreads;
+  S.sz = S.sb + kThr;
   __syncthreads();
   uint32_t parity = 0;
   unsigned epoch = 0;
+  int held = -1;  // block (Tile) of the records in shared memory, of grid held_k
+  int held_k = -1;
   for (int s = 0; s < A.macro_steps; ++s) {
     unsigned on = 0;
     int total = 0;
@@ -122,55 +172,49 @@ __global__ void __launch_bounds__(kEnsThreads, 3) k_ensemble(EnsArgs A) {
         on |= 1u << k;
         total += A.g[k].tiles.ntiles * A.g[k].ngroups;
       }
+    // the block's share: a tile's members follow one another, for its records;
+    // single members are dealt out, for the neighbours' state in the L2 (one
+    // member on level 7 with one on level 8: 458 -> 430 us a step)
+    int r0 = blockIdx.x, r1 = total, dr = gridDim.x;
+    if (!A.single) {
+      r0 = static_cast<int>(static_cast<long long>(total) * blockIdx.x / gridDim.x);
+      r1 = static_cast<int>(static_cast<long long>(total) * (blockIdx.x + 1) / gridDim.x);
+      dr = 1;
+    }
     for (int st = 0; st < 4; ++st) {
-      for (int item = blockIdx.x; item < total; item += gridDim.x) {
-        int k = 0, r = item;
-        for (;; ++k) {
-          if (!(on >> k & 1u)) continue;
-          const int n = A.g[k].tiles.ntiles * A.g[k].ngroups;
-          if (r < n) break;
-          r -= n;
-        }
-        const GridDev &G = A.g[k];
-        const int grp = r / G.tiles.ntiles, tile = r - grp * G.tiles.ntiles;
-        const Tile T(G.tiles.head + 5 * tile);
-        if (threadIdx.x == 0) {
-          // the last item's records have been read (barrier below); order
+      for (int r = r0; r < r1; r += dr) {
+        const Item I(A, on, r);
+        const GridDev &G = A.g[I.k];
+        const Tile T(G.tiles.head + 5 * I.tile);
+        const TileFields F = member_fields(G, st, I.m);
+        const bool fresh = held != T.block || held_k != I.k;
+        if (fresh && threadIdx.x == 0) {
+          // the last tile's records have been read (barrier below); order
           // those reads before the copy's writes
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           bulk_load(smem, G.tiles.data + T.block, T.bytes, &mbar);
         }
-        const int m0 = grp * G.group, m1 = min(G.members, m0 + G.group);
-        for (int m = m0; m < m1; ++m) {
-          const size_t oh = static_cast<size_t>(m) * G.nv, ou = static_cast<size_t>(m) * G.ne;
-          TileFields F;
-          F.hd = (st == 0 ? G.yn_h : (st == 2 ? G.yb_h : G.ya_h)) + oh;
-          F.u = (st == 0 ? G.yn_u : (st == 2 ? G.yb_u : G.ya_u)) + ou;
-          F.h_out = (st == 0 ? G.ya_h : (st == 1 ? G.yb_h : (st == 2 ? G.ya_h : G.yn_h))) + oh;
-          F.u_out = (st == 0 ? G.ya_u : (st == 1 ? G.yb_u : (st == 2 ? G.ya_u : G.yn_u))) + ou;
-          F.yn_h = G.yn_h + oh;
-          F.yn_u = G.yn_u + ou;
-          F.acc_h = G.acc_h + oh;
-          F.acc_u = G.acc_u + ou;
-          F.tend_h = F.tend_u = nullptr;
-          TileOwn<kEnsThreads> own;
-          own.load(T, F, st);
-          if (m == m0) {
-            if (!tc05::mbar_wait(&mbar, parity, A.flags, 32)) return;
-            parity ^= 1u;
-          }
-          own.rim(T, F, S);
-          own.store(T, F, S);
-          __syncthreads();
-          tile_triangles<kEnsThreads>(T, S, G.h_ref, A.pv_on, A.flags);
-          __syncthreads();
-          tile_cells(T, S, F, own, st, G.dt, G.grav, G.h_ref);
-          __syncthreads();
-          tile_edges(T, S, F, own, st, G.dt, G.erad, A.mom_on);
-          // the next member (or tile) overwrites depths, velocities, records;
-          // the edges read neither depths nor velocities
-          if (m + 1 == m1) __syncthreads();
+        held = T.block;
+        held_k = I.k;
+        TileOwn<kThr, V> own;
+        own.template load<!kPair>(T, F, st);
+        if (fresh) {
+          if (!tc05::mbar_wait(&mbar, parity, A.flags, 32)) return;
+          parity ^= 1u;
         }
+        own.rim(T, F, S);
+        own.store(T, F, S);
+        __syncthreads();
+        tile_triangles<kThr>(T, S, G.h_ref, A.pv_on, A.flags);
+        __syncthreads();
+        tile_cells(T, S, F, own, st, G.dt, G.grav, G.h_ref);
+        // by pairs there are no registers to hold these over the cells
+        if (kPair) own.load_edges(T, F, st);
+        __syncthreads();
+        tile_edges(T, S, F, own, st, G.dt, G.erad, A.mom_on);
+        // another tile's records may come over these; the edges read neither
+        // depths nor velocities
+        __syncthreads();
       }
       if (!grid_barrier(A, epoch++)) return;
     }
@@ -216,6 +260,7 @@ struct Ens {
   int *h_flags = nullptr;
   cudaStream_t stream = nullptr;
   int blocks_per_sm = 0;  // 0: as many as fit
+  bool pairs = false;     // members two at a time
   size_t smem = 0;
   EnsArgs args{};         // the parts that stay: sizes, members
   bool any_state = false;
@@ -292,6 +337,10 @@ int fill_tiles(Ens *E, const Layout &L, const TileLayout &T, const int4 *head, u
   return IMODEL_SWM_OK;
 }
 
+using EnsKernel = void (*)(EnsArgs);
+EnsKernel kernel(const Ens *E) { return E->pairs ? k_ensemble<Pair> : k_ensemble<float>; }
+int threads(const Ens *E) { return E->pairs ? kEnsThreads<Pair> : kEnsThreads<float>; }
+
 int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t *members) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
@@ -302,11 +351,23 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
   E->ngrids = ngrids;
   size_t maxn = 0;
   int rc;
-  int64_t cells = 0;
+  int64_t cells = 0, paired = 0;
+  for (int k = 0; k < ngrids; ++k) {
+    const int64_t nv = std::max(0, meshes[k].nv), m = std::max(0, members[k]);
+    cells += nv * m;
+    paired += nv * (m + m % 2);
+  }
+  // Two members at a time where there are tiles enough for every block, unless
+  // a third of what is stepped would be members alone.  us a step of the first
+  // grid, by pairs and singly: 4 members on level 4 with 2 on level 5 45, 40;
+  //  8 with 4 52, 58; 16 with 8 62, 70; 3 on level 6 with 3 on level 7
+  // 232, 244; 3 on level 6 with 1 on level 7 154, 115.
+  E->args.single = 1;
   for (int k = 0; k < ngrids; ++k)
-    cells += static_cast<int64_t>(std::max(0, meshes[k].nv)) * std::max(0, members[k]);
+    if (members[k] > 1) E->args.single = 0;
+  E->pairs = cells >= 60000 && 3 * paired <= 4 * cells;
   const int cap = std::min(tile_cap(static_cast<int>(std::min<int64_t>(cells, INT32_MAX))),
-                           kEnsThreads);
+                           threads(E));
   for (int k = 0; k < ngrids; ++k) {
     if (members[k] < 1) return fail(E, IMODEL_SWM_EINVAL, "every grid needs at least one member");
     Layout L;
@@ -327,6 +388,8 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
     W.nv = L.nv;
     W.ne = L.ne;
     W.members = G.members;
+    W.group = E->pairs ? 2 : 1;
+    W.ngroups = (W.members + W.group - 1) / W.group;
     W.grav = static_cast<float>(L.grav);
     W.erad = static_cast<float>(L.erad);
     // a tile's limits shrink with its size: one of these always fits
@@ -362,28 +425,12 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
       if ((rc = zalloc(E, b, static_cast<size_t>(L.ne) * M))) return rc;
   }
   EnsArgs &A = E->args;
-  E->smem = A.smem_block + sizeof(float) * (static_cast<size_t>(A.smem_h) + A.smem_u + A.smem_t +
-                                            kEnsThreads + 6 * kEnsThreads);
+  E->smem = A.smem_block + (E->pairs ? sizeof(Pair) : sizeof(float)) *
+                               (static_cast<size_t>(A.smem_h) + A.smem_u + A.smem_t +
+                                7 * threads(E));
   constexpr int kMost = 227 * 1024 - 1024;
   if (E->smem > kMost) return fail(E, IMODEL_SWM_EINVAL, "a tile does not fit an SM");
-  EK(cudaFuncSetAttribute(k_ensemble, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
-  // Members per work item: a tile's records come in once for all of them,
-  // but every block should have several items for the blocks to end a stage
-  // together.  One eighth of a block's tile-members is the step of the
-  // longest share over the mean.
-  int sms = 0, occ = 0;
-  EK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
-  EK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, kEnsThreads, E->smem));
-  int64_t visits = 0;
-  for (int k = 0; k < ngrids; ++k)
-    visits += static_cast<int64_t>(E->g[k].dev.tiles.ntiles) * members[k];
-  const int64_t want = std::max<int64_t>(1, visits / (8 * static_cast<int64_t>(sms) *
-                                                      std::max(1, occ)));
-  for (int k = 0; k < ngrids; ++k) {
-    GridDev &W = E->g[k].dev;
-    W.group = static_cast<int>(std::min<int64_t>(want, W.members));
-    W.ngroups = (W.members + W.group - 1) / W.group;
-  }
+  EK(cudaFuncSetAttribute(kernel(E), cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
   if ((rc = zalloc(E, &E->stage_h, maxn)) || (rc = zalloc(E, &E->stage_u, maxn)) ||
       (rc = zalloc(E, &E->bar, 1)) || (rc = zalloc(E, &E->flags, 1)))
     return rc;
@@ -429,13 +476,13 @@ int ens_launch(Ens *E, const double *dt, const int32_t *nsteps, int bps) {
   EK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   EK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   if (!coop) return fail(E, IMODEL_SWM_ECUDA, "device does not support cooperative launch");
-  EK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, kEnsThreads, E->smem));
+  EK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel(E), threads(E), E->smem));
   if (occ < 1) return fail(E, IMODEL_SWM_ECUDA, "ensemble kernel does not fit an SM");
   const int per_sm = (bps > 0 && bps <= occ) ? bps : occ;
   EK(cudaMemsetAsync(E->bar, 0, sizeof(unsigned), E->stream));
   void *args[] = {&A};
-  EK(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_ensemble), dim3(sms * per_sm),
-                                 dim3(kEnsThreads), args, E->smem, E->stream));
+  EK(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel(E)), dim3(sms * per_sm),
+                                 dim3(threads(E)), args, E->smem, E->stream));
   return IMODEL_SWM_OK;
 }
 
@@ -562,7 +609,7 @@ int imodel_swm_ensemble_tune(void *ens, const double *dt, int32_t nsteps, int32_
   float best = 1e30f;
   int bbps = E->blocks_per_sm, occ = 0;
   int rc = IMODEL_SWM_OK;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, imodel::k_ensemble, imodel::kEnsThreads,
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, imodel::kernel(E), imodel::threads(E),
                                                 E->smem);
   for (int bps = occ; bps >= 1 && rc == IMODEL_SWM_OK; --bps) {
     cudaEventRecord(e0, E->stream);
@@ -585,7 +632,7 @@ int imodel_swm_ensemble_tune(void *ens, const double *dt, int32_t nsteps, int32_
   cudaEventDestroy(e1);
   if (rc) return rc;
   E->blocks_per_sm = bbps;
-  choice[0] = imodel::kEnsThreads;
+  choice[0] = imodel::threads(E);
   choice[1] = bbps;
   choice[2] = 0;
   return IMODEL_SWM_OK;

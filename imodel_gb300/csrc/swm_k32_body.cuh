@@ -4,6 +4,7 @@
 // stage and the ensemble kernel (swm_tile.cuh).
 #pragma once
 #include "swm_common.cuh"
+#include "swm_pair.cuh"
 
 namespace imodel {
 
@@ -22,58 +23,67 @@ struct PriorWait {
 
 // Which products are fused into a sum is written out in the functions below,
 // not left to the compiler: the separate kernels, the fused stage and the
-// ensemble kernel give the same bits.
+// ensemble kernel give the same bits.  V: float, or Pair for two members.
 
 // ode_rk4 stage update (swm.f90:2647-2678) in FP32
-__device__ __forceinline__ float rk_stage32(int stage, float k, float yn, float *acc, float dt) {
+template <class V>
+__device__ __forceinline__ V rk_stage32(int stage, V k, V yn, V *acc, float dt) {
   if (stage == 0) {
     *acc = k;
-    return fmaf(0.5f * dt, k, yn);
+    return vfma(all<V>(0.5f * dt), k, yn);
   } else if (stage == 1) {
-    *acc = fmaf(2.0f, k, *acc);
-    return fmaf(0.5f * dt, k, yn);
+    *acc = vfma(all<V>(2.0f), k, *acc);
+    return vfma(all<V>(0.5f * dt), k, yn);
   } else if (stage == 2) {
-    *acc = fmaf(2.0f, k, *acc);
-    return fmaf(dt, k, yn);
+    *acc = vfma(all<V>(2.0f), k, *acc);
+    return vfma(all<V>(dt), k, yn);
   }
-  return fmaf(__fmul_rn(dt, __fadd_rn(*acc, k)), 1.0f / 6.0f, yn);
+  return vfma(vmul(all<V>(dt), vadd(*acc, k)), all<V>(1.0f / 6.0f), yn);
+}
+
+// scalar_elem_divide with its guard, swm_operators.f90:1604-1606
+__device__ __forceinline__ float guarded_div(float a, float b, int *flags) {
+  if (fabsf(b) < 1.1920928955078125e-12f) {
+    atomicOr(flags, 1);
+    return 0.0f;
+  }
+  return a / b;
+}
+__device__ __forceinline__ Pair guarded_div(Pair a, Pair b, int *flags) {
+  return Pair{guarded_div(a.x, b.x, flags), guarded_div(a.y, b.y, flags)};
 }
 
 // q_t = (curl u / A + f) / h_t  (vort_tr + scalar_hx2tr + scalar_elem_divide)
 // from a triangle's decoded record: edges, cells, circulation and kite
 // coefficients, Coriolis parameter; the sums run in slot order 0, 1, 2
-template <class Wait>
+template <class Wait, class V>
 __device__ __forceinline__ void tri_core(int t, const int (&ed)[3], const int (&cv)[3],
                                          const float (&circ)[3], const float (&kite)[3],
-                                         float f, const float *__restrict__ hd,
-                                         const float *__restrict__ u, float *__restrict__ q_tr,
+                                         float f, const V *__restrict__ hd,
+                                         const V *__restrict__ u, V *__restrict__ q_tr,
                                          float h_ref, int pv_on, int *flags,
                                          const float *__restrict__ kt = nullptr,
-                                         float *__restrict__ coefvort = nullptr,
-                                         float *__restrict__ ht_out = nullptr) {
+                                         typename ValueOf<V>::type *__restrict__ coefvort =
+                                             nullptr,
+                                         typename ValueOf<V>::type *__restrict__ ht_out =
+                                             nullptr) {
   IMODEL_WAIT(Wait, hd, u, q_tr, coefvort, ht_out);
-  float eta = f;
-  float ht = 0.0f, z = 0.0f;
+  V eta = all<V>(f);
+  V ht = all<V>(0.0f), z = all<V>(0.0f);
 #pragma unroll
   for (int s = 0; s < 3; ++s) {
-    const float us = u[ed[s]];
-    eta = fmaf(circ[s], us, eta);
-    z = fmaf(circ[s], us, z);
-    ht = fmaf(kite[s], hd[cv[s]], ht);
+    const V us = u[ed[s]], c = all<V>(circ[s]);
+    eta = vfma(c, us, eta);
+    z = vfma(c, us, z);
+    ht = vfma(all<V>(kite[s]), hd[cv[s]], ht);
   }
   // with diffusion on: K_tr times the relative vorticity
-  if (coefvort) coefvort[t] = kt[t] * z;
-  ht += h_ref;
+  if (coefvort) coefvort[t] = vmul(all<V>(kt[t]), z);
+  ht = padd(ht, all<V>(h_ref));
   // gass18: the depth at the triangle for the rhombus PV of the edges
   if (ht_out) ht_out[t] = ht;
-  float q = 0.0f;
-  if (pv_on) {
-    // scalar_elem_divide guard, swm_operators.f90:1604-1606
-    if (fabsf(ht) < 1.1920928955078125e-12f)
-      atomicOr(flags, 1);
-    else
-      q = eta / ht;
-  }
+  V q = all<V>(0.0f);
+  if (pv_on) q = guarded_div(eta, ht, flags);
   q_tr[t] = q;
 }
 
@@ -148,29 +158,33 @@ __device__ __forceinline__ void tri_body16(const DevMesh &M, int t, const float 
 // shares its weight and q_i + q_j between both its terms (five operations a
 // pair, where summing each edge's row took ten), and the pair's work cancels
 // exactly in the weight.  S(j) = R(0) + ... + R(j - 1), w = (S(j) - 1/2) - S(i).
-template <int N>
-__device__ __forceinline__ void trsk_cell(const float (&G)[6], const float (&qs)[6],
-                                          const float (&R)[6], unsigned tneg, float (&Z)[6]) {
-  float S[N], a[N];
-  S[0] = 0.0f;
+//
+// A row's terms with the smaller edges come first, all with a minus: they are
+// summed without it, and the sum turned once.
+template <int N, class V>
+__device__ __forceinline__ void trsk_cell(const V (&G)[6], const V (&qs)[6], const float (&R)[6],
+                                          unsigned tneg, V (&Z)[6]) {
+  V S[N], a[N];
+  S[0] = all<V>(0.0f);
 #pragma unroll
-  for (int j = 1; j < N; ++j) S[j] = S[j - 1] + R[j - 1];
+  for (int j = 1; j < N; ++j) S[j] = padd(S[j - 1], all<V>(R[j - 1]));
 #pragma unroll
-  for (int i = 0; i < N; ++i) a[i] = 0.0f;
+  for (int i = 0; i < N; ++i) a[i] = all<V>(0.0f);
 #pragma unroll
   for (int j = 1; j < N; ++j) {
-    const float Sh = S[j] - 0.5f;
+    const V Sh = padd(S[j], all<V>(-0.5f));
 #pragma unroll
     for (int i = 0; i < j; ++i) {
-      const float t = __fmul_rn(Sh - S[i], __fadd_rn(qs[i], qs[j]));
-      a[i] = fmaf(t, G[j], a[i]);
-      a[j] = fmaf(-t, G[i], a[j]);
+      const V t = vmul(psub(Sh, S[i]), vadd(qs[i], qs[j]));
+      a[i] = vfma(t, G[j], a[i]);
+      a[j] = vfma(t, G[i], a[j]);
     }
+    a[j] = vneg(a[j]);
   }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const float z = 0.5f * a[i];
-    Z[i] = ((tneg >> i) & 1u) ? -z : z;
+    const V z = pmul(all<V>(0.5f), a[i]);
+    Z[i] = ((tneg >> i) & 1u) ? vneg(z) : z;
   }
 }
 
@@ -179,36 +193,39 @@ __device__ __forceinline__ void trsk_cell(const float (&G)[6], const float (&qs)
 // returns the sum of the fluxes out of the cell.  kEdgePV: qt holds the PV of
 // the cell's edges (formed by the edge pre-pass, APVM's upwinding included)
 // instead of the PV of its triangles.
-template <bool kEdgePV = false, bool kZ = true>
-__device__ __forceinline__ float cell_terms(int i, uint32_t meta, const float (&R)[6],
-                                            const float2 (&kd)[6], const float (&ue)[6],
-                                            const float (&hn)[6], const float (&qt)[6], float hi,
-                                            float bt, float inva, float *__restrict__ bern,
-                                            float *__restrict__ zflux, float grav, float h_ref,
-                                            const float *__restrict__ kcv = nullptr,
-                                            float *__restrict__ coefdiv = nullptr) {
+template <bool kEdgePV = false, bool kZ = true, class V = float>
+__device__ __forceinline__ V cell_terms(int i, uint32_t meta, const float (&R)[6],
+                                        const float2 (&kd)[6], const V (&ue)[6],
+                                        const V (&hn)[6], const V (&qt)[6], V hi, float bt,
+                                        float inva, V *__restrict__ bern, V *__restrict__ zflux,
+                                        float grav, float h_ref,
+                                        const float *__restrict__ kcv = nullptr,
+                                        typename ValueOf<V>::type *__restrict__ coefdiv =
+                                            nullptr) {
   const int n = static_cast<int>(meta & 7u);
   const unsigned tneg = meta >> 8;
-  float G[6], qs[6];
-  float div = 0.0f, ke = 0.0f, du = 0.0f;
-  const float qlast = n == 6 ? qt[5] : (n == 5 ? qt[4] : (n == 4 ? qt[3] : qt[2]));
+  const V half = all<V>(0.5f), href = all<V>(h_ref);
+  V G[6], qs[6];
+  V div = all<V>(0.0f), ke = all<V>(0.0f), du = all<V>(0.0f);
+  const V qlast = n == 6 ? qt[5] : (n == 5 ? qt[4] : (n == 4 ? qt[3] : qt[2]));
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
     // F_e = u_e h_e, h_e the two-cell average (scalar_hx2ed)
-    const float F = __fmul_rn(ue[j], fmaf(0.5f, hi + hn[j], h_ref));
-    G[j] = __fmul_rn(F, kd[j].y);
+    const V F = vmul(ue[j], vfma(half, padd(hi, hn[j]), href));
+    const V d = all<V>(kd[j].y);
+    G[j] = vmul(F, d);
     // q_e: edge j lies between triangles j-1 and j (scalar_tr2ed)
-    qs[j] = kEdgePV ? qt[j] : 0.5f * ((j == 0 ? qlast : qt[j - 1]) + qt[j]);
-    div = __fadd_rn(div, G[j]);
-    ke = fmaf(kd[j].x, __fmul_rn(ue[j], ue[j]), ke);
-    du = fmaf(ue[j], kd[j].y, du);
+    qs[j] = kEdgePV ? qt[j] : pmul(half, padd(j == 0 ? qlast : qt[j - 1], qt[j]));
+    div = vadd(div, G[j]);
+    ke = vfma(all<V>(kd[j].x), vmul(ue[j], ue[j]), ke);
+    du = vfma(ue[j], d, du);
   }
   // with diffusion on: K times the divergence of u
-  if (coefdiv) coefdiv[i] = kcv[i] * (du * inva);
-  bern[i] = fmaf(grav, hi + bt, ke);
+  if (coefdiv) coefdiv[i] = vmul(all<V>(kcv[i]), vmul(du, all<V>(inva)));
+  bern[i] = vfma(all<V>(grav), padd(hi, all<V>(bt)), ke);
   // kZ false (dtred): the edges form their PV flux from the triangles
   if (kZ) {
-    float Z[6];
+    V Z[6];
     if (n == 6)
       trsk_cell<6>(G, qs, R, tneg, Z);
     else if (n == 5)
@@ -329,10 +346,10 @@ __device__ __forceinline__ void cell_body(const DevMesh &M, int i,
 }
 
 // -grad B - (Z_c1 + Z_c2) / l_e of an edge
-__device__ __forceinline__ float edge_terms(float b1, float b2, float z1, float z2, float g,
-                                            float erad) {
-  const float grad = __fmul_rn(b2 - b1, g);
-  return -fmaf(z1 + z2, __fmul_rn(g, erad), grad);
+template <class V>
+__device__ __forceinline__ V edge_terms(V b1, V b2, V z1, V z2, float g, float erad) {
+  const V grad = vmul(psub(b2, b1), all<V>(-g));
+  return vfma(padd(z1, z2), all<V>(__fmul_rn(-g, erad)), grad);
 }
 
 // grad_ed(K div x) - grad_ed_tg(K_tr zeta(x)) of an edge between the cells

@@ -41,74 +41,117 @@ struct Tile {
 };
 
 // one run's fields: stage input, y_n, accumulators, stage output (stage < 0:
-// the tendencies)
+// the tendencies); of two members, the first's, the second's mh and mu further
 struct TileFields {
   const float *hd, *u, *yn_h, *yn_u;
   float *acc_h, *acc_u, *h_out, *u_out, *tend_h, *tend_u;
+  size_t mh = 0, mu = 0;
 };
+// element i; the int index keeps it to one wide multiply-add an address
+template <class V>
+__device__ __forceinline__ V tile_load(const float *p, int i, size_t) {
+  return p[i];
+}
+template <>
+__device__ __forceinline__ Pair tile_load<Pair>(const float *p, int i, size_t m) {
+  return Pair{p[i], (p + m)[i]};
+}
+__device__ __forceinline__ void tile_store(float *p, int i, size_t, float v) { p[i] = v; }
+__device__ __forceinline__ void tile_store(float *p, int i, size_t m, Pair v) {
+  p[i] = v.x;
+  (p + m)[i] = v.y;
+}
 
 // the block's shared arrays: depths, velocities, PV, potential, flux terms
-struct TileShared {
+template <class V>
+struct TileSharedOf {
   unsigned char *block;  // the tile's block
-  float *sh, *su, *sq, *sb, *sz;
+  V *sh, *su, *sq, *sb, *sz;
 };
+using TileShared = TileSharedOf<float>;
 
 // What a thread of nthr reads in order, all of it in flight at once: the own
 // depth and velocities, y_n and the accumulators of the update.  kE rounds
 // cover a tile's own edges (three a cell); loops take what is left.
-template <int nthr>
+template <int nthr, class V = float>
 struct TileOwn {
   static constexpr int kE = 3;
-  float uo[kE], ynu[kE], acu[kE], ho, ynh, ach;
+  V uo[kE], ynu[kE], acu[kE], ho, ynh, ach;
+  // kEdges false: without y_n and the accumulators of the edges (load_edges)
+  template <bool kEdges = true>
   __device__ __forceinline__ void load(const Tile &T, const TileFields &F, int stage) {
     const int tid = threadIdx.x;
-    ho = ynh = ach = 0.0f;
+    ho = all<V>(0.0f), ynh = all<V>(0.0f), ach = all<V>(0.0f);
 #pragma unroll
     for (int r = 0; r < kE; ++r) {
       const int k = tid + r * nthr;
-      uo[r] = ynu[r] = acu[r] = 0.0f;
+      uo[r] = ynu[r] = acu[r] = all<V>(0.0f);
       if (k < T.ne) {
-        uo[r] = F.u[T.e0 + k];
-        if (stage >= 0) ynu[r] = F.yn_u[T.e0 + k];
-        if (stage >= 1) acu[r] = F.acc_u[T.e0 + k];
+        uo[r] = tile_load<V>(F.u, T.e0 + k, F.mu);
+        if (kEdges && stage >= 0) ynu[r] = tile_load<V>(F.yn_u, T.e0 + k, F.mu);
+        if (kEdges && stage >= 1) acu[r] = tile_load<V>(F.acc_u, T.e0 + k, F.mu);
       }
     }
     if (tid < T.nc) {
-      ho = F.hd[T.c0 + tid];
-      if (stage >= 0) ynh = F.yn_h[T.c0 + tid];
-      if (stage >= 1) ach = F.acc_h[T.c0 + tid];
+      ho = tile_load<V>(F.hd, T.c0 + tid, F.mh);
+      if (stage >= 0) ynh = tile_load<V>(F.yn_h, T.c0 + tid, F.mh);
+      if (stage >= 1) ach = tile_load<V>(F.acc_h, T.c0 + tid, F.mh);
+    }
+  }
+  __device__ __forceinline__ void load_edges(const Tile &T, const TileFields &F, int stage) {
+#pragma unroll
+    for (int r = 0; r < kE; ++r) {
+      const int k = threadIdx.x + r * nthr;
+      if (k < T.ne) {
+        ynu[r] = tile_load<V>(F.yn_u, T.e0 + k, F.mu);
+        if (stage >= 1) acu[r] = tile_load<V>(F.acc_u, T.e0 + k, F.mu);
+      }
     }
   }
   // the rim's depths and velocities (the block's index lists have arrived):
-  // fewer than two rounds of velocities, one of depths
-  __device__ __forceinline__ void rim(const Tile &T, const TileFields &F, const TileShared &S) {
+  // fewer than two rounds of velocities, one of depths; loops take the rest
+  __device__ __forceinline__ void rim_load(const Tile &T, const TileFields &F,
+                                           const TileSharedOf<V> &S, V (&v)[3]) {
     const int32_t *hx = reinterpret_cast<const int32_t *>(S.block);
     const int32_t *ux = reinterpret_cast<const int32_t *>(S.block + T.ux);
-    float v[3];
     const int k0 = threadIdx.x, k1 = k0 + nthr, nux = T.nu - T.ne, nhx = T.nh - T.nc;
-    if (k0 < nux) v[0] = F.u[ux[k0]];
-    if (k1 < nux) v[1] = F.u[ux[k1]];
-    if (k0 < nhx) v[2] = F.hd[hx[k0]];
+    if (k0 < nux) v[0] = tile_load<V>(F.u, ux[k0], F.mu);
+    if (k1 < nux) v[1] = tile_load<V>(F.u, ux[k1], F.mu);
+    if (k0 < nhx) v[2] = tile_load<V>(F.hd, hx[k0], F.mh);
+  }
+  __device__ __forceinline__ void rim_store(const Tile &T, const TileFields &F,
+                                            const TileSharedOf<V> &S, const V (&v)[3]) {
+    const int32_t *hx = reinterpret_cast<const int32_t *>(S.block);
+    const int32_t *ux = reinterpret_cast<const int32_t *>(S.block + T.ux);
+    const int k0 = threadIdx.x, k1 = k0 + nthr, nux = T.nu - T.ne, nhx = T.nh - T.nc;
     if (k0 < nux) S.su[T.ne + k0] = v[0];
     if (k1 < nux) S.su[T.ne + k1] = v[1];
     if (k0 < nhx) S.sh[T.nc + k0] = v[2];
-    for (int k = k1 + nthr; k < nux; k += nthr) S.su[T.ne + k] = F.u[ux[k]];
-    for (int k = k1; k < nhx; k += nthr) S.sh[T.nc + k] = F.hd[hx[k]];
+    for (int k = k1 + nthr; k < nux; k += nthr) S.su[T.ne + k] = tile_load<V>(F.u, ux[k], F.mu);
+    for (int k = k1; k < nhx; k += nthr) S.sh[T.nc + k] = tile_load<V>(F.hd, hx[k], F.mh);
   }
-  __device__ __forceinline__ void store(const Tile &T, const TileFields &F, const TileShared &S) {
+  __device__ __forceinline__ void rim(const Tile &T, const TileFields &F,
+                                      const TileSharedOf<V> &S) {
+    V v[3];
+    rim_load(T, F, S, v);
+    rim_store(T, F, S, v);
+  }
+  __device__ __forceinline__ void store(const Tile &T, const TileFields &F,
+                                        const TileSharedOf<V> &S) {
     const int tid = threadIdx.x;
 #pragma unroll
     for (int r = 0; r < kE; ++r)
       if (tid + r * nthr < T.ne) S.su[tid + r * nthr] = uo[r];
-    for (int k = tid + kE * nthr; k < T.ne; k += nthr) S.su[k] = F.u[T.e0 + k];
+    for (int k = tid + kE * nthr; k < T.ne; k += nthr)
+      S.su[k] = tile_load<V>(F.u, T.e0 + k, F.mu);
     if (tid < T.nc) S.sh[tid] = ho;
   }
 };
 
 // PV at the tile's triangles
-template <int nthr>
-__device__ __forceinline__ void tile_triangles(const Tile &T, const TileShared &S, float h_ref,
-                                               int pv_on, int *flags) {
+template <int nthr, class V>
+__device__ __forceinline__ void tile_triangles(const Tile &T, const TileSharedOf<V> &S,
+                                               float h_ref, int pv_on, int *flags) {
   const float4 *ta = reinterpret_cast<const float4 *>(S.block + T.triA);
   const uint4 *tb = reinterpret_cast<const uint4 *>(S.block + T.triB);
   const uint32_t *tc = reinterpret_cast<const uint32_t *>(S.block + T.triC);
@@ -122,8 +165,7 @@ __device__ __forceinline__ void tile_triangles(const Tile &T, const TileShared &
                        static_cast<int>(iv >> 20)};
     const float circ[3] = {a.x, a.y, a.z};
     const float kite[3] = {__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z)};
-    tri_core<NoWait>(k, ed, cv, circ, kite, a.w, S.sh, S.su, S.sq,
-                                      h_ref, pv_on, flags);
+    tri_core<NoWait>(k, ed, cv, circ, kite, a.w, S.sh, S.su, S.sq, h_ref, pv_on, flags);
   }
 }
 
@@ -134,15 +176,16 @@ struct NoCell {
   template <class... P>
   __device__ __forceinline__ void operator()(const P &...) const {}
 };
-template <int nthr, class Cell = NoCell>
-__device__ __forceinline__ void tile_cells(const Tile &T, const TileShared &S,
-                                           const TileFields &F, const TileOwn<nthr> &own,
+template <int nthr, class V, class Cell = NoCell>
+__device__ __forceinline__ void tile_cells(const Tile &T, const TileSharedOf<V> &S,
+                                           const TileFields &F, const TileOwn<nthr, V> &own,
                                            int stage, float dt, float grav, float h_ref,
                                            Cell cell = Cell{}) {
   const int tid = threadIdx.x;
   if (tid >= T.nz) return;
   const uint4 *slot = reinterpret_cast<const uint4 *>(S.block + T.slot) + tid;
-  float R[6], ue[6], hn[6], qt[6];
+  float R[6];
+  V ue[6], hn[6], qt[6];
   float2 kd[6];
   uint32_t word[6];
 #pragma unroll
@@ -159,18 +202,18 @@ __device__ __forceinline__ void tile_cells(const Tile &T, const TileShared &S,
   const float bt = reinterpret_cast<const float *>(S.block + T.bt)[tid];
   const bool mine = tid < T.nc;
   const float inva = mine ? reinterpret_cast<const float *>(S.block + T.inva)[tid] : 0.0f;
-  const float div = cell_terms(tid, meta, R, kd, ue, hn, qt, S.sh[tid], bt, inva, S.sb,
-                                       S.sz, grav, h_ref);
+  const V div = cell_terms(tid, meta, R, kd, ue, hn, qt, S.sh[tid], bt, inva, S.sb, S.sz, grav,
+                           h_ref);
   if (!mine) return;
-  const float masseq = __fmul_rn(-div, inva);
+  const V masseq = vmul(div, all<V>(-inva));
   if (stage < 0) {
-    F.tend_h[T.c0 + tid] = masseq;
+    tile_store(F.tend_h, T.c0 + tid, F.mh, masseq);
     cell(word, ue, kd, meta, bt, inva, 0.0f);
   } else {
-    float a = own.ach;
-    const float hnew = rk_stage32(stage, masseq, own.ynh, &a, dt);
-    F.h_out[T.c0 + tid] = hnew;
-    if (stage < 3) F.acc_h[T.c0 + tid] = a;
+    V a = own.ach;
+    const V hnew = rk_stage32(stage, masseq, own.ynh, &a, dt);
+    tile_store(F.h_out, T.c0 + tid, F.mh, hnew);
+    if (stage < 3) tile_store(F.acc_h, T.c0 + tid, F.mh, a);
     cell(word, ue, kd, meta, bt, inva, hnew);
   }
 }
@@ -180,43 +223,44 @@ __device__ __forceinline__ void tile_cells(const Tile &T, const TileShared &S,
 struct NoForce {
   __device__ __forceinline__ float operator()(int, int, int, float) const { return 0.0f; }
 };
-template <int nthr, class Force = NoForce>
-__device__ __forceinline__ void tile_edges(const Tile &T, const TileShared &S,
-                                           const TileFields &F, const TileOwn<nthr> &own,
+template <int nthr, class V, class Force = NoForce>
+__device__ __forceinline__ void tile_edges(const Tile &T, const TileSharedOf<V> &S,
+                                           const TileFields &F, const TileOwn<nthr, V> &own,
                                            int stage, float dt, float erad, int mom_on,
                                            Force force = Force{}) {
   const int tid = threadIdx.x;
   const uint2 *edge = reinterpret_cast<const uint2 *>(S.block + T.edge);
-  auto tendency = [&](int k) {
+  auto tendency = [&](int k) -> V {
     const uint2 w = edge[k];
     const int c1 = w.x & 1023u, c2 = w.x >> 13 & 1023u;
     const float g = __uint_as_float(w.y);
-    float m = edge_terms(S.sb[c1], S.sb[c2], S.sz[6 * c1 + (w.x >> 10 & 7u)],
-                         S.sz[6 * c2 + (w.x >> 23)], g, erad);
+    V m = edge_terms(S.sb[c1], S.sb[c2], S.sz[6 * c1 + (w.x >> 10 & 7u)],
+                     S.sz[6 * c2 + (w.x >> 23)], g, erad);
     if constexpr (!std::is_same<Force, NoForce>::value) m += force(k, c1, c2, g);
-    return mom_on ? m : 0.0f;
+    return mom_on ? m : all<V>(0.0f);
   };
-  auto update = [&](int k, float m, float yn, float ac) {
+  auto update = [&](int k, V m, V yn, V ac) {
     const int e = T.e0 + k;
     if (stage < 0) {
-      F.tend_u[e] = m;
+      tile_store(F.tend_u, e, F.mu, m);
     } else {
-      F.u_out[e] = rk_stage32(stage, m, yn, &ac, dt);
-      if (stage < 3) F.acc_u[e] = ac;
+      tile_store(F.u_out, e, F.mu, rk_stage32(stage, m, yn, &ac, dt));
+      if (stage < 3) tile_store(F.acc_u, e, F.mu, ac);
     }
   };
   // all reads of the rounds before their writes, which could alias them for
   // all the compiler knows
-  constexpr int kE = TileOwn<nthr>::kE;
-  float m[kE];
+  constexpr int kE = TileOwn<nthr, V>::kE;
+  V m[kE];
 #pragma unroll
-  for (int r = 0; r < kE; ++r) m[r] = tid + r * nthr < T.ne ? tendency(tid + r * nthr) : 0.0f;
+  for (int r = 0; r < kE; ++r)
+    m[r] = tid + r * nthr < T.ne ? tendency(tid + r * nthr) : all<V>(0.0f);
 #pragma unroll
   for (int r = 0; r < kE; ++r)
     if (tid + r * nthr < T.ne) update(tid + r * nthr, m[r], own.ynu[r], own.acu[r]);
   for (int k = tid + kE * nthr; k < T.ne; k += nthr)
-    update(k, tendency(k), stage >= 0 ? F.yn_u[T.e0 + k] : 0.0f,
-           stage >= 1 ? F.acc_u[T.e0 + k] : 0.0f);
+    update(k, tendency(k), stage >= 0 ? tile_load<V>(F.yn_u, T.e0 + k, F.mu) : all<V>(0.0f),
+           stage >= 1 ? tile_load<V>(F.acc_u, T.e0 + k, F.mu) : all<V>(0.0f));
 }
 
 }  // namespace imodel
