@@ -82,9 +82,10 @@ __device__ __forceinline__ float gelu(float z) {
   const float hz = 0.5f * z;
   return fmaf(hz, tanh_fast(u), hz);
 }
-__device__ __forceinline__ float gelu_grad(float z) {
-  const float u = fmaf(z * z, kGca, kGc) * z;
-  const float th = tanh_fast(u);
+__device__ __forceinline__ float gelu_tanh(float z) {
+  return tanh_fast(fmaf(z * z, kGca, kGc) * z);
+}
+__device__ __forceinline__ float gelu_grad(float z, float th) {
   return 0.5f * (1.0f + th) +
          0.5f * z * (1.0f - th * th) * 0.7978845608028654f * (1.0f + 3.0f * 0.044715f * z * z);
 }
@@ -120,24 +121,26 @@ __device__ __forceinline__ uint64_t gelu2x2(float z0, float z1) {
   return f2fma(z, f2pk(tanh_fast(u0), tanh_fast(u1)), z);
 }
 
-// row `r` of a K-major 16-bit operand with `kc` columns, from 64 FP32 values
-__device__ __forceinline__ void store_row64(uint8_t *op, int r, const float (&v)[64], int kc) {
+// columns [c0, c0 + 32) of row `r` of a K-major 16-bit operand with `kc`
+// columns, from 32 FP32 values
+__device__ __forceinline__ void store_row32(uint8_t *op, int r, int c0, const float (&v)[32],
+                                            int kc) {
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < 4; ++c) {
     uint4 q;
     q.x = pack2(v[8 * c + 0], v[8 * c + 1]);
     q.y = pack2(v[8 * c + 2], v[8 * c + 3]);
     q.z = pack2(v[8 * c + 4], v[8 * c + 5]);
     q.w = pack2(v[8 * c + 6], v[8 * c + 7]);
-    *reinterpret_cast<uint4 *>(op + kmaj_off(r, 8 * c, kc)) = q;
+    *reinterpret_cast<uint4 *>(op + kmaj_off(r, c0 + 8 * c, kc)) = q;
   }
 }
 
-// 64 FP32 columns [col, col+64) of this thread's TMEM lane
-__device__ __forceinline__ void ld64(uint32_t taddr, float (&v)[64]) {
+// 32 FP32 columns [col, col+32) of this thread's TMEM lane
+__device__ __forceinline__ void ld32(uint32_t taddr, float (&v)[32]) {
   float t[16];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < 2; ++q) {
     ld16(taddr + 16 * q, t);
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[16 * q + i] = t[i];
@@ -190,88 +193,140 @@ namespace imodel {
 namespace {
 
 // ---- fused forward + backward over a batch ---------------------------------
-// dynamic shared memory: B1 4K | B2 8K | B2T 8K | A2 16K | AW 32K | BW 32K.
+// dynamic shared memory: B1 4K | B2 8K | B2T 8K | A2 16K | AW 36K | BW 36K.
 // A3 (dZ2) takes A2's place, whose product has been waited for, and A1 the
-// last rows of BW, which are written after it: 100 KB, so that two CTAs share
+// last rows of BW, which are written after it: 108 KB, so that two CTAs share
 // an SM (and its 512 TMEM columns) and hide each other's waits for products
 // and rows.  A batch of 65,536 rows is 512 tiles: one CTA an SM took four
 // rounds of them.
-constexpr int TRN_SMEM = 4096 + 8192 + 8192 + 16384 + 32768 + 32768;
+// AW and BW are written down their columns, two bytes a lane: their core
+// matrices are 144 bytes apart along K, so that a warp's four lie in different
+// banks (at 128 bytes every store took four passes).
+constexpr int TRN_K = 144, TRN_ROWS = TM / 8 * TRN_K;  // strides of AW and BW
+__device__ __forceinline__ uint32_t trn_off(int r, int k) {
+  return static_cast<uint32_t>((r >> 3) * TRN_ROWS + (k >> 3) * TRN_K + (r & 7) * 16 + (k & 7) * 2);
+}
+constexpr int TRN_W = 16 * TRN_ROWS;  // bytes of AW, of BW
+constexpr int TRN_SMEM = 4096 + 8192 + 8192 + 16384 + 2 * TRN_W;
 constexpr int TRN_CTAS = 2;  // per SM
 
-__global__ void __launch_bounds__(TM, TRN_CTAS)
+// Sums over the warp of 32 values a lane: lane l returns with the l-th.  Each
+// exchange halves what a lane holds, 31 shuffles where a sum of its own for
+// every value takes 160; the tree, and so the rounding, is the same.
+__device__ __forceinline__ float warp_sum32(float (&p)[32], int lane) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < off; ++i) {
+      const float keep = up ? p[i + off] : p[i], send = up ? p[i] : p[i + off];
+      p[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  return p[0];
+}
+
+// Thread (row, half) of a tile: 32 of the 64 columns of a batch row (a warp
+// reads the TMEM lanes of its number modulo four), so that the products' waits
+// and the chains of a row are covered by 16 warps an SM.  Bound by latency: the
+// chain of a tile's four products and what lies between them.  A step of 65,536
+// rows with its reduction: 93 us with one CTA an SM, 56
+// with two CTAs, 40 with the columns' stores spread over the banks, the sums by
+// halves and the reduction in floats, 30 with two threads a row, the next rows
+// read ahead and the prologue before the wait for the kernel before.
+constexpr int TRN_THREADS = 2 * TM, HALF = NH / 2;
+
+__global__ void __launch_bounds__(TRN_THREADS, TRN_CTAS)
     k_mlp_train(Weights W, const uint16_t *__restrict__ x, const float *__restrict__ t,
                 const float *__restrict__ wts,
                 int64_t n, int64_t batch, uint64_t seed, float inv_batch,
                 float *__restrict__ partials, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t *B1 = smem, *B2 = B1 + 4096, *B2T = B2 + 8192, *A2 = B2T + 8192, *AW = A2 + 16384,
-          *BW = AW + 32768, *A3 = A2, *A1 = BW + 24576;
+          *BW = AW + TRN_W, *A3 = A2, *A1 = BW + TRN_W - 8192;
   __shared__ uint64_t mbar;
   __shared__ uint32_t tslot;
   __shared__ float sb1[NH], sb2[NH], sw3[NH];
+  __shared__ float sy[TM];  // a row's output: first half's sum, then all
   // per-warp sums of dw3, db3 and the loss: each warp adds only to its own
   // entries, and the warps are summed in a fixed order at the end, so the
   // partial gradients do not depend on the order in which warps finish
   __shared__ float sdw3[TM / 32][NH], sdb3[TM / 32], sloss[TM / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < 4096 / 16; i += TM)
-    reinterpret_cast<uint4 *>(B1)[i] = reinterpret_cast<const uint4 *>(W.w1img)[i];
-  for (int i = tid; i < 8192 / 16; i += TM) {
-    reinterpret_cast<uint4 *>(B2)[i] = reinterpret_cast<const uint4 *>(W.w2img)[i];
-    reinterpret_cast<uint4 *>(B2T)[i] = reinterpret_cast<const uint4 *>(W.w2timg)[i];
-  }
+  const int row = tid & (TM - 1), half = tid / TM, c0 = HALF * half;
   // AW rows 88..127 stay zero except row 96 (ones, for the bias sums)
-  for (int i = tid; i < 32768 / 16; i += TM) reinterpret_cast<uint4 *>(AW)[i] = make_uint4(0, 0, 0, 0);
-  if (tid < NH) {
-    sb1[tid] = W.p[OFF_B1 + tid];
-    sb2[tid] = W.p[OFF_B2 + tid];
-    sw3[tid] = W.p[OFF_W3 + tid];
+  for (int i = tid; i < TRN_W / 16; i += TRN_THREADS)
+    reinterpret_cast<uint4 *>(AW)[i] = make_uint4(0, 0, 0, 0);
+  if (tid < NH)
     for (int k = 0; k < TM / 32; ++k) sdw3[k][tid] = 0.0f;
-  }
   if (tid < TM / 32) {
     sdb3[tid] = 0.0f;
     sloss[tid] = 0.0f;
   }
-  const float b3 = W.p[OFF_B3];
-  __syncthreads();
-  *reinterpret_cast<uint16_t *>(AW + kmaj_off(96, tid, TM)) = bf16bits(1.0f);
   if (tid == 0) mbar_init(&mbar, 1);
   if (warp == 0) tmem_alloc(&tslot, 256);
+  const int64_t ntiles = (batch + TM - 1) / TM;
+  // a tile's row of the data set, read one tile ahead
+  bool live = false;
+  uint4 c[3];
+  float target = 0.0f, wt = 0.0f;
+  auto fetch = [&](int64_t tile) {
+    const int64_t pos = tile * TM + row;  // position in the batch
+    live = tile < ntiles && pos < batch;
+    c[0] = c[1] = c[2] = make_uint4(0, 0, 0, 0);
+    target = wt = 0.0f;
+    if (!live) return;
+    // seed 0: rows 0..batch-1 in order; otherwise rows drawn with replacement
+    const int64_t k = seed == 0 ? pos
+                                : static_cast<int64_t>(splitmix(seed ^ static_cast<uint64_t>(pos)) %
+                                                       static_cast<uint64_t>(n));
+    const uint4 *src = reinterpret_cast<const uint4 *>(x + k * NIN);
+    c[0] = src[0];
+    c[1] = src[1];
+    c[2] = src[2];
+    target = t[k];
+    wt = wts ? wts[k] : 1.0f;  // sample weight
+  };
+  fetch(blockIdx.x);
+  // the weights come from the kernel before
+  after_prior<true>(W.p, W.w1img, W.w2img, W.w2timg, partials);
+  for (int i = tid; i < 4096 / 16; i += TRN_THREADS)
+    reinterpret_cast<uint4 *>(B1)[i] = reinterpret_cast<const uint4 *>(W.w1img)[i];
+  for (int i = tid; i < 8192 / 16; i += TRN_THREADS) {
+    reinterpret_cast<uint4 *>(B2)[i] = reinterpret_cast<const uint4 *>(W.w2img)[i];
+    reinterpret_cast<uint4 *>(B2T)[i] = reinterpret_cast<const uint4 *>(W.w2timg)[i];
+  }
+  if (tid < NH) {
+    sb1[tid] = W.p[OFF_B1 + tid];
+    sb2[tid] = W.p[OFF_B2 + tid];
+    sw3[tid] = W.p[OFF_W3 + tid];
+  }
+  const float b3 = W.p[OFF_B3];
+  __syncthreads();
+  if (half == 0) *reinterpret_cast<uint16_t *>(AW + trn_off(96, row)) = bf16bits(1.0f);
   fence_async_smem();
   sync_cta();
   const uint32_t tmem = tslot;
-  const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+  const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
   const uint32_t id64 = idesc_bf16(TM, NH), id128 = idesc_bf16(TM, 128);
   uint32_t phase = 0;
   bool ok = true;
   bool first = true;
-  const int64_t ntiles = (batch + TM - 1) / TM;
   for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-    const int64_t pos = tile * TM + tid;  // position in the batch
-    const bool live = pos < batch;
-    // seed 0: rows 0..batch-1 in order; otherwise rows drawn with replacement
-    const int64_t row =
-        !live ? 0
-              : (seed == 0 ? pos
-                           : static_cast<int64_t>(splitmix(seed ^ static_cast<uint64_t>(pos)) %
-                                                  static_cast<uint64_t>(n)));
     // --- inputs: A1 (row-major) and X^T rows 64..87 of AW ----------------
-    uint4 c[3] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-    if (live) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(x + row * NIN);
-      c[0] = src[0];
-      c[1] = src[1];
-      c[2] = src[2];
+    if (half == 0) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4 *>(A1 + kmaj_off(row, 8 * q, K1)) = c[q];
+      *reinterpret_cast<uint4 *>(A1 + kmaj_off(row, 24, K1)) = make_uint4(0, 0, 0, 0);
+    } else {
+      const uint16_t *xs = reinterpret_cast<const uint16_t *>(c);
+#pragma unroll
+      for (int i = 0; i < NIN; ++i)
+        *reinterpret_cast<uint16_t *>(AW + trn_off(64 + i, row)) = xs[i];
     }
-    const float target = live ? t[row] : 0.0f;
-    const float wt = live ? (wts ? wts[row] : 1.0f) : 0.0f;  // sample weight
-#pragma unroll
-    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4 *>(A1 + kmaj_off(tid, 8 * q, K1)) = c[q];
-    *reinterpret_cast<uint4 *>(A1 + kmaj_off(tid, 24, K1)) = make_uint4(0, 0, 0, 0);
-    const uint16_t *xs = reinterpret_cast<const uint16_t *>(c);
-#pragma unroll
-    for (int i = 0; i < NIN; ++i) *reinterpret_cast<uint16_t *>(AW + kmaj_off(64 + i, tid, TM)) = xs[i];
+    const bool alive = live;
+    const float aim = target, weight = wt;
+    fetch(tile + gridDim.x);
     fence_async_smem();
     sync_cta();
     if (tid == 0) {
@@ -283,15 +338,15 @@ __global__ void __launch_bounds__(TM, TRN_CTAS)
     ok = __syncthreads_and(mbar_wait(&mbar, phase, err, ERR_WAIT)) != 0;
     phase ^= 1u;
     fence_after_sync();
-    float v[64];
+    float v[HALF];
     if (ok) {  // H1 = GELU(Z1 + b1): A2 (row-major) and AW rows 0..63 (H1^T)
-      ld64(tmem + lane_base, v);
+      ld32(tmem + lane_base + c0, v);
 #pragma unroll
-      for (int j = 0; j < NH; ++j) v[j] = gelu(v[j] + sb1[j]);
-      store_row64(A2, tid, v, NH);
+      for (int j = 0; j < HALF; ++j) v[j] = gelu(v[j] + sb1[c0 + j]);
+      store_row32(A2, row, c0, v, NH);
 #pragma unroll
-      for (int j = 0; j < NH; ++j)
-        *reinterpret_cast<uint16_t *>(AW + kmaj_off(j, tid, TM)) = live ? bf16bits(v[j]) : 0;
+      for (int j = 0; j < HALF; ++j)
+        *reinterpret_cast<uint16_t *>(AW + trn_off(c0 + j, row)) = alive ? bf16bits(v[j]) : 0;
     }
     fence_async_smem();
     sync_cta();
@@ -307,32 +362,49 @@ __global__ void __launch_bounds__(TM, TRN_CTAS)
     }
     fence_after_sync();
     if (ok) {  // output, loss, dZ2
-      ld64(tmem + lane_base + 64, v);
-      float h2[64];
+      ld32(tmem + lane_base + 64 + c0, v);
+      float h2[HALF];
       float yv = b3;
 #pragma unroll
-      for (int j = 0; j < NH; ++j) {
-        v[j] += sb2[j];
-        h2[j] = gelu(v[j]);
-        yv += h2[j] * sw3[j];
+      for (int j = 0; j < HALF; ++j) {
+        const float z = v[j] + sb2[c0 + j], th = gelu_tanh(z), hz = 0.5f * z;
+        h2[j] = fmaf(hz, th, hz);  // gelu(z)
+        v[j] = gelu_grad(z, th);
       }
-      const float r = live ? yv - target : 0.0f;
-      const float dy = 2.0f * wt * r * inv_batch;
-      float ls = warp_sum(wt * r * r), sdy = warp_sum(dy);
-      if (lane == 0) {
-        sloss[warp] += ls;
-        sdb3[warp] += sdy;
+      // the row's sum runs through the first half's columns, then the second's
+      if (half == 0) {
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) yv = fmaf(h2[j], sw3[j], yv);
+        sy[row] = yv;
+      }
+      __syncthreads();
+      if (half == 1) {
+        yv = sy[row];
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) yv = fmaf(h2[j], sw3[c0 + j], yv);
+        sy[row] = yv;
+      }
+      __syncthreads();
+      yv = sy[row];
+      const float r = alive ? yv - aim : 0.0f;
+      const float dy = 2.0f * weight * r * inv_batch;
+      if (half == 0) {
+        const float ls = warp_sum(weight * r * r), sdy = warp_sum(dy);
+        if (lane == 0) {
+          sloss[warp] += ls;
+          sdb3[warp] += sdy;
+        }
       }
 #pragma unroll
-      for (int j = 0; j < NH; ++j) {
-        const float dw = warp_sum(h2[j] * dy);
-        if (lane == 0) sdw3[warp][j] += dw;
-        v[j] = dy * sw3[j] * gelu_grad(v[j]);  // dZ2
+      for (int j = 0; j < HALF; ++j) {
+        h2[j] *= dy;
+        v[j] = dy * sw3[c0 + j] * v[j];  // dZ2
       }
-      store_row64(A3, tid, v, NH);
+      sdw3[warp & 3][c0 + lane] += warp_sum32(h2, lane);
+      store_row32(A3, row, c0, v, NH);
 #pragma unroll
-      for (int j = 0; j < NH; ++j)
-        *reinterpret_cast<uint16_t *>(BW + kmaj_off(j, tid, TM)) = bf16bits(v[j]);
+      for (int j = 0; j < HALF; ++j)
+        *reinterpret_cast<uint16_t *>(BW + trn_off(c0 + j, row)) = bf16bits(v[j]);
     }
     fence_async_smem();
     sync_cta();
@@ -348,21 +420,22 @@ __global__ void __launch_bounds__(TM, TRN_CTAS)
     }
     fence_after_sync();
     if (ok) {  // dZ1 = dH1 * GELU'(Z1): BW rows 64..127
-      float z1[64];
-      ld64(tmem + lane_base, z1);
-      ld64(tmem + lane_base + 64, v);
+      float z1[HALF];
+      ld32(tmem + lane_base + c0, z1);
+      ld32(tmem + lane_base + 64 + c0, v);
 #pragma unroll
-      for (int j = 0; j < NH; ++j) {
-        const float dz1 = v[j] * gelu_grad(z1[j] + sb1[j]);
-        *reinterpret_cast<uint16_t *>(BW + kmaj_off(64 + j, tid, TM)) = bf16bits(dz1);
+      for (int j = 0; j < HALF; ++j) {
+        const float z = z1[j] + sb1[c0 + j], dz1 = v[j] * gelu_grad(z, gelu_tanh(z));
+        *reinterpret_cast<uint16_t *>(BW + trn_off(64 + c0 + j, row)) = bf16bits(dz1);
       }
     }
     fence_async_smem();
     sync_cta();
     if (ok && tid == 0) {  // DW += AW BW^T over the 128 batch rows of the tile
       for (int s = 0; s < TM / 16; ++s)
-        mma(tmem + 128, smem_desc(smem_u32(AW) + 256 * s, 128, TM * 16),
-            smem_desc(smem_u32(BW) + 256 * s, 128, TM * 16), id128, (first && s == 0) ? 0u : 1u);
+        mma(tmem + 128, smem_desc(smem_u32(AW) + 2 * TRN_K * s, TRN_K, TRN_ROWS),
+            smem_desc(smem_u32(BW) + 2 * TRN_K * s, TRN_K, TRN_ROWS), id128,
+            (first && s == 0) ? 0u : 1u);
       commit(&mbar);
     }
     if (ok) {  // ok is uniform across the CTA
@@ -372,27 +445,27 @@ __global__ void __launch_bounds__(TM, TRN_CTAS)
     first = false;
     sync_cta();
   }
-  // partial gradients of this CTA
+  // partial gradients of this CTA, each half its columns
   float *out = partials + static_cast<int64_t>(blockIdx.x) * NPART;
   if (ok && !first) {
-    float dw[64];
+    float dw[HALF];
     // columns 0..63 of DW: rows 0..63 -> dW2^T; row 96 -> db2
-    ld64(tmem + lane_base + 128, dw);
-    if (tid < NH) {
+    ld32(tmem + lane_base + 128 + c0, dw);
+    if (row < NH) {
 #pragma unroll
-      for (int o = 0; o < NH; ++o) out[OFF_W2 + o * NH + tid] = dw[o];
-    } else if (tid == 96) {
+      for (int o = 0; o < HALF; ++o) out[OFF_W2 + (c0 + o) * NH + row] = dw[o];
+    } else if (row == 96) {
 #pragma unroll
-      for (int o = 0; o < NH; ++o) out[OFF_B2 + o] = dw[o];
+      for (int o = 0; o < HALF; ++o) out[OFF_B2 + c0 + o] = dw[o];
     }
     // columns 64..127: rows 64..87 -> dW1^T; row 96 -> db1
-    ld64(tmem + lane_base + 192, dw);
-    if (tid >= 64 && tid < 64 + NIN) {
+    ld32(tmem + lane_base + 192 + c0, dw);
+    if (row >= 64 && row < 64 + NIN) {
 #pragma unroll
-      for (int o = 0; o < NH; ++o) out[OFF_W1 + o * NIN + (tid - 64)] = dw[o];
-    } else if (tid == 96) {
+      for (int o = 0; o < HALF; ++o) out[OFF_W1 + (c0 + o) * NIN + (row - 64)] = dw[o];
+    } else if (row == 96) {
 #pragma unroll
-      for (int o = 0; o < NH; ++o) out[OFF_B1 + o] = dw[o];
+      for (int o = 0; o < HALF; ++o) out[OFF_B1 + c0 + o] = dw[o];
     }
   } else if (tid < NH) {
     for (int o = 0; o < NH; ++o) out[OFF_W2 + o * NH + tid] = 0.0f;
@@ -411,25 +484,55 @@ __global__ void __launch_bounds__(TM, TRN_CTAS)
   if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
-// Sum of the CTAs' partial gradients in a fixed order, in FP64: a block takes
-// 32 parameters, its warp w every kRed-th partial from w on, and the warps'
-// sums are added in order.  (One thread a parameter added 152 values in a row,
-// 27 us a step: FP64 additions are slow here and 5826 threads are few.)  With
-// ADAM the parameter's update follows at once, and its BF16 images with it.
+// Sum of the CTAs' partial gradients in a fixed order: a block takes 32
+// parameters, its warp w every kRed-th partial from w on, and the warps' sums
+// are added in order, in FP64.  A warp's own sum is kept in three floats that
+// take up each other's rounding errors (TwoSum, Knuth 1969): together they hold
+// the sum beyond FP64's precision, and FP64 additions, two a cycle and SM here,
+// bounded the kernel (16.1 us at 304 partials, 7.5 with these).  (One thread a parameter,
+// 152 values in a row, took 27.)  With ADAM the parameter's update follows at
+// once, and its BF16 images with it.
 constexpr int kRed = 16;
 struct AdamArgs {
   float *p, *m, *v, *loss;
   uint16_t *w1img, *w2img, *w2timg;
   float lr, b1, b2, eps, c1, c2;
 };
+// a = a + b rounded; returns the error of it
+__device__ __forceinline__ float two_sum(float &a, float b) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+  a = s;
+  return e;
+}
 template <bool ADAM>
 __global__ void __launch_bounds__(32 * kRed) k_reduce(const float *__restrict__ partials, int nblk,
                                                       float *__restrict__ grad, AdamArgs A) {
   __shared__ double part[kRed][32];
   const int lane = threadIdx.x & 31, w0 = threadIdx.x >> 5, q = blockIdx.x * 32 + lane;
+  after_prior<true>(partials, grad, A.p, A.m, A.v, A.loss, A.w1img, A.w2img, A.w2timg);
   double s = 0.0;
-  if (q < NPART)
-    for (int b = w0; b < nblk; b += kRed) s += partials[static_cast<int64_t>(b) * NPART + q];
+  if (q < NPART) {
+    const float *p = partials + q;
+    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
+    constexpr int kBatch = 10;  // loads in flight
+    for (int b = w0; b < nblk; b += kBatch * kRed) {
+      float x[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        x[k] = b + k * kRed < nblk ? p[static_cast<int64_t>(b + k * kRed) * NPART] : 0.0f;
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        const float e = two_sum(s0, x[k]);
+        s2 += two_sum(s1, e);
+      }
+    }
+    s = static_cast<double>(s0) + (static_cast<double>(s1) + static_cast<double>(s2));
+    if (!isfinite(s)) {  // an infinity, or a sum beyond FP32's range
+      s = 0.0;
+      for (int b = w0; b < nblk; b += kRed) s += p[static_cast<int64_t>(b) * NPART];
+    }
+  }
   part[w0][lane] = s;
   __syncthreads();
   if (w0 != 0 || q >= NPART) return;
@@ -522,15 +625,14 @@ int run_grad(Mlp *P, const uint16_t *x, const float *t, const float *w, int64_t 
              uint64_t seed, const AdamArgs *A) {
   const int64_t ntiles = (batch + TM - 1) / TM;
   const int nblk = static_cast<int>(std::min<int64_t>(ntiles, TRN_CTAS * P->sms));
-  k_mlp_train<<<nblk, TM, TRN_SMEM, P->stream>>>(weights(P), x, t, w, n, batch, seed,
-                                                 1.0f / static_cast<float>(batch), P->partials,
-                                                 P->d_err);
+  launch_pdl_smem(k_mlp_train, nblk, TRN_THREADS, TRN_SMEM, P->stream, weights(P), x, t, w, n, batch, seed,
+                  1.0f / static_cast<float>(batch), P->partials, P->d_err);
   MK(cudaGetLastError());
   constexpr int blocks = (NPART + 31) / 32;
   if (A)
-    k_reduce<true><<<blocks, 32 * kRed, 0, P->stream>>>(P->partials, nblk, nullptr, *A);
+    launch_pdl(k_reduce<true>, blocks, 32 * kRed, P->stream, P->partials, nblk, nullptr, *A);
   else
-    k_reduce<false><<<blocks, 32 * kRed, 0, P->stream>>>(P->partials, nblk, P->g, AdamArgs{});
+    launch_pdl(k_reduce<false>, blocks, 32 * kRed, P->stream, P->partials, nblk, P->g, AdamArgs{});
   MK(cudaGetLastError());
   return IMODEL_SWM_OK;
 }
