@@ -49,6 +49,12 @@ struct Handle {
   int *d_flags = nullptr;
   int *h_flags = nullptr;      // pinned
   double *h_result = nullptr;  // pinned
+  // small states (kSmallState) pass through one page-locked area (h, then u),
+  // got on the first such call: a kernel reads or writes it over the host link
+  double *h_small = nullptr;
+  bool small_none = false;  // it was refused: pageable copies instead
+  bool small_busy = false;  // work that uses it may be in flight
+  double *out_h = nullptr, *out_u = nullptr;  // where read_flags copies it to
   Work<double> W64{};
   Work<float> W32{};
   cudaStream_t stream = nullptr;
@@ -213,6 +219,7 @@ int alloc_work(Handle *H, Work<T> &W) {
 }
 
 int set_error(Handle *H, int code, const std::string &msg) {
+  H->out_h = H->out_u = nullptr;  // the caller's arrays are not the next call's
   H->err = msg;
   return code;
 }
@@ -280,6 +287,48 @@ void *host_view(Handle *H, const void *p, size_t bytes) {
   return static_cast<char *>(a.devicePointer);
 }
 
+// Up to this many bytes of state the calls for pageable copies cost more than
+// copying once more on the host.  us, by the page-locked area and by pageable
+// copies: tendency at level 3 (26 KB) FP64 34, 73; set and get at level 5
+// (328 KB) 27 and 31, 49 and 46; at level 6 (1.3 MB) 85 and 77, 57 and 53.
+constexpr size_t kSmallState = 512 * 1024;
+
+HostMap host_map(const Handle *H) { return {H->nv, H->ne, H->d_cell_o2n, H->d_edge_o2n}; }
+
+// the page-locked area, idle, for a small state; nullptr for a large one
+double *small_area(Handle *H) {
+  const size_t bytes = sizeof(double) * (static_cast<size_t>(H->nv) + H->ne);
+  if (bytes > kSmallState || H->small_none) return nullptr;
+  if (!H->h_small && cudaMallocHost(&H->h_small, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    H->h_small = nullptr;
+    H->small_none = true;
+    return nullptr;
+  }
+  if (H->small_busy && cudaStreamSynchronize(H->stream) != cudaSuccess) return nullptr;
+  H->small_busy = true;
+  H->out_h = H->out_u = nullptr;
+  return H->h_small;
+}
+double *small_in(Handle *H, const double *h, const double *u) {
+  double *p = small_area(H);
+  if (p) {
+    std::memcpy(p, h, sizeof(double) * H->nv);
+    std::memcpy(p + H->nv, u, sizeof(double) * H->ne);
+  }
+  return p;
+}
+// h, u: the caller's arrays, which read_flags fills
+double *small_out(Handle *H, double *h, double *u) {
+  // the area's input is read by work in front in the same stream
+  double *p = H->small_busy && H->h_small && !H->out_h ? H->h_small : small_area(H);
+  if (p) {
+    H->out_h = h;
+    H->out_u = u;
+  }
+  return p;
+}
+
 // host FP64 arrays (reference order) -> device state yn and the
 // "last stage input" ya, as after the reference's initial tendency call
 // (swm.f90:214)
@@ -321,22 +370,22 @@ int load_state(Handle *H, const double *h, const double *u, bool new_run) {
   }
   const double *hz = static_cast<const double *>(host_view(H, h, sizeof(double) * H->nv));
   const double *uz = static_cast<const double *>(host_view(H, u, sizeof(double) * H->ne));
+  if (!(hz && uz) && (hz = small_in(H, h, u))) uz = hz + H->nv;
   if (hz && uz) {
-    // page-locked arrays: one kernel per array reads them over the host link
-    // in order and writes yn and ya in device order (no staging copy)
-    // (and, with the learned correction on, the guard's checkpoint)
+    // page-locked arrays, or a small state in the handle's own: a kernel
+    // reads them over the host link in order and writes yn and ya in device
+    // order (no staging copy) (and, with the learned correction on, the
+    // guard's checkpoint)
     if (H->precision == IMODEL_SWM_FP64) {
       Work<double> &W = H->W64;
-      launch_load_host<double>(H->nv, H->d_cell_o2n, hz, W.yn_h, W.ya_h, nullptr, 0.0, H->stream);
-      launch_load_host<double>(H->ne, H->d_edge_o2n, uz, W.yn_u, W.ya_u, nullptr, 0.0, H->stream);
+      launch_load_host<double>(host_map(H), hz, uz, {W.yn_h, W.ya_h, nullptr},
+                               {W.yn_u, W.ya_u, nullptr}, 0.0, H->stream);
       H->ck_fresh = false;
     } else {
       Work<float> &W = H->W32;
       const bool ck = H->learned_on;
-      launch_load_host(H->nv, H->d_cell_o2n, hz, W.yn_h, W.ya_h, ck ? H->ck_h : nullptr,
-                       H->h_ref, H->stream);
-      launch_load_host(H->ne, H->d_edge_o2n, uz, W.yn_u, W.ya_u, ck ? H->ck_u : nullptr, 0.0,
-                       H->stream);
+      launch_load_host<float>(host_map(H), hz, uz, {W.yn_h, W.ya_h, ck ? H->ck_h : nullptr},
+                              {W.yn_u, W.ya_u, ck ? H->ck_u : nullptr}, H->h_ref, H->stream);
       H->ck_fresh = ck;
     }
   } else if (H->precision == IMODEL_SWM_FP64) {
@@ -374,15 +423,16 @@ int load_state(Handle *H, const double *h, const double *u, bool new_run) {
 int store_state(Handle *H, double *h, double *u) {
   double *hz = static_cast<double *>(host_view(H, h, sizeof(double) * H->nv));
   double *uz = static_cast<double *>(host_view(H, u, sizeof(double) * H->ne));
+  if (!(hz && uz) && (hz = small_out(H, h, u))) uz = hz + H->nv;
   if (hz && uz) {
     // page-locked arrays: written in order over the host link by the
     // kernels that undo the permutation (no staging copy)
     if (H->precision == IMODEL_SWM_FP64) {
-      launch_store_host(H->nv, H->d_cell_o2n, H->W64.yn_h, hz, 0.0, H->d_flags, H->stream);
-      launch_store_host(H->ne, H->d_edge_o2n, H->W64.yn_u, uz, 0.0, H->d_flags, H->stream);
+      launch_store_host<double>(host_map(H), H->W64.yn_h, H->W64.yn_u, hz, uz, 0.0, H->d_flags,
+                                H->stream);
     } else {
-      launch_store_host(H->nv, H->d_cell_o2n, H->W32.yn_h, hz, H->h_ref, H->d_flags, H->stream);
-      launch_store_host(H->ne, H->d_edge_o2n, H->W32.yn_u, uz, 0.0, H->d_flags, H->stream);
+      launch_store_host<float>(host_map(H), H->W32.yn_h, H->W32.yn_u, hz, uz, H->h_ref, H->d_flags,
+                               H->stream);
     }
     CK(cudaGetLastError());
     return IMODEL_SWM_OK;
@@ -404,10 +454,16 @@ int store_state(Handle *H, double *h, double *u) {
 
 // reads and clears the device flags (synchronising the stream)
 int read_flags(Handle *H, int *f) {
-  CK(cudaMemcpyAsync(H->h_flags, H->d_flags, sizeof(int), cudaMemcpyDeviceToHost, H->stream));
-  CK(cudaMemsetAsync(H->d_flags, 0, sizeof(int), H->stream));
+  launch_take_flags(H->d_flags, H->h_flags, H->stream);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(H->stream));
   *f = *H->h_flags;
+  if (H->out_h) {
+    std::memcpy(H->out_h, H->h_small, sizeof(double) * H->nv);
+    std::memcpy(H->out_u, H->h_small + H->nv, sizeof(double) * H->ne);
+  }
+  H->out_h = H->out_u = nullptr;
+  H->small_busy = false;
   return IMODEL_SWM_OK;
 }
 
@@ -953,6 +1009,7 @@ void destroy(Handle *H) {
   if (H->stream) cudaStreamSynchronize(H->stream);
   for (void *p : H->allocs) cudaFree(p);
   if (H->h_flags) cudaFreeHost(H->h_flags);
+  if (H->h_small) cudaFreeHost(H->h_small);
   if (H->h_result) cudaFreeHost(H->h_result);
   if (H->side) cudaStreamSynchronize(H->side);
   if (H->ev_steps) cudaEventDestroy(H->ev_steps);
@@ -1085,6 +1142,7 @@ int imodel_swm_set_state(void *handle, const double *h, const double *u) {
   if (rc) return rc;
   if (cudaStreamSynchronize(H->stream) != cudaSuccess)
     return imodel::set_error(H, IMODEL_SWM_ECUDA, "stream synchronize failed");
+  H->small_busy = false;
   return IMODEL_SWM_OK;
 }
 
@@ -1123,12 +1181,35 @@ int imodel_swm_tendency(void *handle, const double *h, const double *u, double *
     H->h_ref = static_cast<double>(H->W32.h_ref);
     H->href_fixed = true;
   }
+  // the tendency input becomes the "last stage input" the diagnostics use
+  if (double *z = imodel::small_in(H, h, u)) {
+    const imodel::HostMap N = imodel::host_map(H);
+    if (H->precision == IMODEL_SWM_FP64) {
+      auto &W = H->W64;
+      imodel::launch_load_host<double>(N, z, z + H->nv, {nullptr, W.ya_h, nullptr},
+                                       {nullptr, W.ya_u, nullptr}, 0.0, H->stream);
+      imodel::launch_stage64(H->M, W, W.ya_h, W.ya_u, nullptr, nullptr, -1, 0.0, H->stream);
+      z = imodel::small_out(H, masseq, momeq);
+      imodel::launch_store_host<double>(N, W.tend_h, W.tend_u, z, z + H->nv, 0.0, nullptr,
+                                        H->stream);
+    } else {
+      auto &W = H->W32;
+      imodel::launch_load_host<float>(N, z, z + H->nv, {nullptr, W.ya_h, nullptr},
+                                      {nullptr, W.ya_u, nullptr}, H->h_ref, H->stream);
+      imodel::launch_stage32(H->M, W, W.ya_h, W.ya_u, nullptr, nullptr, -1, 0.0f, H->stream);
+      z = imodel::small_out(H, masseq, momeq);
+      imodel::launch_store_host<float>(N, W.tend_h, W.tend_u, z, z + H->nv, 0.0, nullptr,
+                                       H->stream);
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return imodel::set_error(H, IMODEL_SWM_ECUDA, cudaGetErrorString(e));
+    return imodel::check_flags(H);
+  }
   cudaError_t e;
   e = cudaMemcpyAsync(H->d_stage_h, h, sizeof(double) * H->nv, cudaMemcpyHostToDevice, H->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(H->d_stage_u, u, sizeof(double) * H->ne, cudaMemcpyHostToDevice, H->stream);
   if (e != cudaSuccess) return imodel::set_error(H, IMODEL_SWM_ECUDA, cudaGetErrorString(e));
-  // the tendency input becomes the "last stage input" the diagnostics use
   if (H->precision == IMODEL_SWM_FP64) {
     auto &W = H->W64;
     imodel::launch_gather_in(H->nv, H->d_cell_n2o, H->d_stage_h, W.ya_h, 0.0, H->stream);

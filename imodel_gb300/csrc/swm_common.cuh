@@ -378,17 +378,26 @@ void launch_scatter_out(int n, const int32_t *n2o, const double *src, double *ds
                         int *flags, cudaStream_t s);
 void launch_scatter_out32(int n, const int32_t *n2o, const float *src, double *dst,
                           double shift, int *flags, cudaStream_t s);
-// the same conversions straight between a page-locked host array (reference
-// order, read or written in order over the host link) and the device state:
-// load writes yn, ya and (when not NULL) ck; store raises bit 1 of *flags on
-// NaN/Inf
+// the same conversions straight between page-locked host arrays (reference
+// order, read or written in order over the host link) and the device state, h
+// and u in one launch: load writes yn and ck (unless NULL) and ya; store raises
+// bit 1 of *flags (unless NULL) on NaN/Inf
+struct HostMap {
+  int nv, ne;
+  const int32_t *cell, *edge;  // reference order -> device order
+};
 template <class T>
-void launch_load_host(int n, const int32_t *o2n, const double *src, T *yn, T *ya, T *ck,
-                      double shift, cudaStream_t s);
+struct HostTo {
+  T *yn, *ya, *ck;
+};
 template <class T>
-void launch_store_host(int n, const int32_t *o2n, const T *src, double *dst, double shift,
-                       int *flags, cudaStream_t s);
-
+void launch_load_host(const HostMap &N, const double *h, const double *u, HostTo<T> to_h,
+                      HostTo<T> to_u, double shift, cudaStream_t s);
+template <class T>
+void launch_store_host(const HostMap &N, const T *src_h, const T *src_u, double *h, double *u,
+                       double shift, int *flags, cudaStream_t s);
+// *host = *flags, *flags = 0 (host: page-locked)
+void launch_take_flags(int *flags, int *host, cudaStream_t s);
 
 // Compensated FP64 integrals.  Scratch: partial sums, 2 doubles per block
 // and quantity; result[kDiagQ] on the device.

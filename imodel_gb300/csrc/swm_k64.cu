@@ -671,31 +671,44 @@ __global__ void k_scatter_out(int n, const int32_t *__restrict__ n2o, const T *_
   }
 }
 
-// j runs over the reference order, so that the host array is read (or
-// written) in order; the device side takes the permutation
+// j runs over the reference order (h, then u), so that the host arrays are read
+// (or written) in order; the device side takes the permutation
 template <class T>
-__global__ void k_load_host(int n, const int32_t *__restrict__ o2n,
-                            const double *__restrict__ src, T *__restrict__ yn,
-                            T *__restrict__ ya, T *__restrict__ ck, double shift) {
+__global__ void k_load_host(HostMap N, const double *__restrict__ h, const double *__restrict__ u,
+                            HostTo<T> to_h, HostTo<T> to_u, double shift) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) {
-    const T v = static_cast<T>(src[j] - shift);
-    const int i = o2n[j];
-    yn[i] = v;
-    ya[i] = v;
-    if (ck) ck[i] = v;
-  }
+  const bool cell = j < N.nv;
+  if (j >= N.nv + N.ne) return;
+  const int k = cell ? j : j - N.nv;
+  const double x = cell ? h[k] - shift : u[k];
+  const int i = cell ? N.cell[k] : N.edge[k];
+  after_prior<true>();
+  const T v = static_cast<T>(x);
+  const HostTo<T> to = cell ? to_h : to_u;
+  if (to.yn) to.yn[i] = v;
+  to.ya[i] = v;
+  if (to.ck) to.ck[i] = v;
 }
 
 template <class T>
-__global__ void k_store_host(int n, const int32_t *__restrict__ o2n, const T *__restrict__ src,
-                             double *__restrict__ dst, double shift, int *flags) {
+__global__ void k_store_host(HostMap N, const T *__restrict__ src_h, const T *__restrict__ src_u,
+                             double *__restrict__ h, double *__restrict__ u, double shift,
+                             int *flags) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) {
-    const double v = static_cast<double>(src[o2n[j]]) + shift;
-    dst[j] = v;
-    if (!isfinite(v)) atomicOr(flags, 2);
-  }
+  const bool cell = j < N.nv;
+  if (j >= N.nv + N.ne) return;
+  const int k = cell ? j : j - N.nv;
+  const int i = cell ? N.cell[k] : N.edge[k];
+  after_prior<true>(src_h, src_u, h, u);
+  const double v = cell ? static_cast<double>(src_h[i]) + shift : static_cast<double>(src_u[i]);
+  (cell ? h : u)[k] = v;
+  if (flags && !isfinite(v)) atomicOr(flags, 2);
+}
+
+__global__ void k_take_flags(int *flags, int *host) {
+  after_prior<true>(flags, host);
+  *host = *flags;
+  *flags = 0;
 }
 
 // vecrecon_trsk_tg, interpack.f90:3852-3976 (var%pos == 6)
@@ -1138,23 +1151,27 @@ void launch_scatter_out32(int n, const int32_t *n2o, const float *src, double *d
 }
 
 template <class T>
-void launch_load_host(int n, const int32_t *o2n, const double *src, T *yn, T *ya, T *ck,
-                      double shift, cudaStream_t s) {
-  k_load_host<T><<<nblocks(n, 256), 256, 0, s>>>(n, o2n, src, yn, ya, ck, shift);
+void launch_load_host(const HostMap &N, const double *h, const double *u, HostTo<T> to_h,
+                      HostTo<T> to_u, double shift, cudaStream_t s) {
+  launch_pdl(k_load_host<T>, nblocks(N.nv + N.ne, 256), 256, s, N, h, u, to_h, to_u, shift);
 }
 template <class T>
-void launch_store_host(int n, const int32_t *o2n, const T *src, double *dst, double shift,
-                       int *flags, cudaStream_t s) {
-  k_store_host<T><<<nblocks(n, 256), 256, 0, s>>>(n, o2n, src, dst, shift, flags);
+void launch_store_host(const HostMap &N, const T *src_h, const T *src_u, double *h, double *u,
+                       double shift, int *flags, cudaStream_t s) {
+  launch_pdl(k_store_host<T>, nblocks(N.nv + N.ne, 256), 256, s, N, src_h, src_u, h, u, shift,
+             flags);
 }
-template void launch_load_host<double>(int, const int32_t *, const double *, double *, double *,
-                                       double *, double, cudaStream_t);
-template void launch_load_host<float>(int, const int32_t *, const double *, float *, float *,
-                                      float *, double, cudaStream_t);
-template void launch_store_host<double>(int, const int32_t *, const double *, double *, double,
-                                        int *, cudaStream_t);
-template void launch_store_host<float>(int, const int32_t *, const float *, double *, double,
-                                       int *, cudaStream_t);
+template void launch_load_host<double>(const HostMap &, const double *, const double *,
+                                       HostTo<double>, HostTo<double>, double, cudaStream_t);
+template void launch_load_host<float>(const HostMap &, const double *, const double *,
+                                      HostTo<float>, HostTo<float>, double, cudaStream_t);
+template void launch_store_host<double>(const HostMap &, const double *, const double *, double *,
+                                        double *, double, int *, cudaStream_t);
+template void launch_store_host<float>(const HostMap &, const float *, const float *, double *,
+                                       double *, double, int *, cudaStream_t);
+void launch_take_flags(int *flags, int *host, cudaStream_t s) {
+  launch_pdl(k_take_flags, 1, 1, s, flags, host);
+}
 
 void launch_trsk_tangent(const DevMesh &M, const double *u, double *utg, cudaStream_t s) {
   k_trsk_tangent<<<nblocks(M.ne, 256), 256, 0, s>>>(M, u, utg);
