@@ -2,12 +2,14 @@
 //
 // A handle owns the device copy of the mesh layout, the state buffers of
 // classic RK4 and one CUDA stream.  One RK4 step is 4 stages x 3 or 4 kernels;
-// it is captured once into a CUDA graph per time step length and replayed.
+// it is captured into CUDA graphs (StepGraphs), per time step length, and replayed.
 #include <cuda.h>  // pointer-attribute types only; the driver call is resolved at run time
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <climits>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -22,6 +24,68 @@
 
 namespace imodel {
 namespace {
+
+// The launches of one step, captured for one time step length, and of kMany
+// steps: within a graph a step's first kernel starts as the last one's blocks
+// end (after_prior), between graphs after it has ended and the next graph has
+// been taken up.  us a step, by ones and by eights: the fused FP32 step at level
+// 5 14.4, 11.0, level 7 37.1, 33.9, level 8 153.5, 148.5; FP64 at level 5 53.4,
+// 52.4.  Making the second graph costs about 3.5 us a node, what 34 steps of the
+// four-kernel step save at level 5, or some 300 of the twelve-kernel FP64 step:
+// it is made once as many steps have been taken.
+struct StepGraphs {
+  static constexpr int kMany = 8;
+  cudaGraphExec_t one = nullptr, many = nullptr;
+  double dt = 0.0;
+  int64_t steps = 0, from = 0;  // steps with this dt; when `many` is made
+
+  void drop() {
+    if (one) cudaGraphExecDestroy(one);
+    if (many) cudaGraphExecDestroy(many);
+    one = many = nullptr;
+    steps = 0;
+  }
+  template <class F>
+  static cudaError_t capture(cudaStream_t s, int n, F step, cudaGraphExec_t *exec,
+                             size_t *nodes) {
+    cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    for (int k = 0; k < n; ++k) step();
+    cudaGraph_t g = nullptr;
+    if ((e = cudaStreamEndCapture(s, &g)) != cudaSuccess) return e;
+    e = cudaGraphGetNodes(g, nullptr, nodes);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
+    if (e != cudaSuccess) *exec = nullptr;
+    cudaGraphDestroy(g);
+    return e;
+  }
+  // n steps, each enqueued by step()
+  template <class F>
+  cudaError_t replay(cudaStream_t s, double dt_, int n, F step) {
+    size_t nodes = 0;
+    cudaError_t e = cudaSuccess;
+    if (!one || dt != dt_) {
+      drop();
+      if ((e = capture(s, 1, step, &one, &nodes)) != cudaSuccess) return e;
+      dt = dt_;
+      from = nodes <= 4 ? 32 : 32 * static_cast<int64_t>(nodes);
+    }
+    steps += n;
+    if (!many && n >= kMany && steps >= from) {
+      if (capture(s, kMany, step, &many, &nodes) != cudaSuccess) {
+        cudaGetLastError();  // go on with single steps
+        many = nullptr;
+        from = INT64_MAX;
+      }
+    }
+    int k = 0;
+    for (; many && k + kMany <= n; k += kMany)
+      if ((e = cudaGraphLaunch(many, s)) != cudaSuccess) return e;
+    for (; k < n; ++k)
+      if ((e = cudaGraphLaunch(one, s)) != cudaSuccess) return e;
+    return cudaSuccess;
+  }
+};
 
 struct Handle {
   // gass18 on a grid whose connecting edges do not follow the cells'
@@ -58,8 +122,7 @@ struct Handle {
   Work<double> W64{};
   Work<float> W32{};
   cudaStream_t stream = nullptr;
-  cudaGraphExec_t graph = nullptr;
-  double graph_dt = 0.0;
+  StepGraphs graphs;
   bool state_set = false;
   // learned TRSK correction: mode 1 the per-step network (FP32, cell-centred
   // variant), mode 2 the learned TRSK weights (kite fractions corrected once
@@ -243,26 +306,6 @@ void enqueue_step(Handle *H, double dt) {
   }
 }
 
-int ensure_graph(Handle *H, double dt) {
-  if (H->graph && H->graph_dt == dt) return IMODEL_SWM_OK;
-  if (H->graph) {
-    cudaGraphExecDestroy(H->graph);
-    H->graph = nullptr;
-  }
-  cudaGraph_t g = nullptr;
-  CK(cudaStreamBeginCapture(H->stream, cudaStreamCaptureModeThreadLocal));
-  enqueue_step(H, dt);
-  CK(cudaStreamEndCapture(H->stream, &g));
-  cudaError_t e = cudaGraphInstantiate(&H->graph, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    H->graph = nullptr;
-    return set_error(H, IMODEL_SWM_ECUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-  }
-  H->graph_dt = dt;
-  return IMODEL_SWM_OK;
-}
-
 // A device address of a caller's host array of `bytes` bytes when the array
 // lies wholly inside page-locked memory known to CUDA (cudaMallocHost,
 // cudaHostAlloc, cudaHostRegister) and mapped for this handle's device;
@@ -350,10 +393,7 @@ void learned_switch(Handle *H, bool on) {
     // 1's three kernels
     H->W32.tiles.ntiles = on ? H->ntiles : 0;
   }
-  if (H->graph) {
-    cudaGraphExecDestroy(H->graph);
-    H->graph = nullptr;
-  }
+  H->graphs.drop();
 }
 
 int load_state(Handle *H, const double *h, const double *u, bool new_run) {
@@ -614,10 +654,8 @@ int learned_guard(Handle *H, bool *tripped, int steps) {
 }
 
 int launch_steps(Handle *H, double dt, int nsteps) {
-  int rc = ensure_graph(H, dt);
-  if (rc) return rc;
   H->ck_fresh = false;
-  for (int k = 0; k < nsteps; ++k) CK(cudaGraphLaunch(H->graph, H->stream));
+  CK(H->graphs.replay(H->stream, dt, nsteps, [=] { enqueue_step(H, dt); }));
   return IMODEL_SWM_OK;
 }
 
@@ -1005,7 +1043,7 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
 
 void destroy(Handle *H) {
   if (!H) return;
-  if (H->graph) cudaGraphExecDestroy(H->graph);
+  H->graphs.drop();
   if (H->stream) cudaStreamSynchronize(H->stream);
   for (void *p : H->allocs) cudaFree(p);
   if (H->h_flags) cudaFreeHost(H->h_flags);
@@ -1408,14 +1446,14 @@ int imodel_swm_autotune(void *handle, double dt, int32_t nsteps, int32_t choice[
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   auto trial = [&](const imodel::Tune &t) -> float {
     W.tune = t;
-    if (H->graph) {
-      cudaGraphExecDestroy(H->graph);
-      H->graph = nullptr;
-    }
-    if (e != cudaSuccess || imodel::ensure_graph(H, dt)) return 1e30f;
-    if ((e = cudaGraphLaunch(H->graph, H->stream)) != cudaSuccess) return 1e30f;  // warm-up
+    H->graphs.drop();
+    auto run = [&](int n) {
+      return H->graphs.replay(H->stream, dt, n, [=] { imodel::enqueue_step(H, dt); });
+    };
+    if (e == cudaSuccess) e = run(1);  // warm-up
+    if (e != cudaSuccess) return 1e30f;
     cudaEventRecord(e0, H->stream);
-    for (int k = 0; k < nsteps && e == cudaSuccess; ++k) e = cudaGraphLaunch(H->graph, H->stream);
+    e = run(nsteps);
     cudaEventRecord(e1, H->stream);
     float ms = 1e30f;
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -1467,10 +1505,7 @@ int imodel_swm_autotune(void *handle, double dt, int32_t nsteps, int32_t choice[
       }
     }
   W.tune = best;
-  if (H->graph) {
-    cudaGraphExecDestroy(H->graph);
-    H->graph = nullptr;
-  }
+  H->graphs.drop();
   cpy(W.yn_h, sp, bh);
   cpy(W.yn_u, sp + bh, bu);
   cpy(W.ya_h, sp + bh + bu, bh);
@@ -1517,10 +1552,7 @@ int imodel_swm_set_tuning(void *handle, const int32_t choice[6]) {
     t.mlp_gather = choice[5];
   }
   H->W32.tune = t;
-  if (H->graph) {
-    cudaGraphExecDestroy(H->graph);
-    H->graph = nullptr;
-  }
+  H->graphs.drop();
   return IMODEL_SWM_OK;
 }
 
@@ -1538,10 +1570,7 @@ int imodel_swm_set_diffusion(void *handle, double k2, double k4) {
                      : imodel::setup_diffusion(H, H->W32, k2, k4, nullptr, nullptr);
   // the captured step no longer matches the options, whether or not the
   // set-up succeeded (a failure leaves the terms off)
-  if (H->graph) {
-    cudaGraphExecDestroy(H->graph);
-    H->graph = nullptr;
-  }
+  H->graphs.drop();
   return rc;
 }
 
@@ -1561,10 +1590,7 @@ int imodel_swm_set_diffusion_fields(void *handle, const double *k2_hx, const dou
   const int rc = H->precision == IMODEL_SWM_FP64
                      ? imodel::setup_diffusion(H, H->W64, 0.0, 0.0, k2_hx, k4_hx)
                      : imodel::setup_diffusion(H, H->W32, 0.0, 0.0, k2_hx, k4_hx);
-  if (H->graph) {
-    cudaGraphExecDestroy(H->graph);
-    H->graph = nullptr;
-  }
+  H->graphs.drop();
   return rc;
 }
 
@@ -1609,10 +1635,7 @@ int imodel_swm_set_apvm(void *handle, double pvspar, double dt) {
   // and 2 run before their cell kernel when APVM is on
   const int rc = fp32 ? imodel::setup_apvm(H, H->W32, pvspar, dt)
                       : imodel::setup_apvm(H, H->W64, pvspar, dt);
-  if (H->graph) {
-    cudaGraphExecDestroy(H->graph);
-    H->graph = nullptr;
-  }
+  H->graphs.drop();
   return rc;
 }
 
@@ -1679,8 +1702,7 @@ struct Moist {
   float *f_q[5][4] = {};
   bool state_set = false;
   // one step's launches, captured once per dt and replayed
-  cudaGraphExec_t graph = nullptr;
-  double graph_dt = 0.0;
+  imodel::StepGraphs graphs;
 };
 
 // host array (reference order, nv or ne values) -> device array (device order)
@@ -1847,30 +1869,11 @@ void moist_step64(Moist *X, double dt) {
   }
 }
 
-// X->graph: one step's launches for this dt (captured anew when dt changes)
-int moist_graph(Moist *X, double dt) {
-  Handle *H = X->H;
-  if (X->graph && X->graph_dt == dt) return IMODEL_SWM_OK;
-  if (X->graph) {
-    cudaGraphExecDestroy(X->graph);
-    X->graph = nullptr;
-  }
-  cudaGraph_t g = nullptr;
-  CK(cudaStreamBeginCapture(H->stream, cudaStreamCaptureModeThreadLocal));
+void moist_step(Moist *X, double dt) {
   if (X->fp32)
     moist_step32(X, dt);
   else
     moist_step64(X, dt);
-  CK(cudaStreamEndCapture(H->stream, &g));
-  cudaError_t e = cudaGraphInstantiate(&X->graph, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    X->graph = nullptr;
-    return imodel::set_error(H, IMODEL_SWM_ECUDA,
-                             std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-  }
-  X->graph_dt = dt;
-  return IMODEL_SWM_OK;
 }
 }  // namespace
 
@@ -2009,11 +2012,8 @@ int imodel_moist_advance(void *handle, double dt, int32_t nsteps) {
   if (nsteps < 0 || !(dt > 0) || !std::isfinite(dt))
     return imodel::set_error(H, IMODEL_SWM_EINVAL, "bad dt or nsteps");
   if (cudaSetDevice(H->device) != cudaSuccess) return IMODEL_SWM_ECUDA;
-  int rc = moist_graph(X, dt);
-  if (rc) return rc;
-  for (int step = 0; step < nsteps; ++step)
-    if (cudaGraphLaunch(X->graph, H->stream) != cudaSuccess)
-      return imodel::set_error(H, IMODEL_SWM_ECUDA, "cudaGraphLaunch failed");
+  const cudaError_t e = X->graphs.replay(H->stream, dt, nsteps, [=] { moist_step(X, dt); });
+  if (e != cudaSuccess) return imodel::set_error(H, IMODEL_SWM_ECUDA, cudaGetErrorString(e));
   if (cudaGetLastError() != cudaSuccess) return imodel::set_error(H, IMODEL_SWM_ECUDA, "launch failed");
   return imodel::check_flags(H);
 }
@@ -2045,7 +2045,7 @@ int imodel_moist_get_state(void *handle, double *const y[7]) {
 int imodel_moist_destroy(void *handle) {
   Moist *X = static_cast<Moist *>(handle);
   if (!X) return IMODEL_SWM_OK;
-  if (X->graph) cudaGraphExecDestroy(X->graph);
+  X->graphs.drop();
   imodel::destroy(X->H);
   delete X;
   return IMODEL_SWM_OK;
