@@ -39,7 +39,7 @@ struct DevMesh {
   const float2 *c_kd;   // [6][nv] {KE weight, ttgout*d}
   const uint2 *e_vs2;   // [ne] both cell words of an edge
   // the triangle records with 16-bit indices against per-warp bases
-  // (variant 2; swm_layout.h): {e0|e1, e2|c0, c1|c2, circ 0}, {circ 1,
+  // (variants 1 and 2; swm_layout.h): {e0|e1, e2|c0, c1|c2, circ 0}, {circ 1,
   // circ 2, kite 0, kite 1}, {kite 2, f} [nt], warp bases {edge, cell (-1:
   // use the 32-bit records)}
   const uint4 *t_c16A;
@@ -99,8 +99,7 @@ struct DevMesh64 : DevMesh {
 //   variant 1: triangle -> cell (cell-centred TRSK, writes the PV flux
 //              contribution of each cell edge) -> edge (sums two cells); one
 //              kernel over tiles where fused_stage() holds (the same bits)
-//   variant 2: variant 1 reading the triangle records with 16-bit indices
-//              (40 instead of 52 bytes per triangle)
+//   variant 2: variant 1's separate kernels throughout (no tiles)
 struct Tune {
   int variant = 1;
   int bs_tri = 256, bs_pre = 256, bs_cell = 256, bs_edge = 256;
@@ -285,7 +284,9 @@ inline int launches_per_stage(int precision_fp32, int variant, bool dif_on = fal
   if (!precision_fp32 && scheme == 3) n += 1;  // dtred: the triangle reconstruction of uh q
   // (the last gradients are formed in k_edge32v2)
   const bool in_edge = precision_fp32 && variant >= 1 && scheme != 3;
-  if (dif_on)
+  // APVM's kernels take hyperdiffusion's first application with them
+  const bool in_apvm = in_edge && apvm_on && dif_k4 && scheme == 0;
+  if (dif_on && !in_apvm)
     n += (dif_k4 ? 3 : 1) - (in_edge ? 1 : 0) + ((precision_fp32 && variant == 0) ? 1 : 0);
   // FP32 variants 1 and 2: the edge pre-pass for APVM's or gass18's edge PV
   if (precision_fp32 && variant >= 1 && (apvm_on || scheme == 2)) n += 1;

@@ -39,8 +39,11 @@ __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__re
                                                     float coef,
                                                     const float *__restrict__ qw,
                                                     const float *__restrict__ ht, int pv_on,
-                                                    int *flags) {
-  after_prior<true>(hd, u, q_tr, uh, q_ed, qg, vhx, ht);
+                                                    int *flags,
+                                                    const float *__restrict__ coefdiv,
+                                                    const float *__restrict__ coefvort,
+                                                    float *__restrict__ lap) {
+  after_prior<true>(hd, u, q_tr, uh, q_ed, qg, vhx, ht, coefdiv, coefvort, lap);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -75,6 +78,8 @@ __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__re
                  (a1.z + a2.z) * (b1.z + b2.z));
   }
   q_ed[e] = q;
+  // hyperdiffusion: the first application, with the indices that are here
+  if (lap) lap[e] = edge_lap(M, e, c1, c2, __ldg(&M.e_grad32[e]), coefdiv, coefvort);
 }
 
 // The two reconstructions apvm reads, in FP32 with the layout's weights
@@ -85,11 +90,16 @@ __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__re
 // and the gathers: a triangle reads 64 B of records in four wide loads and the
 // PV across its three edges (it went through the edges' records for them, two
 // more dependent loads), and the vectors are written as 16-byte records, one
-// gather each for the edges.
+// gather each for the edges.  coefdiv (hyperdiffusion on): K div u of the cells,
+// whose velocities are here; with the first edge gradients formed in the edge
+// pre-pass and their divergence and vorticity in the cell kernel's launch, five
+// launches a stage do what seven did (level 8 574 -> 529 us a step).
 __global__ void __launch_bounds__(256) k_apvm32(DevMesh M, const float *__restrict__ q_tr,
                                                 const float *__restrict__ u,
                                                 float4 *__restrict__ qg,
-                                                float4 *__restrict__ vhx, int nbt) {
+                                                float4 *__restrict__ vhx, int nbt,
+                                                const float *__restrict__ kcv,
+                                                float *__restrict__ coefdiv) {
   float v[3] = {0.0f, 0.0f, 0.0f}, p[3];
   int i;
   float4 *out;
@@ -120,7 +130,10 @@ __global__ void __launch_bounds__(256) k_apvm32(DevMesh M, const float *__restri
     for (int j = 0; j < 6; ++j) ed[j] = j < n ? __ldg(&M.c_ed[j * nv + c]) : 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) p[k] = __ldg(&M.c_p32[k * nv + c]);
-    after_prior<true>(q_tr, u, qg, vhx);
+    float dw[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) dw[j] = coefdiv ? __ldg(&M.c_div32[j * nv + c]) : 0.0f;
+    after_prior<true>(q_tr, u, qg, vhx, coefdiv);
     float ue[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) ue[j] = j < n ? u[ed[j]] : 0.0f;
@@ -130,6 +143,12 @@ __global__ void __launch_bounds__(256) k_apvm32(DevMesh M, const float *__restri
 #pragma unroll
       for (int k = 0; k < 3; ++k)
         v[k] = fmaf(ue[j], __ldg(&M.c_apw32[(3 * j + k) * nv + c]), v[k]);
+    if (coefdiv) {
+      float d = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 6; ++j) d = fmaf(ue[j], dw[j], d);
+      coefdiv[c] = kcv[c] * d;
+    }
     i = c;
     out = vhx;
   }
@@ -235,6 +254,20 @@ __global__ void __launch_bounds__(512) k_edge32(DevMesh M, const float *__restri
     yout[e] = rk_stage32(stage, momeq, yn[e], acc + e, dt);
 }
 
+// K_tr zeta(x) of triangle t
+template <class Wait>
+__device__ __forceinline__ void vort_lap(const DevMesh &M, int t, const float *__restrict__ x,
+                                         const float *__restrict__ kt,
+                                         float *__restrict__ coefvort) {
+  const int4 a = __ldg(&M.t_recA[t]), b = __ldg(&M.t_recB[t]);
+  const float c = __ldg(&M.t_recC[t].x), k = __ldg(&kt[t]);
+  IMODEL_WAIT(Wait, x, coefvort);
+  float z = __int_as_float(b.z) * x[a.x];
+  z += __int_as_float(b.w) * x[a.y];
+  z += c * x[a.z];
+  coefvort[t] = k * z;
+}
+
 // ---- diffusion and hyperdiffusion (diffusion_ed, swm_operators.f90:855-975)
 // coefdiv = K div x at the cells (blocks [0, nbc)), coefvort = K_tr zeta(x)
 // at the triangles (the blocks after), with the folded FP32 coefficients of
@@ -256,12 +289,7 @@ __global__ void __launch_bounds__(256) k_difcv32(DevMesh M, const float *__restr
   } else {
     const int t = (blockIdx.x - nbc) * blockDim.x + threadIdx.x;
     if (t >= M.nt) return;
-    const int4 a = __ldg(&M.t_recA[t]), b = __ldg(&M.t_recB[t]);
-    const float4 c = __ldg(&M.t_recC[t]);
-    float z = __int_as_float(b.z) * x[a.x];
-    z += __int_as_float(b.w) * x[a.y];
-    z += c.x * x[a.z];
-    coefvort[t] = __ldg(&kt[t]) * z;
+    vort_lap<NoWait>(M, t, x, kt, coefvort);
   }
 }
 
@@ -279,8 +307,10 @@ __global__ void __launch_bounds__(256) k_diflap32(DevMesh M, const float *__rest
 
 // ---- cell-centred TRSK (variant 1), bodies in swm_k32_body.cuh ------------
 // kEdgePV: q_tr is the edges' PV from the edge pre-pass (APVM); kZ false:
-// no PV-flux terms (dtred forms its PV flux at the triangles)
-template <class Wait, bool kEdgePV, bool kZ = true>
+// no PV-flux terms (dtred forms its PV flux at the triangles).  kLap: with the
+// second application of hyperdiffusion, K div lap from the cell's slots and, in
+// the blocks from nbc on, K_tr zeta(lap) of the triangles.
+template <class Wait, bool kEdgePV, bool kZ = true, bool kLap = false>
 __global__ void __launch_bounds__(512) k_cell32v2(DevMesh M, const float *__restrict__ hd,
                                                   const float *__restrict__ u,
                                                   const float *__restrict__ q_tr,
@@ -292,11 +322,19 @@ __global__ void __launch_bounds__(512) k_cell32v2(DevMesh M, const float *__rest
                                                   float *__restrict__ tend, int stage, float dt,
                                                   float grav, float h_ref,
                                                   const float *__restrict__ kcv,
-                                                  float *__restrict__ coefdiv) {
+                                                  float *__restrict__ coefdiv,
+                                                  const float *__restrict__ lap, int nbc,
+                                                  const float *__restrict__ kt,
+                                                  float *__restrict__ coefvort) {
+  if (kLap && static_cast<int>(blockIdx.x) >= nbc) {
+    const int t = (blockIdx.x - nbc) * blockDim.x + threadIdx.x;
+    if (t < M.nt) vort_lap<Wait>(M, t, lap, kt, coefvort);
+    return;
+  }
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M.nv) return;
-  cell_body<kEdgePV, kZ, Wait>(M, i, hd, u, q_tr, bern, zflux, yn, acc,
-                                          yout, tend, stage, dt, grav, h_ref, kcv, coefdiv);
+  cell_body<kEdgePV, kZ, Wait>(M, i, hd, u, q_tr, bern, zflux, yn, acc, yout, tend, stage, dt,
+                               grav, h_ref, kcv, coefdiv, kLap ? lap : nullptr);
 }
 
 // ---- pxt16 in the cell-centred form (variants 1, 2) ------------------------
@@ -576,7 +614,9 @@ __global__ void __launch_bounds__(512) k_edge32d(DevMesh M, const float *__restr
     yout[e] = rk_stage32(stage, momeq, yn[e], acc + e, dt);
 }
 
-// ---- variant 2: the triangle kernel on records with 16-bit indices -------
+// ---- variants 1 and 2: the triangle kernel on records with 16-bit indices --
+// (40 bytes a triangle where the 32-bit records have 52: 17.5 us at level 8
+// against 20.4; gass18 wants the triangle depths of k_tri32)
 template <class Wait>
 __global__ void __launch_bounds__(512) k_tri32c(DevMesh M, const float *__restrict__ hd,
                                                 const float *__restrict__ u,
@@ -752,7 +792,7 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
   if (dtred1)
     launch_pdl(k_tri32d, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M, h_in, u_in, W.q_tr, W.h_ref,
                W.pv_on, W.flags, D.kt, cvort, W.vhq);
-  else if (T.variant == 2 && W.scheme != IMODEL_SWM_GASS18)
+  else if (T.variant >= 1 && W.scheme != IMODEL_SWM_GASS18)
     launch_wait(k_tri32c<PriorWait>, k_tri32c<NoWait>, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M,
                h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort);
   else
@@ -768,12 +808,17 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
     // APVM (swm_operators.f90:1495-1502) and pxt16's distance-weighted q_e:
     // the PV of every edge from the edge pre-pass, read by the cells in
     // place of the triangle average
+    // hyperdiffusion beside APVM: K div u from APVM's cells, the first edge
+    // gradients in the pre-pass, div and zeta of them in the cell kernel
+    const bool lap_in = A.on && D.k4 && !pxt && !gass && !dtred1;
     if (A.on)
-      launch_pdl(k_apvm32, nbt + nbc, 256, s, M, W.q_tr, u_in, qg4, vhx4, nbt);
+      launch_pdl(k_apvm32, nbt + nbc, 256, s, M, W.q_tr, u_in, qg4, vhx4, nbt, D.kcv,
+                 lap_in ? D.coefdiv : nullptr);
     if (A.on || gass)
       launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr,
                  nullptr, W.q_ed, W.h_ref, A.on ? qg4 : nullptr, vhx4, A.coef,
-                 pxt || gass ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags);
+                 pxt || gass ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags,
+                 D.coefdiv, D.coefvort, lap_in ? D.lap : nullptr);
     if (ev) cudaEventRecord(ev[2], s);
     if (gass)
       launch_pdl(k_cell32g, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern,
@@ -791,17 +836,24 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
       launch_wait(k_cell32v2<PriorWait, false, false>, k_cell32v2<NoWait, false, false>,
                  nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux,
                  W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ?
-                 D.coefdiv : nullptr);
-    else if (A.on)
+                 D.coefdiv : nullptr, nullptr, 0, nullptr, nullptr);
+    else if (lap_in) {
+      const int nc = nblocks(M.nv, T.bs_cell);
+      launch_wait(k_cell32v2<PriorWait, true, true, true>, k_cell32v2<NoWait, true, true, true>,
+                  nc + nblocks(M.nt, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern,
+                  W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv,
+                  D.coefdiv, D.lap, nc, D.kt, D.coefvort);
+    } else if (A.on)
       launch_wait(k_cell32v2<PriorWait, true>, k_cell32v2<NoWait, true>, nblocks(M.nv, T.bs_cell),
                  T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern, W.zflux, W.yn_h, W.acc_h, h_out,
-                 W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr);
+                 W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr, nullptr, 0,
+                 nullptr, nullptr);
     else
       launch_wait(k_cell32v2<PriorWait, false>, k_cell32v2<NoWait, false>, nblocks(M.nv,
                  T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux, W.yn_h,
                  W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv :
-                 nullptr);
-    diffusion_tail(!dtred1);
+                 nullptr, nullptr, 0, nullptr, nullptr);
+    if (!lap_in) diffusion_tail(!dtred1);
     EdgeDif E;
     if (D.on) {
       if (D.k2 && D.k4) E.lap = D.lap;
@@ -821,14 +873,14 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
     return;
   }
   if (ev) cudaEventRecord(ev[1], s);
-  if (A.on) launch_pdl(k_apvm32, nbt + nbc, 256, s, M, W.q_tr, u_in, qg4, vhx4, nbt);
+  if (A.on) launch_pdl(k_apvm32, nbt + nbc, 256, s, M, W.q_tr, u_in, qg4, vhx4, nbt, nullptr, nullptr);
   // the method wrappers (variant 0 only): pxt16 (distance-weighted q_e,
   // Perot KE, pered), gass18 (rhombus PV, connecting-edge PV), dtred
   const int sch = W.scheme;
   const bool pxt = sch == IMODEL_SWM_PXT16, gass = sch == IMODEL_SWM_GASS18;
   launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr, W.uh,
              W.q_ed, W.h_ref, A.on ? qg4 : nullptr, vhx4, A.coef, pxt || gass ? M.e_qw32 : nullptr,
-             gass ? W.h_trs : nullptr, W.pv_on, W.flags);
+             gass ? W.h_trs : nullptr, W.pv_on, W.flags, nullptr, nullptr, nullptr);
   if (ev) cudaEventRecord(ev[2], s);
   launch_pdl(k_cell32, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.uh, W.bern,
              W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, pxt ? 1 : 0);

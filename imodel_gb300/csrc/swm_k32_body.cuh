@@ -201,7 +201,8 @@ __device__ __forceinline__ V cell_terms(int i, uint32_t meta, const float (&R)[6
                                         float grav, float h_ref,
                                         const float *__restrict__ kcv = nullptr,
                                         typename ValueOf<V>::type *__restrict__ coefdiv =
-                                            nullptr) {
+                                            nullptr,
+                                        const typename ValueOf<V>::type *dv = nullptr) {
   const int n = static_cast<int>(meta & 7u);
   const unsigned tneg = meta >> 8;
   const V half = all<V>(0.5f), href = all<V>(h_ref);
@@ -218,9 +219,9 @@ __device__ __forceinline__ V cell_terms(int i, uint32_t meta, const float (&R)[6
     qs[j] = kEdgePV ? qt[j] : pmul(half, padd(j == 0 ? qlast : qt[j - 1], qt[j]));
     div = vadd(div, G[j]);
     ke = vfma(all<V>(kd[j].x), vmul(ue[j], ue[j]), ke);
-    du = vfma(ue[j], d, du);
+    du = vfma(dv ? dv[j] : ue[j], d, du);
   }
-  // with diffusion on: K times the divergence of u
+  // with diffusion on: K times the divergence of u (or of dv)
   if (coefdiv) coefdiv[i] = vmul(all<V>(kcv[i]), vmul(du, all<V>(inva)));
   bern[i] = vfma(all<V>(grav), padd(hi, all<V>(bt)), ke);
   // kZ false (dtred): the edges form their PV flux from the triangles
@@ -252,9 +253,10 @@ __device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)
                                           float *__restrict__ tend, int stage, float dt,
                                           float grav, float h_ref,
                                           const float *__restrict__ kcv = nullptr,
-                                          float *__restrict__ coefdiv = nullptr) {
+                                          float *__restrict__ coefdiv = nullptr,
+                                         const float *dv = nullptr) {
   const float div = cell_terms<kEdgePV, kZ>(i, meta, R, kd, ue, hn, qt, hi, bt, inva, bern,
-                                                zflux, grav, h_ref, kcv, coefdiv);
+                                                zflux, grav, h_ref, kcv, coefdiv, dv);
   const float masseq = __fmul_rn(-div, inva);
   if (stage < 0) {
     tend[i] = masseq;
@@ -271,7 +273,8 @@ __device__ __forceinline__ void cell_math(int i, uint32_t meta, const float (&R)
 // ttgout*d} of each slot (unused pentagon slots repeat slot 0 with zero
 // weights), gathering its neighbours' values.  The cell's own values come in
 // as arguments: h (deviation) hi, b bt, 1/(A a) inva, y_n ynv and the RK
-// accumulator accv (read for stages 1-3).
+// accumulator accv (read for stages 1-3).  lap: coefdiv holds its divergence
+// in place of u's.
 template <bool kEdgePV, bool kZ>
 __device__ __forceinline__ void cell_core(int i, uint32_t meta,
                                           const int (&ed)[6], const int (&nb)[6],
@@ -284,17 +287,20 @@ __device__ __forceinline__ void cell_core(int i, uint32_t meta,
                                           float *__restrict__ acc, float *__restrict__ yout,
                                           float *__restrict__ tend, int stage, float dt,
                                           float grav, float h_ref, const float *__restrict__ kcv = nullptr,
-                                          float *__restrict__ coefdiv = nullptr) {
-  float ue[6], hn[6], qt[6];
+                                          float *__restrict__ coefdiv = nullptr,
+                                          const float *__restrict__ lap = nullptr) {
+  float ue[6], hn[6], qt[6], dv[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
     ue[j] = u[ed[j]];
     hn[j] = hd[nb[j]];
+    if (lap) dv[j] = lap[ed[j]];
     // kEdgePV: q_tr is the edges' PV, indexed by the slot's edge
     qt[j] = q_tr[kEdgePV ? ed[j] : tr[j]];
   }
   cell_math<kEdgePV, kZ>(i, meta, R, kd, ue, hn, qt, hi, bt, inva, ynv, accv, bern, zflux,
-                             acc, yout, tend, stage, dt, grav, h_ref, kcv, coefdiv);
+                             acc, yout, tend, stage, dt, grav, h_ref, kcv, coefdiv,
+                         lap ? dv : nullptr);
 }
 
 // the cell's own values from global memory
@@ -320,7 +326,8 @@ __device__ __forceinline__ void cell_body(const DevMesh &M, int i,
                                           float *__restrict__ yout, float *__restrict__ tend,
                                           int stage, float dt, float grav, float h_ref,
                                           const float *__restrict__ kcv = nullptr,
-                                          float *__restrict__ coefdiv = nullptr) {
+                                          float *__restrict__ coefdiv = nullptr,
+                                          const float *__restrict__ lap = nullptr) {
   const int nv = M.nv;
   const uint32_t meta = __ldg(&M.c_meta[i]);
   int ed[6], nb[6], tr[6];
@@ -337,12 +344,12 @@ __device__ __forceinline__ void cell_body(const DevMesh &M, int i,
     tr[j] = pk.z;
     R[j] = __int_as_float(pk.w);
   }
-  IMODEL_WAIT(Wait, hd, u, q_tr, bern, zflux, yn, acc, yout, tend, coefdiv);
+  IMODEL_WAIT(Wait, hd, u, q_tr, bern, zflux, yn, acc, yout, tend, coefdiv, lap);
   float hi, bt, inva, ynv, accv;
   cell_own(M, i, hd, yn, acc, stage, hi, bt, inva, ynv, accv);
   cell_core<kEdgePV, kZ>(i, meta, ed, nb, tr, R, kd, hi, bt, inva, ynv, accv, hd, u,
                                  q_tr, bern, zflux, acc, yout, tend, stage, dt, grav, h_ref, kcv,
-                                 coefdiv);
+                                 coefdiv, lap);
 }
 
 // -grad B - (Z_c1 + Z_c2) / l_e of an edge

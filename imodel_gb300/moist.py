@@ -226,7 +226,7 @@ class Moist:
         self._check(self.lib.imodel_moist_advance(self._handle, dt, nsteps))
 
     def get_state(self) -> dict:
-        out = [np.zeros(self.grid.ne if k == "u" else self.grid.nv) for k in FIELDS]
+        out = [np.empty(self.grid.ne if k == "u" else self.grid.nv) for k in FIELDS]
         arr = (_capi.c_f64p * 7)(*[_capi.as_f64p(a) for a in out])
         self._check(self.lib.imodel_moist_get_state(self._handle, arr))
         return dict(zip(FIELDS, out))

@@ -222,10 +222,8 @@ int imodel_swm_advance(void *handle, double dt, int32_t nsteps);
  * triangle, edge pre-pass, cell and edge kernels, gather groups of the
  * learned-correction kernel}; variant 0 uses the 10-entry edge stencil,
  * variant 1 the cell-centred TRSK sum (one kernel per stage over tiles for
- * plain trsk10 steps, three kernels with options on), variant 2 three kernels
- * with triangle records holding 16-bit indices (bit-identical results); the
- * last entry is
- * 2, 3 or 4 with the
+ * plain trsk10 steps, separate kernels with options on), variant 2 the separate
+ * kernels throughout (bit-identical results); the last entry is 2, 3 or 4 with the
  * learned correction on (its kernel has 6 warp groups, the rest run the
  * epilogue) and 0 without it.  The FP64 path has a single configuration and
  * returns it. */
