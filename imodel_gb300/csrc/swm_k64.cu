@@ -316,15 +316,17 @@ __global__ void __launch_bounds__(256)
   if (scheme == IMODEL_SWM_PXT16) {
     // kinetic_energy_hx, perhx branch (:1172-1173): half the squared
     // vector_edhx2hx_perot (:454-509, HTC) of u; c_off = ed%c%p - v%p
-    double v0 = 0.0, v1 = 0.0, v2 = 0.0, su[6], dl[6];
+    double su[6], dl[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       const int ed = static_cast<int>(es[j] & 0x7FFFFFFFu);
       su[j] = flip(es[j], u[ed]);
       dl[j] = M.e_dleng[ed];
     }
+    double v0 = su[0] * M.c_off[i] * dl[0], v1 = su[0] * M.c_off[nv + i] * dl[0],
+           v2 = su[0] * M.c_off[2 * nv + i] * dl[0];
 #pragma unroll
-    for (int j = 0; j < 6; ++j)
+    for (int j = 1; j < 6; ++j)
       if (j < n) {
         v0 = v0 + su[j] * M.c_off[(3 * j) * nv + i] * dl[j];
         v1 = v1 + su[j] * M.c_off[(3 * j + 1) * nv + i] * dl[j];
@@ -474,14 +476,13 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh64 M, const double *__re
   } else {
     // pered: at each of the edge's cells the Perot reconstruction of
     // uh (q_e + q_k) / 2 over the cell's edges, projected on the tangent
-    // plane; their average (halved together: 0.5 x + 0.5 y and 0.5 (x + y)
-    // are the same rounding)
+    // plane; twice their average (0.5 x + 0.5 y and 0.5 (x + y) are the same
+    // rounding, and the projection is linear in powers of two)
     const double qe = q2[e];
     double vc[2][3];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int c = M.e_v[i * ne + e];
-      double a0 = 0.0, a1 = 0.0, a2 = 0.0;
       const int n = M.c_nnb[c];
       double f[6], d[6];
 #pragma unroll
@@ -491,8 +492,10 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh64 M, const double *__re
         f[j] = flip(es, uh2[l2]) * (qe + q2[l2]);
         d[j] = M.e_d8[l2];
       }
+      double a0 = f[0] * M.c_off[c] * d[0], a1 = f[0] * M.c_off[nv + c] * d[0],
+             a2 = f[0] * M.c_off[2 * nv + c] * d[0];
 #pragma unroll
-      for (int j = 0; j < 6; ++j)
+      for (int j = 1; j < 6; ++j)
         if (j < n) {
           a0 = a0 + f[j] * M.c_off[(3 * j) * nv + c] * d[j];
           a1 = a1 + f[j] * M.c_off[(3 * j + 1) * nv + c] * d[j];
@@ -508,12 +511,13 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh64 M, const double *__re
       vc[i][1] = a1;
       vc[i][2] = a2;
     }
-    v0 = 0.5 * (vc[0][0] + vc[1][0]);
-    v1 = 0.5 * (vc[0][1] + vc[1][1]);
-    v2 = 0.5 * (vc[0][2] + vc[1][2]);
+    v0 = vc[0][0] + vc[1][0];
+    v1 = vc[0][1] + vc[1][1];
+    v2 = vc[0][2] + vc[1][2];
   }
   proj_sphere(v0, v1, v2, M.e_c[e], M.e_c[ne + e], M.e_c[2 * ne + e], M.e_nrm[e], M.e_rnrm[e]);
-  const double q = -(v0 * M.e_nr[e] + v1 * M.e_nr[ne + e] + v2 * M.e_nr[2 * ne + e]);
+  double q = -(v0 * M.e_nr[e] + v1 * M.e_nr[ne + e] + v2 * M.e_nr[2 * ne + e]);
+  if (scheme != IMODEL_SWM_DTRED) q = 0.5 * q;
   edge_update64(e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
 }
 
