@@ -273,8 +273,8 @@ struct TileLayout {
   size_t data_bytes = 0;  // of all blocks
   HVec<TileHead> head;    // [ntiles]
   // per tile the device indices of its other depths (the ring cells, then the
-  // rest), other edges and triangles, each ascending; from them
-  // launch_fill_tiles writes the blocks on the GPU
+  // rest), other edges and triangles, in any order; launch_fill_tiles sorts
+  // them and writes the blocks on the GPU
   HVec<int32_t> lists;
 };
 // Cuts a trsk10 layout into tiles of at most cap cells with flux terms; false

@@ -220,6 +220,26 @@ __device__ __forceinline__ int place(const int32_t *v, int n, int k) {
   return lo;
 }
 
+// a[0, n) ascending, by the whole block: bitonic sort in its mirrored form
+// (Batcher 1968), every exchange towards ascending order, so that the places
+// from n on need not exist
+__device__ __forceinline__ void sort_block(int32_t *a, int n) {
+  for (int k = 2; k < 2 * n; k *= 2)
+    for (int j = k / 2; j > 0; j /= 2) {
+      const int mask = j == k / 2 ? k - 1 : j;
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int l = i ^ mask;
+        if (l > i && l < n && a[i] > a[l]) {
+          const int32_t t = a[i];
+          a[i] = a[l];
+          a[l] = t;
+        }
+      }
+    }
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(256) k_fill_tiles(DevMesh M, const int4 *head,
                                                     const int32_t *lists, unsigned char *data) {
   // the lists (below 1024 entries each): ring cells and other depths, other
@@ -231,10 +251,15 @@ __global__ void __launch_bounds__(256) k_fill_tiles(DevMesh M, const int4 *head,
   unsigned char *block = data + 16 * static_cast<size_t>(T.block);
   int32_t *hx = reinterpret_cast<int32_t *>(block);
   int32_t *ux = reinterpret_cast<int32_t *>(block + T.ux);
-  for (int k = threadIdx.x; k < nhx; k += blockDim.x) hx[k] = lh[k] = src[k];
-  for (int k = threadIdx.x; k < nux; k += blockDim.x) ux[k] = lu[k] = src[nhx + k];
+  for (int k = threadIdx.x; k < nhx; k += blockDim.x) lh[k] = src[k];
+  for (int k = threadIdx.x; k < nux; k += blockDim.x) lu[k] = src[nhx + k];
   for (int k = threadIdx.x; k < T.nt; k += blockDim.x) lt[k] = src[nhx + nux + k];
-  __syncthreads();
+  sort_block(lh, nring);
+  sort_block(lh + nring, nhx - nring);
+  sort_block(lu, nux);
+  sort_block(lt, T.nt);
+  for (int k = threadIdx.x; k < nhx; k += blockDim.x) hx[k] = lh[k];
+  for (int k = threadIdx.x; k < nux; k += blockDim.x) ux[k] = lu[k];
   // local numbers: depths own, ring, others; edges own, others
   auto cell = [&](int c) -> uint32_t {
     if (c >= T.c0 && c < T.c0 + T.nc) return c - T.c0;

@@ -137,7 +137,6 @@ bool build_tiles(const Layout &L, int cap, TileLayout &T) {
           const int hi = std::max(L.e_v[e], L.e_v[NE + e]);
           if (cells.add(hi)) Q.z.push_back(hi);
         }
-        std::sort(Q.z.begin(), Q.z.end());
         auto around = [&](int c) {
           for (int j = 0; j < L.c_nnb[c]; ++j) {
             const int nb = L.c_nb[j * NV + c], t = L.c_tr[j * NV + c], e = L.c_ed[j * NV + c];
@@ -154,9 +153,6 @@ bool build_tiles(const Layout &L, int cap, TileLayout &T) {
             if (edges.add(e)) Q.ux.push_back(e);
             if (cells.add(v)) Q.hx.push_back(v);
           }
-        std::sort(Q.hx.begin(), Q.hx.end());
-        std::sort(Q.ux.begin(), Q.ux.end());
-        std::sort(Q.tri.begin(), Q.tri.end());
         const int nz = c1 - c0 + static_cast<int>(Q.z.size());
         const int nh = nz + static_cast<int>(Q.hx.size());
         const int nu = e1 - e0 + static_cast<int>(Q.ux.size());
