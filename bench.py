@@ -223,19 +223,24 @@ class Dist:
             self.dist.destroy_process_group()
 
 
-def kernel_bytes(nv, ne, nt, precision, variant=0):
+def kernel_bytes(nv, ne, nt, precision, variant=0, fused=False):
     """Algorithmic bytes of one launch of each stage kernel: every array
     element the kernel reads or writes counted once (gathered arrays count
-    once per element, not once per gather)."""
+    once per element, not once per gather).  fused: one kernel a stage, timed
+    in the cell kernel's slot."""
     w = 4 if precision == "fp32" else 8
+    if fused:
+        # records: triangle 36 B, cell slots 6 x 16 B and 3 words, edge 8 B;
+        # h and u: input, y_n, acc r/w, output (tiles' rims not counted)
+        return {"triangle": 0, "edge_pre": 0, "edge": 0,
+                "cell": nt * 36 + nv * (6 * 16 + 12) + ne * 8 + (nv + ne) * 5 * w}
     # triangle: f, 3 circulation coefs, 3 edge idx, 3 kite coefs, 3 cell idx,
     # q out; gathers u and h
     tri = nt * (w + 3 * w + 3 * 4 + 3 * w + 3 * 4 + w) + ne * w + nv * w
     if precision == "fp32" and variant in (1, 2):
-        if variant == 2:
-            # the triangle record: 40 bytes (6 16-bit indices, f in the
-            # record), 8 bytes of bases per warp of 32 triangles
-            tri = nt * (40 + 8 / 32 + w) + ne * w + nv * w
+        # the triangle record: 40 bytes (6 16-bit indices, f in the
+        # record), 8 bytes of bases per warp of 32 triangles
+        tri = nt * (40 + 8 / 32 + w) + ne * w + nv * w
         # cell: meta, 1/(A a), b, 6 slots x (edge, neighbour, triangle idx,
         # kite fraction, KE weight, ttgout*d); h, y_n, acc r/w, y_out, B out,
         # 6 PV-flux contributions out; gathers u and q
@@ -254,13 +259,14 @@ def kernel_bytes(nv, ne, nt, precision, variant=0):
     return {"triangle": tri, "edge_pre": edge_pre, "cell": cell, "edge": edge}
 
 
-def kernel_names(variant):
-    if variant == 2:
-        return {"triangle": "k_tri32c", "edge_pre": "", "cell": "k_cell32v2",
+def kernel_names(variant, fused=False):
+    if fused:
+        return {"cell": "k_stage32"}
+    if variant in (1, 2):
+        return {"triangle": "k_tri32c", "edge_pre": "k_edge_pre32", "cell": "k_cell32v2",
                 "edge": "k_edge32v2"}
-    v2 = "v2" if variant == 1 else ""
-    return {"triangle": "k_tri32", "edge_pre": "k_edge_pre32", "cell": "k_cell32" + v2,
-            "edge": "k_edge32" + v2}
+    return {"triangle": "k_tri32", "edge_pre": "k_edge_pre32", "cell": "k_cell32",
+            "edge": "k_edge32"}
 
 
 def load_peaks():
@@ -358,7 +364,9 @@ MLP_FLOP_PER_EDGE = 2 * (24 * 64 + 64 * 64 + 64)
 # benchmark's level by the number of cells, as the traffic grows with them.
 # DRAM bytes per cell of one launch (ncu at icos level 8, an RK stage that
 # reads the accumulator)
-TRAFFIC_PER_CELL = {"k_cell32v2": 133.779e6 / 655362}
+TRAFFIC_PER_CELL = {"k_cell32v2": 133.779e6 / 655362, "k_stage32": 877.0e6 / 2621442}
+TRAFFIC_SOURCE = {"k_cell32v2": "ncu capture at icos level 8, scaled by cells",
+                  "k_stage32": "ncu capture at icos level 9, scaled by cells"}
 
 
 def load_tflops():
@@ -526,8 +534,9 @@ def main():
 
         peak, peak_kind = load_peaks()
         variant = rh["tuning"]["variant"]
-        kb = kernel_bytes(g.nv, g.ne, g.nt, "fp32", variant)
-        prof = {k: v for k, v in rh["prof"].items() if k != "edge_pre" or kb["edge_pre"]}
+        fused = rh["main_kernel"] == "k_stage32"
+        kb = kernel_bytes(g.nv, g.ne, g.nt, "fp32", variant, fused)
+        prof = {k: v for k, v in rh["prof"].items() if kb[k]}
         dom = max(prof, key=prof.get)
         achieved = kb[dom] / (prof[dom] / 1000.0) / 1e9
         # whole-step bytes: the 2000 B/cell-step model and this layout's own
@@ -535,7 +544,7 @@ def main():
         layout_step = 4 * sum(kb.values())
         sec_step = rh["ms"] / args.steps / 1000.0
         kernel_ms = dict(prof)
-        kname = kernel_names(variant)[dom]
+        kname = kernel_names(variant, fused)[dom]
         traffic = TRAFFIC_PER_CELL[kname] * g.nv if kname in TRAFFIC_PER_CELL else None
         wc, we = g.hx_areag, g.ed_leng * g.edhx_leng / 2.0
         err = {}
@@ -564,7 +573,7 @@ def main():
                          "achieved": achieved,
                          "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_kind, "traffic": traffic,
-                         "traffic_source": "ncu capture at icos level 8, scaled by cells",
+                         "traffic_source": TRAFFIC_SOURCE.get(kname),
                          "algorithmic_bytes_per_launch": kb[dom]},
             "step_roofline": {
                 "bytes_per_cell_step_model": 2000.0,
