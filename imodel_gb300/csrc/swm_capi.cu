@@ -1832,12 +1832,8 @@ void moist_step64(Moist *X, double dt) {
       A.upw1 = X->upw1;
       const double *h_in = swm ? in(st, W.yn_h, W.ya_h, W.yb_h) : W.yn_h;
       const double *u_in = swm ? in(st, W.yn_u, W.ya_u, W.yb_u) : W.yn_u;
-      if (swm)
-        imodel::launch_stage64(H->M, W, h_in, u_in, nullptr, nullptr, -1, dt, H->stream);
       A.h_in = h_in;
       A.u_in = u_in;
-      A.tend_h = W.tend_h;
-      A.tend_u = W.tend_u;
       A.yn_h = W.yn_h;
       A.acc_h = W.acc_h;
       A.h_out = out(st, W.yn_h, W.ya_h, W.yb_h);
@@ -1862,7 +1858,11 @@ void moist_step64(Moist *X, double dt) {
       A.qc = X->qc;
       A.qr = X->qr;
       A.flags = H->d_flags;
-      imodel::launch_moist_stage(H->M, A, H->stream);
+      if (swm)
+        imodel::launch_stage64(H->M, W, h_in, u_in, nullptr, nullptr, -1, dt, H->stream, nullptr,
+                               &A);
+      else
+        imodel::launch_moist_tracer(H->M, A, H->stream);
     }
     imodel::launch_moist_q(H->nv, W.yn_h, X->q[1][0], X->q[2][0], X->q[3][0], X->qv, X->qc,
                            X->qr, H->d_flags, H->stream);

@@ -233,7 +233,8 @@ void launch_consts64(DevMesh64 &M, double *p, cudaStream_t s);
 // kernels of the stage, for per-kernel timing outside graph capture.
 void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_in,
                     const double *u_in, double *h_out, double *u_out, int stage,
-                    double dt, cudaStream_t s, cudaEvent_t *ev = nullptr);
+                    double dt, cudaStream_t s, cudaEvent_t *ev = nullptr,
+                    const struct MoistArgs *moist = nullptr);
 // The learned corrections' error proxy: per block part[2 b] = sum w (a -
 // b)^2 and part[2 b + 1] = sum w (b - c)^2 over the edges, in FP64, w = l d
 // / 2 (e_area32); nblk blocks of 256 threads
@@ -302,17 +303,20 @@ void launch_dif_coefs(const DevMesh &M, const double *kf, double k, bool take_sq
                       float *kc32, double *kt64, float *kt32, cudaStream_t s);
 
 
-// One RK stage of the moist shallow-water model (swm_moist.cu).  Tracer k of
-// {h theta, h qv, h qc, h qr, h tracer} is advanced when bit k of `active`
-// is set; swm != 0 adds the shallow-water terms (the caller has written
-// tend_h and tend_u with a tendency evaluation of the stage input),
-// the thermal momentum source and the water sources.
+// One RK stage of the moist shallow-water model.  Tracer k of {h theta, h qv,
+// h qc, h qr, h tracer} is advanced when bit k of `active` is set; swm != 0: with
+// the shallow-water terms, the thermal momentum source and the water sources, in
+// launch_stage64's own kernels (swm_k64.cuh): three launches a stage where the
+// tendency and two kernels after it took five, level 6 224 -> 210 us a step,
+// level 5 111 -> 93.
+// initialize_moist_swm_fields (moist_swm.f90:730-732)
+constexpr double kLscale = 10.0, kGammaR = 0.001, kQprecip = 0.0001;
 struct MoistArgs {
   int stage = 0;
   double dt = 0.0;
   int swm = 0, active = 0;
   int upw1 = 0;  // tracer advection: 0 "trsk" (centred), 1 "upw1" (upwind)
-  const double *u_in = nullptr, *h_in = nullptr, *tend_u = nullptr, *tend_h = nullptr;
+  const double *u_in = nullptr, *h_in = nullptr;
   double *yn_u = nullptr, *acc_u = nullptr, *u_out = nullptr;
   double *yn_h = nullptr, *acc_h = nullptr, *h_out = nullptr;
   const double *q_in[5] = {};
@@ -330,7 +334,9 @@ struct MoistArgs {
 // q0 ex20 in place
 void launch_moist_consts(const DevMesh64 &M, const double *th, double *ex20, double q0,
                          double *gthb, cudaStream_t s);
-void launch_moist_stage(const DevMesh64 &M, const MoistArgs &A, cudaStream_t s);
+// the tracers alone (swm == 0); with the shallow-water terms launch_stage64
+// takes the arguments
+void launch_moist_tracer(const DevMesh64 &M, const MoistArgs &A, cudaStream_t s);
 void launch_moist_q(int nv, const double *h, const double *hqv, const double *hqc,
                     const double *hqr, double *qv, double *qc, double *qr, int *flags,
                     cudaStream_t s);

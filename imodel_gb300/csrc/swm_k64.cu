@@ -6,34 +6,14 @@
 // so that the FP64 step reproduces the reference arithmetic of
 // src/swm.f90:2416-2683 and src/swm_operators.f90 bit for bit.
 #include <cmath>
+#include <type_traits>
 
 #include "imodel_swm.h"
 #include "swm_common.cuh"
-#include "swm_div.cuh"
+#include "swm_k64.cuh"
 
 namespace imodel {
 namespace {
-
-// constants.f90:45 -- eps = epsilon(1.) (float epsilon)
-constexpr double kEps = 1.1920928955078125e-07;
-
-// ode_rk4, swm.f90:2647-2678.  dt is half the time step in stages 0 and 1: dt
-// k / 2 and (dt / 2) k are the same rounding (a power of two), and acc + 2 k
-// is one fused operation with an exact product.
-__device__ __forceinline__ double rk_stage(int stage, double k, double yn, double *acc,
-                                           double dt) {
-  if (stage == 0) {
-    *acc = k;
-    return yn + dt * k;
-  } else if (stage == 1) {
-    *acc = __fma_rn(2.0, k, *acc);
-    return yn + dt * k;
-  } else if (stage == 2) {
-    *acc = __fma_rn(2.0, k, *acc);
-    return yn + dt * k;
-  }
-  return yn + div_by(dt * (*acc + k), 6.0, kSixth);
-}
 
 // What bounds the FP64 step: GB300's FP64 pipe (2 operations per cycle and
 // SM), not memory -- the kernels below are counted in FP64 operations.  Three
@@ -67,6 +47,7 @@ __device__ __forceinline__ void edge_flux64(const DevMesh64 &M, int e, const dou
 // of the circumcentre (bary, pxt16) or scalar_edtr2trcc of h_ed (:286-343,
 // gass18, which also keeps eta and h_tr for the rhombus PV).  The blocks
 // after: the edges' fluxes, which the next launch reads beside q.
+template <class Moist>
 __global__ void __launch_bounds__(256) k_tri64(DevMesh64 M, const double *__restrict__ h,
                                                const double *__restrict__ u,
                                                double *__restrict__ q_tr, int pv_on,
@@ -75,11 +56,13 @@ __global__ void __launch_bounds__(256) k_tri64(DevMesh64 M, const double *__rest
                                                double *__restrict__ eta_t,
                                                double *__restrict__ h_trs,
                                                double *__restrict__ uh2,
-                                               double2 *__restrict__ fe, int nbt) {
+                                               double2 *__restrict__ fe, int nbt, Moist Q) {
   after_prior<false>(h, u, q_tr, coefvort, eta_t, h_trs, uh2, fe);
   if (static_cast<int>(blockIdx.x) >= nbt) {
     const int e = (blockIdx.x - nbt) * blockDim.x + threadIdx.x;
-    if (e < M.ne) edge_flux64(M, e, h, u, uh2, fe);
+    if (e >= M.ne) return;
+    edge_flux64(M, e, h, u, uh2, fe);
+    if constexpr (std::is_same<Moist, MoistArgs>::value) moist_flux64(M, Q, e);
     return;
   }
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -267,6 +250,7 @@ __device__ __forceinline__ double edge_pv2(const DevMesh64 &M, int e,
 // (:1162-1171), Bernoulli potential (swm.f90:2533-2536) and the
 // mass-equation RK stage.  The blocks after: q2, twice the edges' PV.  The
 // two do not read each other; sharing a launch fills the chip on small grids.
+template <class Moist>
 __global__ void __launch_bounds__(256)
     k_cell64(DevMesh64 M, const double *__restrict__ h, const double *__restrict__ u,
              const double2 *__restrict__ fe, double *__restrict__ bern,
@@ -276,7 +260,7 @@ __global__ void __launch_bounds__(256)
              const double *__restrict__ q_tr, const double *__restrict__ qg,
              const double *__restrict__ vhx, double coef, int scheme,
              const double *__restrict__ eta_t, const double *__restrict__ h_trs, int pv_on,
-             int *flags) {
+             int *flags, Moist Q) {
   if (static_cast<int>(blockIdx.x) >= nbc) {
     after_prior<false>(q2, q_tr, qg, vhx, eta_t, h_trs);
     const int e = (blockIdx.x - nbc) * blockDim.x + threadIdx.x;
@@ -342,6 +326,10 @@ __global__ void __launch_bounds__(256)
   }
   bern[i] = M.grav * (h[i] + M.c_bt[i]) + ke;
   const double masseq = -divuh;
+  if constexpr (std::is_same<Moist, MoistArgs>::value) {
+    moist_cell64<true>(M, Q, i, masseq);
+    return;
+  }
   if (stage < 0)
     tend[i] = masseq;
   else
@@ -350,25 +338,30 @@ __global__ void __launch_bounds__(256)
 
 // the momentum tendency from its two terms (swm.f90:2578-2594) and the RK
 // stage
-__device__ __forceinline__ void edge_update64(int e, double g, double q,
+template <class Moist = NoMoist>
+__device__ __forceinline__ void edge_update64(const DevMesh64 &M, int e, double g, double q,
                                               const double *__restrict__ yn,
                                               double *__restrict__ acc,
                                               double *__restrict__ yout,
                                               double *__restrict__ tend, int stage, double dt,
                                               int mom_on, const double *__restrict__ dif1,
-                                              const double *__restrict__ dif2) {
+                                              const double *__restrict__ dif2,
+                                              const Moist &Q = Moist{}) {
   double momeq = -g - q;
   // diffusion, then hyperdiffusion (swm.f90:2578-2589)
   if (dif1) momeq = momeq + dif1[e];
   if (dif2) momeq = momeq - dif2[e];
   if (!mom_on) momeq = 0.0;
-  if (stage < 0)
+  if constexpr (std::is_same<Moist, MoistArgs>::value)
+    moist_edge64(M, Q, e, momeq);
+  else if (stage < 0)
     tend[e] = momeq;
   else
     yout[e] = rk_stage(stage, momeq, yn[e], acc + e, dt);
 }
 
 // grad_ed (:511-548) + coriolis_ed TRSK (:1283-1308) and the momentum RK stage
+template <class Moist>
 __global__ void __launch_bounds__(256) k_edge64(DevMesh64 M, const double *__restrict__ bern,
                                                 const double *__restrict__ uh2,
                                                 const double *__restrict__ q2,
@@ -379,7 +372,7 @@ __global__ void __launch_bounds__(256) k_edge64(DevMesh64 M, const double *__res
                                                 double dt, int mom_on,
                                                 const double *__restrict__ dif1,
                                                 const double *__restrict__ dif2,
-                                                const int32_t *__restrict__ stq) {
+                                                const int32_t *__restrict__ stq, Moist Q) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -413,7 +406,7 @@ __global__ void __launch_bounds__(256) k_edge64(DevMesh64 M, const double *__res
     if (s < ns) q = s == 0 ? t : q + t;
   }
   q = div_by(q, l, rl);
-  edge_update64(e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
+  edge_update64(M, e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2, Q);
 }
 
 // dtred: vector_edhx2tr_perot (:345-406, HTC) of uh at the triangle
@@ -518,7 +511,7 @@ __global__ void __launch_bounds__(256) k_edge64r(DevMesh64 M, const double *__re
   proj_sphere(v0, v1, v2, M.e_c[e], M.e_c[ne + e], M.e_c[2 * ne + e], M.e_nrm[e], M.e_rnrm[e]);
   double q = -(v0 * M.e_nr[e] + v1 * M.e_nr[ne + e] + v2 * M.e_nr[2 * ne + e]);
   if (scheme != IMODEL_SWM_DTRED) q = 0.5 * q;
-  edge_update64(e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
+  edge_update64(M, e, g, q, yn, acc, yout, tend, stage, dt, mom_on, dif1, dif2);
 }
 
 // diffusion_ed (swm_operators.f90:855-895), first half: coefdiv = K
@@ -1043,7 +1036,7 @@ inline int nblocks(int n, int t) { return (n + t - 1) / t; }
 
 void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_in,
                     const double *u_in, double *h_out, double *u_out, int stage, double dt,
-                    cudaStream_t s, cudaEvent_t *ev) {
+                    cudaStream_t s, cudaEvent_t *ev, const MoistArgs *moist) {
   if (ev) cudaEventRecord(ev[0], s);
   // diffusion: the triangle and cell kernels also write K_tr zeta(u) and
   // K div u; the edge gradients follow them (and, with hyperdiffusion, the
@@ -1053,8 +1046,14 @@ void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_i
   if (stage == 0 || stage == 1) dt = dt * 0.5;  // rk_stage
   const int bt = block64(M.nt), bc = block64(M.nv), be = block64(M.ne);
   const int nbt = nblocks(M.nt, bt);
-  launch_pdl(k_tri64, nbt + nblocks(M.ne, bt), bt, s, M, h_in, u_in, W.q_tr, W.pv_on, W.flags,
-             D.kt, D.on ? D.coefvort : nullptr, sch, W.eta_t, W.h_trs, W.uh, W.fe, nbt);
+  auto tri = [&](auto kernel, const auto &Q) {
+    launch_pdl(kernel, nbt + nblocks(M.ne, bt), bt, s, M, h_in, u_in, W.q_tr, W.pv_on, W.flags,
+               D.kt, D.on ? D.coefvort : nullptr, sch, W.eta_t, W.h_trs, W.uh, W.fe, nbt, Q);
+  };
+  if (moist)
+    tri(k_tri64<MoistArgs>, *moist);
+  else
+    tri(k_tri64<NoMoist>, NoMoist{});
   if (ev) cudaEventRecord(ev[1], s);
   const Apvm<double> &A = W.apvm;
   if (A.on) {
@@ -1065,10 +1064,16 @@ void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_i
     launch_pdl(k_vhq64, nblocks(M.nt, bt), bt, s, M, W.uh, W.q_tr, W.vhq);
   if (ev) cudaEventRecord(ev[2], s);
   const int nbc = nblocks(M.nv, bc);
-  launch_pdl(k_cell64, nbc + nblocks(M.ne, bc), bc, s, M, h_in, u_in, W.fe, W.bern, W.yn_h,
-             W.acc_h, h_out, W.tend_h, stage, dt, D.kcv, D.on ? D.coefdiv : nullptr, nbc, W.q_ed,
-             W.q_tr, A.on ? A.qg : nullptr, A.vhx, A.coef, sch, W.eta_t, W.h_trs, W.pv_on,
-             W.flags);
+  auto cell = [&](auto kernel, const auto &Q) {
+    launch_pdl(kernel, nbc + nblocks(M.ne, bc), bc, s, M, h_in, u_in, W.fe, W.bern, W.yn_h,
+               W.acc_h, h_out, W.tend_h, stage, dt, D.kcv, D.on ? D.coefdiv : nullptr, nbc,
+               W.q_ed, W.q_tr, A.on ? A.qg : nullptr, A.vhx, A.coef, sch, W.eta_t, W.h_trs,
+               W.pv_on, W.flags, Q);
+  };
+  if (moist)
+    cell(k_cell64<MoistArgs>, *moist);
+  else
+    cell(k_cell64<NoMoist>, NoMoist{});
   if (D.on) {
     launch_pdl(k_diflap64, nblocks(M.ne, be), be, s, M, D.coefdiv, D.coefvort, D.lap);
     if (D.k4) {
@@ -1082,10 +1087,17 @@ void launch_stage64(const DevMesh64 &M, const Work<double> &W, const double *h_i
     launch_pdl(k_edge64r, nblocks(M.ne, be), be, s, M, W.bern, W.uh, W.q_ed, W.vhq, W.yn_u,
                W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, D.k2 ? D.lap : nullptr, D.k4 ?
                D.lap2 : nullptr, sch);
-  else
-    launch_pdl(k_edge64, nblocks(M.ne, be), be, s, M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u,
-               u_out, W.tend_u, stage, dt, W.mom_on, D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 :
-               nullptr, sch == IMODEL_SWM_GASS18 ? M.e_stq : nullptr);
+  else {
+    auto edge = [&](auto kernel, const auto &Q) {
+      launch_pdl(kernel, nblocks(M.ne, be), be, s, M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u, u_out,
+                 W.tend_u, stage, dt, W.mom_on, D.k2 ? D.lap : nullptr, D.k4 ? D.lap2 : nullptr,
+                 sch == IMODEL_SWM_GASS18 ? M.e_stq : nullptr, Q);
+    };
+    if (moist)
+      edge(k_edge64<MoistArgs>, *moist);
+    else
+      edge(k_edge64<NoMoist>, NoMoist{});
+  }
   if (ev) cudaEventRecord(ev[4], s);
 }
 

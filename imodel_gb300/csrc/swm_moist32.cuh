@@ -5,9 +5,6 @@
 
 namespace imodel {
 
-// initialize_moist_swm_fields (moist_swm.f90:730-732)
-constexpr double kLscale = 10.0, kGammaR = 0.001, kQprecip = 0.0001;
-
 // the thermal momentum source g/2 grad(h h theta) / h_e + g theta_e grad(b)
 // (moist_swm.f90:1299-1315) of an edge from its cells' depth deviations and
 // h theta; gr = 1 / (l erad), gthb the second term
