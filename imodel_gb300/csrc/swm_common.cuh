@@ -137,16 +137,17 @@ template <class P>
 __device__ __forceinline__ void pin_ptr(P &p) {
   asm volatile("" : "+l"(p));
 }
-template <bool early, class... P>
+template <bool early, bool tiles = false, class... P>
 __device__ __forceinline__ void after_prior(P &...p) {
-  if (early && gridDim.x < kPdlGrid) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (early && (tiles || gridDim.x < kPdlGrid)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   (pin_ptr(p), ...);
 }
 inline bool pdl_grid(int grid) { return static_cast<unsigned>(grid) < kPdlGrid; }
 // launches k, which calls after_prior, so that it may start before the kernel
 // before it in the stream has finished (on grids below kPdlGrid)
-template <class... P, class... A>
+// tiles: on any grid (the kernel calls after_prior<true, true>)
+template <bool tiles = false, class... P, class... A>
 inline void launch_pdl_smem(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s,
                             A &&...a) {
   cudaLaunchConfig_t c{};
@@ -158,7 +159,7 @@ inline void launch_pdl_smem(void (*k)(P...), int grid, int block, size_t smem, c
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
-  c.numAttrs = pdl_grid(grid) ? 1 : 0;
+  c.numAttrs = tiles || pdl_grid(grid) ? 1 : 0;
   cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
 }
 template <class... P, class... A>
@@ -400,9 +401,11 @@ struct HostTo {
 template <class T>
 void launch_load_host(const HostMap &N, const double *h, const double *u, HostTo<T> to_h,
                       HostTo<T> to_u, double shift, cudaStream_t s);
+// take (with flags NULL): also *host = *take, *take = 0
 template <class T>
 void launch_store_host(const HostMap &N, const T *src_h, const T *src_u, double *h, double *u,
-                       double shift, int *flags, cudaStream_t s);
+                       double shift, int *flags, cudaStream_t s, int *take = nullptr,
+                       int *host = nullptr);
 // *host = *flags, *flags = 0 (host: page-locked)
 void launch_take_flags(int *flags, int *host, cudaStream_t s);
 

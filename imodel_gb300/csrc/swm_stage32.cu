@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kThr, kThr == 256 ? 3 : 4)
   S.sq = S.su + D.max_u;
   S.sb = S.sq + D.max_t;
   S.sz = reinterpret_cast<float *>(smem + T.triA);
-  after_prior<true>(hd, u, yn_h, acc_h, h_out, yn_u, acc_u, u_out, tend_h, tend_u);
+  after_prior<true, true>(hd, u, yn_h, acc_h, h_out, yn_u, acc_u, u_out, tend_h, tend_u);
   const TileFields F{hd, u, yn_h, yn_u, acc_h, acc_u, h_out, u_out, tend_h, tend_u};
   TileOwn<kThr> own;
   own.load(T, F, kStage);
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kThr, 3)
 #pragma unroll
   for (int r = 0; r < TileOwn<kThr>::kE; ++r)
     gthb[r] = tid + r * kThr < T.ne ? A.gthb[T.e0 + tid + r * kThr] : 0.0f;
-  after_prior<true>();
+  after_prior<true, true>();
   const TileFields F{A.h_in,  A.u_in,  A.yn_h, A.yn_u,  A.acc_h,
                      A.acc_u, A.h_out, A.u_out, nullptr, nullptr};
   TileOwn<kThr> own;
@@ -382,7 +382,7 @@ bool fused_moist_ok(const TileDev &T) {
 void launch_moist_stage32_fused(const DevMesh &M, const Work<float> &W, const MoistArgs32 &A,
                                 cudaStream_t s) {
   const TileDev &T = W.tiles;
-  launch_pdl_smem(moist_kernel(T, A.stage), T.ntiles, threads(T), moist_smem(T), s, T, A,
+  launch_pdl_smem<true>(moist_kernel(T, A.stage), T.ntiles, threads(T), moist_smem(T), s, T, A,
                   static_cast<float>(M.grav), static_cast<float>(M.erad), W.pv_on, W.mom_on);
 }
 
@@ -401,7 +401,7 @@ void launch_stage32_fused(const DevMesh &M, const Work<float> &W, const float *h
                           const float *u_in, float *h_out, float *u_out, int stage, float dt,
                           cudaStream_t s) {
   const TileDev &T = W.tiles;
-  launch_pdl_smem(stage_kernel(T, stage), T.ntiles, threads(T), fused_smem(T), s, T, h_in, u_in,
+  launch_pdl_smem<true>(stage_kernel(T, stage), T.ntiles, threads(T), fused_smem(T), s, T, h_in, u_in,
                   W.yn_h, W.acc_h, h_out, W.yn_u, W.acc_u, u_out, W.tend_h, W.tend_u, dt,
                   static_cast<float>(M.grav), static_cast<float>(M.erad), W.h_ref, W.pv_on,
                   W.mom_on, W.flags);
