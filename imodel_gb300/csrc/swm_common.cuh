@@ -127,9 +127,11 @@ struct TileDev {
 // successor start at once rather than as this kernel's blocks end.  Per step:
 // FP32 level 5 27.0 us with plain launches, 24.1 with the wait alone, 20.9
 // with the early start; level 7 50.7, 49.3, 43.7; the moist FP32 step at level
-// 8 432, 422, 412.  At level 9 (10,000 blocks and more) nothing is gained and
-// the early start costs 3 % of the cell kernel.  The FP64 kernels keep the
-// wait alone (level 5 69.9 us plain, 57.7 with the wait, 63.6 early; pxt16 at
+// 8 432, 422, 412.  At level 9 (10,000 blocks and more) the separate kernels gain
+// nothing and the early start costs 3 % of the cell kernel; the tiles' kernels
+// (tiles) start early on every grid, as the next stage's first tiles are copied
+// in while the last ones run (level 9 553 us a step -> 539, the moist step 873
+// -> 854).  The FP64 kernels keep the wait alone (level 5 69.9 us plain, 57.7 with the wait, 63.6 early; pxt16 at
 // level 6 325, 323, 422): their blocks must spread evenly over the FP64 pipes,
 // and blocks that start early take the places first freed.
 constexpr unsigned kPdlGrid = 8192;
@@ -401,11 +403,9 @@ struct HostTo {
 template <class T>
 void launch_load_host(const HostMap &N, const double *h, const double *u, HostTo<T> to_h,
                       HostTo<T> to_u, double shift, cudaStream_t s);
-// take (with flags NULL): also *host = *take, *take = 0
 template <class T>
 void launch_store_host(const HostMap &N, const T *src_h, const T *src_u, double *h, double *u,
-                       double shift, int *flags, cudaStream_t s, int *take = nullptr,
-                       int *host = nullptr);
+                       double shift, int *flags, cudaStream_t s);
 // *host = *flags, *flags = 0 (host: page-locked)
 void launch_take_flags(int *flags, int *host, cudaStream_t s);
 
