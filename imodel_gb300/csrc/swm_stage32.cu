@@ -382,7 +382,7 @@ bool fused_moist_ok(const TileDev &T) {
 void launch_moist_stage32_fused(const DevMesh &M, const Work<float> &W, const MoistArgs32 &A,
                                 cudaStream_t s) {
   const TileDev &T = W.tiles;
-  launch_pdl_smem<true>(moist_kernel(T, A.stage), T.ntiles, threads(T), moist_smem(T), s, T, A,
+  launch_pdl_smem(moist_kernel(T, A.stage), T.ntiles, threads(T), moist_smem(T), s, T, A,
                   static_cast<float>(M.grav), static_cast<float>(M.erad), W.pv_on, W.mom_on);
 }
 
@@ -401,7 +401,7 @@ void launch_stage32_fused(const DevMesh &M, const Work<float> &W, const float *h
                           const float *u_in, float *h_out, float *u_out, int stage, float dt,
                           cudaStream_t s) {
   const TileDev &T = W.tiles;
-  launch_pdl_smem<true>(stage_kernel(T, stage), T.ntiles, threads(T), fused_smem(T), s, T, h_in, u_in,
+  launch_pdl_smem(stage_kernel(T, stage), T.ntiles, threads(T), fused_smem(T), s, T, h_in, u_in,
                   W.yn_h, W.acc_h, h_out, W.yn_u, W.acc_u, u_out, W.tend_h, W.tend_u, dt,
                   static_cast<float>(M.grav), static_cast<float>(M.erad), W.h_ref, W.pv_on,
                   W.mom_on, W.flags);
