@@ -338,6 +338,20 @@ constexpr size_t kSmallState = 512 * 1024;
 
 HostMap host_map(const Handle *H) { return {H->nv, H->ne, H->d_cell_o2n, H->d_edge_o2n}; }
 
+// whether the host can copy a and b itself (a device address is left to
+// cudaMemcpyAsync, which refuses it)
+bool host_arrays(const void *a, const void *b) {
+  for (const void *p : {a, b}) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (at.type == cudaMemoryTypeDevice) return false;
+  }
+  return true;
+}
+
 // the page-locked area, idle, for a small state; nullptr for a large one
 double *small_area(Handle *H) {
   const size_t bytes = sizeof(double) * (static_cast<size_t>(H->nv) + H->ne);
@@ -354,7 +368,7 @@ double *small_area(Handle *H) {
   return H->h_small;
 }
 double *small_in(Handle *H, const double *h, const double *u) {
-  double *p = small_area(H);
+  double *p = host_arrays(h, u) ? small_area(H) : nullptr;
   if (p) {
     std::memcpy(p, h, sizeof(double) * H->nv);
     std::memcpy(p + H->nv, u, sizeof(double) * H->ne);
@@ -363,6 +377,7 @@ double *small_in(Handle *H, const double *h, const double *u) {
 }
 // h, u: the caller's arrays, which read_flags fills
 double *small_out(Handle *H, double *h, double *u) {
+  if (!host_arrays(h, u)) return nullptr;
   // the area's input is read by work in front in the same stream
   double *p = H->small_busy && H->h_small && !H->out_h ? H->h_small : small_area(H);
   if (p) {
@@ -1220,7 +1235,8 @@ int imodel_swm_tendency(void *handle, const double *h, const double *u, double *
     H->href_fixed = true;
   }
   // the tendency input becomes the "last stage input" the diagnostics use
-  if (double *z = imodel::small_in(H, h, u)) {
+  double *z = imodel::host_arrays(masseq, momeq) ? imodel::small_in(H, h, u) : nullptr;
+  if (z) {
     const imodel::HostMap N = imodel::host_map(H);
     if (H->precision == IMODEL_SWM_FP64) {
       auto &W = H->W64;

@@ -677,10 +677,10 @@ __global__ void k_load_host(HostMap N, const double *__restrict__ h, const doubl
   const bool cell = j < N.nv;
   if (j >= N.nv + N.ne) return;
   const int k = cell ? j : j - N.nv;
-  const double x = cell ? h[k] - shift : u[k];
   const int i = cell ? N.cell[k] : N.edge[k];
-  after_prior<true>();
-  const T v = static_cast<T>(x);
+  // the caller's arrays may be what the work in front writes
+  after_prior<true>(h, u);
+  const T v = static_cast<T>(cell ? h[k] - shift : u[k]);
   const HostTo<T> to = cell ? to_h : to_u;
   if (to.yn) to.yn[i] = v;
   to.ya[i] = v;
