@@ -194,8 +194,8 @@ namespace {
 
 // ---- fused forward + backward over a batch ---------------------------------
 // dynamic shared memory: B1 4K | B2 8K | B2T 8K | A2 16K | AW 36K | BW 36K.
-// A3 (dZ2) takes A2's place, whose product has been waited for, and A1 the
-// last rows of BW, which are written after it: 108 KB, so that two CTAs share
+// A1 (the inputs), A2 and A3 (dZ2) take turns in one place, each written when the
+// product of the one before has been waited for: 108 KB, so that two CTAs share
 // an SM (and its 512 TMEM columns) and hide each other's waits for products
 // and rows.  A batch of 65,536 rows is 512 tiles: one CTA an SM took four
 // rounds of them.
@@ -232,8 +232,9 @@ __device__ __forceinline__ float warp_sum32(float (&p)[32], int lane) {
 // chain of a tile's four products and what lies between them.  A step of 65,536
 // rows with its reduction: 93 us with one CTA an SM, 56
 // with two CTAs, 40 with the columns' stores spread over the banks, the sums by
-// halves and the reduction in floats, 30 with two threads a row, the next rows
-// read ahead and the prologue before the wait for the kernel before.
+// halves and the reduction in floats, 30.3 with two threads a row, the next rows
+// read ahead and the prologue before the wait for the kernel before, 29.7 with a
+// tile's last product waited for with the next tile's first.
 constexpr int TRN_THREADS = 2 * TM, HALF = NH / 2;
 
 __global__ void __launch_bounds__(TRN_THREADS, TRN_CTAS)
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(TRN_THREADS, TRN_CTAS)
                 float *__restrict__ partials, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t *B1 = smem, *B2 = B1 + 4096, *B2T = B2 + 8192, *A2 = B2T + 8192, *AW = A2 + 16384,
-          *BW = AW + TRN_W, *A3 = A2, *A1 = BW + TRN_W - 8192;
+          *BW = AW + TRN_W, *A3 = A2, *A1 = A2;
   __shared__ uint64_t mbar;
   __shared__ uint32_t tslot;
   __shared__ float sb1[NH], sb2[NH], sw3[NH];
@@ -313,20 +314,12 @@ __global__ void __launch_bounds__(TRN_THREADS, TRN_CTAS)
   bool ok = true;
   bool first = true;
   for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-    // --- inputs: A1 (row-major) and X^T rows 64..87 of AW ----------------
+    // --- inputs: A1 (row-major); the tile before's last product may be running
     if (half == 0) {
 #pragma unroll
       for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4 *>(A1 + kmaj_off(row, 8 * q, K1)) = c[q];
       *reinterpret_cast<uint4 *>(A1 + kmaj_off(row, 24, K1)) = make_uint4(0, 0, 0, 0);
-    } else {
-      const uint16_t *xs = reinterpret_cast<const uint16_t *>(c);
-#pragma unroll
-      for (int i = 0; i < NIN; ++i)
-        *reinterpret_cast<uint16_t *>(AW + trn_off(64 + i, row)) = xs[i];
     }
-    const bool alive = live;
-    const float aim = target, weight = wt;
-    fetch(tile + gridDim.x);
     fence_async_smem();
     sync_cta();
     if (tid == 0) {
@@ -335,9 +328,19 @@ __global__ void __launch_bounds__(TRN_THREADS, TRN_CTAS)
             smem_desc(smem_u32(B1) + 256 * s, 128, K1 * 16), id64, s);
       commit(&mbar);
     }
+    // (this also waits for the tile before's last product)
     ok = __syncthreads_and(mbar_wait(&mbar, phase, err, ERR_WAIT)) != 0;
     phase ^= 1u;
     fence_after_sync();
+    if (half == 1) {  // X^T, rows 64..87 of AW
+      const uint16_t *xs = reinterpret_cast<const uint16_t *>(c);
+#pragma unroll
+      for (int i = 0; i < NIN; ++i)
+        *reinterpret_cast<uint16_t *>(AW + trn_off(64 + i, row)) = xs[i];
+    }
+    const bool alive = live;
+    const float aim = target, weight = wt;
+    fetch(tile + gridDim.x);
     float v[HALF];
     if (ok) {  // H1 = GELU(Z1 + b1): A2 (row-major) and AW rows 0..63 (H1^T)
       ld32(tmem + lane_base + c0, v);
@@ -436,14 +439,13 @@ __global__ void __launch_bounds__(TRN_THREADS, TRN_CTAS)
         mma(tmem + 128, smem_desc(smem_u32(AW) + 2 * TRN_K * s, TRN_K, TRN_ROWS),
             smem_desc(smem_u32(BW) + 2 * TRN_K * s, TRN_K, TRN_ROWS), id128,
             (first && s == 0) ? 0u : 1u);
-      commit(&mbar);
-    }
-    if (ok) {  // ok is uniform across the CTA
-      ok = __syncthreads_and(mbar_wait(&mbar, phase, err, ERR_WAIT)) != 0;
-      phase ^= 1u;
     }
     first = false;
-    sync_cta();
+  }
+  if (ok && !first) {  // the last tile's last product
+    if (tid == 0) commit(&mbar);
+    ok = __syncthreads_and(mbar_wait(&mbar, phase, err, ERR_WAIT)) != 0;
+    fence_after_sync();
   }
   // partial gradients of this CTA, each half its columns
   float *out = partials + static_cast<int64_t>(blockIdx.x) * NPART;
