@@ -10,12 +10,13 @@
 // with the same bits.
 //
 // What bounds it: at level 9 HBM (about 256 B of records and 80 B of state a
-// cell and stage, 5.85 TB/s measured, 0.88 of a copy's rate), where the three
+// cell and stage, 6.3 TB/s measured, 0.94 of a copy's rate), where the three
 // kernels move 440 B; below level 8 the latency of a block's own chain (copy,
 // gather, three phases), so a block issues all loads of its thread at once
 // and the copies before the wait.  Per step against the three kernels: level
-// 9 738 -> 551 us, 8 189 -> 153, 7 43.7 -> 37.1, 6 24.8 -> 16.5, 5 20.9 ->
-// 12.4 to 14.4.  Loading the records into registers phase by phase and the
+// 9 738 -> 553 us, 8 189 -> 154, 7 43.7 -> 37.1, 6 24.8 -> 16.5, 5 20.9 ->
+// 12.4; with the early start on every grid and eight steps a graph 538, 149,
+// 33.8, 14.3, 11.0.  Loading the records into registers phase by phase and the
 // state in loops instead took 982 us at level 9.
 #include "imodel_swm.h"
 #include "swm_layout.h"
