@@ -1867,7 +1867,7 @@ void moist_step64(Moist *X, double dt) {
       A.uphi = X->uphi;
       A.dts = st < 2 ? dt * 0.5 : dt;
       A.hgrav = H->M.grav * 0.5;
-      A.rdt = dt >= 0x1p-500 && dt <= 0x1p500 ? 1.0 / dt : std::nan("");
+      A.rdt = dt >= imodel::kRecipLow && dt <= imodel::kRecipHigh ? 1.0 / dt : std::nan("");
       A.gthb = X->gthb;
       A.q0ex = X->ex20;
       A.qv = X->qv;

@@ -226,6 +226,8 @@ struct Work {
   int mom_on;        // testcase >= 2: momentum tendency kept, else zeroed
 };
 
+// divisors outside get NaN for a reciprocal (swm_div.cuh)
+constexpr double kRecipLow = 0x1p-64, kRecipHigh = 0x1p500;
 // M's derived FP64 constants, in consts64_size(M) doubles at p
 size_t consts64_size(const DevMesh64 &M);
 void launch_consts64(DevMesh64 &M, double *p, cudaStream_t s);

@@ -19,8 +19,10 @@ static __device__ __noinline__ double div_full(double a, double b) { return a / 
 // floating-point division when the divisor is known in advance", IEEE Trans.
 // Comput. 53, 2004).  Three FP64 operations; a / b compiles to about ten on
 // GB300's FP64 pipe, which bounds the step.  A quotient outside 2^-895 ..
-// 2^896 (zero, infinities, NaN and whatever the layout marked with rb = NaN
-// among them) takes the division itself, so every input gets a / b.
+// 2^896 (zero, infinities, NaN and every divisor with rb = NaN among them)
+// takes the division itself, so every input gets a / b.  rb is given for |b|
+// from kRecipLow to kRecipHigh: a smaller b with a quotient in range could have
+// a remainder below the normal numbers.
 __device__ __forceinline__ double div_by(double a, double b, double rb) {
   const double q = a * rb;
   const double z = __fma_rn(__fma_rn(-q, b, a), rb, q);

@@ -592,7 +592,7 @@ __global__ void k_dif_coefs(DevMesh M, const double *__restrict__ kf, double k, 
 // normal range
 __device__ __forceinline__ double recip(double b) {
   const double a = fabs(b);
-  return a >= 0x1p-500 && a <= 0x1p500 ? 1.0 / b : __longlong_as_double(0x7FF8000000000000LL);
+  return a >= kRecipLow && a <= kRecipHigh ? 1.0 / b : __longlong_as_double(0x7FF8000000000000LL);
 }
 __device__ __forceinline__ double norm3(const double *p, int n, int i) {
   const double p0 = p[i], p1 = p[n + i], p2 = p[2 * n + i];
@@ -1114,7 +1114,7 @@ void launch_consts64(DevMesh64 &M, double *p, cudaStream_t s) {
     p += n;
     return q;
   };
-  M.rerad = M.erad >= 0x1p-500 && M.erad <= 0x1p500 ? 1.0 / M.erad : std::nan("");
+  M.rerad = M.erad >= kRecipLow && M.erad <= kRecipHigh ? 1.0 / M.erad : std::nan("");
   M.c_rareag = take(nv);
   M.c_rcellarea = take(nv);
   M.c_eds = reinterpret_cast<const uint32_t *>(take(3 * nv));

@@ -57,7 +57,7 @@ __global__ void k_moist_q(int nv, const double *__restrict__ h, const double *__
     atomicOr(flags, 1);
     return;
   }
-  const double r = fabs(hi) <= 0x1p500 ? 1.0 / hi : __longlong_as_double(0x7FF8000000000000LL);
+  const double r = fabs(hi) <= kRecipHigh ? 1.0 / hi : __longlong_as_double(0x7FF8000000000000LL);
   qv[i] = div_by(hqv[i], hi, r);
   qc[i] = div_by(hqc[i], hi, r);
   qr[i] = div_by(hqr[i], hi, r);
