@@ -951,29 +951,49 @@ __global__ void __launch_bounds__(kRedThreads) k_diag(DevMesh M, const T *__rest
     const double q = ht != 0.0 ? diag_div(eta, ht) : 0.0;
     part[Q_ENS] += A * ht * (q * q) * 0.5;
   }
-  KSum acc[kDiagQ];
-#pragma unroll
-  for (int q = 0; q < kDiagQ; ++q) acc[q] = KSum{part[q], 0.0};
-  // max-type entries are reduced with max, not a sum: pre-reduce them (their
-  // sums, all zero, are overwritten below)
-  const int kMaxQ[3] = {Q_MAXDIV, Q_NAN, Q_UMAX};
-  double mx[3] = {maxdiv, nan, umax};
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-    for (int off = 16; off > 0; off >>= 1)
-      mx[k] = fmax(mx[k], __shfl_down_sync(0xffffffffu, mx[k], off));
-  __shared__ double smax[3][kRedThreads / 32];
+  // The block's sums, with few FP64 operations, which bound a small grid's call
+  // (608 blocks; with 12 compensated sums a warp and the maxima in FP64 a call
+  // took 65 us at level 5, 114 at level 7, with these 40 and 90): eight sums go
+  // down the warp by halves, nine additions where a sum of its own for each takes
+  // 40, in the same tree; the maxima, none of them negative, as integers.
+  static_assert(Q_ADIV2 == 7 && Q_MAXDIV == 8 && Q_NAN == 9 && Q_UMAX == 10 && kDiagQ == 12, "");
+  __shared__ double sh[kRedThreads / 32][8];
+  __shared__ long long smax[3][kRedThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-    for (int k = 0; k < 3; ++k) smax[k][warp] = mx[k];
+#pragma unroll
+  for (int off = 16, n = 4; off >= 4; off >>= 1, n >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      const double keep = up ? part[k + n] : part[k], send = up ? part[k] : part[k + n];
+      part[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  part[0] += __shfl_xor_sync(0xffffffffu, part[0], 2);
+  part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
+  if ((lane & 3) == 0) sh[warp][lane >> 2] = part[0];
+  const double mx[3] = {maxdiv, nan, umax};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    long long m = __double_as_longlong(mx[k]);
+    for (int off = 16; off > 0; off >>= 1)
+      m = max(m, __shfl_down_sync(0xffffffffu, m, off));
+    if (lane == 0) smax[k][warp] = m;
+  }
   __syncthreads();
-  double bm[3] = {0.0, 0.0, 0.0};
-  for (int k = 0; k < 3; ++k)
-    for (int w = 0; w < kRedThreads / 32; ++w) bm[k] = fmax(bm[k], smax[k][w]);
-  block_reduce_store<kDiagQ>(acc, scratch);
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) scratch[(kMaxQ[k] * gridDim.x + blockIdx.x) * 2] = bm[k];
+  if (threadIdx.x < kDiagQ) {
+    const int q = threadIdx.x;
+    KSum t{0.0, 0.0};
+    if (q <= Q_ADIV2) {
+      for (int w = 0; w < kRedThreads / 32; ++w) t.merge(KSum{sh[w][q], 0.0});
+    } else if (q <= Q_UMAX) {
+      long long m = 0;
+      for (int w = 0; w < kRedThreads / 32; ++w) m = max(m, smax[q - Q_MAXDIV][w]);
+      t.s = __longlong_as_double(m);
+    }
+    scratch[(q * gridDim.x + blockIdx.x) * 2] = t.s;
+    scratch[(q * gridDim.x + blockIdx.x) * 2 + 1] = t.c;
+  }
 }
 
 // error_calc partials (swm.f90:3492-3543): weights A_i (cells) and l*d/2
