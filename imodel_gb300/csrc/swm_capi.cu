@@ -109,10 +109,10 @@ struct Handle {
   CUresult (*range_attr)(void *, CUpointer_attribute, CUdeviceptr) = nullptr;
   double *d_stage_h = nullptr, *d_stage_u = nullptr;  // FP64, reference order
   double *d_ref_h = nullptr, *d_ref_u = nullptr;      // FP64, device order
-  double *d_scratch = nullptr, *d_result = nullptr;
+  double *d_scratch = nullptr;
   int *d_flags = nullptr;
   int *h_flags = nullptr;      // pinned
-  double *h_result = nullptr;  // pinned
+  double *h_result = nullptr;  // pinned, written by k_finalize
   // small states (kSmallState) pass through one page-locked area (h, then u),
   // got on the first such call: a kernel reads or writes it over the host link
   double *h_small = nullptr;
@@ -547,20 +547,18 @@ int check_flags(Handle *H) {
 }
 
 // total energy of the current state (compensated FP64 integral) and max |u|
-// enqueues it on stream s, with the read-back into h_result
+// enqueues it on stream s, into h_result
 int enqueue_energy(Handle *H, cudaStream_t s) {
   if (H->precision == IMODEL_SWM_FP64) {
     auto &W = H->W64;
-    launch_diag<double>(H->M, W, W.yn_h, W.yn_u, W.ya_h, W.ya_u, H->d_scratch, H->d_result, s,
+    launch_diag<double>(H->M, W, W.yn_h, W.yn_u, W.ya_h, W.ya_u, H->d_scratch, H->h_result, s,
                         true);
   } else {
     auto &W = H->W32;
-    launch_diag<float>(H->M, W, W.yn_h, W.yn_u, W.ya_h, W.ya_u, H->d_scratch, H->d_result, s,
+    launch_diag<float>(H->M, W, W.yn_h, W.yn_u, W.ya_h, W.ya_u, H->d_scratch, H->h_result, s,
                        true);
   }
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(H->h_result, H->d_result, sizeof(double) * kDiagQ, cudaMemcpyDeviceToHost,
-                     s));
   return IMODEL_SWM_OK;
 }
 
@@ -1000,7 +998,7 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
   if ((rc = dalloc(H, &H->d_stage_h, L.nv)) || (rc = dalloc(H, &H->d_stage_u, L.ne)) ||
       (rc = dalloc(H, &H->d_ref_h, L.nv)) || (rc = dalloc(H, &H->d_ref_u, L.ne)) ||
       (rc = dalloc(H, &H->d_scratch, static_cast<size_t>(2) * kRedBlocks * 16)) ||
-      (rc = dalloc(H, &H->d_result, 16)) || (rc = dalloc(H, &H->d_flags, 1)))
+      (rc = dalloc(H, &H->d_flags, 1)))
     return rc;
   CK(cudaMallocHost(&H->h_flags, sizeof(int)));
   CK(cudaMallocHost(&H->h_result, 16 * sizeof(double)));
@@ -1296,16 +1294,13 @@ int imodel_swm_diagnostics(void *handle, imodel_swm_diag *out) {
   if (H->precision == IMODEL_SWM_FP64) {
     auto &W = H->W64;
     imodel::launch_diag<double>(H->M, W, W.yn_h, W.yn_u, W.ya_h, W.ya_u, H->d_scratch,
-                                H->d_result, H->stream);
+                                H->h_result, H->stream);
   } else {
     auto &W = H->W32;
     imodel::launch_diag<float>(H->M, W, W.yn_h, W.yn_u, W.ya_h, W.ya_u, H->d_scratch,
-                               H->d_result, H->stream);
+                               H->h_result, H->stream);
   }
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(H->h_result, H->d_result, sizeof(double) * imodel::kDiagQ,
-                        cudaMemcpyDeviceToHost, H->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
   if (e != cudaSuccess) return imodel::set_error(H, IMODEL_SWM_ECUDA, cudaGetErrorString(e));
   const double *r = H->h_result;
@@ -1343,14 +1338,11 @@ int imodel_swm_errors(void *handle, const double *h_ref, const double *u_ref, do
   imodel::launch_gather_in(H->ne, H->d_edge_n2o, H->d_stage_u, H->d_ref_u, 0.0, H->stream);
   if (H->precision == IMODEL_SWM_FP64)
     imodel::launch_errors<double>(H->M, H->W64.yn_h, H->W64.yn_u, 0.0, H->d_ref_h, H->d_ref_u,
-                                  H->d_scratch, H->d_result, H->stream);
+                                  H->d_scratch, H->h_result, H->stream);
   else
     imodel::launch_errors<float>(H->M, H->W32.yn_h, H->W32.yn_u, H->h_ref, H->d_ref_h,
-                                 H->d_ref_u, H->d_scratch, H->d_result, H->stream);
+                                 H->d_ref_u, H->d_scratch, H->h_result, H->stream);
   e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(H->h_result, H->d_result, sizeof(double) * 8, cudaMemcpyDeviceToHost,
-                        H->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
   if (e != cudaSuccess) return imodel::set_error(H, IMODEL_SWM_ECUDA, cudaGetErrorString(e));
   const double *r = H->h_result;

@@ -781,6 +781,7 @@ __global__ void k_finalize(const double *__restrict__ scratch, int nblk, int nq,
   // and 3 across the warps) rather than by one thread in a row: FP64
   // operations have a long latency on this GPU
   const int q = blockIdx.x;
+  after_prior<true>(scratch, result);
   if (q >= nq) return;
   static_assert(kRedThreads == 256, "8 warps per block");
   __shared__ double ss[8], sc[8];
@@ -1224,7 +1225,7 @@ void launch_diag(const DevMesh &M, const Work<T> &W, const T *h, const T *u, con
     k_diag<T, true><<<kRedBlocks, kRedThreads, 0, s>>>(M, h, u, hs, us,
                                                         static_cast<double>(W.h_ref), scratch);
   const unsigned maxmask = (1u << Q_MAXDIV) | (1u << Q_NAN) | (1u << Q_UMAX);
-  k_finalize<<<kDiagQ, kRedThreads, 0, s>>>(scratch, kRedBlocks, kDiagQ, maxmask, result);
+  launch_pdl(k_finalize, kDiagQ, kRedThreads, s, scratch, kRedBlocks, kDiagQ, maxmask, result);
 }
 template void launch_diag<double>(const DevMesh &, const Work<double> &, const double *,
                                   const double *, const double *, const double *, double *,
@@ -1238,7 +1239,7 @@ void launch_errors(const DevMesh &M, const T *h, const T *u, double h_ref, const
                    const double *uref, double *scratch, double *result, cudaStream_t s) {
   k_errors<T><<<kRedBlocks, kRedThreads, 0, s>>>(M, h, u, h_ref, href, uref, scratch);
   const unsigned maxmask = (1u << 2) | (1u << 3) | (1u << 6) | (1u << 7);
-  k_finalize<<<8, kRedThreads, 0, s>>>(scratch, kRedBlocks, 8, maxmask, result);
+  launch_pdl(k_finalize, 8, kRedThreads, s, scratch, kRedBlocks, 8, maxmask, result);
 }
 template void launch_errors<double>(const DevMesh &, const double *, const double *, double,
                                     const double *, const double *, double *, double *,
