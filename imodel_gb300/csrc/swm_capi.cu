@@ -118,7 +118,6 @@ struct Handle {
   double *h_small = nullptr;
   bool small_none = false;  // it was refused: pageable copies instead
   bool small_busy = false;  // work that uses it may be in flight
-  double *out_h = nullptr, *out_u = nullptr;  // where read_flags copies it to
   Work<double> W64{};
   Work<float> W32{};
   cudaStream_t stream = nullptr;
@@ -282,7 +281,6 @@ int alloc_work(Handle *H, Work<T> &W) {
 }
 
 int set_error(Handle *H, int code, const std::string &msg) {
-  H->out_h = H->out_u = nullptr;  // the caller's arrays are not the next call's
   H->err = msg;
   return code;
 }
@@ -364,7 +362,6 @@ double *small_area(Handle *H) {
   }
   if (H->small_busy && cudaStreamSynchronize(H->stream) != cudaSuccess) return nullptr;
   H->small_busy = true;
-  H->out_h = H->out_u = nullptr;
   return H->h_small;
 }
 double *small_in(Handle *H, const double *h, const double *u) {
@@ -375,15 +372,17 @@ double *small_in(Handle *H, const double *h, const double *u) {
   }
   return p;
 }
-// h, u: the caller's arrays, which read_flags fills
-double *small_out(Handle *H, double *h, double *u) {
+// The caller's arrays (h, u) that a call's results go to from the area, once
+// the work is done (read_flags): an object of that call, as the arrays are the
+// caller's only until it returns.  Null: the results need no such copy.
+struct SmallOut {
+  double *h = nullptr, *u = nullptr;
+};
+// the area for results, after the work in front in the stream has read its input
+double *small_out(Handle *H, double *h, double *u, SmallOut *out) {
   if (!host_arrays(h, u)) return nullptr;
-  // the area's input is read by work in front in the same stream
-  double *p = H->small_busy && H->h_small && !H->out_h ? H->h_small : small_area(H);
-  if (p) {
-    H->out_h = h;
-    H->out_u = u;
-  }
+  double *p = H->small_busy && H->h_small ? H->h_small : small_area(H);
+  if (p) *out = {h, u};
   return p;
 }
 
@@ -475,10 +474,12 @@ int load_state(Handle *H, const double *h, const double *u, bool new_run) {
   return IMODEL_SWM_OK;
 }
 
-int store_state(Handle *H, double *h, double *u) {
+// the state to h and u; what goes through the area arrives with read_flags(out)
+int store_state(Handle *H, double *h, double *u, SmallOut *out) {
+  *out = {};
   double *hz = static_cast<double *>(host_view(H, h, sizeof(double) * H->nv));
   double *uz = static_cast<double *>(host_view(H, u, sizeof(double) * H->ne));
-  if (!(hz && uz) && (hz = small_out(H, h, u))) uz = hz + H->nv;
+  if (!(hz && uz) && (hz = small_out(H, h, u, out))) uz = hz + H->nv;
   if (hz && uz) {
     // page-locked arrays: written in order over the host link by the
     // kernels that undo the permutation (no staging copy)
@@ -507,17 +508,17 @@ int store_state(Handle *H, double *h, double *u) {
   return IMODEL_SWM_OK;
 }
 
-// reads and clears the device flags (synchronising the stream)
-int read_flags(Handle *H, int *f) {
+// reads and clears the device flags (synchronising the stream), and hands over
+// what the call's results in the area go to
+int read_flags(Handle *H, int *f, const SmallOut &out = {}) {
   launch_take_flags(H->d_flags, H->h_flags, H->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(H->stream));
   *f = *H->h_flags;
-  if (H->out_h) {
-    std::memcpy(H->out_h, H->h_small, sizeof(double) * H->nv);
-    std::memcpy(H->out_u, H->h_small + H->nv, sizeof(double) * H->ne);
+  if (out.h) {
+    std::memcpy(out.h, H->h_small, sizeof(double) * H->nv);
+    std::memcpy(out.u, H->h_small + H->nv, sizeof(double) * H->ne);
   }
-  H->out_h = H->out_u = nullptr;
   H->small_busy = false;
   return IMODEL_SWM_OK;
 }
@@ -540,9 +541,9 @@ int flags_status(Handle *H, int f) {
   return IMODEL_SWM_OK;
 }
 
-int check_flags(Handle *H) {
+int check_flags(Handle *H, const SmallOut &out = {}) {
   int f = 0;
-  const int rc = read_flags(H, &f);
+  const int rc = read_flags(H, &f, out);
   return rc ? rc : flags_status(H, f);
 }
 
@@ -733,27 +734,28 @@ int step_host(Handle *H, double *h, double *u, double dt, int nsteps) {
   if (rc) return rc;
   const bool overlap = H->learned_active && H->te_ref_set && H->side && nsteps > 0 &&
                        nsteps <= kGuardSteps && std::isfinite(dt);
+  SmallOut out;
   if (!overlap) {
-    if ((rc = advance(H, dt, nsteps)) || (rc = store_state(H, h, u))) return rc;
-    return check_flags(H);
+    if ((rc = advance(H, dt, nsteps)) || (rc = store_state(H, h, u, &out))) return rc;
+    return check_flags(H, out);
   }
   if ((rc = save_checkpoint(H)) || (rc = launch_steps(H, dt, nsteps))) return rc;
   CK(cudaEventRecord(H->ev_steps, H->stream));
   CK(cudaStreamWaitEvent(H->side, H->ev_steps, 0));
   if ((rc = enqueue_energy(H, H->side))) return rc;
   CK(cudaEventRecord(H->ev_side, H->side));
-  if ((rc = store_state(H, h, u))) return rc;
+  if ((rc = store_state(H, h, u, &out))) return rc;
   CK(cudaStreamWaitEvent(H->stream, H->ev_side, 0));
   int f = 0;
-  if ((rc = read_flags(H, &f))) return rc;
+  if ((rc = read_flags(H, &f, out))) return rc;
   const double te = H->h_result[Q_PE] + H->h_result[Q_KE];
   bool trip = guard_decide(H, te, H->h_result[Q_UMAX]);
   if (!trip && (rc = error_proxy(H, nsteps, &trip))) return rc;
   if (!trip) return flags_status(H, f);
   if ((rc = roll_back(H)) || (rc = launch_steps(H, dt, nsteps)) ||
-      (rc = store_state(H, h, u)))
+      (rc = store_state(H, h, u, &out)))
     return rc;
-  return check_flags(H);
+  return check_flags(H, out);
 }
 
 // the guard's bounds and the error proxy's buffer (FP32 learned handles)
@@ -1202,9 +1204,10 @@ int imodel_swm_get_state(void *handle, double *h, double *u) {
   if (!H || !h || !u) return IMODEL_SWM_EINVAL;
   if (!H->state_set) return imodel::set_error(H, IMODEL_SWM_ESTATE, "no state set");
   if (cudaSetDevice(H->device) != cudaSuccess) return IMODEL_SWM_ECUDA;
-  int rc = imodel::store_state(H, h, u);
+  imodel::SmallOut out;
+  int rc = imodel::store_state(H, h, u, &out);
   if (rc) return rc;
-  return imodel::check_flags(H);
+  return imodel::check_flags(H, out);
 }
 
 int imodel_swm_advance(void *handle, double dt, int32_t nsteps) {
@@ -1241,7 +1244,6 @@ int imodel_swm_tendency(void *handle, const double *h, const double *u, double *
       imodel::launch_load_host<double>(N, z, z + H->nv, {nullptr, W.ya_h, nullptr},
                                        {nullptr, W.ya_u, nullptr}, 0.0, H->stream);
       imodel::launch_stage64(H->M, W, W.ya_h, W.ya_u, nullptr, nullptr, -1, 0.0, H->stream);
-      z = imodel::small_out(H, masseq, momeq);
       imodel::launch_store_host<double>(N, W.tend_h, W.tend_u, z, z + H->nv, 0.0, nullptr,
                                         H->stream);
     } else {
@@ -1249,13 +1251,12 @@ int imodel_swm_tendency(void *handle, const double *h, const double *u, double *
       imodel::launch_load_host<float>(N, z, z + H->nv, {nullptr, W.ya_h, nullptr},
                                       {nullptr, W.ya_u, nullptr}, H->h_ref, H->stream);
       imodel::launch_stage32(H->M, W, W.ya_h, W.ya_u, nullptr, nullptr, -1, 0.0f, H->stream);
-      z = imodel::small_out(H, masseq, momeq);
       imodel::launch_store_host<float>(N, W.tend_h, W.tend_u, z, z + H->nv, 0.0, nullptr,
                                        H->stream);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return imodel::set_error(H, IMODEL_SWM_ECUDA, cudaGetErrorString(e));
-    return imodel::check_flags(H);
+    return imodel::check_flags(H, {masseq, momeq});
   }
   cudaError_t e;
   e = cudaMemcpyAsync(H->d_stage_h, h, sizeof(double) * H->nv, cudaMemcpyHostToDevice, H->stream);
