@@ -511,8 +511,7 @@ int store_state(Handle *H, double *h, double *u, SmallOut *out) {
 // reads and clears the device flags (synchronising the stream), and hands over
 // what the call's results in the area go to
 int read_flags(Handle *H, int *f, const SmallOut &out = {}) {
-  launch_take_flags(H->d_flags, H->h_flags, H->stream);
-  CK(cudaGetLastError());
+  CK(launch_take_flags(H->d_flags, H->h_flags, H->stream));
   CK(cudaStreamSynchronize(H->stream));
   *f = *H->h_flags;
   if (out.h) {

@@ -148,9 +148,10 @@ __device__ __forceinline__ void after_prior(P &...p) {
 inline bool pdl_grid(int grid) { return static_cast<unsigned>(grid) < kPdlGrid; }
 // launches k, which calls after_prior, so that it may start before the kernel
 // before it in the stream has finished (level 8 FP64, whose grids are above
-// kPdlGrid: 1597 us a step without, 1593 with)
+// kPdlGrid: 1597 us a step without, 1593 with); the launch's own status, with
+// which no error that something else left in the thread is mixed up
 template <class... P, class... A>
-inline void launch_pdl_smem(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s,
+inline cudaError_t launch_pdl_smem(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s,
                             A &&...a) {
   cudaLaunchConfig_t c{};
   c.gridDim = dim3(grid);
@@ -162,11 +163,11 @@ inline void launch_pdl_smem(void (*k)(P...), int grid, int block, size_t smem, c
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
   c.numAttrs = 1;
-  cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
+  return cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
 }
 template <class... P, class... A>
-inline void launch_pdl(void (*k)(P...), int grid, int block, cudaStream_t s, A &&...a) {
-  launch_pdl_smem(k, grid, block, 0, s, a...);
+inline cudaError_t launch_pdl(void (*k)(P...), int grid, int block, cudaStream_t s, A &&...a) {
+  return launch_pdl_smem(k, grid, block, 0, s, a...);
 }
 
 // Laplacian diffusion and hyperdiffusion of the momentum (diffusion_ed,
@@ -409,7 +410,7 @@ template <class T>
 void launch_store_host(const HostMap &N, const T *src_h, const T *src_u, double *h, double *u,
                        double shift, int *flags, cudaStream_t s);
 // *host = *flags, *flags = 0 (host: page-locked)
-void launch_take_flags(int *flags, int *host, cudaStream_t s);
+cudaError_t launch_take_flags(int *flags, int *host, cudaStream_t s);
 
 // Compensated FP64 integrals.  Scratch: partial sums, 2 doubles per block
 // and quantity; result[kDiagQ] on the device.

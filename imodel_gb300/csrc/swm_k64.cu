@@ -1206,8 +1206,8 @@ template void launch_store_host<double>(const HostMap &, const double *, const d
                                         double *, double, int *, cudaStream_t);
 template void launch_store_host<float>(const HostMap &, const float *, const float *, double *,
                                        double *, double, int *, cudaStream_t);
-void launch_take_flags(int *flags, int *host, cudaStream_t s) {
-  launch_pdl(k_take_flags, 1, 1, s, flags, host);
+cudaError_t launch_take_flags(int *flags, int *host, cudaStream_t s) {
+  return launch_pdl(k_take_flags, 1, 1, s, flags, host);
 }
 
 void launch_trsk_tangent(const DevMesh &M, const double *u, double *utg, cudaStream_t s) {

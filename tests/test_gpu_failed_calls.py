@@ -47,3 +47,24 @@ def test_a_failed_call_keeps_no_address_of_the_caller(grid_at, precision, call):
     m.get_state()
     assert np.all(ho == -1.0) and np.all(uo == -2.0)
     m.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_steps_do_not_fail_on_an_error_of_something_else(grid_at, precision):
+    """advance checks its own launches: another part of the program that ran
+    out of memory does not make it fail."""
+    g = grid_at(3)
+    h, u = swm.initialize_fields_tc2(g)
+    out = []
+    for leave in (False, True):
+        m = SWM(g, precision)
+        m.set_state(h, u)
+        if leave:
+            _leave_an_error()
+        m.advance(300.0, 3)
+        if leave:
+            ctypes.CDLL("libcudart.so.13").cudaGetLastError()
+        out.append(m.get_state())
+        m.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
