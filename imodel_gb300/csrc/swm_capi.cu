@@ -227,7 +227,7 @@ int dalloc(Handle *H, T **p, size_t n) {
 }
 
 // the tiles of the fused FP32 stage (none when the layout does not fit)
-int upload_tiles(Handle *H, const Layout &L) {
+int make_tiles(Handle *H, const Layout &L) {
   TileLayout T;
   if (!build_tiles(L, tile_cap(L.nv), T)) return IMODEL_SWM_OK;
   TileDev D;
@@ -259,6 +259,22 @@ int upload_tiles(Handle *H, const Layout &L) {
   CK(f);
   H->W32.tiles = D;
   H->ntiles = D.ntiles;
+  return IMODEL_SWM_OK;
+}
+// The last allocation of a create: the separate kernels need no tiles, so
+// without memory for them (0.6 GB at level 9) the handle steps with those.
+int upload_tiles(Handle *H, const Layout &L) {
+  const size_t kept = H->allocs.size();
+  int rc;
+  try {
+    rc = make_tiles(H, L);
+  } catch (const std::bad_alloc &) {
+    rc = IMODEL_SWM_ENOMEM;
+  }
+  if (rc != IMODEL_SWM_ENOMEM) return rc;
+  cudaGetLastError();
+  for (; H->allocs.size() > kept; H->allocs.pop_back()) cudaFree(H->allocs.back());
+  H->err.clear();
   return IMODEL_SWM_OK;
 }
 
@@ -978,9 +994,6 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
     launch_consts64(M, p, nullptr);  // the stream of the uploads and the zero-fill
     CK(cudaGetLastError());
   }
-  if (H->precision == IMODEL_SWM_FP32 && scheme == IMODEL_SWM_TRSK10 &&
-      (rc = upload_tiles(H, L)))
-    return rc;
   H->d_cell_n2o = const_cast<int32_t *>(cn2o);
   H->d_edge_n2o = const_cast<int32_t *>(en2o);
   const int32_t *co2n = nullptr, *eo2n = nullptr;
@@ -1051,6 +1064,9 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
       H->learned_on = H->learned_active = true;
     }
   }
+  if (H->precision == IMODEL_SWM_FP32 && scheme == IMODEL_SWM_TRSK10 &&
+      (rc = upload_tiles(H, L)))
+    return rc;
   CK(cudaDeviceSynchronize());
   return IMODEL_SWM_OK;
 }
