@@ -41,6 +41,8 @@ def test_a_failed_call_keeps_no_address_of_the_caller(grid_at, precision, call):
     assert rc == _capi.ECUDA or rc == _capi.ENOMEM
     # the arrays are the program's again: no later call writes to them
     ho[:], uo[:] = -1.0, -2.0
+    m.advance(300.0, 1)
+    assert np.all(ho == -1.0) and np.all(uo == -2.0)
     m.set_state(h, u)
     m.advance(300.0, 1)
     m.diagnostics()
