@@ -145,7 +145,6 @@ __device__ __forceinline__ void after_prior(P &...p) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   (pin_ptr(p), ...);
 }
-inline bool pdl_grid(int grid) { return static_cast<unsigned>(grid) < kPdlGrid; }
 // launches k, which calls after_prior, so that it may start before the kernel
 // before it in the stream has finished (level 8 FP64, whose grids are above
 // kPdlGrid: 1597 us a step without, 1593 with); the launch's own status, with

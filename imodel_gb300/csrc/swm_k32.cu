@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(512) k_tri32(DevMesh M, const float *__restric
 // (scalar_tr2ed), the circumcentre-distance weights of pxt16 (qw) or
 // gass18's rhombus PV (qw and the triangle depths ht: (w1 eta1 + w2 eta2) /
 // (w1 h1 + w2 h2), eta = q h, with scalar_elem_divide's guard)
+template <class Wait>
 __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__restrict__ hd,
                                                     const float *__restrict__ u,
                                                     const float *__restrict__ q_tr,
@@ -43,7 +44,7 @@ __global__ void __launch_bounds__(512) k_edge_pre32(DevMesh M, const float *__re
                                                     const float *__restrict__ coefdiv,
                                                     const float *__restrict__ coefvort,
                                                     float *__restrict__ lap) {
-  after_prior<true>(hd, u, q_tr, uh, q_ed, qg, vhx, ht, coefdiv, coefvort, lap);
+  IMODEL_WAIT(Wait, hd, u, q_tr, uh, q_ed, qg, vhx, ht, coefdiv, coefvort, lap);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(256) k_apvm32(DevMesh M, const float *__restri
 }
 
 // -div F, K, Bernoulli potential g (h - h_ref + b) + K, mass RK stage
+template <class Wait>
 __global__ void __launch_bounds__(512) k_cell32(DevMesh M, const float *__restrict__ hd,
                                                 const float *__restrict__ u,
                                                 const float *__restrict__ uh,
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(512) k_cell32(DevMesh M, const float *__restri
                                                 float *__restrict__ yout,
                                                 float *__restrict__ tend, int stage, float dt,
                                                 float grav, int perot) {
-  after_prior<true>(hd, u, uh, bern, yn, acc, yout, tend);
+  IMODEL_WAIT(Wait, hd, u, uh, bern, yn, acc, yout, tend);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nv = M.nv;
   if (i >= nv) return;
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(512) k_cell32(DevMesh M, const float *__restri
 }
 
 // -grad B - TRSK PV flux, momentum RK stage
+template <class Wait>
 __global__ void __launch_bounds__(512) k_edge32(DevMesh M, const float *__restrict__ bern,
                                                 const float *__restrict__ uh,
                                                 const float *__restrict__ q_ed,
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(512) k_edge32(DevMesh M, const float *__restri
                                                 const float *__restrict__ dif2,
                                                 const int32_t *__restrict__ stq,
                                                 const float *__restrict__ q_tr, int dtred) {
-  after_prior<true>(bern, uh, q_ed, yn, acc, yout, tend, dif1, dif2, q_tr);
+  IMODEL_WAIT(Wait, bern, uh, q_ed, yn, acc, yout, tend, dif1, dif2, q_tr);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne;
   if (e >= ne) return;
@@ -548,6 +551,7 @@ __global__ void __launch_bounds__(512) k_cell32g(DevMesh M, const float *__restr
 // q_t P_t once per triangle (uh_s = u_s (h_ref + the mean of the two
 // corners on edge s), the edge pre-pass's F bit for bit); the edge kernel
 // projects the two triangles' vectors on its normal.
+template <class Wait>
 __global__ void __launch_bounds__(512) k_tri32d(DevMesh M, const float *__restrict__ hd,
                                                 const float *__restrict__ u,
                                                 float *__restrict__ q_tr, float h_ref,
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(512) k_tri32d(DevMesh M, const float *__restri
   const int ed[3] = {a.x, a.y, a.z}, cv[3] = {a.w, b.x, b.y};
   const float circ[3] = {__int_as_float(b.z), __int_as_float(b.w), c.x};
   const float kite[3] = {c.y, c.z, c.w};
-  after_prior<true>(hd, u, q_tr, coefvort, wq);
+  IMODEL_WAIT(Wait, hd, u, q_tr, coefvort, wq);
   tri_core<NoWait>(t, ed, cv, circ, kite, __ldg(&M.t_f32[t]), hd, u,
                                     q_tr, h_ref, pv_on, flags, kt, coefvort, nullptr);
   const float q = q_tr[t];
@@ -583,6 +587,7 @@ __global__ void __launch_bounds__(512) k_tri32d(DevMesh M, const float *__restri
 }
 
 // -grad B - Q_e and the momentum RK stage of edge e (dtred)
+template <class Wait>
 __global__ void __launch_bounds__(512) k_edge32d(DevMesh M, const float *__restrict__ bern,
                                                  const float *__restrict__ wq,
                                                  const float *__restrict__ yn,
@@ -591,7 +596,7 @@ __global__ void __launch_bounds__(512) k_edge32d(DevMesh M, const float *__restr
                                                  float *__restrict__ tend, int stage, float dt,
                                                  int mom_on, const float *__restrict__ dif1,
                                                  const float *__restrict__ dif2) {
-  after_prior<true>(bern, wq, yn, acc, yout, tend, dif1, dif2);
+  IMODEL_WAIT(Wait, bern, wq, yn, acc, yout, tend, dif1, dif2);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = M.ne, nt = M.nt;
   if (e >= ne) return;
@@ -733,12 +738,15 @@ __global__ void __launch_bounds__(256) k_departure(DevMesh M, const float *__res
 
 inline int nblocks(int n, int t) { return (n + t - 1) / t; }
 
-// kp, the instance that waits for its predecessor itself, on small grids; kn
-// without the wait on large ones
+// kp, the instance that waits for its predecessor itself, on grids of fewer
+// than `limit` blocks; kn, without the wait, on larger ones.  Level 9, us a step
+// with the wait in variant 0's kernels on every grid and by this rule: 1944,
+// 1858; with APVM 2514, 2428; pxt16 2068, 1981; gass18 2376, 2304; dtred 1186,
+// 1172.
 template <class... P, class... A>
-void launch_wait(void (*kp)(P...), void (*kn)(P...), int grid, int block, cudaStream_t s,
-                 A &&...a) {
-  if (pdl_grid(grid))
+void launch_wait(void (*kp)(P...), void (*kn)(P...), unsigned limit, int grid, int block,
+                 cudaStream_t s, A &&...a) {
+  if (static_cast<unsigned>(grid) < limit)
     launch_pdl(kp, grid, block, s, a...);
   else
     kn<<<grid, block, 0, s>>>(static_cast<P>(a)...);
@@ -790,15 +798,15 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
   // gass18 needs the triangle depths of the 32-bit triangle kernel, dtred
   // the Perot vectors of its own
   if (dtred1)
-    launch_pdl(k_tri32d, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M, h_in, u_in, W.q_tr, W.h_ref,
-               W.pv_on, W.flags, D.kt, cvort, W.vhq);
+    launch_wait(k_tri32d<PriorWait>, k_tri32d<NoWait>, kPdlGrid, nblocks(M.nt, T.bs_tri),
+                T.bs_tri, s, M, h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort, W.vhq);
   else if (T.variant >= 1 && W.scheme != IMODEL_SWM_GASS18)
-    launch_wait(k_tri32c<PriorWait>, k_tri32c<NoWait>, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M,
-               h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort);
+    launch_wait(k_tri32c<PriorWait>, k_tri32c<NoWait>, kPdlGrid, nblocks(M.nt, T.bs_tri),
+                T.bs_tri, s, M, h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort);
   else
-    launch_wait(k_tri32<PriorWait>, k_tri32<NoWait>, nblocks(M.nt, T.bs_tri), T.bs_tri, s, M,
-               h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort, W.scheme ==
-               IMODEL_SWM_GASS18 ? W.h_trs : nullptr);
+    launch_wait(k_tri32<PriorWait>, k_tri32<NoWait>, kPdlGrid, nblocks(M.nt, T.bs_tri), T.bs_tri,
+                s, M, h_in, u_in, W.q_tr, W.h_ref, W.pv_on, W.flags, D.kt, cvort,
+                W.scheme == IMODEL_SWM_GASS18 ? W.h_trs : nullptr);
   if (T.variant >= 1) {
     if (ev) cudaEventRecord(ev[1], s);
     // learned correction: formed once per step from the first stage's state
@@ -815,10 +823,11 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
       launch_pdl(k_apvm32, nbt + nbc, 256, s, M, W.q_tr, u_in, qg4, vhx4, nbt, D.kcv,
                  lap_in ? D.coefdiv : nullptr);
     if (A.on || gass)
-      launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr,
-                 nullptr, W.q_ed, W.h_ref, A.on ? qg4 : nullptr, vhx4, A.coef,
-                 pxt || gass ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on, W.flags,
-                 D.coefdiv, D.coefvort, lap_in ? D.lap : nullptr);
+      launch_wait(k_edge_pre32<PriorWait>, k_edge_pre32<NoWait>, kPdlGrid,
+                  nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr, nullptr, W.q_ed,
+                  W.h_ref, A.on ? qg4 : nullptr, vhx4, A.coef, pxt || gass ? M.e_qw32 : nullptr,
+                  gass ? W.h_trs : nullptr, W.pv_on, W.flags, D.coefdiv, D.coefvort,
+                  lap_in ? D.lap : nullptr);
     if (ev) cudaEventRecord(ev[2], s);
     if (gass)
       launch_pdl(k_cell32g, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern,
@@ -833,26 +842,26 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
                  W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref,
                  D.kcv, D.on ? D.coefdiv : nullptr);
     else if (dtred1)
-      launch_wait(k_cell32v2<PriorWait, false, false>, k_cell32v2<NoWait, false, false>,
-                 nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux,
-                 W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ?
-                 D.coefdiv : nullptr, nullptr, 0, nullptr, nullptr);
+      launch_wait(k_cell32v2<PriorWait, false, false>, k_cell32v2<NoWait, false, false>, kPdlGrid,
+                  nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux,
+                  W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv,
+                  D.on ? D.coefdiv : nullptr, nullptr, 0, nullptr, nullptr);
     else if (lap_in) {
       const int nc = nblocks(M.nv, T.bs_cell);
       launch_wait(k_cell32v2<PriorWait, true, true, true>, k_cell32v2<NoWait, true, true, true>,
-                  nc + nblocks(M.nt, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern,
-                  W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv,
-                  D.coefdiv, D.lap, nc, D.kt, D.coefvort);
+                  kPdlGrid, nc + nblocks(M.nt, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed,
+                  W.bern, W.zflux, W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref,
+                  D.kcv, D.coefdiv, D.lap, nc, D.kt, D.coefvort);
     } else if (A.on)
-      launch_wait(k_cell32v2<PriorWait, true>, k_cell32v2<NoWait, true>, nblocks(M.nv, T.bs_cell),
-                 T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern, W.zflux, W.yn_h, W.acc_h, h_out,
-                 W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv : nullptr, nullptr, 0,
-                 nullptr, nullptr);
+      launch_wait(k_cell32v2<PriorWait, true>, k_cell32v2<NoWait, true>, kPdlGrid,
+                  nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_ed, W.bern, W.zflux,
+                  W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv,
+                  D.on ? D.coefdiv : nullptr, nullptr, 0, nullptr, nullptr);
     else
-      launch_wait(k_cell32v2<PriorWait, false>, k_cell32v2<NoWait, false>, nblocks(M.nv,
-                 T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux, W.yn_h,
-                 W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv, D.on ? D.coefdiv :
-                 nullptr, nullptr, 0, nullptr, nullptr);
+      launch_wait(k_cell32v2<PriorWait, false>, k_cell32v2<NoWait, false>, kPdlGrid,
+                  nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.q_tr, W.bern, W.zflux,
+                  W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, W.h_ref, D.kcv,
+                  D.on ? D.coefdiv : nullptr, nullptr, 0, nullptr, nullptr);
     if (!lap_in) diffusion_tail(!dtred1);
     EdgeDif E;
     if (D.on) {
@@ -863,12 +872,14 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
     }
     if (ev) cudaEventRecord(ev[3], s);
     if (dtred1)
-      launch_pdl(k_edge32d, nblocks(M.ne, T.bs_edge), T.bs_edge, s, M, W.bern, W.vhq, W.yn_u,
-                 W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2);
+      launch_wait(k_edge32d<PriorWait>, k_edge32d<NoWait>, kPdlGrid, nblocks(M.ne, T.bs_edge),
+                  T.bs_edge, s, M, W.bern, W.vhq, W.yn_u, W.acc_u, u_out, W.tend_u, stage, dt,
+                  W.mom_on, dif1, dif2);
     else
-      launch_wait(k_edge32v2<PriorWait>, k_edge32v2<NoWait>, nblocks((M.ne + 1) / 2, T.bs_edge),
-                 T.bs_edge, s, M, W.bern, W.zflux, W.yn_u, W.acc_u, u_out, W.tend_u, stage, dt,
-                 W.mom_on, static_cast<float>(M.erad), W.learned ? W.learned->corr : nullptr, E);
+      launch_wait(k_edge32v2<PriorWait>, k_edge32v2<NoWait>, kPdlGrid,
+                  nblocks((M.ne + 1) / 2, T.bs_edge), T.bs_edge, s, M, W.bern, W.zflux, W.yn_u,
+                  W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, static_cast<float>(M.erad),
+                  W.learned ? W.learned->corr : nullptr, E);
     if (ev) cudaEventRecord(ev[4], s);
     return;
   }
@@ -878,17 +889,26 @@ void launch_stage32(const DevMesh &M, const Work<float> &W, const float *h_in,
   // Perot KE, pered), gass18 (rhombus PV, connecting-edge PV), dtred
   const int sch = W.scheme;
   const bool pxt = sch == IMODEL_SWM_PXT16, gass = sch == IMODEL_SWM_GASS18;
-  launch_pdl(k_edge_pre32, nblocks(M.ne, T.bs_pre), T.bs_pre, s, M, h_in, u_in, W.q_tr, W.uh,
-             W.q_ed, W.h_ref, A.on ? qg4 : nullptr, vhx4, A.coef, pxt || gass ? M.e_qw32 : nullptr,
-             gass ? W.h_trs : nullptr, W.pv_on, W.flags, nullptr, nullptr, nullptr);
+  launch_wait(k_edge_pre32<PriorWait>, k_edge_pre32<NoWait>, kPdlGrid, nblocks(M.ne, T.bs_pre),
+              T.bs_pre, s, M, h_in, u_in, W.q_tr, W.uh, W.q_ed, W.h_ref, A.on ? qg4 : nullptr,
+              vhx4, A.coef, pxt || gass ? M.e_qw32 : nullptr, gass ? W.h_trs : nullptr, W.pv_on,
+              W.flags, nullptr, nullptr, nullptr);
   if (ev) cudaEventRecord(ev[2], s);
-  launch_pdl(k_cell32, nblocks(M.nv, T.bs_cell), T.bs_cell, s, M, h_in, u_in, W.uh, W.bern,
-             W.yn_h, W.acc_h, h_out, W.tend_h, stage, dt, grav, pxt ? 1 : 0);
+  launch_wait(k_cell32<PriorWait>, k_cell32<NoWait>, kPdlGrid, nblocks(M.nv, T.bs_cell),
+              T.bs_cell, s, M, h_in, u_in, W.uh, W.bern, W.yn_h, W.acc_h, h_out, W.tend_h, stage,
+              dt, grav, pxt ? 1 : 0);
   diffusion_tail(false);
   if (ev) cudaEventRecord(ev[3], s);
-  launch_pdl(k_edge32, nblocks(M.ne, T.bs_edge), T.bs_edge, s, M, W.bern, W.uh, W.q_ed, W.yn_u,
-             W.acc_u, u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2, gass ? M.e_stq : nullptr,
-             W.q_tr, sch == IMODEL_SWM_DTRED ? 1 : 0);
+  // The ten-entry stencil's blocks are long: where several rounds of them follow,
+  // those that start early hold up the cells' (us a step with the wait and
+  // without, level 7 and 8: 139.8 and 541, 127.2 and 528; gass18 198.7 and 658,
+  // 195.9 and 642; level 6 has 480 blocks, and 60.6 with it, 62.5 without).
+  // dtred's edges read their triangles alone (level 8: 328, 334).
+  const bool dtred = sch == IMODEL_SWM_DTRED;
+  launch_wait(k_edge32<PriorWait>, k_edge32<NoWait>, dtred ? kPdlGrid : kPdlGrid / 8,
+              nblocks(M.ne, T.bs_edge), T.bs_edge, s, M, W.bern, W.uh, W.q_ed, W.yn_u, W.acc_u,
+              u_out, W.tend_u, stage, dt, W.mom_on, dif1, dif2, gass ? M.e_stq : nullptr, W.q_tr,
+              dtred ? 1 : 0);
   if (ev) cudaEventRecord(ev[4], s);
 }
 
