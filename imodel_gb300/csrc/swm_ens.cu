@@ -302,38 +302,62 @@ int zalloc(Ens *E, T **p, size_t n) {
   return IMODEL_SWM_OK;
 }
 
-// the tiles' blocks, from a copy of the layout's arrays that is not kept
+// the tiles' blocks, from a copy of the layout's arrays that is not kept: in one
+// allocation, as getting and freeing each of the twelve took longer than all
+// copies
 int fill_tiles(Ens *E, const Layout &L, const TileLayout &T, const int4 *head, uint4 *data) {
-  const size_t kept = E->allocs.size();
-  DevMesh M;
-  std::memset(&M, 0, sizeof(M));
-  M.nv = L.nv;
-  M.ne = L.ne;
-  M.nt = L.nt;
-  const std::vector<float> bt32(L.nv, 0.0f);
-  const int32_t *ra = nullptr, *rb = nullptr, *rc3 = nullptr, *pk = nullptr, *lists = nullptr;
-  const float *kd = nullptr;
-  const uint32_t *vs2 = nullptr;
-  int rc;
-  if ((rc = up(E, L.t_recA, &ra)) || (rc = up(E, L.t_recB, &rb)) || (rc = up(E, L.t_recC, &rc3)) ||
-      (rc = up(E, L.t_f32, &M.t_f32)) || (rc = up(E, L.c_meta, &M.c_meta)) ||
-      (rc = up(E, L.c_inva32, &M.c_inva32)) || (rc = up(E, bt32, &M.c_bt32)) ||
-      (rc = up(E, L.e_grad32, &M.e_grad32)) || (rc = up(E, L.c_pk, &pk)) ||
-      (rc = up(E, L.c_kd, &kd)) || (rc = up(E, L.e_vs2, &vs2)) || (rc = up(E, T.lists, &lists)))
-    return rc;
-  M.t_recA = reinterpret_cast<const int4 *>(ra);
-  M.t_recB = reinterpret_cast<const int4 *>(rb);
-  M.t_recC = reinterpret_cast<const float4 *>(rc3);
-  M.c_pk = reinterpret_cast<const int4 *>(pk);
-  M.c_kd = reinterpret_cast<const float2 *>(kd);
-  M.e_vs2 = reinterpret_cast<const uint2 *>(vs2);
-  launch_fill_tiles(M, T.ntiles, head, lists, data, nullptr);
-  EK(cudaGetLastError());
-  EK(cudaStreamSynchronize(nullptr));
-  while (E->allocs.size() > kept) {
-    EK(cudaFree(E->allocs.back()));
-    E->allocs.pop_back();
+  size_t bytes = 0;
+  auto place = [&bytes](size_t n) {  // 256-byte aligned, as cudaMalloc would
+    const size_t at = bytes;
+    bytes += (n + 255) & ~static_cast<size_t>(255);
+    return at;
+  };
+  auto size = [](const auto &v) { return v.size() * sizeof(v[0]); };
+  const size_t ra = place(size(L.t_recA)), rb = place(size(L.t_recB)), rc = place(size(L.t_recC)),
+               f = place(size(L.t_f32)), meta = place(size(L.c_meta)),
+               inva = place(size(L.c_inva32)), bt = place(sizeof(float) * L.nv),
+               gr = place(size(L.e_grad32)), pk = place(size(L.c_pk)), kd = place(size(L.c_kd)),
+               vs2 = place(size(L.e_vs2)), li = place(size(T.lists));
+  char *p = nullptr;
+  EK(cudaMalloc(&p, bytes));
+  cudaError_t e = cudaMemsetAsync(p + bt, 0, sizeof(float) * L.nv, nullptr);
+  auto copy = [&](size_t at, const auto &v) {
+    if (e == cudaSuccess) e = cudaMemcpy(p + at, v.data(), size(v), cudaMemcpyHostToDevice);
+  };
+  copy(ra, L.t_recA);
+  copy(rb, L.t_recB);
+  copy(rc, L.t_recC);
+  copy(f, L.t_f32);
+  copy(meta, L.c_meta);
+  copy(inva, L.c_inva32);
+  copy(gr, L.e_grad32);
+  copy(pk, L.c_pk);
+  copy(kd, L.c_kd);
+  copy(vs2, L.e_vs2);
+  copy(li, T.lists);
+  if (e == cudaSuccess) {
+    DevMesh M;
+    std::memset(&M, 0, sizeof(M));
+    M.nv = L.nv;
+    M.ne = L.ne;
+    M.nt = L.nt;
+    M.t_recA = reinterpret_cast<const int4 *>(p + ra);
+    M.t_recB = reinterpret_cast<const int4 *>(p + rb);
+    M.t_recC = reinterpret_cast<const float4 *>(p + rc);
+    M.t_f32 = reinterpret_cast<const float *>(p + f);
+    M.c_meta = reinterpret_cast<const uint32_t *>(p + meta);
+    M.c_inva32 = reinterpret_cast<const float *>(p + inva);
+    M.c_bt32 = reinterpret_cast<const float *>(p + bt);
+    M.e_grad32 = reinterpret_cast<const float *>(p + gr);
+    M.c_pk = reinterpret_cast<const int4 *>(p + pk);
+    M.c_kd = reinterpret_cast<const float2 *>(p + kd);
+    M.e_vs2 = reinterpret_cast<const uint2 *>(p + vs2);
+    launch_fill_tiles(M, T.ntiles, head, reinterpret_cast<const int32_t *>(p + li), data, nullptr);
+    e = cudaGetLastError();
   }
+  const cudaError_t g = cudaFree(p);  // waits for the kernel
+  EK(e);
+  EK(g);
   return IMODEL_SWM_OK;
 }
 
