@@ -109,6 +109,7 @@ SWM_SYMBOLS = [
     "imodel_swm_get_state", "imodel_swm_advance", "imodel_swm_profile",
     "imodel_swm_autotune", "imodel_swm_set_tuning", "imodel_swm_set_diffusion",
     "imodel_swm_set_diffusion_fields", "imodel_swm_set_apvm", "imodel_swm_test_fail_alloc",
+    "imodel_swm_test_tune_search",
     "imodel_swm_learned_weights", "imodel_swm_learned_error_proxy",
     "imodel_swm_test_layout_digest",
     "imodel_swm_launch_count",

@@ -20,6 +20,7 @@
 #include "imodel_moist.h"
 #include "imodel_swm.h"
 #include "swm_common.cuh"
+#include "swm_tune.h"
 #include "swm_layout.h"
 
 namespace imodel {
@@ -59,6 +60,15 @@ struct StepGraphs {
     cudaGraphDestroy(g);
     return e;
   }
+  // the graph of kMany steps beside the one of a step
+  template <class F>
+  void make_many(cudaStream_t s, F step) {
+    size_t nodes = 0;
+    if (many || from == INT64_MAX || capture(s, kMany, step, &many, &nodes) == cudaSuccess) return;
+    cudaGetLastError();  // go on with single steps
+    many = nullptr;
+    from = INT64_MAX;
+  }
   // n steps, each enqueued by step()
   template <class F>
   cudaError_t replay(cudaStream_t s, double dt_, int n, F step) {
@@ -71,13 +81,7 @@ struct StepGraphs {
       from = nodes <= 4 ? 32 : 32 * static_cast<int64_t>(nodes);
     }
     steps += n;
-    if (!many && n >= kMany && steps >= from) {
-      if (capture(s, kMany, step, &many, &nodes) != cudaSuccess) {
-        cudaGetLastError();  // go on with single steps
-        many = nullptr;
-        from = INT64_MAX;
-      }
-    }
+    if (n >= kMany && steps >= from) make_many(s, step);
     int k = 0;
     for (; many && k + kMany <= n; k += kMany)
       if ((e = cudaGraphLaunch(many, s)) != cudaSuccess) return e;
@@ -1476,6 +1480,9 @@ int imodel_swm_autotune(void *handle, double dt, int32_t nsteps, int32_t choice[
     };
     if (e == cudaSuccess) e = run(1);  // warm-up
     if (e != cudaSuccess) return 1e30f;
+    // the many-step graph too, so that only steps lie between the events
+    if (nsteps >= imodel::StepGraphs::kMany)
+      H->graphs.make_many(H->stream, [=] { imodel::enqueue_step(H, dt); });
     cudaEventRecord(e0, H->stream);
     e = run(nsteps);
     cudaEventRecord(e1, H->stream);
@@ -1484,50 +1491,15 @@ int imodel_swm_autotune(void *handle, double dt, int32_t nsteps, int32_t choice[
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
     return e == cudaSuccess ? ms : 1e30f;
   };
-  const int sizes[3] = {128, 256, 512};
-  imodel::Tune best;
-  float best_ms = 1e30f;
+  imodel::TuneSpace space;
   // the learned correction is wired into the cell-centred variants only
-  for (int v = H->learned_mode == 1 ? 1 : 0; v <= (H->v0_only ? 0 : 2); ++v)
-    for (int b : sizes) {
-      imodel::Tune t;
-      t.variant = v;
-      t.bs_tri = t.bs_pre = t.bs_cell = t.bs_edge = b;
-      const float ms = trial(t);
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = t;
-      }
-    }
-  // refine the block size of each kernel with the others fixed
-  int imodel::Tune::*fields[4] = {&imodel::Tune::bs_tri, &imodel::Tune::bs_pre,
-                                  &imodel::Tune::bs_cell, &imodel::Tune::bs_edge};
-  for (int f = 0; f < 4; ++f) {
-    if (f == 1 && best.variant >= 1) continue;
-    for (int b : sizes) {
-      if (best.*fields[f] == b) continue;
-      imodel::Tune t = best;
-      t.*fields[f] = b;
-      const float ms = trial(t);
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = t;
-      }
-    }
-  }
-  // the learned-correction kernel's split of warps between gathering and
-  // the epilogue
-  if (H->learned_active && H->learned_mode == 1)
-    for (int g = 2; g <= 4; ++g) {
-      if (best.mlp_gather == g) continue;
-      imodel::Tune t = best;
-      t.mlp_gather = g;
-      const float ms = trial(t);
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = t;
-      }
-    }
+  space.stencil = H->learned_mode != 1;
+  space.cells = !H->v0_only;
+  imodel::Work<float> one = W;
+  one.tune.variant = 1;
+  space.fused = imodel::fused_stage(one);
+  space.network = H->learned_active && H->learned_mode == 1;
+  const imodel::Tune best = imodel::search_tune(space, trial);
   W.tune = best;
   H->graphs.drop();
   cpy(W.yn_h, sp, bh);
@@ -1640,6 +1612,32 @@ int imodel_swm_learned_error_proxy(void *handle, double *value) {
 int imodel_swm_test_fail_alloc(int32_t after) {
   if (after < 0) return IMODEL_SWM_EINVAL;
   imodel::g_fail_alloc_after.store(after);
+  return IMODEL_SWM_OK;
+}
+
+int imodel_swm_test_tune_search(const int32_t space[4], float (*trial)(const int32_t *),
+                                int32_t choice[6]) {
+  if (!space || !trial || !choice) return IMODEL_SWM_EINVAL;
+  imodel::TuneSpace S;
+  S.stencil = space[0] != 0;
+  S.cells = space[1] != 0;
+  S.fused = space[2] != 0;
+  S.network = space[3] != 0;
+  auto put = [](const imodel::Tune &t, int32_t *c) {
+    c[0] = t.variant;
+    c[1] = t.bs_tri;
+    c[2] = t.bs_pre;
+    c[3] = t.bs_cell;
+    c[4] = t.bs_edge;
+    c[5] = t.mlp_gather;
+  };
+  put(imodel::search_tune(S,
+                          [&](const imodel::Tune &t) {
+                            int32_t c[6];
+                            put(t, c);
+                            return trial(c);
+                          }),
+      choice);
   return IMODEL_SWM_OK;
 }
 

@@ -224,7 +224,9 @@ int imodel_swm_advance(void *handle, double dt, int32_t nsteps);
  * learned-correction kernel}; variant 0 uses the 10-entry edge stencil,
  * variant 1 the cell-centred TRSK sum (one kernel per stage over tiles for
  * plain trsk10 steps, separate kernels with options on), variant 2 the separate
- * kernels throughout (bit-identical results); the last entry is 2, 3 or 4 with the
+ * kernels throughout (bit-identical results).  The one-kernel stage takes no
+ * block sizes: those beside it are the separate kernels' fastest, for when an
+ * option is switched on.  The last entry is 2, 3 or 4 with the
  * learned correction on (its kernel has 6 warp groups, the rest run the
  * epilogue) and 0 without it.  The FP64 path has a single configuration and
  * returns it. */
@@ -285,6 +287,12 @@ int imodel_swm_test_layout_digest(const imodel_swm_mesh *m, int32_t scheme, int3
  * off).  It lets tests check that a failed set-up (set_apvm,
  * set_diffusion*) leaves the handle stepping correctly without the option. */
 int imodel_swm_test_fail_alloc(int32_t after);
+/* Test hook with no counterpart in the reference and no GPU use: the
+ * autotuner's search with the caller's times.  space = {stencil variant,
+ * cell-centred variants, variant 1 fused, learned-correction kernel} (0 or 1
+ * each); trial is given a configuration (as in choice) and returns its time. */
+int imodel_swm_test_tune_search(const int32_t space[4], float (*trial)(const int32_t *),
+                                int32_t choice[6]);
 /* Launches issued by one advance call for nsteps steps (kernels only). */
 int imodel_swm_launch_count(void *handle, int32_t nsteps, int64_t *count);
 /* Runs nsteps RK4 steps kernel by kernel (no graph) with CUDA events around
