@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kEnsThreads<V>, std::is_same<V, Pair>::value ?
         TileOwn<kThr, V> own;
         own.template load<!kPair>(T, F, st);
         if (fresh) {
-          if (!tc05::mbar_wait(&mbar, parity, A.flags, 32)) return;
+          if (!tc05::mbar_wait<2>(&mbar, parity, A.flags, 32)) return;
           parity ^= 1u;
         }
         own.rim(T, F, S);

@@ -61,12 +61,10 @@ __global__ void __launch_bounds__(kThr, kThr == 256 ? 3 : 4)
   TileOwn<kThr> own;
   own.load(T, F, kStage);
   __syncthreads();  // the barriers are initialised
-  if (T.slot > 0) {
-    if (!tc05::mbar_wait(&mbar[0], 0, flags, 32)) return;
-    own.rim(T, F, S);
-  }
+  // (without its lists the block still waits for its records)
+  if (T.slot > 0 && tc05::mbar_wait<2, true>(&mbar[0], 0, flags, 32)) own.rim(T, F, S);
   own.store(T, F, S);
-  if (!tc05::mbar_wait(&mbar[1], 0, flags, 32)) return;
+  if (!tc05::mbar_wait<2, true>(&mbar[1], 0, flags, 32)) return;
   __syncthreads();
   tile_triangles<kThr>(T, S, h_ref, pv_on, flags);
   __syncthreads();
@@ -136,8 +134,7 @@ __global__ void __launch_bounds__(kThr, 3)
     qc = A.qc[c];
   }
   __syncthreads();  // the barriers are initialised
-  if (T.slot > 0) {
-    if (!tc05::mbar_wait(&mbar[0], 0, A.flags, 32)) return;
+  if (T.slot > 0 && tc05::mbar_wait<2>(&mbar[0], 0, A.flags, 32)) {
     own.rim(T, F, S);
     const int32_t *hx = reinterpret_cast<const int32_t *>(smem);
     for (int q = tid; q < T.nh - T.nc; q += kThr) {
@@ -151,7 +148,7 @@ __global__ void __launch_bounds__(kThr, 3)
 #pragma unroll
   for (int k = 0; k < kTr; ++k)
     if (own_cell && (A.active >> k & 1)) tr[k * D.max_h + tid] = qi[k];
-  if (!tc05::mbar_wait(&mbar[1], 0, A.flags, 32)) return;
+  if (!tc05::mbar_wait<2>(&mbar[1], 0, A.flags, 32)) return;
   __syncthreads();
   tile_triangles<kThr>(T, S, A.h_ref, pv_on, A.flags);
   __syncthreads();

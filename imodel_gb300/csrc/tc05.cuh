@@ -82,20 +82,38 @@ __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count) {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// bounded wait for phase `parity` of the mbarrier; false (and *err |= flag)
-// if it did not complete
+// whether phase `parity` of the mbarrier is complete
+__device__ __forceinline__ bool mbar_done(uint64_t *mbar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(smem_u32(mbar)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// bounded wait for phase `parity` of the mbarrier: *err |= flag after 2^20
+// polls, and false if it is not complete after kRounds times as many (2: the
+// caller leaves next, and what it has in flight would write to memory that is
+// another block's by then).  kShort: the polls as a loop of one, for kernels of
+// few microseconds, where the code's length shows (the fused stage at level 5
+// 11.1 -> 10.5 us a step); the moist stage at level 8, at its register limit,
+// takes 262 with the loop that the compiler unrolls and 270 with this one.
+template <int kRounds = 1, bool kShort = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, int *err, int flag) {
-  for (int it = 0; it < (1 << 20); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(smem_u32(mbar)), "r"(parity)
-        : "memory");
-    if (done) return true;
+#pragma unroll 1
+  for (int round = 0; round < kRounds; ++round) {
+    if constexpr (kShort) {
+#pragma unroll 1
+      for (int it = 0; it < (1 << 20); ++it)
+        if (mbar_done(mbar, parity)) return true;
+    } else {
+      for (int it = 0; it < (1 << 20); ++it)
+        if (mbar_done(mbar, parity)) return true;
+    }
+    atomicOr(err, flag);
   }
-  atomicOr(err, flag);
   return false;
 }
 
