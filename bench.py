@@ -231,9 +231,12 @@ def kernel_bytes(nv, ne, nt, precision, variant=0, fused=False):
     w = 4 if precision == "fp32" else 8
     if fused:
         # records: triangle 36 B, cell slots 6 x 16 B and 3 words, edge 8 B;
-        # h and u: input, y_n, acc r/w, output (tiles' rims not counted)
+        # h and u, the mean of the four stages that the profile averages: input,
+        # y_n, acc r/w, output; stage 0 reads y_n as its input and only writes
+        # acc, stage 3 does not write it (tiles' rims not counted)
+        state = (3 + 5 + 5 + 4) / 4
         return {"triangle": 0, "edge_pre": 0, "edge": 0,
-                "cell": nt * 36 + nv * (6 * 16 + 12) + ne * 8 + (nv + ne) * 5 * w}
+                "cell": nt * 36 + nv * (6 * 16 + 12) + ne * 8 + (nv + ne) * state * w}
     # triangle: f, 3 circulation coefs, 3 edge idx, 3 kite coefs, 3 cell idx,
     # q out; gathers u and h
     tri = nt * (w + 3 * w + 3 * 4 + 3 * w + 3 * 4 + w) + ne * w + nv * w
@@ -362,9 +365,10 @@ MLP_FLOP_PER_EDGE = 2 * (24 * 64 + 64 * 64 + 64)
 # DRAM bytes (read + write) per unit of a launch, from one ncu capture of the
 # kernel at icos level 8 (128.0 MB for 655,362 cells), scaled to the
 # benchmark's level by the number of cells, as the traffic grows with them.
-# DRAM bytes per cell of one launch (ncu at icos level 8, an RK stage that
-# reads the accumulator)
-TRAFFIC_PER_CELL = {"k_cell32v2": 133.779e6 / 655362, "k_stage32": 877.0e6 / 2621442}
+# DRAM bytes per cell of one launch (ncu; the separate kernels in an RK stage
+# that reads the accumulator, the fused stage the mean of its four stages)
+TRAFFIC_PER_CELL = {"k_cell32v2": 133.779e6 / 655362,
+                    "k_stage32": (792.1e6 + 873.9e6 + 873.1e6 + 836.5e6) / 4 / 2621442}
 TRAFFIC_SOURCE = {"k_cell32v2": "ncu capture at icos level 8, scaled by cells",
                   "k_stage32": "ncu capture at icos level 9, scaled by cells"}
 
