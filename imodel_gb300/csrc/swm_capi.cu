@@ -1153,7 +1153,7 @@ int setup_diffusion(Handle *H, Work<T> &W, double k2, double k4, const double *k
 template <class T>
 int setup_apvm(Handle *H, Work<T> &W, double pvspar, double dt) {
   Apvm<T> &A = W.apvm;
-  // off until all three buffers exist: a failed allocation leaves the handle
+  // off until all buffers exist: a failed allocation leaves the handle
   // stepping without APVM instead of launching through a null buffer
   A.on = false;
   if (!(pvspar > 0)) return IMODEL_SWM_OK;
@@ -1161,7 +1161,8 @@ int setup_apvm(Handle *H, Work<T> &W, double pvspar, double dt) {
   const size_t k = sizeof(T) == sizeof(float) ? 4 : 3;
   if ((!A.qg && (rc = dalloc(H, &A.qg, k * static_cast<size_t>(H->nt)))) ||
       (!A.vhx && (rc = dalloc(H, &A.vhx, k * static_cast<size_t>(H->nv)))) ||
-      (!A.qge && (rc = dalloc(H, &A.qge, static_cast<size_t>(H->ne)))))
+      (sizeof(T) == sizeof(double) && !A.qge &&
+       (rc = dalloc(H, &A.qge, static_cast<size_t>(H->ne)))))
     return rc;
   A.coef = static_cast<T>(pvspar * dt);
   A.on = true;

@@ -48,7 +48,6 @@ __device__ __forceinline__ Pair all<Pair>(float a) {
 __device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
 // the same where no fused operation can arise: the compiler schedules plain
 // operators better than the intrinsics (level 7 38.9 -> 37.2 us a step)
 __device__ __forceinline__ float padd(float a, float b) { return a + b; }
