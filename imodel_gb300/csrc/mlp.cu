@@ -718,8 +718,6 @@ int imodel_mlp_create(int32_t device, void **mlp) {
   MK(cudaMemset(P->v, 0, imodel::NPART * sizeof(float)));
   MK(cudaMemset(P->d_err, 0, sizeof(int)));
   MK(cudaMallocHost(&P->h_err, sizeof(int)));
-  // the zero-fill (default stream) comes before what P->stream writes
-  MK(cudaStreamSynchronize(nullptr));
   return IMODEL_SWM_OK;
 }
 

@@ -1132,11 +1132,9 @@ int setup_diffusion(Handle *H, Work<T> &W, double k2, double k4, const double *k
   // sqrt(hx2tr(K4)), and then also replaces the Laplacian's coefficients
   const double *kf = k4on ? kf4 : kf2;
   double *kf_dev = nullptr;
-  const size_t nv = static_cast<size_t>(H->nv);
-  if (kf && !H->d_kf && (rc = dalloc(H, &H->d_kf, 2 * nv))) return rc;
-  // the zero-fill (default stream) comes before what H->stream writes
-  CK(cudaStreamSynchronize(nullptr));
   if (kf) {
+    const size_t nv = static_cast<size_t>(H->nv);
+    if (!H->d_kf && (rc = dalloc(H, &H->d_kf, 2 * nv))) return rc;
     CK(cudaMemcpyAsync(H->d_kf, kf, nv * sizeof(double), cudaMemcpyHostToDevice, H->stream));
     launch_gather_in(H->nv, H->d_cell_n2o, H->d_kf, H->d_kf + nv, 0.0, H->stream);
     kf_dev = H->d_kf + nv;
@@ -1166,8 +1164,6 @@ int setup_apvm(Handle *H, Work<T> &W, double pvspar, double dt) {
       (sizeof(T) == sizeof(double) && !A.qge &&
        (rc = dalloc(H, &A.qge, static_cast<size_t>(H->ne)))))
     return rc;
-  // the zero-fill (default stream) comes before what the steps write
-  CK(cudaStreamSynchronize(nullptr));
   A.coef = static_cast<T>(pvspar * dt);
   A.on = true;
   return IMODEL_SWM_OK;

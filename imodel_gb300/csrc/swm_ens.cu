@@ -459,8 +459,6 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
       (rc = zalloc(E, &E->bar, 1)) || (rc = zalloc(E, &E->flags, 1)))
     return rc;
   EK(cudaMallocHost(&E->h_flags, sizeof(int)));
-  // the zero-fill (default stream) comes before what E->stream writes
-  EK(cudaStreamSynchronize(nullptr));
   return IMODEL_SWM_OK;
 }
 
