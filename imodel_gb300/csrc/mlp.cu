@@ -713,10 +713,10 @@ int imodel_mlp_create(int32_t device, void **mlp) {
                                   sizeof(float)));
   MK(cudaMalloc(&P->img, (imodel::NH * imodel::K1 + 2 * imodel::NH * imodel::NH) * 2));
   MK(cudaMalloc(&P->d_err, sizeof(int)));
-  MK(cudaMemset(P->p, 0, imodel::NPART * sizeof(float)));
-  MK(cudaMemset(P->m, 0, imodel::NPART * sizeof(float)));
-  MK(cudaMemset(P->v, 0, imodel::NPART * sizeof(float)));
-  MK(cudaMemset(P->d_err, 0, sizeof(int)));
+  MK(cudaMemsetAsync(P->p, 0, imodel::NPART * sizeof(float), P->stream));
+  MK(cudaMemsetAsync(P->m, 0, imodel::NPART * sizeof(float), P->stream));
+  MK(cudaMemsetAsync(P->v, 0, imodel::NPART * sizeof(float), P->stream));
+  MK(cudaMemsetAsync(P->d_err, 0, sizeof(int), P->stream));
   MK(cudaMallocHost(&P->h_err, sizeof(int)));
   return IMODEL_SWM_OK;
 }

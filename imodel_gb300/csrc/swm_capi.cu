@@ -125,6 +125,10 @@ struct Handle {
   Work<double> W64{};
   Work<float> W32{};
   cudaStream_t stream = nullptr;
+  // where new buffers are zero-filled: the default stream with the uploads of a
+  // create, which waits for all of it at its end; afterwards `stream`, whose
+  // kernels use them next
+  cudaStream_t fill = nullptr;
   StepGraphs graphs;
   bool state_set = false;
   // learned TRSK correction: mode 1 the per-step network (FP32, cell-centred
@@ -225,7 +229,7 @@ int dalloc(Handle *H, T **p, size_t n) {
   }
   CK(cudaMalloc(&q, (n > 0 ? n : 1) * sizeof(T)));
   H->allocs.push_back(q);
-  CK(cudaMemset(q, 0, (n > 0 ? n : 1) * sizeof(T)));
+  CK(cudaMemsetAsync(q, 0, (n > 0 ? n : 1) * sizeof(T), H->fill));
   *p = static_cast<T *>(q);
   return IMODEL_SWM_OK;
 }
@@ -1072,6 +1076,7 @@ int create(Handle *H, const imodel_swm_mesh *m, const imodel_swm_opts *o) {
       (rc = upload_tiles(H, L)))
     return rc;
   CK(cudaDeviceSynchronize());
+  H->fill = H->stream;
   return IMODEL_SWM_OK;
 }
 
@@ -1947,9 +1952,6 @@ int imodel_moist_create(const imodel_swm_mesh *m, const imodel_moist_opts *o, vo
     for (int k = 0; k < 5; ++k)
       for (int b = 0; b < 4; ++b)
         if ((rc = imodel::dalloc(H, &X->f_q[k][b], nv))) return rc;
-    // the buffers' zero-fill (default stream) comes before what H->stream writes
-    if (cudaStreamSynchronize(nullptr) != cudaSuccess)
-      return imodel::set_error(H, IMODEL_SWM_ECUDA, "stream synchronize failed");
     if ((rc = moist_in32(H, o->theta, th, false, 0.0)) ||
         (rc = moist_in32(H, ex.data(), X->f_ex20, false, 0.0)))
       return rc;
@@ -1966,9 +1968,6 @@ int imodel_moist_create(const imodel_swm_mesh *m, const imodel_moist_opts *o, vo
         if ((rc = imodel::dalloc(H, &X->q[k][b], nv))) return rc;
     if ((rc = imodel::dalloc(H, &X->uphi, 5 * ne)) || (rc = imodel::dalloc(H, &X->gthb, ne)))
       return rc;
-    // the buffers' zero-fill (default stream) comes before what H->stream writes
-    if (cudaStreamSynchronize(nullptr) != cudaSuccess)
-      return imodel::set_error(H, IMODEL_SWM_ECUDA, "stream synchronize failed");
     if ((rc = moist_in(H, o->theta, X->th, false)) || (rc = moist_in(H, ex.data(), X->ex20, false)))
       return rc;
     imodel::launch_moist_consts(H->M, X->th, X->ex20, X->q0, X->gthb, H->stream);

@@ -292,12 +292,14 @@ int up(Ens *E, const std::vector<V, A> &v, const V **dst) {
   return IMODEL_SWM_OK;
 }
 
+// zero-filled on s, the stream that uses the buffer first (the tiles' blocks are
+// written on the default stream, behind the uploads)
 template <class T>
-int zalloc(Ens *E, T **p, size_t n) {
+int zalloc(Ens *E, T **p, size_t n, cudaStream_t s) {
   void *q = nullptr;
   EK(cudaMalloc(&q, (n ? n : 1) * sizeof(T)));
   E->allocs.push_back(q);
-  EK(cudaMemset(q, 0, (n ? n : 1) * sizeof(T)));
+  EK(cudaMemsetAsync(q, 0, (n ? n : 1) * sizeof(T), s));
   *p = static_cast<T *>(q);
   return IMODEL_SWM_OK;
 }
@@ -428,7 +430,7 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
     const TileHead *head = nullptr;
     uint4 *data = nullptr;
     const int32_t *cn2o = nullptr, *en2o = nullptr;
-    if ((rc = up(E, T.head, &head)) || (rc = zalloc(E, &data, T.data_bytes / sizeof(uint4))) ||
+    if ((rc = up(E, T.head, &head)) || (rc = zalloc(E, &data, T.data_bytes / sizeof(uint4), nullptr)) ||
         (rc = up(E, L.cell_n2o, &cn2o)) || (rc = up(E, L.edge_n2o, &en2o)))
       return rc;
     D.head = reinterpret_cast<const int4 *>(head);
@@ -443,10 +445,10 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
     A.smem_t = std::max(A.smem_t, T.max_t);
     float **bv[] = {&W.yn_h, &W.ya_h, &W.yb_h, &W.acc_h};
     for (float **b : bv)
-      if ((rc = zalloc(E, b, static_cast<size_t>(L.nv) * M))) return rc;
+      if ((rc = zalloc(E, b, static_cast<size_t>(L.nv) * M, E->stream))) return rc;
     float **be[] = {&W.yn_u, &W.ya_u, &W.yb_u, &W.acc_u};
     for (float **b : be)
-      if ((rc = zalloc(E, b, static_cast<size_t>(L.ne) * M))) return rc;
+      if ((rc = zalloc(E, b, static_cast<size_t>(L.ne) * M, E->stream))) return rc;
   }
   EnsArgs &A = E->args;
   E->smem = A.smem_block + (E->pairs ? sizeof(Pair) : sizeof(float)) *
@@ -455,8 +457,9 @@ int ens_create(Ens *E, const imodel_swm_mesh *meshes, int ngrids, const int32_t 
   constexpr int kMost = 227 * 1024 - 1024;
   if (E->smem > kMost) return fail(E, IMODEL_SWM_EINVAL, "a tile does not fit an SM");
   EK(cudaFuncSetAttribute(kernel(E), cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
-  if ((rc = zalloc(E, &E->stage_h, maxn)) || (rc = zalloc(E, &E->stage_u, maxn)) ||
-      (rc = zalloc(E, &E->bar, 1)) || (rc = zalloc(E, &E->flags, 1)))
+  if ((rc = zalloc(E, &E->stage_h, maxn, E->stream)) ||
+      (rc = zalloc(E, &E->stage_u, maxn, E->stream)) ||
+      (rc = zalloc(E, &E->bar, 1, E->stream)) || (rc = zalloc(E, &E->flags, 1, E->stream)))
     return rc;
   EK(cudaMallocHost(&E->h_flags, sizeof(int)));
   return IMODEL_SWM_OK;
