@@ -30,10 +30,11 @@ namespace {
 // steps: within a graph a step's first kernel starts as the last one's blocks
 // end (after_prior), between graphs after it has ended and the next graph has
 // been taken up.  us a step, by ones and by eights: the fused FP32 step at level
-// 5 14.4, 11.0, level 7 37.1, 33.9, level 8 153.5, 148.5; FP64 at level 5 53.4,
-// 52.4.  Making the second graph costs about 3.5 us a node, what 34 steps of the
-// four-kernel step save at level 5, or some 300 of the twelve-kernel FP64 step:
-// it is made once as many steps have been taken.
+// 5 12.4, 10.6, level 7 37.8, 33.7, level 8 153.2, 149.3; FP64 at level 5 53.4,
+// 52.9.  Making the second graph costs about 3.5 us a node, what 27 steps of the
+// four-kernel step save at level 7, 62 at level 5, or some 600 of the
+// twelve-kernel FP64 step: it is made after 32 steps of the one and 32 a node
+// of the others.
 struct StepGraphs {
   static constexpr int kMany = 8;
   cudaGraphExec_t one = nullptr, many = nullptr;

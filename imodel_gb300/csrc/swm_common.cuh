@@ -118,22 +118,24 @@ struct TileDev {
 
 // Programmatic dependent launch: a kernel of a step may start while its
 // predecessor still runs, load what is fixed (indices, geometry) and then
-// wait for it.  after_prior(x, ...) is that wait; every pointer to data that a
-// kernel of the step writes must be passed to it, so that no load through it
-// can be moved above the wait (a __restrict__ const pointer's loads count as
-// invariant otherwise).
+// wait for it.  after_prior(x, ...) is that wait; every __restrict__ pointer
+// to data that a kernel of the step writes must be passed to it, so that no load
+// through it can be moved above the wait (a __restrict__ const pointer's loads
+// count as invariant otherwise).  Pointers that come in a structure (MoistArgs,
+// EdgeDif) carry no such promise: their loads stay behind the wait by themselves.
 //
 // early (the FP32 kernels): on grids of fewer than kPdlGrid blocks let the
 // successor start at once rather than as this kernel's blocks end.  Per step:
 // FP32 level 5 27.0 us with plain launches, 24.1 with the wait alone, 20.9
 // with the early start; level 7 50.7, 49.3, 43.7; the moist FP32 step at level
 // 8 432, 422, 412.  At level 9 (10,000 blocks and more) the separate kernels gain
-// nothing and the early start costs 3 % of the cell kernel; the tiles' kernels
-// (tiles) start early on every grid, as the next stage's first tiles are copied
-// in while the last ones run (level 9 553 us a step -> 539, the moist step 873
-// -> 854).  The FP64 kernels keep the wait alone (level 5 69.9 us plain, 57.7 with the wait, 63.6 early; pxt16 at
-// level 6 325, 323, 422): their blocks must spread evenly over the FP64 pipes,
-// and blocks that start early take the places first freed.
+// nothing, and the early start and the wait cost 2 to 3 % of the step: they have
+// instances without (launch_wait).  The tiles' kernels (tiles) start early on
+// every grid, as the next stage's first tiles are copied in while the last ones
+// run (level 9 553 us a step -> 539, the moist step 873 -> 854).  The FP64 kernels
+// keep the wait alone (level 5 69.9 us plain, 57.7 with the wait, 63.6 early;
+// pxt16 at level 6 325, 323, 422): their blocks must spread evenly over the FP64
+// pipes, and blocks that start early take the places first freed.
 constexpr unsigned kPdlGrid = 8192;
 template <class P>
 __device__ __forceinline__ void pin_ptr(P &p) {

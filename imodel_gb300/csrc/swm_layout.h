@@ -245,7 +245,7 @@ uint16_t bf16_bits(float v);
 // velocities around it: to step its edges it forms the flux terms of nz cells
 // (its own and the edges' other cells), for which it reads nh depths (those
 // cells, then their other neighbours), nu velocities (own edges, then others)
-// and forms the PV of nt triangles.  Local numbers are below 1024 (10 bits).
+// and forms the PV of nt triangles.  There are at most 1024 of each (10 bits).
 struct TileHead {
   int32_t c0, nc, nz, nh;
   int32_t e0, ne, nu, nt;
@@ -278,7 +278,7 @@ struct TileLayout {
   HVec<int32_t> lists;
 };
 // Cuts a trsk10 layout into tiles of at most cap cells with flux terms; false
-// when a tile has 1024 or more of something (the caller then does without).
+// when a tile has more than 1024 of something (the caller then does without).
 bool build_tiles(const Layout &L, int cap, TileLayout &T);
 
 // Inputs of the learned TRSK weights (imodel_gb300/learned_weights.py): 24

@@ -15,8 +15,8 @@
 // gather, three phases), so a block issues all loads of its thread at once
 // and the copies before the wait.  Per step against the three kernels: level
 // 9 738 -> 553 us, 8 189 -> 154, 7 43.7 -> 37.1, 6 24.8 -> 16.5, 5 20.9 ->
-// 12.4; with the early start on every grid and eight steps a graph 538, 149,
-// 33.8, 14.3, 11.0.  Loading the records into registers phase by phase and the
+// 12.4; with the early start on every grid, eight steps a graph and short polls
+// 537, 149, 33.7, 14.2, 10.5.  Loading the records into registers phase by phase and the
 // state in loops instead took 982 us at level 9.
 #include "imodel_swm.h"
 #include "swm_layout.h"
@@ -240,7 +240,7 @@ __device__ __forceinline__ void sort_block(int32_t *a, int n) {
 
 __global__ void __launch_bounds__(256) k_fill_tiles(DevMesh M, const int4 *head,
                                                     const int32_t *lists, unsigned char *data) {
-  // the lists (below 1024 entries each): ring cells and other depths, other
+  // the lists (at most 1024 entries each): ring cells and other depths, other
   // edges, triangles
   __shared__ int32_t lh[1024], lu[1024], lt[1024];
   const Tile T(head + 5 * blockIdx.x);

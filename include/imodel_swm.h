@@ -171,7 +171,9 @@ typedef struct imodel_swm_diag {
 } imodel_swm_diag;
 
 /* Creates a handle: copies the mesh, reorders cells along a space-filling
- * curve, builds the padded-CSR connectivity and uploads everything.  On
+ * curve, builds the padded-CSR connectivity and uploads everything.  An FP32
+ * trsk10 handle that finds no device memory for the fused stage's tiles steps
+ * with the separate kernels (the same bits).  On
  * failure *handle is still set, so that imodel_swm_last_error() can explain
  * the failure; it must be released with imodel_swm_destroy() either way. */
 int imodel_swm_create(const imodel_swm_mesh *m, const imodel_swm_opts *o,
